@@ -81,6 +81,7 @@ extern "C" int bgt_ctx_destroy(bgt_ctx *c)
     for (auto &kv : c->cache) bgt_batch_destroy(kv.second);
     c->cache.clear();
     for (auto &p : c->scratch) cudaFree(p.ptr);
+    if (c->pinned.ptr) cudaFreeHost(c->pinned.ptr);
     if (c->own) cudaStreamDestroy(c->own);
     delete c;
     return BGT_OK;
@@ -109,6 +110,25 @@ int bgt::ctx_scratch(bgt_ctx *c, int slot, size_t bytes, void **out)
         size_t nb = std::max(bytes, (size_t)4096);
         cudaError_t e = cudaMalloc(&s.ptr, nb);
         if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(scratch)");
+        s.bytes = nb;
+    }
+    *out = s.ptr;
+    return BGT_OK;
+}
+
+int bgt::ctx_pinned(bgt_ctx *c, size_t bytes, void **out)
+{
+    Scratch &s = c->pinned;
+    if (s.bytes < bytes) {
+        if (s.ptr) {
+            cudaStreamSynchronize(c->stream);
+            cudaFreeHost(s.ptr);
+            s.ptr = nullptr;
+            s.bytes = 0;
+        }
+        const size_t nb = std::max(bytes + bytes / 4, (size_t)65536);
+        cudaError_t e = cudaMallocHost(&s.ptr, nb);
+        if (e != cudaSuccess) return cuda_fail(e, "cudaMallocHost");
         s.bytes = nb;
     }
     *out = s.ptr;

@@ -45,6 +45,9 @@ size_t dtype_size(int dtype);
 int default_cfg(int dims, int W, int H, int D);
 int tuned_cfg(int dims, int W, int H, int D);
 int ctx_scratch(bgt_ctx *c, int slot, size_t bytes, void **out);
+// Pinned host buffer of at least `bytes` (grown, never shrunk), for readbacks
+// that end before the call returns.
+int ctx_pinned(bgt_ctx *c, size_t bytes, void **out);
 int single_batch(bgt_ctx *c, int dims, int W, int H, int D, bgt_batch **out);
 int batch_check(bgt_batch *b);
 int batch_set_input_extent(bgt_batch *b, int id, int inW, int inH, int inD);
@@ -70,6 +73,8 @@ struct DevSegs {
 // Device ExtractSegmentsV on a packed image (P words per row): arrays left in
 // the context's scratch, or copied to host memory.
 int segments_device_arrays(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, int D, int P, DevSegs *out);
+// The same as one cooperative launch (segments_graph.cu); 1 = beyond its index range.
+int segments_graph(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, int D, int P, DevSegs *out);
 int segments_packed(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, int D, int P, HostSegs *out);
 // Exclusive prefix sum of n ints on the context's stream (CUB temporary
 // storage in scratch slot `slot`).
@@ -83,6 +88,8 @@ struct bgt_ctx {
     cudaStream_t own = nullptr;
     cudaStream_t stream = nullptr;
     std::vector<bgt::Scratch> scratch;
+    bgt::Scratch pinned;
+    size_t seg_chains = 0, seg_nodes = 0;  // list sizes of the segment extraction (grown on demand)
     std::map<std::tuple<int, int, int, int>, bgt_batch *> cache;
 };
 

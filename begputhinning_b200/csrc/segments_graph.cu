@@ -1,0 +1,678 @@
+// segments_graph.cu -- ExtractSegmentsV as one cooperative launch
+// (2D/ExtractSegments.cpp:16-127, 3D/ExtractSegments.cpp:135-251), bit-exact
+// in content and order, with no sequential part left.
+//
+// The reference visits the nodes (points without exactly two foreground
+// neighbours) in raster order; a visit walks -v branches, each along a run of
+// two-neighbour points (a chain) or one step to a neighbouring node, zeroes
+// what it walks over and adds 1 to the value of the node it ends at.  Two
+// facts make every node's output independent of the others' visits:
+//  * an edge (a chain, or two adjacent nodes) is always walked by the node
+//    that comes first in raster order.  A node starts with one unit of budget
+//    per neighbour; each earlier neighbour's walk takes exactly one of them
+//    and exactly one of its edges, so at its visit the budget equals the
+//    edges that are left, and all of them are walked;
+//  * hence the arrivals at a node before its visit are its edges to earlier
+//    nodes, and its segments, in the scan order of its neighbours, are its
+//    edges to later nodes, chains that lead nowhere, and chains back to
+//    itself, followed by one single-point segment per unit of budget left
+//    over (neighbours on the frame, an isolated point).
+// A walk that meets no nonzero point stays where it is and ends on the same
+// point again: at the end of a chain that leads to the frame, and at the far
+// end of a chain back to its own node, whose far end then counts as one more
+// (two-point) segment of that node.  tests/test_segment_edges.py checks this
+// closed form against the oracle on thinned and on raw masks.
+//
+// What is left is list ranking: every chain point has to know the two ends
+// of its chain and its distance to them.  Each chain point is two half-edges
+// (leaving it through its first or second neighbour); pointer jumping over
+// the half-edges takes about log4(longest chain) rounds, after which every
+// point writes its own coordinates at its place in the output.  Phases (grid
+// barriers in between):
+//   A  node and chain masks per packed word (bit-sliced neighbour counts)
+//   B  block prefix sums -> raster-ordered node and chain lists
+//   C  half-edges: successor or, next to a node or the frame, terminal
+//   J  pointer jumping until no half-edge finishes any more (the rest are
+//      cycles without a node, which the reference never walks)
+//   D  segments and points per node;  E  prefix sums, node outputs
+//   F  chain points write their coordinates
+//
+// Bound: latency -- about 7 + log4(longest chain) grid barriers of 1-2 us,
+// and in phase A of a volume the read of its packed words.  Measured on a
+// B200, whole ExtractSegmentsV call, against a walk that followed each chain
+// with one thread and ran the nodes from a queue in the order of their
+// dependences: 2048^2 stroke image (226 k points) 5.72 -> 0.51 ms, 256^3
+// volume (2.3 k points) 0.86 -> 0.15 ms; CenterlineExtraction of a 512^2
+// image 1.24 -> 0.35 ms.
+#include <algorithm>
+#include <cstdlib>
+#include <cstring>
+
+#include "host.h"
+#include "kernels.cuh"
+
+namespace bgt {
+
+namespace {
+constexpr int kSegThreads = 512;
+constexpr int kSegWarps = kSegThreads / 32;
+constexpr uint32_t kFin = 0x80000000u;      // half-edge pair: the pointer is a terminal half-edge
+constexpr uint32_t kNone = 0xffffffffu;     // no exit node / not walked from this end
+constexpr int kMaxRounds = 64;
+constexpr size_t kSegHeaderBytes = 64;
+// sync block: [0] barrier arrivals, [1] status, then per jump round: finished, left over
+constexpr int kSyncInts = 2 + 2 * kMaxRounds;
+
+__host__ __device__ inline size_t seg_up16(size_t v) { return (v + 15) & ~size_t(15); }
+
+// Output block: header, start[S + 1], is_end[S], x[N], y[N], z[N].
+struct SegLayout {
+    size_t start, is_end, x, y, z, total;
+};
+__host__ __device__ inline SegLayout seg_layout(unsigned S, unsigned N, int dims)
+{
+    SegLayout L;
+    L.start = kSegHeaderBytes;
+    L.is_end = L.start + seg_up16((size_t)(S + 1) * 4);
+    L.x = L.is_end + seg_up16(S);
+    L.y = L.x + seg_up16((size_t)N * 2);
+    L.z = L.y + seg_up16((size_t)N * 2);
+    L.total = L.z + (dims == 3 ? seg_up16((size_t)N * 2) : 0);
+    return L;
+}
+
+struct SegArgs {
+    const uint32_t *buf;  // packed image, P words per row
+    int W, H, D, P;
+    uint32_t ww, nw;      // used words per row, used words in all
+    FastDiv dww, dH;
+    uint4 *rec;           // per used word with foreground: node mask, chain mask, node rank, chain index
+    // chain points
+    uint2 *cpt;           // row, x
+    uint16_t *cdir;       // its two neighbours (window cells): low | high << 8
+    unsigned long long *pair;  // per half-edge: steps << 32 | kFin? | half-edge reached
+    uint32_t *cexit;      // terminal half-edge -> rank of its node (kNone: the chain leads nowhere)
+    uint32_t *cbase;      // terminal half-edge -> output index of the chain's first point walked from its node
+    uint32_t cap_c;
+    // nodes
+    uint2 *npt;           // row, x
+    uint8_t *ndeg;        // foreground neighbours
+    uint2 *ncnt;          // segments, points
+    uint32_t cap_n;
+    uint2 *bsum, *bsum2;  // per block: nodes and chain points; segments and points
+    int *sync;
+    uint8_t *out;
+    unsigned long long out_bytes;
+    long long timeout_ns;
+};
+
+// Header of the output block.
+struct SegHeader {
+    uint32_t nodes, chains, segs, pts;
+    int status;  // 0 done, 1 lists too small, 2 output too small, 4 a wait ran out, 8 sums past 32 bits
+};
+
+// Grid barrier (cooperative launch: every block is resident).  Bounded; false
+// once any block gave up.
+__device__ bool seg_barrier(const SegArgs &a, unsigned &gen)
+{
+    __shared__ int ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        gen++;
+        __threadfence();
+        atomicAdd(a.sync, 1);
+        const int target = (int)(gen * gridDim.x);
+        const unsigned long long t_end = globaltimer() + (unsigned long long)a.timeout_ns;
+        bool good = true;
+        for (int spin = 0; ld_acquire(a.sync) < target; spin++)
+            if ((spin & 255) == 255 && globaltimer() > t_end) {
+                good = false;
+                break;
+            }
+        if (!good) atomicOr(a.sync + 1, 4);
+        ok = good && !(ld_acquire(a.sync + 1) & 4);
+    }
+    __syncthreads();
+    const bool r = ok;
+    __syncthreads();
+    return r;
+}
+
+// Exclusive prefix sum over the block of two counters packed in 64 bits.
+__device__ unsigned long long seg_exscan(unsigned long long v, unsigned long long *total)
+{
+    __shared__ unsigned long long wsum[kSegWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned long long x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(kFull, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) wsum[warp] = x;
+    __syncthreads();
+    unsigned long long before = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < kSegWarps; w++) {
+        const unsigned long long s = wsum[w];
+        if (w < warp) before += s;
+        all += s;
+    }
+    __syncthreads();
+    *total = all;
+    return before + x - v;
+}
+
+// Sums of the per-block totals before this block, and of all blocks.
+__device__ void seg_block_prefix(const uint2 *sums, unsigned long long (&before)[2], unsigned long long (&all)[2])
+{
+    unsigned long long b0 = 0, b1 = 0, s0 = 0, s1 = 0;
+    for (unsigned k = threadIdx.x; k < gridDim.x; k += kSegThreads) {
+        const uint2 v = __ldcg(sums + k);
+        s0 += v.x;
+        s1 += v.y;
+        if (k < blockIdx.x) {
+            b0 += v.x;
+            b1 += v.y;
+        }
+    }
+    unsigned long long t;
+    seg_exscan(b0, &t);
+    before[0] = t;
+    seg_exscan(b1, &t);
+    before[1] = t;
+    seg_exscan(s0, &t);
+    all[0] = t;
+    seg_exscan(s1, &t);
+    all[1] = t;
+}
+
+template <int DIMS>
+struct Win {
+    static constexpr int C = DIMS == 2 ? 4 : 13;  // centre cell; a cell before it precedes the point in raster order
+};
+
+// Foreground bits of the 3x3 (x3) window of the interior point (row, x),
+// cells in the reference's scan order, the centre cleared.
+template <int DIMS>
+__device__ __forceinline__ uint32_t seg_window(const SegArgs &a, uint32_t row, uint32_t x)
+{
+    const uint32_t j0 = (x - 1) >> 5, j1 = (x + 1) >> 5, sh = (x - 1) & 31u;
+    uint32_t w = 0;
+#pragma unroll
+    for (int k = 0; k < (DIMS == 2 ? 3 : 9); k++) {
+        const int dz = DIMS == 2 ? 0 : k / 3 - 1, dy = DIMS == 2 ? k - 1 : k % 3 - 1;
+        const uint32_t *p = a.buf + (size_t)((long long)row + (long long)dz * a.H + dy) * a.P;
+        w |= (__funnelshift_r(__ldg(p + j0), __ldg(p + j1), sh) & 7u) << (3 * k);
+    }
+    return w & ~(1u << Win<DIMS>::C);
+}
+
+// Cells of the window that are interior (points when they are foreground).
+template <int DIMS>
+__device__ __forceinline__ uint32_t seg_interior(const SegArgs &a, uint32_t row, uint32_t x)
+{
+    constexpr uint32_t all = DIMS == 2 ? 0x1FFu : 0x7FFFFFFu;
+    constexpr uint32_t xl = DIMS == 2 ? 0x49u : 0x1249249u, yl = DIMS == 2 ? 0x7u : 0x1C0E07u;
+    uint32_t y = row, m = all;
+    if (DIMS == 3) {
+        const uint32_t z = fdiv(a.dH, row);
+        y = row - z * (uint32_t)a.H;
+        if (z == 1) m &= ~0x1FFu;
+        if (z + 2 == (uint32_t)a.D) m &= ~(0x1FFu << 18);
+    }
+    if (x == 1) m &= ~xl;
+    if (x + 2 == (uint32_t)a.W) m &= ~(xl << 2);
+    if (y == 1) m &= ~yl;
+    if (y + 2 == (uint32_t)a.H) m &= ~(yl << 6);
+    return m;
+}
+
+// The point in window cell q of (row, x): true for a node (id = its rank),
+// false for a chain point (id = its index).
+__device__ __forceinline__ bool seg_point(const SegArgs &a, uint32_t row, uint32_t x, int q, uint32_t &id)
+{
+    const int dz = q / 9, dy = (q / 3) % 3, dx = q % 3;  // 2D callers add 9 (the middle plane)
+    const uint32_t r = (uint32_t)((long long)row + (long long)(dz - 1) * a.H + (dy - 1));
+    const uint32_t xx = x + (uint32_t)dx - 1u;
+    const uint4 w = __ldcg(a.rec + (size_t)r * a.ww + (xx >> 5));
+    const uint32_t b = 1u << (xx & 31u);
+    const bool node = (w.x & b) != 0u;
+    id = node ? w.z + __popc(w.x & (b - 1u)) : w.w + __popc(w.y & (b - 1u));
+    return node;
+}
+
+// Phases A and B: masks, counts, lists.
+template <int DIMS>
+__device__ __forceinline__ void seg_masks(const SegArgs &a, uint32_t i, uint32_t c, uint32_t &nodes, uint32_t &chains)
+{
+    const uint32_t row = fdiv(a.dww, i), j = i - row * a.ww;
+    uint32_t y = row, z = 0;
+    if (DIMS == 3) {
+        z = fdiv(a.dH, row);
+        y = row - z * (uint32_t)a.H;
+    }
+    nodes = chains = 0;
+    if (y == 0 || y + 1 >= (uint32_t)a.H || (DIMS == 3 && (z == 0 || z + 1 >= (uint32_t)a.D))) return;
+    uint32_t pts = c;
+    if (j == 0) pts &= ~1u;
+    const int last = a.W - 2 - (int)(j * 32);  // highest interior bit of the word
+    if (last < 0) return;
+    if (last < 31) pts &= (2u << last) - 1u;
+    if (!pts) return;
+    // counts modulo 2, and "at least two", "at least four": exactly two = the second and neither of the others
+    uint32_t c0 = 0, c1 = 0, big = 0;
+    auto add = [&](uint32_t v) {
+        const uint32_t t = c0 & v;
+        c0 ^= v;
+        big |= c1 & t;
+        c1 ^= t;
+    };
+#pragma unroll
+    for (int k = 0; k < (DIMS == 2 ? 3 : 9); k++) {
+        const int dz = DIMS == 2 ? 0 : k / 3 - 1, dy = DIMS == 2 ? k - 1 : k % 3 - 1;
+        const uint32_t *p = a.buf + (size_t)((long long)row + (long long)dz * a.H + dy) * a.P + j;
+        const uint32_t m = __ldg(p), l = j > 0 ? __ldg(p - 1) : 0u, r = j + 1 < a.ww ? __ldg(p + 1) : 0u;
+        add(at_xm1(m, l));
+        if (dz != 0 || dy != 0) add(m);
+        add(at_xp1(m, r));
+    }
+    const uint32_t two = c1 & ~c0 & ~big;
+    nodes = pts & ~two;
+    chains = pts & two;
+}
+
+// What node r does at its visit; with EMIT its segments and end points are
+// written from segment si and point pi on (and the chains it walks learn
+// where their points go), else only counted.
+template <int DIMS, bool EMIT>
+__device__ __forceinline__ uint2 seg_visit(const SegArgs &a, uint32_t r, uint32_t si, uint32_t pi, int32_t *start,
+                                           uint8_t *is_end, int16_t *px, int16_t *py, int16_t *pz)
+{
+    constexpr int C = Win<DIMS>::C, q0 = DIMS == 2 ? 9 : 0;
+    const uint2 at = __ldcg(a.npt + r);
+    const uint32_t win = seg_window<DIMS>(a, at.x, at.y);
+    uint32_t todo = win & seg_interior<DIMS>(a, at.x, at.y);
+    const int n = __popc(win);
+    const uint32_t pi0 = pi, si0 = si;
+    uint32_t arrivals = 0;
+    auto put = [&](uint32_t k, uint2 p) {
+        uint32_t y = p.x, z = 0;
+        if (DIMS == 3) {
+            z = fdiv(a.dH, p.x);
+            y = p.x - z * (uint32_t)a.H;
+            pz[k] = (int16_t)z;
+        }
+        px[k] = (int16_t)p.y;
+        py[k] = (int16_t)y;
+    };
+    // a segment of `len` chain points that starts at r and ends at `end`
+    auto segment = [&](uint32_t len, uint2 end, bool e) {
+        if (EMIT) {
+            start[si] = (int32_t)pi;
+            is_end[si] = e || n < 2;
+            put(pi, at);
+            put(pi + 1 + len, end);
+        }
+        si++;
+        pi += len + 2;
+    };
+    while (todo) {
+        const int q = __ffs(todo) - 1;
+        todo &= todo - 1;
+        uint32_t id;
+        if (seg_point(a, at.x, at.y, q + q0, id)) {
+            if (q < C) {
+                arrivals++;
+                continue;
+            }
+            if (EMIT) segment(0, __ldcg(a.npt + id), __ldcg(a.ndeg + id) < 2);
+            else segment(0, at, false);
+            continue;
+        }
+        const int back = 2 * C - q;
+        const int sr = (__ldcg(a.cdir + id) & 0xff) == back ? 0 : 1;  // the side of the chain point that r is on
+        const unsigned long long pr = __ldcg(a.pair + 2 * (size_t)id + (1 - sr));
+        const uint32_t t = (uint32_t)pr & ~kFin, len = (uint32_t)(pr >> 32) + 1;
+        const uint32_t e = __ldcg(a.cexit + t);
+        const uint32_t home = 2 * id + sr;  // terminal half-edge of this end of the chain
+        if (e == kNone) {  // leads to the frame: the last point again
+            if (EMIT) a.cbase[home] = pi + 1;
+            segment(len, EMIT ? __ldcg(a.cpt + (t >> 1)) : at, false);
+        } else if (e == r) {
+            const uint16_t fd = __ldcg(a.cdir + (t >> 1));
+            const int far_q = 2 * C - ((t & 1) ? fd >> 8 : fd & 0xff);  // the cell of r that holds the far end
+            if (q < far_q) {
+                if (EMIT) a.cbase[home] = pi + 1;
+                segment(len, EMIT ? __ldcg(a.cpt + (t >> 1)) : at, false);
+            } else {
+                if (EMIT) a.cbase[home] = kNone;
+                segment(0, EMIT ? __ldcg(a.cpt + id) : at, false);
+            }
+        } else if (e > r) {
+            if (EMIT) {
+                a.cbase[home] = pi + 1;
+                segment(len, __ldcg(a.npt + e), __ldcg(a.ndeg + e) < 2);
+            } else {
+                segment(len, at, false);
+            }
+        } else {
+            if (EMIT) a.cbase[home] = kNone;
+            arrivals++;
+        }
+    }
+    // the rest of the budget: single points
+    for (int left = max(n, 1) - (int)arrivals - (int)(si - si0); left > 0; left--) {
+        if (EMIT) {
+            start[si] = (int32_t)pi;
+            is_end[si] = n < 2;
+            put(pi, at);
+        }
+        si++;
+        pi++;
+    }
+    if (!EMIT) a.ndeg[r] = (uint8_t)n;
+    return make_uint2(si - si0, pi - pi0);
+}
+
+template <int DIMS>
+__global__ void __launch_bounds__(kSegThreads, 1) segments_graph_kernel(const SegArgs a)
+{
+    unsigned gen = 0;
+    const uint32_t tid = blockIdx.x * kSegThreads + threadIdx.x, nthr = gridDim.x * kSegThreads;
+    SegHeader *hdr = reinterpret_cast<SegHeader *>(a.out);
+    unsigned long long total, before[2], all[2];
+
+    // A: masks and counts of this block's range of words
+    const uint32_t per = (a.nw + gridDim.x - 1) / gridDim.x;
+    const uint32_t w0 = min(a.nw, per * blockIdx.x), w1 = min(a.nw, w0 + per);
+    unsigned long long cnt = 0;
+    for (uint32_t i = w0 + threadIdx.x; i < w1; i += kSegThreads) {
+        const uint32_t row = fdiv(a.dww, i);
+        const uint32_t c = __ldg(a.buf + (size_t)row * a.P + (i - row * a.ww));
+        if (!c) continue;
+        uint32_t nodes, chains;
+        seg_masks<DIMS>(a, i, c, nodes, chains);
+        a.rec[i] = make_uint4(nodes, chains, 0u, 0u);
+        cnt += (unsigned long long)__popc(nodes) << 32 | __popc(chains);
+    }
+    seg_exscan(cnt, &total);
+    if (threadIdx.x == 0) a.bsum[blockIdx.x] = make_uint2((uint32_t)(total >> 32), (uint32_t)total);
+    if (!seg_barrier(a, gen)) return;
+
+    // B: lists in raster order
+    seg_block_prefix(a.bsum, before, all);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *hdr = SegHeader{(uint32_t)min(all[0], (unsigned long long)kNone), (uint32_t)min(all[1], (unsigned long long)kNone),
+                         0u, 0u, all[0] > a.cap_n || all[1] > a.cap_c ? 1 : 0};
+    }
+    if (all[0] > a.cap_n || all[1] > a.cap_c) return;
+    const uint32_t nn = (uint32_t)all[0], nc = (uint32_t)all[1];
+    uint32_t no = (uint32_t)before[0], co = (uint32_t)before[1];
+    for (uint32_t base = w0; base < w1; base += kSegThreads) {
+        const uint32_t i = base + threadIdx.x;
+        uint32_t row = 0, c = 0;
+        uint4 rc = make_uint4(0u, 0u, 0u, 0u);
+        if (i < w1) {
+            row = fdiv(a.dww, i);
+            c = __ldg(a.buf + (size_t)row * a.P + (i - row * a.ww));
+            if (c) rc = __ldcg(a.rec + i);
+        }
+        if (!__syncthreads_or((rc.x | rc.y) != 0u)) continue;
+        const unsigned long long o =
+            seg_exscan((unsigned long long)__popc(rc.x) << 32 | __popc(rc.y), &total);
+        if (c) {
+            uint32_t ni = no + (uint32_t)(o >> 32), ci = co + (uint32_t)o;
+            a.rec[i] = make_uint4(rc.x, rc.y, ni, ci);
+            const uint32_t x0 = (i - row * a.ww) * 32;
+            for (uint32_t m = rc.x; m; m &= m - 1) a.npt[ni++] = make_uint2(row, x0 + __ffs(m) - 1);
+            for (uint32_t m = rc.y; m; m &= m - 1) a.cpt[ci++] = make_uint2(row, x0 + __ffs(m) - 1);
+        }
+        no += (uint32_t)(total >> 32);
+        co += (uint32_t)total;
+    }
+    if (!seg_barrier(a, gen)) return;
+
+    // C: half-edges
+    constexpr int C = Win<DIMS>::C, q0 = DIMS == 2 ? 9 : 0;
+    for (uint32_t k = tid; k < nc; k += nthr) {
+        const uint2 at = __ldcg(a.cpt + k);
+        const uint32_t win = seg_window<DIMS>(a, at.x, at.y), in = seg_interior<DIMS>(a, at.x, at.y);
+        const int q2[2] = {__ffs(win) - 1, 31 - __clz(win)};
+        a.cdir[k] = (uint16_t)(q2[0] | q2[1] << 8);
+#pragma unroll
+        for (int s = 0; s < 2; s++) {
+            const int q = q2[s];
+            const uint32_t h = 2 * k + s;
+            uint32_t id = kNone;
+            const bool inner = (in >> q) & 1u;
+            if (!inner || seg_point(a, at.x, at.y, q + q0, id)) {
+                a.pair[h] = kFin | h;
+                a.cexit[h] = id;
+                a.cbase[h] = kNone;
+                continue;
+            }
+            // the neighbour's side that does not lead back here
+            const int qq = q + q0;
+            const uint32_t r = (uint32_t)((long long)at.x + (long long)(qq / 9 - 1) * a.H + ((qq / 3) % 3 - 1));
+            const uint32_t nwin = seg_window<DIMS>(a, r, at.y + (uint32_t)(qq % 3) - 1u);
+            const uint32_t s2 = (__ffs(nwin) - 1) == 2 * C - q ? 1u : 0u;
+            a.pair[h] = 1ull << 32 | (2 * id + s2);
+        }
+    }
+    if (!seg_barrier(a, gen)) return;
+
+    // J: pointer jumping.  Pairs are read and written whole (8 bytes), so a
+    // reader sees an older or a newer pair, both true.  Of the half-edges of
+    // a path that are not finished the one nearest its terminal points at a
+    // finished one, so a round in which none finishes leaves only cycles.
+    for (int round = 0; round < kMaxRounds; round++) {
+        bool fin = false, left = false;
+        for (uint32_t h = tid; h < 2 * nc; h += nthr) {
+            unsigned long long v = __ldcg(a.pair + h);
+            if ((uint32_t)v & kFin) continue;
+            uint32_t p = (uint32_t)v, d = (uint32_t)(v >> 32);
+#pragma unroll 1
+            for (int k = 0; k < 4 && !(p & kFin); k++) {
+                const unsigned long long u = __ldcg(a.pair + p);
+                p = (uint32_t)u;
+                d += (uint32_t)(u >> 32);
+            }
+            __stcg(a.pair + h, (unsigned long long)d << 32 | p);
+            if (p & kFin) fin = true;
+            else left = true;
+        }
+        const int any_left = __syncthreads_or(left), any_fin = __syncthreads_or(fin);
+        if (threadIdx.x == 0) {
+            if (any_fin) atomicOr(a.sync + 2 + 2 * round, 1);
+            if (any_left) atomicOr(a.sync + 3 + 2 * round, 1);
+        }
+        if (!seg_barrier(a, gen)) return;
+        if (!__ldcg(a.sync + 2 + 2 * round) || !__ldcg(a.sync + 3 + 2 * round)) break;
+    }
+
+    // D: segments and points per node (a contiguous range of nodes per block)
+    const uint32_t nper = (nn + gridDim.x - 1) / gridDim.x;
+    const uint32_t n0 = min(nn, nper * blockIdx.x), n1 = min(nn, n0 + nper);
+    unsigned long long s0 = 0, s1 = 0;
+    for (uint32_t r = n0 + threadIdx.x; r < n1; r += kSegThreads) {
+        const uint2 v = seg_visit<DIMS, false>(a, r, 0, 0, nullptr, nullptr, nullptr, nullptr, nullptr);
+        a.ncnt[r] = v;
+        s0 += v.x;
+        s1 += v.y;
+    }
+    seg_exscan(s0, &total);
+    s0 = total;
+    seg_exscan(s1, &total);
+    s1 = total;
+    if (threadIdx.x == 0) {
+        a.bsum2[blockIdx.x] = make_uint2((uint32_t)s0, (uint32_t)s1);
+        if (s0 >> 31 || s1 >> 31) atomicOr(a.sync + 1, 8);
+    }
+    if (!seg_barrier(a, gen)) return;
+
+    // E: output ranges, node outputs
+    seg_block_prefix(a.bsum2, before, all);
+    const bool wide = (ld_acquire(a.sync + 1) & 8) || all[0] >> 31 || all[1] >> 31;
+    const SegLayout L = seg_layout((unsigned)all[0], (unsigned)all[1], DIMS);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        hdr->segs = (uint32_t)all[0];
+        hdr->pts = (uint32_t)all[1];
+        hdr->status = wide ? 8 : L.total > a.out_bytes ? 2 : 0;
+    }
+    if (wide || L.total > a.out_bytes) return;
+    int32_t *start = reinterpret_cast<int32_t *>(a.out + L.start);
+    uint8_t *is_end = a.out + L.is_end;
+    int16_t *px = reinterpret_cast<int16_t *>(a.out + L.x), *py = reinterpret_cast<int16_t *>(a.out + L.y),
+            *pz = reinterpret_cast<int16_t *>(a.out + L.z);
+    if (blockIdx.x == 0 && threadIdx.x == 0) start[all[0]] = (int32_t)all[1];
+    uint32_t so = (uint32_t)before[0], po = (uint32_t)before[1];
+    for (uint32_t base = n0; base < n1; base += kSegThreads) {
+        const uint32_t r = base + threadIdx.x;
+        const uint2 v = r < n1 ? __ldcg(a.ncnt + r) : make_uint2(0u, 0u);
+        const unsigned long long o = seg_exscan((unsigned long long)v.x << 32 | v.y, &total);
+        if (r < n1)
+            seg_visit<DIMS, true>(a, r, so + (uint32_t)(o >> 32), po + (uint32_t)o, start, is_end, px, py, pz);
+        so += (uint32_t)(total >> 32);
+        po += (uint32_t)total;
+    }
+    if (!seg_barrier(a, gen)) return;
+
+    // F: chain points
+    for (uint32_t k = tid; k < nc; k += nthr) {
+        uint32_t pos = kNone;
+#pragma unroll
+        for (int s = 0; s < 2; s++) {
+            const unsigned long long v = __ldcg(a.pair + 2 * (size_t)k + s);
+            if (!((uint32_t)v & kFin)) continue;  // a cycle without a node
+            const uint32_t b = __ldcg(a.cbase + ((uint32_t)v & ~kFin));
+            if (b != kNone) pos = b + (uint32_t)(v >> 32);
+        }
+        if (pos == kNone) continue;
+        const uint2 at = __ldcg(a.cpt + k);
+        uint32_t y = at.x;
+        if (DIMS == 3) {
+            const uint32_t z = fdiv(a.dH, at.x);
+            y = at.x - z * (uint32_t)a.H;
+            pz[pos] = (int16_t)z;
+        }
+        px[pos] = (int16_t)at.y;
+        py[pos] = (int16_t)y;
+    }
+}
+}  // namespace
+
+// Device segment extraction of a packed image.  Returns BGT_OK with *out
+// filled (arrays in the context's scratch until its next extraction), 1 when
+// the image is beyond this path's index range, or an error.  The lists and
+// the output live in scratch sized by what the context has met so far; an
+// image that needs more reports its counts and is run once more.
+int segments_graph(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, int D, int P, DevSegs *out)
+{
+    *out = DevSegs();
+    const long long rows = (long long)H * D, ww = (W + 31) / 32, nw = rows * ww, npx = (long long)W * rows;
+    if (nw >= (1LL << 31) || rows >= (1LL << 31)) return 1;
+    cudaStream_t st = c->stream;
+    SegArgs a{};
+    a.buf = d_buf;
+    a.W = W;
+    a.H = H;
+    a.D = D;
+    a.P = P;
+    a.ww = (uint32_t)ww;
+    a.nw = (uint32_t)nw;
+    a.dww = make_fastdiv((uint32_t)ww);
+    a.dH = make_fastdiv((uint32_t)H);
+    a.timeout_ns = 2000000000LL;
+    // about two words per thread, one block per SM at most (a barrier costs more with more blocks)
+    const int grid = (int)std::max<long long>(1, std::min<long long>(c->sms, (nw + 2 * kSegThreads - 1) / (2 * kSegThreads)));
+    c->seg_chains = std::max(c->seg_chains, std::max<size_t>(16384, (size_t)npx / (dims == 2 ? 16 : 64)));
+    c->seg_nodes = std::max(c->seg_nodes, std::max<size_t>(4096, (size_t)npx / (dims == 2 ? 64 : 256)));
+    void *p_rec, *p_out, *p_list, *p_sync, *h_pin;
+    int rc;
+    if ((rc = ctx_scratch(c, 30, (size_t)nw * sizeof(uint4), &p_rec)) ||
+        (rc = ctx_scratch(c, 33, kSyncInts * sizeof(int) + 2 * (size_t)c->sms * sizeof(uint2), &p_sync)) ||
+        (rc = ctx_pinned(c, 4096, &h_pin)))
+        return rc;
+    a.rec = (uint4 *)p_rec;
+    a.sync = (int *)p_sync;
+    a.bsum = (uint2 *)((char *)p_sync + kSyncInts * sizeof(int));
+    a.bsum2 = a.bsum + c->sms;
+    size_t out_bytes = 0;
+    for (int attempt = 0; attempt < 4; attempt++) {
+        const size_t nc = c->seg_chains, nn = c->seg_nodes;
+        if (nc >= (1u << 30) || nn >= (1u << 31)) return 1;
+        size_t off = 0;
+        auto take = [&](size_t bytes) {
+            const size_t o = off;
+            off += (bytes + 255) / 256 * 256;
+            return o;
+        };
+        const size_t o_cpt = take(nc * 8), o_cdir = take(nc * 2), o_pair = take(nc * 16), o_exit = take(nc * 8),
+                     o_base = take(nc * 8), o_npt = take(nn * 8), o_deg = take(nn), o_cnt = take(nn * 8);
+        if ((rc = ctx_scratch(c, 31, off, &p_list))) return rc;
+        char *l = (char *)p_list;
+        a.cpt = (uint2 *)(l + o_cpt);
+        a.cdir = (uint16_t *)(l + o_cdir);
+        a.pair = (unsigned long long *)(l + o_pair);
+        a.cexit = (uint32_t *)(l + o_exit);
+        a.cbase = (uint32_t *)(l + o_base);
+        a.npt = (uint2 *)(l + o_npt);
+        a.ndeg = (uint8_t *)(l + o_deg);
+        a.ncnt = (uint2 *)(l + o_cnt);
+        a.cap_c = (uint32_t)nc;
+        a.cap_n = (uint32_t)nn;
+        // points: the chain points and two per segment, about two segments per node
+        out_bytes = std::max(out_bytes, seg_layout((unsigned)std::min<size_t>(4 * nn, 1u << 30),
+                                                   (unsigned)std::min<size_t>(nc + 8 * nn, 1u << 30), dims).total);
+        if ((rc = ctx_scratch(c, 19, out_bytes, &p_out))) return rc;
+        a.out = (uint8_t *)p_out;
+        a.out_bytes = c->scratch[19].bytes;
+        cudaError_t e = cudaMemsetAsync(a.sync, 0, kSyncInts * sizeof(int), st);
+        if (e != cudaSuccess) return cuda_fail(e, "segment sync reset");
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(grid);
+        cfg.blockDim = dim3(kSegThreads);
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        e = dims == 2 ? cudaLaunchKernelEx(&cfg, segments_graph_kernel<2>, a)
+                      : cudaLaunchKernelEx(&cfg, segments_graph_kernel<3>, a);
+        if (e != cudaSuccess) return cuda_fail(e, "segment kernel");
+        int *h_sync = (int *)((char *)h_pin + kSegHeaderBytes);
+        e = cudaMemcpyAsync(h_pin, a.out, sizeof(SegHeader), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(h_sync, a.sync, 2 * sizeof(int), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        if (e != cudaSuccess) return cuda_fail(e, "segment extraction");
+        const SegHeader h = *(const SegHeader *)h_pin;
+        if (h_sync[1] & 4) return fail(BGT_ERR_TIMEOUT, "segment extraction: a device wait gave up");
+        if (h.status == 8) return fail(BGT_ERR_LIMIT, "segment output bound exceeds 2^31 entries");
+        if (h.status == 1) {
+            c->seg_chains = std::max(c->seg_chains, (size_t)h.chains + h.chains / 8);
+            c->seg_nodes = std::max(c->seg_nodes, (size_t)h.nodes + h.nodes / 8);
+            continue;
+        }
+        const SegLayout L = seg_layout(h.segs, h.pts, dims);
+        if (h.status == 2) {
+            out_bytes = L.total;
+            continue;
+        }
+        out->nseg = (int)h.segs;
+        out->npts = (int)h.pts;
+        if (h.segs == 0) return BGT_OK;
+        uint8_t *o = a.out;
+        out->start = (int32_t *)(o + L.start);
+        out->is_end = o + L.is_end;
+        out->px = (int16_t *)(o + L.x);
+        out->py = (int16_t *)(o + L.y);
+        out->pz = dims == 3 ? (int16_t *)(o + L.z) : nullptr;
+        return BGT_OK;
+    }
+    return fail(BGT_ERR_NOMEM, "segment extraction: the counts kept growing");
+}
+
+}  // namespace bgt
