@@ -67,8 +67,12 @@ struct alignas(16) Inst {
     // resident engine (resident.cu)
     int res;                  // 1: thinned by the resident engine, 0: by the tile rings
     int spill;                // set by the resident engine when a volume's bricks do not fit: the rings take it
-    int res_arrive;           // arrivals at the band barrier of a multi-CTA image (all bands, all passes)
-    int res_last;             // last pass in which some band's core changed (-1: none yet)
+    unsigned long long res_meet[2];  // meetings of its CTAs in turn: arrivals (low half), changes reported (high half)
+    int res_bands;            // 3D: boxes the volume is cut into
+    int res_gy;               // 3D: boxes along y (band = z index * res_gy + y index)
+    int res_stride;           // 3D: messages a box may send per iteration (its core words)
+    uint2 *res_msg;           // 3D, several boxes: [2][boxes][res_stride] (word of the volume, value)
+    int *res_cnt;             // ... and their counts [2][boxes]
 };
 
 // Core words of a tile (clamped to the image): the algorithmic unit of a pass.
@@ -206,6 +210,13 @@ __device__ __forceinline__ int ld_acquire(const int *p)
 {
     int v;
     asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long long *p)
+{
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
 

@@ -289,7 +289,6 @@ static void plan_resident(bgt_batch *b)
         in.res = 0;
         if (rings_only || !it.auto_cfg || b->res_grid < 1) continue;
         if (it.dims == 3) {
-            if (!res_fits3d(it.W, it.H, it.D)) continue;
             in.res = 1;
             vols.push_back({(double)it.W * it.H * it.D, i});
         } else {
@@ -299,32 +298,59 @@ static void plan_resident(bgt_batch *b)
     }
     std::stable_sort(vols.begin(), vols.end(), [](auto &x, auto &y) { return x.first > y.first; });
     std::stable_sort(imgs.begin(), imgs.end(), [](auto &x, auto &y) { return x.first > y.first; });
-    // a large volume is cut into z-slabs of whole brick layers (4 planes),
-    // each with two halo layers on either side, so its iterations spread
-    // over several SMs, and so that a slab's non-empty bricks fit one CTA
-    // (counted on the device: a volume is planned for a quarter of its
-    // slab's bricks being non-empty; one that exceeds it goes to the tile
-    // rings); at least 4 core layers per slab
-    constexpr int kHalo3 = 2, kMinLayers = 4;
-    double vox_per_slab = 1.0e6;
-    if (const char *e = getenv("BGT_RES3D_SLAB_VOXELS")) vox_per_slab = std::max(1.0e4, atof(e));
+    // A volume is cut into boxes of rows and planes (full width), gy along y
+    // and gz along z, each with kResHalo3D rows and planes around it: as many
+    // as its share of the batch's work is worth (a box of fewer than
+    // box_words core words gains nothing: meeting costs more than it saves),
+    // and at least as many as make a box fit one CTA with all of its words
+    // non-empty or, where that would take more boxes than the share allows,
+    // with kMinFill of them (a volume that turns out denser goes to the tile
+    // rings).  Of the cuts with that many boxes the one with the smallest
+    // box is taken.
+    constexpr double kMinFill = 0.3, kLastFill = 0.15;
+    double box_words = 3072.0;
+    if (const char *e = getenv("BGT_RES3D_BOX_WORDS")) box_words = std::max(1.0, atof(e));
+    const char *slab = getenv("BGT_RES3D_SLAB_VOXELS");
     for (auto &v : vols) {
         const BatchItem &it = b->items[v.second];
-        const int layers = (it.D + 3) / 4;
-        const int gmax = std::max(1, std::min(layers / kMinLayers, b->res_grid));
-        int G = std::max(1, std::min((int)std::ceil(v.first / vox_per_slab), gmax));
-        auto slab_ok = [&](int g) {
-            const int sl = g == 1 ? layers : (layers + g - 1) / g + 2 * kHalo3;
-            const int cap = res_slots_fit3d(it.W, it.H, 4 * sl);
-            const double bricks = (double)((it.W + 31) / 32) * ((it.H + 31) / 32) * sl;
-            return cap > 0 && 0.25 * bricks <= cap;
+        Inst &in = b->h[v.second];
+        const int wl = (it.W + 31) / 32;
+        const double words = (double)wl * it.H * it.D;
+        auto extent = [](int n, int g) {  // longest box along an axis of n cut into g, halo included
+            return (n + g - 1) / g + (g == 1 ? 0 : g == 2 ? kResHalo3D : 2 * kResHalo3D);
         };
-        while (G < gmax && !slab_ok(G)) G++;
-        while (G > 1 && res_slots_fit3d(it.W, it.H, 4 * ((layers + G - 1) / G + 2 * kHalo3)) == 0) G--;
-        for (int k = 0; k < G; k++) {
-            const int r0 = (int)((long long)k * layers / G), r1 = (int)((long long)(k + 1) * layers / G);
-            b->res_items.push_back(ResItem{v.second, k, G, r0, r1, G > 1 ? kHalo3 : 0});
+        int share = (int)std::ceil(words / std::max(target, box_words));
+        if (slab) share = (int)std::ceil(v.first / std::max(1.0e4, atof(slab)));
+        share = std::max(1, std::min(share, b->res_grid));
+        // the cut into at most `boxes` boxes that hold `fill` with the smallest box, or (fewest) the fewest boxes
+        int gy = 0, gz = 0;
+        auto search = [&](int boxes, double fill, bool fewest) {
+            double best = 1e30;
+            for (int y = 1; y <= std::min(boxes, std::max(1, it.H / kResHalo3D)); y++)
+                for (int z = 1; y * z <= boxes && z <= std::max(1, it.D / kResHalo3D); z++) {
+                    const int ey = extent(it.H, y), ez = extent(it.D, z);
+                    if (res_fill_fit3d(it.W, ey, ez) < fill) continue;
+                    const double cost = (fewest ? 1e9 * y * z : 1e-3 * y * z) + (double)ey * ez;
+                    if (cost < best) best = cost, gy = y, gz = z;
+                }
+            return gy > 0;
+        };
+        const bool ok = search(share, 1.0, false) || search(share, kMinFill, false) ||
+                        search(b->res_grid, kMinFill, true) || search(b->res_grid, kLastFill, true);
+        if (!ok) {
+            in.res = 0;  // cannot be cut into boxes that fit: the rings take it
+            continue;
         }
+        const int G = gy * gz;
+        in.res_gy = gy;
+        in.res_stride = ((it.H + gy - 1) / gy) * ((it.D + gz - 1) / gz) * wl;
+        for (int k = 0; k < G; k++) {
+            const int kz = k / gy, ky = k % gy;
+            const int r0 = (int)((long long)kz * it.D / gz), r1 = (int)((long long)(kz + 1) * it.D / gz);
+            const int c0 = (int)((long long)ky * it.H / gy), c1 = (int)((long long)(ky + 1) * it.H / gy);
+            b->res_items.push_back(ResItem{v.second, k, G, r0, r1, G > 1 ? kResHalo3D : 0, c0, c1});
+        }
+        in.res_bands = G;
         b->any_res3d = true;
     }
     for (auto &m : imgs) {
@@ -347,7 +373,7 @@ static void plan_resident(bgt_batch *b)
         }
         for (int k = 0; k < G; k++) {
             const int r0 = (int)((long long)k * it.H / G), r1 = (int)((long long)(k + 1) * it.H / G);
-            b->res_items.push_back(ResItem{i, k, G, r0, r1, G > 1 ? kHalo : 0});
+            b->res_items.push_back(ResItem{i, k, G, r0, r1, G > 1 ? kHalo : 0, 0, it.W});
         }
     }
     for (int i = 0; i < N; i++)
@@ -386,7 +412,7 @@ static void init_inst(BatchItem &it, Inst &in)
 
 // Offsets of everything a batch keeps in its device pool.
 struct InstOffs {
-    size_t b0, b1, uni, lc, act, list;
+    size_t b0, b1, uni, lc, act, list, msg, cnt;
 };
 struct PoolLayout {
     std::vector<InstOffs> offs;
@@ -412,6 +438,12 @@ static PoolLayout layout_pool(const std::vector<Inst> &h, size_t n_res_items)
         o.act = off; off = align_up(off + (size_t)in.ntiles, 256);
         o.list = off; off = align_up(off + (size_t)in.ntiles * 4, 256);
         total_tiles += in.ntiles;
+        // messages between the boxes of a volume (two iterations' worth)
+        o.msg = o.cnt = 0;
+        if (in.res && in.dims == 3 && in.res_bands > 1) {
+            o.msg = off; off = align_up(off + 2 * (size_t)in.res_bands * in.res_stride * sizeof(uint2), 256);
+            o.cnt = off; off = align_up(off + 2 * (size_t)in.res_bands * 4, 256);
+        }
     }
     // all per-tile "last change" arrays in one block (one memset per run)
     L.off_lc = off;
@@ -510,6 +542,8 @@ extern "C" int bgt_batch_finalize(bgt_batch *b)
         in.lc = (int *)(P + o.lc);
         in.act = (uint8_t *)(P + o.act);
         in.list = (int *)(P + o.list);
+        in.res_msg = o.msg ? (uint2 *)(P + o.msg) : nullptr;
+        in.res_cnt = o.cnt ? (int *)(P + o.cnt) : nullptr;
         in.tmap = b->d_tmaps + kMapsPerInst * i;
         const CfgInfo &c = *cfg_info(in.cfg);
         CUtensorMap *m = &maps[(size_t)kMapsPerInst * i];

@@ -52,9 +52,10 @@ struct Sched {
 // iteration).  Items are taken in order by one fetch-and-add.
 struct ResItem {
     int inst;        // instance index
-    int band, bands; // band index and number of bands (1: the whole instance)
-    int r0, r1;      // 2D: core rows [r0, r1) of the band
-    int halo;        // 2D: halo rows kept on each side of the core (0 for a single band)
+    int band, bands; // band (3D: box) index and number of bands (1: the whole instance)
+    int r0, r1;      // 2D: core rows [r0, r1) of the band; 3D: core planes of the box
+    int halo;        // rows (3D: and planes) kept on each side of the core (0 for a single band)
+    int c0, c1;      // 3D: core rows of the box
 };
 struct ResSched {
     int head;        // next item
@@ -83,10 +84,10 @@ constexpr int kResSmemBytes = 230400;  // dynamic shared memory of one CTA (one 
 int res_smem_bytes();
 // Rows of a W-wide 2D band (core plus halo) that one CTA holds.
 int res_rows_fit2d(int W);
-// Non-empty bricks a D x H x W volume (or slab) may have to fit one CTA (0: its table does not fit).
-int res_slots_fit3d(int W, int H, int D);
-// Whether a D x H x W volume's brick table fits (its bricks are counted on the device).
-bool res_fits3d(int W, int H, int D);
+// Share of the words of a 3D box (ny rows x nz planes, halo included) that may be
+// non-empty for it to fit one CTA (negative: not even an empty one fits).
+double res_fill_fit3d(int W, int ny, int nz);
+constexpr int kResHalo3D = 6;  // one iteration: six subiterations, one row and plane each
 cudaError_t res_occupancy(int *per_sm);  // resident CTAs per SM
 cudaError_t launch_resident(int grid, Inst *d_insts, int ninst, const ResItem *d_items, int nitems,
                             ResSched *d_rs, ResTrace *d_trace, long long timeout_ns, cudaStream_t st);

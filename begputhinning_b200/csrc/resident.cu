@@ -32,18 +32,19 @@
 // reach at most its halo rows; if an iteration before the meeting was
 // already a fixed point, the one at the meeting is too.
 //
-// 3D volume (sparse bricks, one CTA).  Deletion never adds foreground, so
-// bricks of 32 voxels (one word) x 32 rows x 4 planes that are empty at the
-// start stay empty.  Only the non-empty ones are stored: a brick table maps
-// each brick to a slot (0: the all-zero brick), and three slot buffers hold
-// the state (ping-pong) and the iteration's pre-test union.  A warp
-// processes a brick, lane = row, marching through its four planes with a
-// three-plane window of 3x3 (row, word) neighbourhoods loaded from the
-// neighbouring bricks' slots.  Brick activity follows the iteration: a brick
-// whose 3x3x3 brick neighbourhood did not change during the previous
-// iteration has an empty union and cannot change (the argument of the tile
-// engine), so only active bricks are processed.  A volume whose non-empty
-// bricks do not fit is flagged `spill` and left to the tile engine.
+// 3D volume (dense boxes, word lists).  A box of the volume (rows x planes,
+// full width) lies once in shared memory.  Deletion never adds foreground,
+// so the words that are empty at the start are never looked at: each
+// iteration goes over the list of the others, keeps the active ones (a word
+// next to one that changed in the previous iteration: otherwise its union is
+// empty, the argument of the tile engine at word granularity), evaluates the
+// pre-test and U on them, one word per thread, and the words with a non-empty
+// union are the candidates of the five other subiterations.  A subiteration
+// finds its deletions, meets, and applies them, so the state needs no second
+// copy.  A large volume is cut into boxes on several CTAs that trade the
+// words changed near their edges after every iteration.  A volume of which a
+// box has more non-empty words than fit is flagged `spill` and left to the
+// tile engine.
 //
 // Rules, order of directions and termination are those of the tile engine
 // (2D/CUDA_ThinningKernelMultiBlock2D.cuh:104-135,
@@ -59,9 +60,6 @@ namespace bgt {
 namespace {
 constexpr int kWarps = kResThreads / 32;
 constexpr int kSmemBytes = kResSmemBytes;  // dynamic shared memory per CTA
-constexpr int kSlotWords = 129;      // 4 planes x 32 rows, plus one word so slots fall on different banks
-constexpr int kMaxBricks = 16384;    // brick table entries of a resident volume
-constexpr int kBZ = 4;               // planes per brick
 
 __host__ __device__ inline size_t up16(size_t v) { return (v + 15) & ~size_t(15); }
 }  // namespace
@@ -84,11 +82,13 @@ __host__ __device__ inline size_t res_words2d(int W, int nrows)
     return (size_t)pp * (1 + 2 * (size_t)nrows) + (size_t)ns * nch;
 }
 
-// bytes of shared memory a volume with nb bricks of which ns are non-empty needs
-__host__ __device__ inline size_t res_bytes3d(int nb, int ns)
+// bytes of shared memory a box of ny x nz rows of wl words (halo included)
+// needs when `listed` of its words are non-empty
+constexpr size_t kBoxListBytes = 4 + 4 + 4 + 4 + 2;  // list, candidate, union, deletions, active list
+__host__ __device__ inline size_t res_bytes3d(int wl, int ny, int nz, double listed)
 {
-    return up16((size_t)nb * 2) + up16((size_t)(ns + 1) * 4) + up16((size_t)(ns + 1) * 4) +
-           up16((size_t)(ns + 1) * 2) + (size_t)3 * (ns + 1) * kSlotWords * 4;
+    const size_t rows2 = (size_t)(ny + 2) * (nz + 2);
+    return up16((rows2 * (wl + 1) + 1) * 4) + 2 * up16(rows2 * 4) + (size_t)(listed * kBoxListBytes) + 80;
 }
 
 int res_smem_bytes() { return kSmemBytes; }
@@ -104,29 +104,48 @@ int res_rows_fit2d(int W)
     return lo;
 }
 
-int res_slots_fit3d(int W, int H, int D)
+double res_fill_fit3d(int W, int ny, int nz)
 {
-    const long long nb = (long long)((W + 31) / 32) * ((H + 31) / 32) * ((D + kBZ - 1) / kBZ);
-    if (nb > kMaxBricks) return 0;
-    int ns = 0;
-    while (res_bytes3d((int)nb, ns + 1) <= (size_t)kSmemBytes) ns++;
-    return ns;
-}
-
-bool res_fits3d(int W, int H, int D)
-{
-    const long long nb = (long long)((W + 31) / 32) * ((H + 31) / 32) * ((D + kBZ - 1) / kBZ);
-    return nb <= kMaxBricks && res_bytes3d((int)nb, 1) <= (size_t)kSmemBytes;
+    const int wl = (W + 31) / 32;
+    if ((long long)(ny + 2) * (nz + 2) * (wl + 1) >= 65535) return -1.0;  // words are indexed by 16 bits
+    const double words = (double)wl * ny * nz;
+    const size_t base = res_bytes3d(wl, ny, nz, 0.0);
+    if (base > (size_t)kSmemBytes) return -1.0;
+    return std::min(1.0, (double)((size_t)kSmemBytes - base) / kBoxListBytes / words);
 }
 
 // ------------------------------------------------------------ helpers -----
-__device__ __forceinline__ bool res_wait_at_least(const int *p, int target, long long timeout_ns)
+// The CTAs of one instance meet for the k-th time: each adds 1 to the low half
+// of meet[k & 1], and 1 to its high half when something of its own changed
+// since the last meeting; the wait (bounded) ends when all `bands` arrived.
+// Two words in turn, so that a CTA that is already at the next meeting leaves
+// what a late one reads here alone (it cannot get to the one after that).
+// One thread per CTA calls it, after a __syncthreads that follows the CTA's
+// writes to global memory.  Returns 0 when nobody changed anything, 1 when
+// somebody did, 2 when the wait ran out.
+struct MeetState {
+    unsigned k = 0, seen0 = 0, seen1 = 0;  // meetings so far, high halves after the last one of either word
+};
+__device__ __forceinline__ int res_meet(unsigned long long *meet, unsigned bands, bool changed, MeetState &m,
+                                        long long timeout_ns)
 {
+    unsigned long long *w = meet + (m.k & 1);
+    const unsigned arrivals = bands * (m.k / 2 + 1);
+    __threadfence();
+    atomicAdd(w, changed ? (1ull << 32) + 1ull : 1ull);
     const unsigned long long t_end = globaltimer() + (unsigned long long)timeout_ns;
     for (int spin = 0;; spin++) {
-        if (ld_acquire(p) >= target) return true;
-        if ((spin & 63) == 63 && globaltimer() > t_end) return false;
-        __nanosleep(spin < 16 ? 32 : 128);
+        const unsigned long long v = ld_acquire64(w);
+        if ((unsigned)v >= arrivals) {
+            const unsigned n = (unsigned)(v >> 32);
+            const bool some = n != ((m.k & 1) ? m.seen1 : m.seen0);
+            if (m.k & 1) m.seen1 = n;
+            else m.seen0 = n;
+            m.k++;
+            return some ? 1 : 0;
+        }
+        if ((spin & 63) == 63 && globaltimer() > t_end) return 2;
+        if (spin >= 4096) __nanosleep(64);  // partners that have not started yet
     }
 }
 
@@ -137,30 +156,6 @@ __device__ __forceinline__ int res_take(int *c)
     int k = 0;
     if ((threadIdx.x & 31) == 0) k = atomicAdd(c, 1);
     return __shfl_sync(kFull, k, 0);
-}
-
-// Exclusive prefix sum over the CTA of one int per thread; *total gets the sum.
-__device__ int res_block_exscan(int v, int *total)
-{
-    __shared__ int warp_sum[kWarps];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(kFull, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_sum[warp] = x;
-    __syncthreads();
-    int before = 0, all = 0;
-    for (int w = 0; w < kWarps; w++) {
-        const int s = warp_sum[w];
-        if (w < warp) before += s;
-        all += s;
-    }
-    __syncthreads();
-    *total = all;
-    return before + x - v;
 }
 
 // ------------------------------------------------------------ 2D ----------
@@ -375,6 +370,7 @@ __device__ void res_run2d(Inst &in, const ResItem &it, uint32_t *sm, ResSched *S
     __syncthreads();
 
     int result = 0;  // 1 converged, -1 pass cap or failed wait
+    MeetState meet;
     unsigned long long words = 0;
     int q = 0;
     for (;; q++) {
@@ -405,26 +401,13 @@ __device__ void res_run2d(Inst &in, const ResItem &it, uint32_t *sm, ResSched *S
             }
             __syncthreads();
             if (threadIdx.x == 0) {
-                __threadfence();
-                if (any) atomicMax(&in.res_last, q);
-                atomicAdd(&in.res_arrive, 1);
-                int f;
-                if (!res_wait_at_least(&in.res_arrive, it.bands * (e + 1), S->timeout_ns)) {
-                    atomicOr(&S->status, kErrQueueTimeout);
-                    f = 2;
-                } else {
-                    f = ld_acquire(&in.res_last) < q ? 1 : 0;
-                }
-                s_flag = f;
+                s_flag = res_meet(in.res_meet, it.bands, any, meet, S->timeout_ns);
+                if (s_flag == 2) atomicOr(&S->status, kErrQueueTimeout);
             }
             __syncthreads();
             const int f = s_flag;
-            if (f == 1) {
-                result = 1;
-                break;
-            }
-            if (f == 2) {
-                result = -1;
+            if (f != 1) {
+                result = f == 0 ? 1 : -1;
                 break;
             }
             // halo rows: the neighbours' boundary core rows after pass q
@@ -475,187 +458,201 @@ __device__ void res_run2d(Inst &in, const ResItem &it, uint32_t *sm, ResSched *S
 }
 
 // ------------------------------------------------------------ 3D ----------
-struct Vol3D {
-    uint16_t *tab;     // [nbz][nby][nbx] -> slot (0: empty)
-    int *coord;        // slot -> linear brick index
-    uint8_t *act;      // slot: active in this iteration
-    uint8_t *chg;      // slot: changed in this iteration
-    uint8_t *nxt;      // slot: active in the next iteration
-    uint8_t *ufl;      // slot: its pre-test union of this iteration is not empty
-    uint16_t *list;    // active slots of this iteration
-    uint32_t *X, *Y, *U;  // slot buffers (slot 0 = the zero brick)
-    int nbx, nby, nbz, nslots;
+// Entry of a box's word list: word index in shared memory (16 bits), its
+// column in the rows' change masks (5 bits), its distance from the box's core
+// (3 bits, 0 = core), and, in the candidate list, whether it changed.
+constexpr uint32_t kEntChanged = 1u << 24;
+__device__ __forceinline__ uint32_t ent_idx(uint32_t e) { return e & 0xffffu; }
+__device__ __forceinline__ uint32_t ent_col(uint32_t e) { return (e >> 16) & 31u; }
+__device__ __forceinline__ int ent_dist(uint32_t e) { return (int)((e >> 21) & 7u); }
+
+struct Box3D {
+    uint32_t *state;      // [nz + 2][ny + 2] rows of wl words, a zero word between rows, a zero word at the end
+    uint32_t *cidx, *cU, *cdel;  // candidates of this iteration: entry, union, deletions of the subiteration
+    int p, ps;            // words between rows, between planes
 };
 
-// The nine row/word neighbourhood words of one plane (offset `off` within
-// the slots) from the slot bases of the rows above (u), this row (o) and
-// below (d), each for the words x-1, x, x+1.
-__device__ __forceinline__ void res_plane9(const uint32_t *__restrict__ IN, const int (&u)[3], const int (&o)[3],
-                                           const int (&d)[3], int off, uint32_t (&P)[9])
+// The 3x3x3 neighbourhood words of the word at s.
+__device__ __forceinline__ void box_window(const uint32_t *s, int p, int ps, uint32_t (&g)[27])
 {
-    const uint32_t ul = IN[u[0] + off], uc = IN[u[1] + off], ur = IN[u[2] + off];
-    const uint32_t ol = IN[o[0] + off], oc = IN[o[1] + off], orr = IN[o[2] + off];
-    const uint32_t dl = IN[d[0] + off], dc = IN[d[1] + off], dr = IN[d[2] + off];
-    P[0] = at_xm1(uc, ul); P[1] = uc; P[2] = at_xp1(uc, ur);
-    P[3] = at_xm1(oc, ol); P[4] = oc; P[5] = at_xp1(oc, orr);
-    P[6] = at_xm1(dc, dl); P[7] = dc; P[8] = at_xp1(dc, dr);
-}
-
-// Slot bases (word index of this lane's row) of the three x-neighbour bricks
-// in the z-layer dzb (-1, 0, +1) for the rows above, at and below this lane's
-// row; nb27 holds, in lane k < 27, the slot of brick offset
-// (k/9 - 1, (k/3)%3 - 1, k%3 - 1) in (z, y, x).
-__device__ __forceinline__ void res_bases3d(int nb27, int dzb, int (&u)[3], int (&o)[3], int (&d)[3])
-{
-    const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
-        const int so = __shfl_sync(kFull, nb27, 9 * (dzb + 1) + 3 + c);
-        const int su = __shfl_sync(kFull, nb27, 9 * (dzb + 1) + c);
-        const int sd = __shfl_sync(kFull, nb27, 9 * (dzb + 1) + 6 + c);
-        o[c] = so * kSlotWords + lane;
-        u[c] = lane == 0 ? su * kSlotWords + 31 : so * kSlotWords + lane - 1;
-        d[c] = lane == 31 ? sd * kSlotWords : so * kSlotWords + lane + 1;
+    for (int k = 0; k < 9; k++) {
+        const uint32_t *r = s + (k / 3 - 1) * ps + (k % 3 - 1) * p;
+        const uint32_t l = r[-1], c = r[0], n = r[1];
+        g[3 * k] = at_xm1(c, l);
+        g[3 * k + 1] = c;
+        g[3 * k + 2] = at_xp1(c, n);
     }
 }
 
-// Subiteration J (0: pre-test union + U; 1..5: N, E, D, S, W) on brick slot s.
-// J = 0 also ORs the brick's union bits into *uany.
+// Position of this lane's element in a list the warp appends to (-1: none).
+__device__ __forceinline__ int warp_append(bool take, int *count)
+{
+    const unsigned m = __ballot_sync(kFull, take);
+    int base = 0;
+    if ((threadIdx.x & 31) == 0 && m) base = atomicAdd(count, __popc(m));
+    base = __shfl_sync(kFull, base, 0);
+    return take ? base + __popc(m & ((1u << (threadIdx.x & 31)) - 1u)) : -1;
+}
+
+// Subiteration J (1..5: N, E, D, S, W) on the candidates: find the deletions,
+// meet, apply them, meet.  Words farther than 5 - J from the core are left
+// alone: what they read may be wrong by now, and nothing reads them before
+// their owner sends them.
 template <int J>
-__device__ uint32_t res_brick3d(const Vol3D &v, int s, const uint32_t *__restrict__ IN, uint32_t *__restrict__ OUT,
-                                uint32_t *__restrict__ U, uint32_t *uany)
+__device__ __forceinline__ uint32_t box_deletions(const Box3D &b, uint32_t e, uint32_t cand)
 {
-    const int lane = threadIdx.x & 31;
-    const int li = v.coord[s];
-    const int bx = li % v.nbx, by = (li / v.nbx) % v.nby, bz = li / (v.nbx * v.nby);
-    int nb27 = 0;
-    if (lane < 27) {
-        const int zz = bz + lane / 9 - 1, yy = by + (lane / 3) % 3 - 1, xx = bx + lane % 3 - 1;
-        if (zz >= 0 && zz < v.nbz && yy >= 0 && yy < v.nby && xx >= 0 && xx < v.nbx)
-            nb27 = v.tab[(zz * v.nby + yy) * v.nbx + xx];
-    }
-    int u[3], o[3], d[3];
-    uint32_t A[9], B[9], Cn[9];
-    res_bases3d(nb27, -1, u, o, d);
-    res_plane9(IN, u, o, d, 3 * 32, A);  // plane 4bz - 1: last plane of the brick below
-    res_bases3d(nb27, 0, u, o, d);
-    res_plane9(IN, u, o, d, 0, B);
-    const int self = s * kSlotWords + lane;
-    uint32_t chg = 0;
-#pragma unroll 1
-    for (int q = 0; q < kBZ; q++) {
-        if (q == kBZ - 1) res_bases3d(nb27, 1, u, o, d);
-        res_plane9(IN, u, o, d, ((q + 1) & 3) * 32, Cn);
-        const uint32_t val = B[4];
-        uint32_t nv = val;
-        const int widx = self + q * 32;
-        if constexpr (J == 0) {
-            uint32_t un = 0;
-            if (__any_sync(kFull, val != 0u)) {
-                uint32_t g[27];
-#pragma unroll
-                for (int i = 0; i < 9; i++) {
-                    g[i] = A[i];
-                    g[9 + i] = B[i];
-                    g[18 + i] = Cn[i];
-                }
-                const uint32_t du = rule3d<0>(g);
-                un = (du | rule3d<1>(g) | rule3d<2>(g) | rule3d<3>(g) | rule3d<4>(g) | rule3d<5>(g)) & val;
-                nv = val & ~du;
-            }
-            U[widx] = un;
-            *uany |= un;
-        } else {
-            const uint32_t cand = val & U[widx];
-            if (__any_sync(kFull, cand != 0u)) {
-                uint32_t g[27];
-#pragma unroll
-                for (int i = 0; i < 9; i++) {
-                    g[i] = A[i];
-                    g[9 + i] = B[i];
-                    g[18 + i] = Cn[i];
-                }
-                nv = val & ~(cand & rule3d<J>(g));
-            }
-        }
-        OUT[widx] = nv;
-        chg |= val ^ nv;
-#pragma unroll
-        for (int i = 0; i < 9; i++) {
-            A[i] = B[i];
-            B[i] = Cn[i];
-        }
-    }
-    return chg;
+    if (ent_dist(e) > 5 - J || cand == 0u) return 0u;
+    uint32_t g[27];
+    box_window(b.state + ent_idx(e), b.p, b.ps, g);
+    return cand & rule3d<J>(g);
 }
 
-// One volume, or one z-slab of a large volume: brick layers [r0, r1) are
-// the slab's core, `halo` layers on each side (clamped to the volume) are
-// held too and recomputed.  Slabs run whole iterations (pre-test, U, N, E, D,
-// S, W) in lockstep and trade their boundary layers through global memory
-// after each: errors entering at a slab's outer edge move one plane per
-// subiteration (the pre-test's union reads one plane further, inside the
-// same bound), six planes in an iteration, so a halo of two layers (eight
-// planes) keeps the core exact.  Halo bricks and the core bricks next to
-// them are processed in every iteration.
-__device__ void res_run3d(Inst &in, const ResItem &it, uint8_t *smb, ResSched *S, int *take)
+// ... with any number of candidates per thread
+template <int J>
+__device__ __forceinline__ void box_subiteration(const Box3D b, int nc, unsigned &words)
 {
-    __shared__ int s_cnt, s_flag;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    Vol3D v;
-    const int wl = (in.W + 31) >> 5;
-    const int nbz_all = (in.D + kBZ - 1) / kBZ;
-    const bool banded = it.bands > 1;
-    const int c_lo = banded ? it.r0 : 0, c_hi = banded ? it.r1 : nbz_all;
-    const int e_lo = max(0, c_lo - it.halo), e_hi = min(nbz_all, c_hi + it.halo);
-    v.nbx = wl;
-    v.nby = (in.H + 31) >> 5;
-    v.nbz = e_hi - e_lo;
-    const int bz0 = e_lo;
-    const int nb = v.nbx * v.nby * v.nbz;
-    v.tab = reinterpret_cast<uint16_t *>(smb);
-    for (int i = threadIdx.x; i < nb; i += kResThreads) v.tab[i] = 0;
+    bool any = false;
+    for (int c = threadIdx.x; c < nc; c += kResThreads) {
+        const uint32_t e = b.cidx[c];
+        const uint32_t del = box_deletions<J>(b, e, b.state[ent_idx(e)] & b.cU[c]);
+        words += ent_dist(e) == 0;
+        any |= del != 0u;
+        b.cdel[c] = del;
+    }
+    if (!__syncthreads_or(any)) return;
+    for (int c = threadIdx.x; c < nc; c += kResThreads) {
+        const uint32_t del = b.cdel[c];
+        if (del) {
+            const uint32_t e = b.cidx[c];
+            b.state[ent_idx(e)] &= ~del;
+            b.cidx[c] = e | kEntChanged;
+        }
+    }
     __syncthreads();
-    // mark the non-empty bricks: one coalesced pass over the used words of
-    // the held planes (word i of the pass = word i % wl of row i / wl)
+}
+
+// ... with at most one: its word, union and entry stay in registers
+template <int J>
+__device__ __forceinline__ void box_subiteration1(const Box3D b, uint32_t e, uint32_t un, uint32_t &val, unsigned &words)
+{
+    const uint32_t del = box_deletions<J>(b, e, val & un);
+    words += un != 0u && ent_dist(e) == 0;
+    if (!__syncthreads_or(del != 0u)) return;
+    if (del) {
+        val &= ~del;
+        b.state[ent_idx(e)] = val;
+    }
+    __syncthreads();
+}
+
+// One volume, or one box of it: rows [c0, c1) of planes [r0, r1) are the
+// core; `halo` rows and planes around it (clamped to the volume) are held
+// too.  Boxes run whole iterations (pre-test, U, N, E, D, S, W) in lockstep.
+// A wrong value moves one row or plane per subiteration (the pre-test reads
+// the same neighbours as U), so with six halo rows and planes the core is
+// exact after an iteration; then every box sends the words near its core's
+// edge that changed to a list in global memory, the boxes meet, and each
+// takes over what lies in its halo from its neighbours' lists.
+//
+// Bound: the latency of an iteration (about 10 us: six dependent subiterations
+// with two barriers each, then the meeting), not throughput: a box has some
+// hundred active words.  Against warps marching through sparse bricks of
+// 32 x 32 x 4 voxels, every brick of the neighbourhood of a change evaluated
+// whole (24 us per iteration): a 97 x 75 x 66 tree volume 214 -> 72 us, a
+// 187 x 203 x 161 one 955 -> 150 us, a 256^3 one, whose bricks did not fit,
+// 1330 us on the tile rings -> 176 us.
+__device__ void res_run3d(Inst &in, const ResItem &it, uint8_t *smb, ResSched *S)
+{
+    __shared__ int s_n[4];  // lengths: word list, active words, candidates, messages
+    __shared__ int s_flag;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int W = in.W, H = in.H, D = in.D, P = in.P, wl = (W + 31) >> 5;
+    const bool team = it.bands > 1;
+    const int z0 = max(0, it.r0 - it.halo), z1 = min(D, it.r1 + it.halo);
+    const int y0 = max(0, it.c0 - it.halo), y1 = min(H, it.c1 + it.halo);
+    const int nz = z1 - z0, ny = y1 - y0, ny2 = ny + 2, rows2 = (nz + 2) * ny2;
+    int xs = 0;  // words per column of the change masks: 1 << xs
+    while (((wl - 1) >> xs) > 31) xs++;
+    Box3D b;
+    b.p = wl + 1;
+    b.ps = ny2 * b.p;
+    const uint32_t mp = 0xffffffffu / (uint32_t)b.p + 1u;
+    const uint32_t mny = 0xffffffffu / (uint32_t)ny2 + 1u;
+    const int nwords = rows2 * b.p + 1;
+    size_t off = 0;
+    b.state = reinterpret_cast<uint32_t *>(smb);
+    off += up16((size_t)nwords * 4);
+    uint32_t *const act = reinterpret_cast<uint32_t *>(smb + off);
+    off += up16((size_t)rows2 * 4);
+    uint32_t *const chg = reinterpret_cast<uint32_t *>(smb + off);
+    off += up16((size_t)rows2 * 4);
+    uint32_t *const list = reinterpret_cast<uint32_t *>(smb + off);
+    const int list_cap = (int)(((size_t)kSmemBytes - off) / 4);
+
+    for (size_t i = threadIdx.x; i < off / 16; i += kResThreads) reinterpret_cast<uint4 *>(smb)[i] = make_uint4(0, 0, 0, 0);
+    if (threadIdx.x < 4) s_n[threadIdx.x] = 0;
+    __syncthreads();
     const uint32_t *g0 = in.buf[0];
-    const int z_first = kBZ * e_lo, z_end = min(in.D, kBZ * e_hi);
+    // words of the box in raster order, a thread every kResThreads-th one
+    const int nbox = nz * ny * wl;
+    const int qr = kResThreads / wl, dx = kResThreads - qr * wl, dz = qr / ny, dy = qr - dz * ny;
+    struct Pos {
+        int x, y, z;
+    };
+    auto first_pos = [&]() {
+        const int r = (int)threadIdx.x / wl;
+        return Pos{(int)threadIdx.x - r * wl, r % ny, r / ny};
+    };
+    auto advance = [&](Pos &q) {
+        q.x += dx;
+        q.y += dy;
+        q.z += dz;
+        if (q.x >= wl) {
+            q.x -= wl;
+            q.y++;
+        }
+        if (q.y >= ny) {
+            q.y -= ny;
+            q.z++;
+        }
+    };
+    auto index_of = [&](const Pos &q) { return ((q.z + 1) * ny2 + q.y + 1) * b.p + 1 + q.x; };
     {
-        const int nw = (z_end - z_first) * in.H * wl;
-        const size_t base = (size_t)z_first * in.H;
-        for (int i = threadIdx.x; i < nw; i += kResThreads) {
-            const int r = i / wl, x = i - r * wl;
-            if (__ldcg(g0 + (base + r) * in.P + x) != 0u) {
-                const int zl = r / in.H, y = r - zl * in.H;
-                v.tab[((zl / kBZ) * v.nby + (y >> 5)) * v.nbx + x] = 1;
+        constexpr int U = 4;  // loads in flight per thread
+        Pos q = first_pos();
+        for (int i = threadIdx.x; i - lane < nbox; i += U * kResThreads) {
+            uint32_t v[U];
+            Pos at[U];
+#pragma unroll
+            for (int k = 0; k < U; k++) {
+                at[k] = q;
+                v[k] = i + k * kResThreads < nbox ? __ldcg(g0 + ((size_t)(z0 + q.z) * H + (y0 + q.y)) * P + q.x) : 0u;
+                advance(q);
+            }
+#pragma unroll
+            for (int k = 0; k < U; k++) {
+                const int y = y0 + at[k].y, z = z0 + at[k].z;
+                const int d = max(max(max(it.c0 - y, y - it.c1 + 1), max(it.r0 - z, z - it.r1 + 1)), 0);
+                const int idx = v[k] ? index_of(at[k]) : 0;
+                if (v[k]) b.state[idx] = v[k];
+                const int pos = warp_append(v[k] != 0u && d <= 5, &s_n[0]);
+                if (pos >= 0 && pos < list_cap)
+                    list[pos] = (uint32_t)idx | (uint32_t)(at[k].x >> xs) << 16 | (uint32_t)d << 21;
             }
         }
     }
     __syncthreads();
-    // slots in raster order of the bricks
-    const int per = (nb + kResThreads - 1) / kResThreads;
-    const int i0 = min(nb, threadIdx.x * per), i1 = min(nb, i0 + per);
-    int cnt = 0;
-    for (int i = i0; i < i1; i++) cnt += v.tab[i] != 0;
-    int total = 0;
-    const int first = res_block_exscan(cnt, &total);
-    v.nslots = total;
-    const bool fits = res_bytes3d(nb, total) <= (size_t)kSmemBytes;
-    if (banded) {
-        // every slab must fit, or the tile engine takes the whole volume:
-        // the slabs agree before any of them writes anything
+    const int nl = s_n[0];
+    MeetState meet;
+    const bool fits = off + (size_t)nl * kBoxListBytes + 64 <= (size_t)kSmemBytes;
+    if (team) {
+        // every box must fit, or the tile engine takes the whole volume: the
+        // boxes agree before any of them writes anything
         if (threadIdx.x == 0) {
             if (!fits) atomicExch(&in.spill, 1);
-            __threadfence();
-            atomicAdd(&in.res_arrive, 1);
-            int f;
-            if (!res_wait_at_least(&in.res_arrive, it.bands, S->timeout_ns)) {
-                atomicOr(&S->status, kErrQueueTimeout);
-                f = 2;
-            } else {
-                f = ld_acquire(&in.spill) ? 1 : 0;
-            }
-            s_flag = f;
+            s_flag = res_meet(in.res_meet, it.bands, !fits, meet, S->timeout_ns);
+            if (s_flag == 2) atomicOr(&S->status, kErrQueueTimeout);
         }
         __syncthreads();
         if (s_flag) {
@@ -669,218 +666,199 @@ __device__ void res_run3d(Inst &in, const ResItem &it, uint8_t *smb, ResSched *S
         __syncthreads();
         return;
     }
-    size_t off = up16((size_t)nb * 2);
-    v.coord = reinterpret_cast<int *>(smb + off);
-    off += up16((size_t)(total + 1) * 4);
-    v.act = smb + off;
-    v.chg = v.act + (total + 1);
-    v.nxt = v.chg + (total + 1);
-    v.ufl = v.nxt + (total + 1);
-    off += up16((size_t)(total + 1) * 4);
-    v.list = reinterpret_cast<uint16_t *>(smb + off);
-    off += up16((size_t)(total + 1) * 2);
-    v.X = reinterpret_cast<uint32_t *>(smb + off);
-    v.Y = v.X + (size_t)(total + 1) * kSlotWords;
-    v.U = v.Y + (size_t)(total + 1) * kSlotWords;
-    {
-        int sl = first + 1;
-        for (int i = i0; i < i1; i++)
-            if (v.tab[i]) {
-                v.tab[i] = (uint16_t)sl;
-                v.coord[sl] = i;
-                sl++;
-            }
-    }
-    for (int i = threadIdx.x; i < kSlotWords; i += kResThreads) {
-        v.X[i] = 0u;
-        v.Y[i] = 0u;
-        v.U[i] = 0u;
-    }
-    for (int i = threadIdx.x; i <= total; i += kResThreads) {
-        v.act[i] = i > 0;
-        v.chg[i] = 0;
-        v.nxt[i] = 0;
-        v.ufl[i] = 0;
-    }
-    if (threadIdx.x < 2) take[threadIdx.x] = 0;
+    b.cidx = list + nl;
+    b.cU = b.cidx + nl;
+    b.cdel = b.cU + nl;
+    uint16_t *const alist = reinterpret_cast<uint16_t *>(b.cdel + nl);
+    for (int r = threadIdx.x; r < rows2; r += kResThreads) act[r] = kFull;
     __syncthreads();
-    // brick layer (global) of a slot
-    auto layer_of = [&](int s) { return bz0 + v.coord[s] / (v.nbx * v.nby); };
-    // copy the slot's words from / to packed volume g (rows inside the volume only)
-    auto gather = [&](const uint32_t *g, int s, bool both) {
-        const int li = v.coord[s];
-        const int bx = li % v.nbx, by = (li / v.nbx) % v.nby, bz = bz0 + li / (v.nbx * v.nby);
-        const int y = 32 * by + lane;
-#pragma unroll
-        for (int q = 0; q < kBZ; q++) {
-            const int z = kBZ * bz + q;
-            const uint32_t w = (y < in.H && z < in.D) ? __ldcg(g + ((size_t)z * in.H + y) * in.P + bx) : 0u;
-            v.X[s * kSlotWords + q * 32 + lane] = w;
-            if (both) v.Y[s * kSlotWords + q * 32 + lane] = w;
-        }
-    };
-    auto scatter = [&](uint32_t *g, int s) {
-        const int li = v.coord[s];
-        const int bx = li % v.nbx, by = (li / v.nbx) % v.nby, bz = bz0 + li / (v.nbx * v.nby);
-        const int y = 32 * by + lane;
-        if (y >= in.H) return;
-#pragma unroll
-        for (int q = 0; q < kBZ; q++) {
-            const int z = kBZ * bz + q;
-            if (z < in.D) g[((size_t)z * in.H + y) * in.P + bx] = v.X[s * kSlotWords + q * 32 + lane];
-        }
-    };
-    // gather the non-empty bricks (both state buffers)
-    for (int s = warp + 1; s <= total; s += kWarps) gather(g0, s, true);
-    __syncthreads();
-    // layers processed in every iteration of a slab: its halo and the core layers next to it
-    const int keep_lo = it.band > 0 ? c_lo + it.halo : 0;
-    const int keep_hi = it.band + 1 < it.bands ? c_hi - it.halo : nbz_all;
 
+    const int gy = in.res_gy;  // boxes along y
+    const int bz = it.band / gy, by = it.band - bz * gy, gz = it.bands / gy;
     int iter = 0, result = 0;
-    unsigned long long words = 0, bricks = 0;
+    unsigned words = 0, entries = 0;
     const int cap_it = in.pass_cap / 6 + 1;
     for (;; iter++) {
-        if (threadIdx.x == 0) s_cnt = 0;
-        __syncthreads();
-        for (int s = threadIdx.x + 1; s <= total; s += kResThreads)
-            if (v.act[s]) v.list[atomicAdd(&s_cnt, 1)] = (uint16_t)s;
-        __syncthreads();
-        int nact = s_cnt;
-        for (int j = 0; j < 6; j++) {
-            if (j == 1) {
-                // a brick whose union is empty cannot change in the rest of
-                // the iteration (every deletion is of a union voxel), and both
-                // of its buffers already hold its state: only the others go on
-                if (threadIdx.x == 0) s_cnt = 0;
-                __syncthreads();
-                for (int s = threadIdx.x + 1; s <= total; s += kResThreads)
-                    if (v.act[s] && v.ufl[s]) v.list[atomicAdd(&s_cnt, 1)] = (uint16_t)s;
-                __syncthreads();
-                nact = s_cnt;
+        // active words: a word of the row's 3x3 rows that is at most one
+        // column away changed in the previous iteration (otherwise its union
+        // is empty), and some voxel of it misses one of its face neighbours
+        for (int base = warp * 32; base < nl; base += kResThreads) {
+            const int k = base + lane;
+            bool on = false;
+            if (k < nl) {
+                const uint32_t e = list[k], idx = ent_idx(e);
+                if ((act[__umulhi(idx, mp)] >> ent_col(e)) & 1u) {
+                    const uint32_t *s = b.state + idx;
+                    const uint32_t c = *s;
+                    const uint32_t faces = at_xm1(c, s[-1]) & at_xp1(c, s[1]) & s[b.p] & s[-b.p] & s[b.ps] & s[-b.ps];
+                    on = (c & ~faces) != 0u;
+                }
             }
-            if (threadIdx.x == 0) take[(j + 1) & 1] = 0;
-            const uint32_t *IN = (j & 1) ? v.Y : v.X;
-            uint32_t *OUT = (j & 1) ? v.X : v.Y;
-            for (;;) {
-                const int k = res_take(take + (j & 1));
-                if (k >= nact) break;
-                const int s = v.list[k];
-                uint32_t c, uany = 0;
-                switch (j) {
-                case 0: c = res_brick3d<0>(v, s, IN, OUT, v.U, &uany); break;
-                case 1: c = res_brick3d<1>(v, s, IN, OUT, v.U, &uany); break;
-                case 2: c = res_brick3d<2>(v, s, IN, OUT, v.U, &uany); break;
-                case 3: c = res_brick3d<3>(v, s, IN, OUT, v.U, &uany); break;
-                case 4: c = res_brick3d<4>(v, s, IN, OUT, v.U, &uany); break;
-                default: c = res_brick3d<5>(v, s, IN, OUT, v.U, &uany); break;
+            const int pos = warp_append(on, &s_n[1]);
+            if (pos >= 0) alist[pos] = (uint16_t)k;
+        }
+        __syncthreads();
+        const int na = s_n[1];
+        // pre-test and U
+        for (int base = warp * 32; base < na; base += kResThreads) {
+            const int k = base + lane;
+            uint32_t e = 0, un = 0, du = 0;
+            if (k < na) {
+                e = list[alist[k]];
+                const uint32_t *s = b.state + ent_idx(e);
+                uint32_t g[27];
+                box_window(s, b.p, b.ps, g);
+                du = rule3d<0>(g) & g[13];
+                un = (du | rule3d<1>(g) | rule3d<2>(g) | rule3d<3>(g) | rule3d<4>(g) | rule3d<5>(g)) & g[13];
+                words += ent_dist(e) == 0;
+                entries++;
+            }
+            const int c = warp_append(un != 0u, &s_n[2]);
+            if (c >= 0) {
+                b.cidx[c] = e;
+                b.cU[c] = un;
+                b.cdel[c] = du;
+            }
+        }
+        __syncthreads();
+        const int nc = s_n[2];
+        if (nc > kResThreads) {
+            for (int c = threadIdx.x; c < nc; c += kResThreads) {
+                const uint32_t del = b.cdel[c];
+                if (del) {
+                    const uint32_t e = b.cidx[c];
+                    b.state[ent_idx(e)] &= ~del;
+                    b.cidx[c] = e | kEntChanged;
                 }
-                if (j == 0) {
-                    const bool u = __any_sync(kFull, uany != 0u);
-                    if (lane == 0) v.ufl[s] = u;
-                }
-                if (lane == 0) {
-                    const int li = v.coord[s];
-                    const int by = (li / v.nbx) % v.nby, bz = bz0 + li / (v.nbx * v.nby);
-                    if (bz >= c_lo && bz < c_hi) {
-                        words += (unsigned long long)min(32, in.H - 32 * by) * min(kBZ, in.D - kBZ * bz);
-                        bricks++;
-                    }
-                }
-                if (__any_sync(kFull, c != 0u) && lane == 0) v.chg[s] = 1;
             }
             __syncthreads();
+            box_subiteration<1>(b, nc, words);
+            box_subiteration<2>(b, nc, words);
+            box_subiteration<3>(b, nc, words);
+            box_subiteration<4>(b, nc, words);
+            box_subiteration<5>(b, nc, words);
+        } else if (nc > 0) {
+            const int c = threadIdx.x;
+            uint32_t e = 0, un = 0, val = 0, del = 0;
+            if (c < nc) {
+                e = b.cidx[c];
+                un = b.cU[c];
+                del = b.cdel[c];
+                val = b.state[ent_idx(e)];
+            }
+            const uint32_t before = val;
+            if (del) {
+                val &= ~del;
+                b.state[ent_idx(e)] = val;
+            }
+            __syncthreads();
+            box_subiteration1<1>(b, e, un, val, words);
+            box_subiteration1<2>(b, e, un, val, words);
+            box_subiteration1<3>(b, e, un, val, words);
+            box_subiteration1<4>(b, e, un, val, words);
+            box_subiteration1<5>(b, e, un, val, words);
+            if (val != before) b.cidx[c] = e | kEntChanged;
         }
-        // next iteration's bricks: the 3x3x3 brick neighbourhoods of the
-        // changed ones; `core` = a core brick changed
-        int core = 0;
-        for (int s = threadIdx.x + 1; s <= total; s += kResThreads) {
-            const int bzs = layer_of(s);
-            if (banded && (bzs < keep_lo || bzs >= keep_hi)) v.nxt[s] = 1;
-            if (!v.chg[s]) continue;
-            if (bzs >= c_lo && bzs < c_hi) core = 1;
-            const int li = v.coord[s];
-            const int bx = li % v.nbx, by = (li / v.nbx) % v.nby, bz = li / (v.nbx * v.nby);
-            for (int dz = -1; dz <= 1; dz++) {
-                const int zz = bz + dz;
-                if (zz < 0 || zz >= v.nbz) continue;
-                for (int dy = -1; dy <= 1; dy++) {
-                    const int yy = by + dy;
-                    if (yy < 0 || yy >= v.nby) continue;
-                    for (int dx = -1; dx <= 1; dx++) {
-                        const int xx = bx + dx;
-                        if (xx < 0 || xx >= v.nbx) continue;
-                        const int n = v.tab[(zz * v.nby + yy) * v.nbx + xx];
-                        if (n) v.nxt[n] = 1;
-                    }
-                }
+        // changed words of the core: marks, and messages to the boxes around
+        bool core = false;
+        uint2 *msg = nullptr;
+        if (team) msg = in.res_msg + ((size_t)(iter & 1) * it.bands + it.band) * in.res_stride;
+        for (int c = threadIdx.x; c < nc; c += kResThreads) {
+            const uint32_t e = b.cidx[c];
+            if (!(e & kEntChanged) || ent_dist(e) != 0) continue;
+            core = true;
+            const uint32_t idx = ent_idx(e), row = __umulhi(idx, mp);
+            atomicOr(&chg[row], 1u << ent_col(e));
+            if (!team) continue;
+            const int zz = (int)__umulhi(row, mny), y = y0 + (int)row - zz * ny2 - 1, z = z0 + zz - 1;
+            const int h = it.halo;
+            if ((it.r0 > 0 && z < it.r0 + h) || (it.r1 < D && z >= it.r1 - h) || (it.c0 > 0 && y < it.c0 + h) ||
+                (it.c1 < H && y >= it.c1 - h)) {
+                const int x = (int)idx - (int)row * b.p - 1;
+                msg[atomicAdd(&s_n[3], 1)] = make_uint2(((uint32_t)z * (uint32_t)H + (uint32_t)y) * (uint32_t)wl + (uint32_t)x,
+                                                        b.state[idx]);
             }
         }
-        const bool any_core = __syncthreads_or(core);
-        if (!banded) {
-            if (!any_core) {
+        const bool any = __syncthreads_or(core);
+        bool any_chg = any;
+        if (!team) {
+            if (!any) {
                 result = 1;
                 break;
             }
         } else {
-            // trade boundary layers with the neighbouring slabs (state in X)
-            uint32_t *gx = in.buf[(iter + 1) & 1];  // buf[0] holds the start state other slabs may still load
-            for (int s = warp + 1; s <= total; s += kWarps) {
-                const int bzs = layer_of(s);
-                const bool out_lo = it.band > 0 && bzs >= c_lo && bzs < c_lo + it.halo;
-                const bool out_hi = it.band + 1 < it.bands && bzs >= c_hi - it.halo && bzs < c_hi;
-                if (out_lo || out_hi) scatter(gx, s);
-            }
-            __syncthreads();
             if (threadIdx.x == 0) {
-                __threadfence();
-                if (any_core) atomicMax(&in.res_last, iter);
-                atomicAdd(&in.res_arrive, 1);
-                int f;
-                if (!res_wait_at_least(&in.res_arrive, it.bands * (iter + 2), S->timeout_ns)) {
-                    atomicOr(&S->status, kErrQueueTimeout);
-                    f = 2;
-                } else {
-                    f = ld_acquire(&in.res_last) < iter ? 1 : 0;
-                }
-                s_flag = f;
+                in.res_cnt[(iter & 1) * it.bands + it.band] = s_n[3];
+                s_flag = res_meet(in.res_meet, it.bands, any, meet, S->timeout_ns);
+                if (s_flag == 2) atomicOr(&S->status, kErrQueueTimeout);
             }
             __syncthreads();
             const int f = s_flag;
-            if (f == 1) {
-                result = 1;
+            if (f != 1) {
+                result = f == 0 ? 1 : -1;
                 break;
             }
-            if (f == 2) {
-                result = -1;
-                break;
+            // three warps per neighbouring box take over its messages
+            const int k8 = warp & 7, k9 = k8 < 4 ? k8 : k8 + 1;
+            const int nbz = bz + k9 / 3 - 1, nby = by + k9 % 3 - 1;
+            if (nbz >= 0 && nbz < gz && nby >= 0 && nby < gy) {
+                const int nb = nbz * gy + nby;
+                const uint2 *m = in.res_msg + ((size_t)(iter & 1) * it.bands + nb) * in.res_stride;
+                const int k0 = (warp >> 3) * 32 + lane;
+                // the first message is loaded beside the count, whether it is one or not
+                uint2 v = k0 < in.res_stride ? __ldcg(m + k0) : make_uint2(0u, 0u);
+                const int n = __ldcg(in.res_cnt + (iter & 1) * it.bands + nb);
+                for (int k = k0; k < n;) {
+                    const int r = (int)(v.x / (uint32_t)wl), x = (int)v.x - r * wl, z = r / H, y = r - z * H;
+                    if (z >= z0 && z < z1 && y >= y0 && y < y1) {
+                        const int row = (z - z0 + 1) * ny2 + (y - y0 + 1);
+                        b.state[row * b.p + 1 + x] = v.y;
+                        atomicOr(&chg[row], 1u << (x >> xs));
+                        any_chg = true;
+                    }
+                    k += (kWarps / 8) * 32;
+                    if (k < n) v = __ldcg(m + k);
+                }
             }
-            for (int s = warp + 1; s <= total; s += kWarps) {
-                const int bzs = layer_of(s);
-                if (bzs < c_lo || bzs >= c_hi) gather(gx, s, true);
-            }
-        }
-        for (int s = threadIdx.x + 1; s <= total; s += kResThreads) {
-            v.act[s] = v.nxt[s];
-            v.nxt[s] = 0;
-            v.chg[s] = 0;
+            any_chg = __syncthreads_or(any_chg);
         }
         if (iter + 1 >= cap_it) {
             if (threadIdx.x == 0) atomicOr(&S->status, kErrPassLimit);
             result = -1;
             break;
         }
+        // rows to look at in the next iteration
+        for (int r = threadIdx.x + ny2; r < rows2 - ny2; r += kResThreads) {
+            uint32_t m = 0;
+            if (any_chg) {
+                const uint32_t *c = chg + r;
+#pragma unroll
+                for (int k = 0; k < 9; k++) m |= c[(k / 3 - 1) * ny2 + (k % 3 - 1)];
+            }
+            act[r] = m | m << 1 | m >> 1;
+        }
+        if (threadIdx.x >= 1 && threadIdx.x < 4) s_n[threadIdx.x] = 0;
+        __syncthreads();
+        if (any_chg)
+            for (int r = threadIdx.x; r < rows2; r += kResThreads) chg[r] = 0u;
+        // (chg is next written after the barriers of the next iteration)
     }
     __syncthreads();
-    // the converged core (in X after the sixth subiteration) -> buf[0]
-    uint32_t *g0w = in.buf[0];
-    for (int s = warp + 1; s <= total; s += kWarps) {
-        const int bzs = layer_of(s);
-        if (bzs >= c_lo && bzs < c_hi) scatter(g0w, s);
+    // the converged core -> buf[0]
+    {
+        uint32_t *g0w = in.buf[0];
+        Pos q = first_pos();
+        for (int i = threadIdx.x; i < nbox; i += kResThreads, advance(q)) {
+            const int y = y0 + q.y, z = z0 + q.z;
+            if (y >= it.c0 && y < it.c1 && z >= it.r0 && z < it.r1)
+                g0w[((size_t)z * H + y) * P + q.x] = b.state[index_of(q)];
+        }
     }
+    words = __reduce_add_sync(kFull, words);
+    entries = __reduce_add_sync(kFull, entries);
     if (lane == 0 && words) {
-        atomicAdd(&in.work_words, words);
-        atomicAdd(&in.tiles_run, bricks);
+        atomicAdd(&in.work_words, (unsigned long long)words);
+        atomicAdd(&in.tiles_run, (unsigned long long)entries);
     }
     if (threadIdx.x == 0) {
         if (it.band == 0) in.passes_run = 6 * (iter + 1);
@@ -894,8 +872,7 @@ __global__ void resident_reset_kernel(Inst *insts, int n, ResSched *S, int nitem
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         Inst &in = insts[i];
-        in.res_arrive = 0;
-        in.res_last = -1;
+        in.res_meet[0] = in.res_meet[1] = 0;
         in.spill = 0;
         if (in.res) {
             in.converged = 1;  // lowered to -1 by a band that fails
@@ -937,7 +914,7 @@ __global__ void __launch_bounds__(kResThreads, kResCtasPerSm)
         if (in.dims == 2)
             res_run2d(in, it, reinterpret_cast<uint32_t *>(res_smem), S, s_take);
         else
-            res_run3d(in, it, res_smem, S, s_take);
+            res_run3d(in, it, res_smem, S);
         if (threadIdx.x == 0) trace[k] = ResTrace{t0, (long long)globaltimer(), res_smid(), 0};
     }
 }

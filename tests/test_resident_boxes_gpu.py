@@ -1,0 +1,56 @@
+"""GPU parity of the resident kernel's 3D boxes (begputhinning_b200/csrc/resident.cu)
+against the oracle: one box, cuts along y, along z and along both, boxes whose
+cores are as thin as the halo, ragged and word-boundary widths, change masks
+with more than one word per column, and a volume that spills to the tile
+rings."""
+import numpy as np
+import pytest
+
+from oracle import pyoracle as po
+from tests.helpers import blobs3d, random3d
+
+pytestmark = pytest.mark.gpu
+
+
+def _thin(ctx, vols, grid=0):
+    import torch
+    from begputhinning_b200 import Batch
+    b = Batch(ctx)
+    ids = [b.add(v.shape) for v in vols]
+    if grid:
+        b.set_grid(grid)
+    b.finalize()
+    ins = [torch.from_numpy(v).cuda() for v in vols]
+    outs = [torch.full_like(t, 7) for t in ins]
+    for i, t, o in zip(ids, ins, outs):
+        b.set_io(i, t, o)
+    for _ in range(2):
+        b.run()
+    res = [o.cpu().numpy() for o in outs], [b.plan(i) for i in ids], [b.stats(i) for i in ids]
+    b.close()
+    return res
+
+
+@pytest.mark.parametrize("box_words", [20, 200, 3000, 1000000])
+@pytest.mark.parametrize("shape", [(13, 14, 31), (12, 70, 32), (70, 12, 33), (40, 41, 65), (7, 90, 97), (25, 24, 1100)])
+def test_boxes(ctx, shape, box_words, monkeypatch):
+    monkeypatch.setenv("BGT_RES3D_BOX_WORDS", str(box_words))
+    rng = np.random.default_rng(sum(shape))
+    vols = [random3d(rng, *shape, 0.5), blobs3d(rng, *shape, max(2, np.prod(shape) // 2000), rmax=9),
+            np.ones(shape, np.uint8)]
+    for v in vols:  # one volume per batch: its share of the work is the whole grid
+        (got,), (plan,), (stat,) = _thin(ctx, [v])
+        want, _ = po.thin3d(v)
+        assert plan[0] and stat["converged"] == 1
+        assert np.array_equal(got, want), f"plan {plan}: {(got != want).sum()} voxels differ"
+
+
+@pytest.mark.parametrize("density", [0.02, 0.6])
+def test_boxes_spill(ctx, density):
+    """Few CTAs: the sparse volume fits its boxes, the dense one does not and goes to the tile rings."""
+    rng = np.random.default_rng(3)
+    vols = [random3d(rng, 70, 130, 130, density), blobs3d(rng, 30, 30, 40, 5)]
+    got, plans, stats = _thin(ctx, vols, grid=3)
+    for g, v, s in zip(got, vols, stats):
+        assert s["converged"] == 1
+        assert np.array_equal(g, po.thin3d(v)[0]), f"{plans}"
