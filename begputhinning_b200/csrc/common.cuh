@@ -66,7 +66,6 @@ struct alignas(16) Inst {
     unsigned long long work_words;  // packed core words processed (sum over passes and tiles)
     // resident engine (resident.cu)
     int res;                  // 1: thinned by the resident engine, 0: by the tile rings
-    int spill;                // set by the resident engine when a volume's bricks do not fit: the rings take it
     unsigned long long res_meet[2];  // meetings of its CTAs in turn: arrivals (low half), changes reported (high half)
     int res_bands;            // 3D: boxes the volume is cut into
     int res_gy;               // 3D: boxes along y (band = z index * res_gy + y index)

@@ -276,7 +276,6 @@ static void plan_resident(bgt_batch *b)
     constexpr int kHalo = kResHalo2D, kMinCore = 32;  // 2D band halo
     b->res_items.clear();
     b->any_ring = false;
-    b->any_res3d = false;
     const int N = (int)b->items.size();
     const bool rings_only = b->engine_mode == 1 || (getenv("BGT_ENGINE") && !strcmp(getenv("BGT_ENGINE"), "rings"));
     double total = 0;
@@ -301,13 +300,10 @@ static void plan_resident(bgt_batch *b)
     // A volume is cut into boxes of rows and planes (full width), gy along y
     // and gz along z, each with kResHalo3D rows and planes around it: as many
     // as its share of the batch's work is worth (a box of fewer than
-    // box_words core words gains nothing: meeting costs more than it saves),
-    // and at least as many as make a box fit one CTA with all of its words
-    // non-empty or, where that would take more boxes than the share allows,
-    // with kMinFill of them (a volume that turns out denser goes to the tile
-    // rings).  Of the cuts with that many boxes the one with the smallest
-    // box is taken.
-    constexpr double kMinFill = 0.3, kLastFill = 0.15;
+    // box_words core words gains nothing: meeting costs more than it saves;
+    // 1500 to 5000 words measured the same on lone volumes, 16000 25% longer),
+    // or as few as fit one CTA each.  Of the cuts with that many boxes the one
+    // with the smallest box is taken.
     double box_words = 3072.0;
     if (const char *e = getenv("BGT_RES3D_BOX_WORDS")) box_words = std::max(1.0, atof(e));
     const char *slab = getenv("BGT_RES3D_SLAB_VOXELS");
@@ -322,21 +318,20 @@ static void plan_resident(bgt_batch *b)
         int share = (int)std::ceil(words / std::max(target, box_words));
         if (slab) share = (int)std::ceil(v.first / std::max(1.0e4, atof(slab)));
         share = std::max(1, std::min(share, b->res_grid));
-        // the cut into at most `boxes` boxes that hold `fill` with the smallest box, or (fewest) the fewest boxes
+        // the cut into at most `boxes` boxes with the smallest box, or (fewest) the fewest boxes
         int gy = 0, gz = 0;
-        auto search = [&](int boxes, double fill, bool fewest) {
+        auto search = [&](int boxes, bool fewest) {
             double best = 1e30;
             for (int y = 1; y <= std::min(boxes, std::max(1, it.H / kResHalo3D)); y++)
                 for (int z = 1; y * z <= boxes && z <= std::max(1, it.D / kResHalo3D); z++) {
                     const int ey = extent(it.H, y), ez = extent(it.D, z);
-                    if (res_fill_fit3d(it.W, ey, ez) < fill) continue;
+                    if (!res_fits3d(it.W, ey, ez)) continue;
                     const double cost = (fewest ? 1e9 * y * z : 1e-3 * y * z) + (double)ey * ez;
                     if (cost < best) best = cost, gy = y, gz = z;
                 }
             return gy > 0;
         };
-        const bool ok = search(share, 1.0, false) || search(share, kMinFill, false) ||
-                        search(b->res_grid, kMinFill, true) || search(b->res_grid, kLastFill, true);
+        const bool ok = search(share, false) || search(b->res_grid, true);
         if (!ok) {
             in.res = 0;  // cannot be cut into boxes that fit: the rings take it
             continue;
@@ -351,7 +346,6 @@ static void plan_resident(bgt_batch *b)
             b->res_items.push_back(ResItem{v.second, k, G, r0, r1, G > 1 ? kResHalo3D : 0, c0, c1});
         }
         in.res_bands = G;
-        b->any_res3d = true;
     }
     for (auto &m : imgs) {
         const int i = m.second;
@@ -664,8 +658,8 @@ extern "C" int bgt_batch_stage_ms(bgt_batch *b, float *pack_ms, float *engine_ms
 }
 
 // The engine stage of the last run split into the resident kernel and the
-// tile-ring engine that follows it (volumes that spilled, instances the
-// resident engine does not take).
+// tile-ring engine that follows it (instances the resident engine does not
+// take).
 extern "C" int bgt_batch_engine_ms(bgt_batch *b, float *resident_ms, float *rings_ms)
 {
     if (!b || !b->finalized) return fail(BGT_ERR_STATE, "batch not finalized");
@@ -863,11 +857,13 @@ static int enqueue_engine(bgt_batch *b, cudaStream_t st, bool capturing)
 {
     const int N = (int)b->items.size();
     stage_event(b->ev[0], st, capturing);
-    cudaError_t e = cudaMemsetAsync(b->d_lc, 0x80, b->lc_bytes, st);
+    cudaError_t e = cudaSuccess;
+    if (b->any_ring) e = cudaMemsetAsync(b->d_lc, 0x80, b->lc_bytes, st);
     if (e == cudaSuccess) e = launch_pack_all(b->d_insts, b->d_io, N, b->pack_words, b->bytes_only, st);
     if (e != cudaSuccess) return cuda_fail(e, "pack");
-    sched_reset_kernel<<<std::min<unsigned>(1024, (b->cap + 255) / 256), 256, 0, st>>>(
-        b->d_sched, b->d_seq, b->d_item, b->cap, 20000000000LL, b->grid);
+    if (b->any_ring)
+        sched_reset_kernel<<<std::min<unsigned>(1024, (b->cap + 255) / 256), 256, 0, st>>>(
+            b->d_sched, b->d_seq, b->d_item, b->cap, 20000000000LL, b->grid);
     stage_event(b->ev[1], st, capturing);
     // bands of an image wait for one another only for the length of one
     // iteration of the slowest band: 4 s is far beyond any legitimate wait
@@ -875,7 +871,7 @@ static int enqueue_engine(bgt_batch *b, cudaStream_t st, bool capturing)
                         b->d_rtrace, 4000000000LL, st);
     if (e != cudaSuccess) return cuda_fail(e, "resident engine launch");
     stage_event(b->ev[2], st, capturing);
-    if (b->any_ring || b->any_res3d) {
+    if (b->any_ring) {
         e = launch_engine(b->grid, b->smem, b->d_insts, N, b->d_sched, st);
         if (e != cudaSuccess) return cuda_fail(e, "engine launch");
     }
@@ -1100,7 +1096,8 @@ int bgt::batch_check(bgt_batch *b)
     cudaError_t e = cudaStreamSynchronize(b->ctx->stream);
     if (e != cudaSuccess) return cuda_fail(e, "batch run");
     int status = 0, rstatus = 0;
-    e = cudaMemcpy(&status, &b->d_sched->status, sizeof(int), cudaMemcpyDeviceToHost);
+    if (b->last_mode != 0 || b->any_ring)
+        e = cudaMemcpy(&status, &b->d_sched->status, sizeof(int), cudaMemcpyDeviceToHost);
     if (e == cudaSuccess && b->last_mode == 0 && !b->res_items.empty())
         e = cudaMemcpy(&rstatus, &b->d_rs->status, sizeof(int), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_fail(e, "status readback");

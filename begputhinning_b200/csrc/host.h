@@ -136,7 +136,6 @@ struct bgt_batch {
     bgt::ResTrace *d_rtrace = nullptr;  // per-item timeline of the last resident run
     int res_grid = 0;
     bool any_ring = false;            // some instance is planned for the tile rings
-    bool any_res3d = false;           // some volume may spill from the resident engine to the rings
     cudaGraphExec_t gexec = nullptr;
     bool graph_valid = false;
     // plain path with the pass loop on the device (bgt_batch_run mode 2)

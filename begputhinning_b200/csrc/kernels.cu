@@ -521,12 +521,10 @@ __global__ void pack_all_kernel(const Inst *__restrict__ insts, const IODesc *__
             ke = k + 1 < n ? io[k + 1].wbegin : total;
             const Inst &in = insts[d.inst];
             buf0 = in.buf[0];
-            // an image thinned by the resident kernel reads only buf[0] and
-            // no tile marks (its bands write buf[1] before reading it); the
-            // tile engine and volumes, which may spill to it, need both
-            const bool res2d = in.res && in.dims == 2;
-            buf1 = res2d ? nullptr : in.buf[1];
-            lc = res2d ? nullptr : in.lc;
+            // the resident kernel reads only buf[0] and no tile marks (its
+            // bands write buf[1] before reading it); the tile engine needs both
+            buf1 = in.res ? nullptr : in.buf[1];
+            lc = in.res ? nullptr : in.lc;
             P = in.P;
             H = in.H;
             tiles_x = in.tiles_x;
@@ -1116,8 +1114,7 @@ __global__ void __launch_bounds__(kThreads) engine_seed_kernel(Inst *insts, int 
 {
     __shared__ uint32_t scratch[2048];
     for (int ii = blockIdx.x; ii < ninst; ii += gridDim.x) {
-        // instances of the resident engine are done unless they spilled
-        if (insts[ii].res && !insts[ii].spill) continue;
+        if (insts[ii].res) continue;  // thinned by the resident engine
         if (threadIdx.x == 0) {
             insts[ii].converged = 0;
             insts[ii].passes_run = 0;

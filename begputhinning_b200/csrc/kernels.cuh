@@ -84,9 +84,8 @@ constexpr int kResSmemBytes = 230400;  // dynamic shared memory of one CTA (one 
 int res_smem_bytes();
 // Rows of a W-wide 2D band (core plus halo) that one CTA holds.
 int res_rows_fit2d(int W);
-// Share of the words of a 3D box (ny rows x nz planes, halo included) that may be
-// non-empty for it to fit one CTA (negative: not even an empty one fits).
-double res_fill_fit3d(int W, int ny, int nz);
+// Whether a 3D box (ny rows x nz planes of a volume W wide, halo included) fits one CTA.
+bool res_fits3d(int W, int ny, int nz);
 constexpr int kResHalo3D = 6;  // one iteration: six subiterations, one row and plane each
 cudaError_t res_occupancy(int *per_sm);  // resident CTAs per SM
 cudaError_t launch_resident(int grid, Inst *d_insts, int ninst, const ResItem *d_items, int nitems,

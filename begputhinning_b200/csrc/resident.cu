@@ -42,9 +42,8 @@
 // union are the candidates of the five other subiterations.  A subiteration
 // finds its deletions, meets, and applies them, so the state needs no second
 // copy.  A large volume is cut into boxes on several CTAs that trade the
-// words changed near their edges after every iteration.  A volume of which a
-// box has more non-empty words than fit is flagged `spill` and left to the
-// tile engine.
+// words changed near their edges after every iteration.  A box with more
+// non-empty words than the lists hold goes over all of its words instead.
 //
 // Rules, order of directions and termination are those of the tile engine
 // (2D/CUDA_ThinningKernelMultiBlock2D.cuh:104-135,
@@ -83,12 +82,13 @@ __host__ __device__ inline size_t res_words2d(int W, int nrows)
 }
 
 // bytes of shared memory a box of ny x nz rows of wl words (halo included)
-// needs when `listed` of its words are non-empty
+// needs: its state, the rows' masks and, in the dense form, two more words
+// per word (the lists take what they find there, up to 44% non-empty words)
 constexpr size_t kBoxListBytes = 4 + 4 + 4 + 4 + 2;  // list, candidate, union, deletions, active list
-__host__ __device__ inline size_t res_bytes3d(int wl, int ny, int nz, double listed)
+__host__ __device__ inline size_t res_bytes3d(int wl, int ny, int nz)
 {
-    const size_t rows2 = (size_t)(ny + 2) * (nz + 2);
-    return up16((rows2 * (wl + 1) + 1) * 4) + 2 * up16(rows2 * 4) + (size_t)(listed * kBoxListBytes) + 80;
+    const size_t rows2 = (size_t)(ny + 2) * (nz + 2), words = rows2 * (wl + 1) + 1;
+    return up16(words * 4) + 2 * up16(rows2 * 4) + 2 * words * 4 + 80;
 }
 
 int res_smem_bytes() { return kSmemBytes; }
@@ -104,14 +104,11 @@ int res_rows_fit2d(int W)
     return lo;
 }
 
-double res_fill_fit3d(int W, int ny, int nz)
+bool res_fits3d(int W, int ny, int nz)
 {
     const int wl = (W + 31) / 32;
-    if ((long long)(ny + 2) * (nz + 2) * (wl + 1) >= 65535) return -1.0;  // words are indexed by 16 bits
-    const double words = (double)wl * ny * nz;
-    const size_t base = res_bytes3d(wl, ny, nz, 0.0);
-    if (base > (size_t)kSmemBytes) return -1.0;
-    return std::min(1.0, (double)((size_t)kSmemBytes - base) / kBoxListBytes / words);
+    // words are indexed by 16 bits
+    return (long long)(ny + 2) * (nz + 2) * (wl + 1) < 65535 && res_bytes3d(wl, ny, nz) <= (size_t)kSmemBytes;
 }
 
 // ------------------------------------------------------------ helpers -----
@@ -617,6 +614,10 @@ __device__ void res_run3d(Inst &in, const ResItem &it, uint8_t *smb, ResSched *S
             q.z++;
         }
     };
+    auto dist_of = [&](const Pos &q) {
+        const int y = y0 + q.y, z = z0 + q.z;
+        return max(max(max(it.c0 - y, y - it.c1 + 1), max(it.r0 - z, z - it.r1 + 1)), 0);
+    };
     auto index_of = [&](const Pos &q) { return ((q.z + 1) * ny2 + q.y + 1) * b.p + 1 + q.x; };
     {
         constexpr int U = 4;  // loads in flight per thread
@@ -632,8 +633,7 @@ __device__ void res_run3d(Inst &in, const ResItem &it, uint8_t *smb, ResSched *S
             }
 #pragma unroll
             for (int k = 0; k < U; k++) {
-                const int y = y0 + at[k].y, z = z0 + at[k].z;
-                const int d = max(max(max(it.c0 - y, y - it.c1 + 1), max(it.r0 - z, z - it.r1 + 1)), 0);
+                const int d = dist_of(at[k]);
                 const int idx = v[k] ? index_of(at[k]) : 0;
                 if (v[k]) b.state[idx] = v[k];
                 const int pos = warp_append(v[k] != 0u && d <= 5, &s_n[0]);
@@ -645,30 +645,12 @@ __device__ void res_run3d(Inst &in, const ResItem &it, uint8_t *smb, ResSched *S
     __syncthreads();
     const int nl = s_n[0];
     MeetState meet;
-    const bool fits = off + (size_t)nl * kBoxListBytes + 64 <= (size_t)kSmemBytes;
-    if (team) {
-        // every box must fit, or the tile engine takes the whole volume: the
-        // boxes agree before any of them writes anything
-        if (threadIdx.x == 0) {
-            if (!fits) atomicExch(&in.spill, 1);
-            s_flag = res_meet(in.res_meet, it.bands, !fits, meet, S->timeout_ns);
-            if (s_flag == 2) atomicOr(&S->status, kErrQueueTimeout);
-        }
-        __syncthreads();
-        if (s_flag) {
-            if (s_flag == 2 && threadIdx.x == 0) atomicMin(&in.converged, -1);
-            __syncthreads();
-            return;
-        }
-    } else if (!fits) {
-        // does not fit: the tile engine thins this volume (nothing here was written to it)
-        if (threadIdx.x == 0) in.spill = 1;
-        __syncthreads();
-        return;
-    }
+    // more non-empty words than the lists hold: go over all words of the box,
+    // with the union and the deletions stored per word
+    const bool dense = off + (size_t)nl * kBoxListBytes + 64 > (size_t)kSmemBytes;
     b.cidx = list + nl;
-    b.cU = b.cidx + nl;
-    b.cdel = b.cU + nl;
+    b.cU = dense ? list : b.cidx + nl;
+    b.cdel = b.cU + (dense ? nwords : nl);
     uint16_t *const alist = reinterpret_cast<uint16_t *>(b.cdel + nl);
     for (int r = threadIdx.x; r < rows2; r += kResThreads) act[r] = kFull;
     __syncthreads();
@@ -678,105 +660,166 @@ __device__ void res_run3d(Inst &in, const ResItem &it, uint8_t *smb, ResSched *S
     int iter = 0, result = 0;
     unsigned words = 0, entries = 0;
     const int cap_it = in.pass_cap / 6 + 1;
+    // a word of the core changed: mark it, and tell the boxes around when it lies near the core's edge
+    auto changed = [&](uint32_t idx, uint32_t col, uint2 *msg) {
+        const uint32_t row = __umulhi(idx, mp);
+        atomicOr(&chg[row], 1u << col);
+        if (!team) return;
+        const int zz = (int)__umulhi(row, mny), y = y0 + (int)row - zz * ny2 - 1, z = z0 + zz - 1;
+        const int h = it.halo;
+        if ((it.r0 > 0 && z < it.r0 + h) || (it.r1 < D && z >= it.r1 - h) || (it.c0 > 0 && y < it.c0 + h) ||
+            (it.c1 < H && y >= it.c1 - h)) {
+            const int x = (int)idx - (int)row * b.p - 1;
+            msg[atomicAdd(&s_n[3], 1)] =
+                make_uint2(((uint32_t)z * (uint32_t)H + (uint32_t)y) * (uint32_t)wl + (uint32_t)x, b.state[idx]);
+        }
+    };
     for (;; iter++) {
-        // active words: a word of the row's 3x3 rows that is at most one
-        // column away changed in the previous iteration (otherwise its union
-        // is empty), and some voxel of it misses one of its face neighbours
-        for (int base = warp * 32; base < nl; base += kResThreads) {
-            const int k = base + lane;
-            bool on = false;
-            if (k < nl) {
-                const uint32_t e = list[k], idx = ent_idx(e);
-                if ((act[__umulhi(idx, mp)] >> ent_col(e)) & 1u) {
-                    const uint32_t *s = b.state + idx;
-                    const uint32_t c = *s;
-                    const uint32_t faces = at_xm1(c, s[-1]) & at_xp1(c, s[1]) & s[b.p] & s[-b.p] & s[b.ps] & s[-b.ps];
-                    on = (c & ~faces) != 0u;
-                }
-            }
-            const int pos = warp_append(on, &s_n[1]);
-            if (pos >= 0) alist[pos] = (uint16_t)k;
-        }
-        __syncthreads();
-        const int na = s_n[1];
-        // pre-test and U
-        for (int base = warp * 32; base < na; base += kResThreads) {
-            const int k = base + lane;
-            uint32_t e = 0, un = 0, du = 0;
-            if (k < na) {
-                e = list[alist[k]];
-                const uint32_t *s = b.state + ent_idx(e);
-                uint32_t g[27];
-                box_window(s, b.p, b.ps, g);
-                du = rule3d<0>(g) & g[13];
-                un = (du | rule3d<1>(g) | rule3d<2>(g) | rule3d<3>(g) | rule3d<4>(g) | rule3d<5>(g)) & g[13];
-                words += ent_dist(e) == 0;
-                entries++;
-            }
-            const int c = warp_append(un != 0u, &s_n[2]);
-            if (c >= 0) {
-                b.cidx[c] = e;
-                b.cU[c] = un;
-                b.cdel[c] = du;
-            }
-        }
-        __syncthreads();
-        const int nc = s_n[2];
-        if (nc > kResThreads) {
-            for (int c = threadIdx.x; c < nc; c += kResThreads) {
-                const uint32_t del = b.cdel[c];
-                if (del) {
-                    const uint32_t e = b.cidx[c];
-                    b.state[ent_idx(e)] &= ~del;
-                    b.cidx[c] = e | kEntChanged;
-                }
-            }
-            __syncthreads();
-            box_subiteration<1>(b, nc, words);
-            box_subiteration<2>(b, nc, words);
-            box_subiteration<3>(b, nc, words);
-            box_subiteration<4>(b, nc, words);
-            box_subiteration<5>(b, nc, words);
-        } else if (nc > 0) {
-            const int c = threadIdx.x;
-            uint32_t e = 0, un = 0, val = 0, del = 0;
-            if (c < nc) {
-                e = b.cidx[c];
-                un = b.cU[c];
-                del = b.cdel[c];
-                val = b.state[ent_idx(e)];
-            }
-            const uint32_t before = val;
-            if (del) {
-                val &= ~del;
-                b.state[ent_idx(e)] = val;
-            }
-            __syncthreads();
-            box_subiteration1<1>(b, e, un, val, words);
-            box_subiteration1<2>(b, e, un, val, words);
-            box_subiteration1<3>(b, e, un, val, words);
-            box_subiteration1<4>(b, e, un, val, words);
-            box_subiteration1<5>(b, e, un, val, words);
-            if (val != before) b.cidx[c] = e | kEntChanged;
-        }
-        // changed words of the core: marks, and messages to the boxes around
         bool core = false;
         uint2 *msg = nullptr;
         if (team) msg = in.res_msg + ((size_t)(iter & 1) * it.bands + it.band) * in.res_stride;
-        for (int c = threadIdx.x; c < nc; c += kResThreads) {
-            const uint32_t e = b.cidx[c];
-            if (!(e & kEntChanged) || ent_dist(e) != 0) continue;
-            core = true;
-            const uint32_t idx = ent_idx(e), row = __umulhi(idx, mp);
-            atomicOr(&chg[row], 1u << ent_col(e));
-            if (!team) continue;
-            const int zz = (int)__umulhi(row, mny), y = y0 + (int)row - zz * ny2 - 1, z = z0 + zz - 1;
-            const int h = it.halo;
-            if ((it.r0 > 0 && z < it.r0 + h) || (it.r1 < D && z >= it.r1 - h) || (it.c0 > 0 && y < it.c0 + h) ||
-                (it.c1 < H && y >= it.c1 - h)) {
-                const int x = (int)idx - (int)row * b.p - 1;
-                msg[atomicAdd(&s_n[3], 1)] = make_uint2(((uint32_t)z * (uint32_t)H + (uint32_t)y) * (uint32_t)wl + (uint32_t)x,
-                                                        b.state[idx]);
+        if (!dense) {
+            // active words: a word of the row's 3x3 rows that is at most one
+            // column away changed in the previous iteration (otherwise its union
+            // is empty), and some voxel of it misses one of its face neighbours
+            for (int base = warp * 32; base < nl; base += kResThreads) {
+                const int k = base + lane;
+                bool on = false;
+                if (k < nl) {
+                    const uint32_t e = list[k], idx = ent_idx(e);
+                    if ((act[__umulhi(idx, mp)] >> ent_col(e)) & 1u) {
+                        const uint32_t *s = b.state + idx;
+                        const uint32_t c = *s;
+                        const uint32_t faces = at_xm1(c, s[-1]) & at_xp1(c, s[1]) & s[b.p] & s[-b.p] & s[b.ps] & s[-b.ps];
+                        on = (c & ~faces) != 0u;
+                    }
+                }
+                const int pos = warp_append(on, &s_n[1]);
+                if (pos >= 0) alist[pos] = (uint16_t)k;
+            }
+            __syncthreads();
+            const int na = s_n[1];
+            // pre-test and U
+            for (int base = warp * 32; base < na; base += kResThreads) {
+                const int k = base + lane;
+                uint32_t e = 0, un = 0, du = 0;
+                if (k < na) {
+                    e = list[alist[k]];
+                    const uint32_t *s = b.state + ent_idx(e);
+                    uint32_t g[27];
+                    box_window(s, b.p, b.ps, g);
+                    du = rule3d<0>(g) & g[13];
+                    un = (du | rule3d<1>(g) | rule3d<2>(g) | rule3d<3>(g) | rule3d<4>(g) | rule3d<5>(g)) & g[13];
+                    words += ent_dist(e) == 0;
+                    entries++;
+                }
+                const int c = warp_append(un != 0u, &s_n[2]);
+                if (c >= 0) {
+                    b.cidx[c] = e;
+                    b.cU[c] = un;
+                    b.cdel[c] = du;
+                }
+            }
+            __syncthreads();
+            const int nc = s_n[2];
+            if (nc > kResThreads) {
+                for (int c = threadIdx.x; c < nc; c += kResThreads) {
+                    const uint32_t del = b.cdel[c];
+                    if (del) {
+                        const uint32_t e = b.cidx[c];
+                        b.state[ent_idx(e)] &= ~del;
+                        b.cidx[c] = e | kEntChanged;
+                    }
+                }
+                __syncthreads();
+                box_subiteration<1>(b, nc, words);
+                box_subiteration<2>(b, nc, words);
+                box_subiteration<3>(b, nc, words);
+                box_subiteration<4>(b, nc, words);
+                box_subiteration<5>(b, nc, words);
+            } else if (nc > 0) {
+                const int c = threadIdx.x;
+                uint32_t e = 0, un = 0, val = 0, del = 0;
+                if (c < nc) {
+                    e = b.cidx[c];
+                    un = b.cU[c];
+                    del = b.cdel[c];
+                    val = b.state[ent_idx(e)];
+                }
+                const uint32_t before = val;
+                if (del) {
+                    val &= ~del;
+                    b.state[ent_idx(e)] = val;
+                }
+                __syncthreads();
+                box_subiteration1<1>(b, e, un, val, words);
+                box_subiteration1<2>(b, e, un, val, words);
+                box_subiteration1<3>(b, e, un, val, words);
+                box_subiteration1<4>(b, e, un, val, words);
+                box_subiteration1<5>(b, e, un, val, words);
+                if (val != before) b.cidx[c] = e | kEntChanged;
+            }
+            for (int c = threadIdx.x; c < nc; c += kResThreads) {
+                const uint32_t e = b.cidx[c];
+                if (!(e & kEntChanged) || ent_dist(e) != 0) continue;
+                core = true;
+                changed(ent_idx(e), ent_col(e), msg);
+            }
+        } else {
+            Pos q = first_pos();
+            for (int i = threadIdx.x; i < nbox; i += kResThreads, advance(q)) {
+                const int idx = index_of(q), d = dist_of(q);
+                const uint32_t *s = b.state + idx;
+                uint32_t un = 0, du = 0;
+                if (d <= 5 && *s && ((act[(q.z + 1) * ny2 + q.y + 1] >> (q.x >> xs)) & 1u)) {
+                    uint32_t g[27];
+                    box_window(s, b.p, b.ps, g);
+                    du = rule3d<0>(g) & g[13];
+                    un = (du | rule3d<1>(g) | rule3d<2>(g) | rule3d<3>(g) | rule3d<4>(g) | rule3d<5>(g)) & g[13];
+                    words += d == 0;
+                    entries++;
+                }
+                b.cU[idx] = un;
+                b.cdel[idx] = du;
+            }
+            __syncthreads();
+#pragma unroll 1
+            for (int j = 0; j < 6; j++) {
+                // deletions of subiteration j were found: apply them, then find the next one's
+                q = first_pos();
+                for (int i = threadIdx.x; i < nbox; i += kResThreads, advance(q)) {
+                    const int idx = index_of(q);
+                    const uint32_t del = b.cdel[idx];
+                    if (del) b.state[idx] &= ~del;
+                }
+                __syncthreads();
+                if (j == 5) break;
+                q = first_pos();
+                for (int i = threadIdx.x; i < nbox; i += kResThreads, advance(q)) {
+                    const int idx = index_of(q), d = dist_of(q);
+                    const uint32_t cand = b.state[idx] & b.cU[idx];
+                    uint32_t del = 0;
+                    if (cand && d <= 4 - j) {
+                        uint32_t g[27];
+                        box_window(b.state + idx, b.p, b.ps, g);
+                        del = cand & (j == 0   ? rule3d<1>(g)
+                                      : j == 1 ? rule3d<2>(g)
+                                      : j == 2 ? rule3d<3>(g)
+                                      : j == 3 ? rule3d<4>(g)
+                                               : rule3d<5>(g));
+                        words += d == 0;
+                    }
+                    b.cdel[idx] = del;
+                }
+                __syncthreads();
+            }
+            // only voxels of the union were deleted: a word changed when it lost some of its union
+            q = first_pos();
+            for (int i = threadIdx.x; i < nbox; i += kResThreads, advance(q)) {
+                const int idx = index_of(q);
+                if (!(b.cU[idx] & ~b.state[idx]) || dist_of(q) != 0) continue;
+                core = true;
+                changed((uint32_t)idx, (uint32_t)(q.x >> xs), msg);
             }
         }
         const bool any = __syncthreads_or(core);
@@ -873,7 +916,6 @@ __global__ void resident_reset_kernel(Inst *insts, int n, ResSched *S, int nitem
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         Inst &in = insts[i];
         in.res_meet[0] = in.res_meet[1] = 0;
-        in.spill = 0;
         if (in.res) {
             in.converged = 1;  // lowered to -1 by a band that fails
             in.passes_run = 0;

@@ -1,8 +1,8 @@
 """GPU parity of the resident kernel's 3D boxes (begputhinning_b200/csrc/resident.cu)
 against the oracle: one box, cuts along y, along z and along both, boxes whose
 cores are as thin as the halo, ragged and word-boundary widths, change masks
-with more than one word per column, and a volume that spills to the tile
-rings."""
+with more than one word per column, and boxes with more non-empty words than
+their lists hold."""
 import numpy as np
 import pytest
 
@@ -46,11 +46,13 @@ def test_boxes(ctx, shape, box_words, monkeypatch):
 
 
 @pytest.mark.parametrize("density", [0.02, 0.6])
-def test_boxes_spill(ctx, density):
-    """Few CTAs: the sparse volume fits its boxes, the dense one does not and goes to the tile rings."""
+def test_boxes_dense(ctx, density):
+    """Few CTAs, so large boxes: the sparse volume's words fit the lists, the
+    dense one's do not and every word is gone over."""
     rng = np.random.default_rng(3)
-    vols = [random3d(rng, 70, 130, 130, density), blobs3d(rng, 30, 30, 40, 5)]
-    got, plans, stats = _thin(ctx, vols, grid=3)
+    vols = [random3d(rng, 70, 130, 126, density), blobs3d(rng, 30, 30, 40, 5)]
+    got, plans, stats = _thin(ctx, vols, grid=12)
+    assert all(p[0] for p in plans)
     for g, v, s in zip(got, vols, stats):
         assert s["converged"] == 1
         assert np.array_equal(g, po.thin3d(v)[0]), f"{plans}"
