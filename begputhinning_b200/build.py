@@ -24,7 +24,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 CU_SOURCES = ["kernels.cu", "resident.cu", "host.cu", "segments.cu", "segments_graph.cu", "centerline.cu", "noalloc.cu", "serve.cu"]
 CXX_SOURCES = ["dropin.cpp"]
-HEADERS = ["common.cuh", "rules.cuh", "tiles.cuh", "kernels.cuh", "host.h"]
+HEADERS = ["common.cuh", "pixels.cuh", "rules.cuh", "tiles.cuh", "kernels.cuh", "host.h"]
 
 LIB = os.path.join(PKG, "libbgt.so")
 SYNTH = os.path.join(PKG, "libbgt_synth.so")

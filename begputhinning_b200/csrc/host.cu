@@ -639,7 +639,8 @@ extern "C" int bgt_batch_set_grid(bgt_batch *b, int ctas)
 }
 
 // Device time of the stages of the last engine run: pack (with the mark
-// reset and scheduler reset), engine (seed + persistent kernel), unpack.
+// reset and scheduler reset), engine (resident kernel with its pixel I/O, seed
+// + persistent kernel), unpack.
 extern "C" int bgt_batch_stage_ms(bgt_batch *b, float *pack_ms, float *engine_ms, float *unpack_ms)
 {
     if (!b || !b->finalized) return fail(BGT_ERR_STATE, "batch not finalized");
@@ -783,19 +784,61 @@ __global__ void sched_reset_kernel(Sched *S, unsigned *seq, int4 *item, unsigned
     }
 }
 
-// Upload the per-instance I/O table used by the batch-wide pack/unpack, in
-// stream order from a host copy the batch keeps (done before any capture).
+// Whether some instance's output overlaps another instance's input.  The
+// resident kernel finishes instances one by one, so such a batch keeps the
+// order "all inputs are read, then all outputs are written".
+static bool io_crosses(const bgt_batch *b)
+{
+    struct Span {
+        uintptr_t lo, hi;
+        int inst;
+    };
+    std::vector<Span> ins;
+    const int N = (int)b->items.size();
+    if (N == 1) return false;
+    auto bytes = [&](int i, bool input) {
+        const Inst &in = b->h[i];
+        const IO &s = b->io[i];
+        const size_t n = input && s.inW ? (size_t)s.inW * s.inH * s.inD : (size_t)in.W * in.H * in.D;
+        return n * dtype_size(s.dtype);
+    };
+    for (int i = 0; i < N; i++) {
+        const uintptr_t p = (uintptr_t)b->io[i].in;
+        ins.push_back(Span{p, p + bytes(i, true), i});
+    }
+    std::sort(ins.begin(), ins.end(), [](const Span &x, const Span &y) { return x.lo < y.lo; });
+    std::vector<uintptr_t> top(N);  // highest end up to here
+    for (int k = 0; k < N; k++) top[k] = std::max(ins[k].hi, k ? top[k - 1] : 0);
+    for (int i = 0; i < N; i++) {
+        if (!b->io[i].out) continue;
+        const uintptr_t lo = (uintptr_t)b->io[i].out, hi = lo + bytes(i, false);
+        int k = (int)(std::lower_bound(ins.begin(), ins.end(), hi, [](const Span &x, uintptr_t v) { return x.lo < v; }) -
+                      ins.begin()) - 1;
+        for (; k >= 0 && top[k] > lo; k--)
+            if (ins[k].hi > lo && ins[k].inst != i) return true;
+    }
+    return false;
+}
+
+// Build the per-instance I/O table and upload it, in stream order from a host
+// copy the batch keeps (done before any capture).  Only instances that the
+// tile rings take, or that the resident kernel finds packed, are packed and
+// unpacked by the batch-wide kernels; a batch of one resident instance passes
+// its table entry to the kernel instead of uploading it.
 static int upload_io(bgt_batch *b)
 {
     if (!b->io_dirty) return BGT_OK;
     const int N = (int)b->items.size();
     std::vector<IODesc> &io = b->io_host;
+    for (int i = 0; i < N; i++)
+        if (!b->io[i].in) return fail(BGT_ERR_STATE, "instance %d has no input", i);
+    b->pixels = !io_crosses(b);
     io.assign(N, IODesc());
     long long w = 0, g = 0;
+    b->bytes_only = true;
     for (int i = 0; i < N; i++) {
         const Inst &in = b->h[i];
         const IO &s = b->io[i];
-        if (!s.in) return fail(BGT_ERR_STATE, "instance %d has no input", i);
         io[i].in = s.in;
         io[i].out = s.out;
         io[i].dtype = s.dtype;
@@ -813,8 +856,12 @@ static int upload_io(bgt_batch *b)
         io[i].dTW = make_fastdiv((uint32_t)in.TW);
         io[i].dTH = make_fastdiv((uint32_t)in.TH);
         io[i].dTZ = make_fastdiv((uint32_t)std::max(1, in.TZ));
+        if (in.res && b->pixels) continue;
+        const int dt = s.dtype;
+        b->bytes_only &= dtype_size(dt) == 1 && (io[i].mode == 0 || dt == BGT_U8 || dt == BGT_BOOL);
         w += (long long)in.P * in.H * in.D;
-        if (dtype_size(s.dtype) == 1 && s.out) {
+        if (!s.out) continue;
+        if (dtype_size(s.dtype) == 1) {
             // unpack unit: 32-byte-aligned chunk of the output
             const uintptr_t o = reinterpret_cast<uintptr_t>(s.out);
             const uintptr_t end = o + (uintptr_t)in.W * in.H * in.D;
@@ -826,61 +873,60 @@ static int upload_io(bgt_batch *b)
     }
     b->pack_words = w;
     b->unpack_words = g;
-    b->any_out = false;
-    b->bytes_only = true;
-    for (int i = 0; i < N; i++) {
-        b->any_out |= b->io[i].out != nullptr;
-        const int dt = io[i].dtype;
-        b->bytes_only &= dtype_size(dt) == 1 && (io[i].mode == 0 || dt == BGT_U8 || dt == BGT_BOOL);
+    if (N > 1 || w > 0) {
+        cudaError_t e = cudaMemcpyAsync(b->d_io, io.data(), (size_t)N * sizeof(IODesc), cudaMemcpyHostToDevice,
+                                        b->ctx->stream);
+        if (e != cudaSuccess) return cuda_fail(e, "I/O table upload");
     }
-    cudaError_t e = cudaMemcpyAsync(b->d_io, io.data(), (size_t)N * sizeof(IODesc), cudaMemcpyHostToDevice,
-                                    b->ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "I/O table upload");
     b->io_dirty = false;
     return BGT_OK;
 }
 
-// Stream-ordered sequence of the engine run (capturable): mark reset, one
-// batch-wide pack (which also marks non-empty tiles), scheduler reset, seed
-// + persistent engine, one batch-wide unpack.
+// Stream-ordered sequence of the engine run (capturable).  The resident
+// kernel reads the pixels of its instances and writes them back; instances of
+// the tile rings go through mark reset, batch-wide pack, scheduler reset, seed
+// and persistent engine, and batch-wide unpack.
 // Stage boundary event: inside a capture it must become an event-record node
 // (cudaEventRecordExternal); outside a capture it is a plain record.
-static void stage_event(cudaEvent_t ev, cudaStream_t st, bool capturing)
+static void stage_event(bgt_batch *b, int k, cudaStream_t st, bool capturing)
 {
+    if (!b->timed) return;
     if (capturing)
-        cudaEventRecordWithFlags(ev, st, cudaEventRecordExternal);
+        cudaEventRecordWithFlags(b->ev[k], st, cudaEventRecordExternal);
     else
-        cudaEventRecord(ev, st);
+        cudaEventRecord(b->ev[k], st);
 }
 
 static int enqueue_engine(bgt_batch *b, cudaStream_t st, bool capturing)
 {
     const int N = (int)b->items.size();
-    stage_event(b->ev[0], st, capturing);
+    stage_event(b, 0, st, capturing);
     cudaError_t e = cudaSuccess;
     if (b->any_ring) e = cudaMemsetAsync(b->d_lc, 0x80, b->lc_bytes, st);
-    if (e == cudaSuccess) e = launch_pack_all(b->d_insts, b->d_io, N, b->pack_words, b->bytes_only, st);
+    if (e == cudaSuccess && b->pack_words > 0)
+        e = launch_pack_all(b->d_insts, b->d_io, N, b->pack_words, b->bytes_only, st);
     if (e != cudaSuccess) return cuda_fail(e, "pack");
     if (b->any_ring)
         sched_reset_kernel<<<std::min<unsigned>(1024, (b->cap + 255) / 256), 256, 0, st>>>(
             b->d_sched, b->d_seq, b->d_item, b->cap, 20000000000LL, b->grid);
-    stage_event(b->ev[1], st, capturing);
+    stage_event(b, 1, st, capturing);
     // bands of an image wait for one another only for the length of one
     // iteration of the slowest band: 4 s is far beyond any legitimate wait
     e = launch_resident(b->res_grid, b->d_insts, N, b->d_res_items, (int)b->res_items.size(), b->d_rs,
-                        b->d_rtrace, 4000000000LL, st);
+                        b->d_rtrace, 4000000000LL, b->d_io, N == 1 && b->pack_words == 0 ? &b->io_host[0] : nullptr,
+                        b->pixels, st);
     if (e != cudaSuccess) return cuda_fail(e, "resident engine launch");
-    stage_event(b->ev[2], st, capturing);
+    stage_event(b, 2, st, capturing);
     if (b->any_ring) {
         e = launch_engine(b->grid, b->smem, b->d_insts, N, b->d_sched, st);
         if (e != cudaSuccess) return cuda_fail(e, "engine launch");
     }
-    stage_event(b->ev[3], st, capturing);
-    if (b->any_out) {
+    stage_event(b, 3, st, capturing);
+    if (b->unpack_words > 0) {
         e = launch_unpack_all(b->d_insts, b->d_io, N, b->unpack_words, st);
         if (e != cudaSuccess) return cuda_fail(e, "unpack");
     }
-    stage_event(b->ev[4], st, capturing);
+    stage_event(b, 4, st, capturing);
     return BGT_OK;
 }
 
@@ -1209,6 +1255,7 @@ int bgt::single_batch(bgt_ctx *c, int dims, int W, int H, int D, bgt_batch **out
     }
     bgt_batch *b = nullptr;
     int rc = bgt_batch_create(c, &b);
+    if (rc == BGT_OK) b->timed = false;  // nobody can ask for its stage times
     if (rc == BGT_OK) rc = dims == 2 ? bgt_batch_add2d(b, W, H, -1, nullptr) : bgt_batch_add3d(b, W, H, D, -1, nullptr);
     if (rc == BGT_OK) rc = bgt_batch_finalize(b);
     if (rc != BGT_OK) {

@@ -120,7 +120,8 @@ struct bgt_batch {
     size_t lc_bytes = 0;
     bgt::IODesc *d_io = nullptr;  // per-instance I/O table of the batch-wide pack/unpack
     bool io_dirty = true;
-    bool any_out = false;
+    bool pixels = true;       // the resident kernel reads and writes the pixels itself (no output overlaps another's input)
+    bool timed = true;        // record the stage boundaries
     bool bytes_only = false;  // every input one byte wide, tested "byte != 0"
     long long pack_words = 0, unpack_words = 0;
     unsigned cap = 0;

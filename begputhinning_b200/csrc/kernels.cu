@@ -5,6 +5,7 @@
 #include <cstdio>
 
 #include "kernels.cuh"
+#include "pixels.cuh"
 #include "tiles.cuh"
 
 namespace bgt {
@@ -223,25 +224,6 @@ cudaError_t launch_rule_table(int dims, int dir, uint32_t *d_out, cudaStream_t s
 }
 
 // ------------------------------------------------------------ pack --------
-// Foreground tests of the reference's binarisation.  2D: (unsigned int)v > 0
-// evaluated on the device (2D/CUDA_DeviceHelperFunctions.cuh:101), i.e. a
-// saturating conversion for floating types.  3D: int(v) > 0 as the host
-// evaluates it (3D/CenterlineExtraction.cpp:44; x86-64 conversion of
-// out-of-range floats gives INT_MIN).
-template <typename T>
-__device__ __forceinline__ bool fg2(T v) { return (unsigned int)v > 0u; }
-template <>
-__device__ __forceinline__ bool fg2<bool>(bool v) { return v; }
-
-template <typename T>
-__device__ __forceinline__ bool fg3(T v) { return (int)v > 0; }
-template <>
-__device__ __forceinline__ bool fg3<float>(float v) { return v >= 1.0f && v < 2147483648.0f; }
-template <>
-__device__ __forceinline__ bool fg3<double>(double v) { return v >= 1.0 && v < 2147483648.0; }
-template <>
-__device__ __forceinline__ bool fg3<bool>(bool v) { return v; }
-
 // One thread per packed word; writes both ping-pong buffers (so tiles that
 // never change hold identical data in both).  The input may be smaller than
 // the instance (inW x inH x inD inside W x H x D, row stride inW); the rest
@@ -350,23 +332,6 @@ cudaError_t launch_unpack(int dtype, const uint32_t *buf, int W, int H, int D, i
 // One launch packs (or unpacks) every instance of a batch: the global word
 // index is mapped to its instance by a binary search over io[].wbegin.
 
-// 32 one-byte pixels starting at p -> bit word.  MSB-of-byte gather:
-// multiplying the MSB mask by 0x00204081 moves bits 7, 15, 23, 31 to 28..31
-// without carries.
-__device__ __forceinline__ uint32_t bytes4_to_bits(uint32_t cmp)
-{
-    return ((cmp & 0x80808080u) * 0x00204081u) >> 28;
-}
-
-// 4 bytes -> 4 bits "byte != 0" (bit k for byte k) with integer ALU ops only:
-// the low seven bits of each byte plus 0x7F carry into the byte's MSB
-// exactly when they are nonzero (no carry leaves the byte), and OR-ing the
-// byte back in covers the MSB itself.
-__device__ __forceinline__ uint32_t nz4_to_bits(uint32_t c)
-{
-    return bytes4_to_bits(((c & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | c);
-}
-
 // 32 bytes at word offset Q (0..3) and byte shift sh of 12 loaded words ->
 // 32 "nonzero" bits
 template <int Q>
@@ -439,49 +404,11 @@ __device__ __forceinline__ uint32_t pack_word(const T *p, int n, long long room 
     return w;
 }
 
-// 32 one-byte pixels from p (n < 32 at a row's ragged end) -> "byte != 0"
-// bits, without branches that depend on p's alignment: three aligned 16-byte
-// loads cover p .. p+31 (they may run past the row into the next one, never
-// past the input: `room` and `lead` as in pack_word), the 12 loaded words are
-// shifted by p's word offset in two conditional-select stages and by its byte
-// offset with funnel shifts, and bits at and past n are cleared.  Words too
-// close to either end of the input take the byte loop.
-__device__ __forceinline__ uint32_t pack_bytes32(const uint8_t *p, int n, long long room, long long lead)
-{
-    const uintptr_t pa = reinterpret_cast<uintptr_t>(p);
-    const unsigned o = (unsigned)(pa & 15u);
-    if ((long long)o <= lead && (long long)(48u - o) <= room) {
-        const uint4 *a16 = reinterpret_cast<const uint4 *>(pa & ~uintptr_t(15));
-        const uint4 A = __ldg(a16), B = __ldg(a16 + 1), C = __ldg(a16 + 2);
-        const uint32_t u[12] = {A.x, A.y, A.z, A.w, B.x, B.y, B.z, B.w, C.x, C.y, C.z, C.w};
-        const bool s2 = (o & 8u) != 0, s1 = (o & 4u) != 0;
-        uint32_t t[10], v[9];
-#pragma unroll
-        for (int i = 0; i < 10; i++) t[i] = s2 ? u[i + 2] : u[i];
-#pragma unroll
-        for (int i = 0; i < 9; i++) v[i] = s1 ? t[i + 1] : t[i];
-        const unsigned sh = (o & 3u) * 8u;
-        uint32_t w = 0;
-#pragma unroll
-        for (int k = 0; k < 8; k++) w |= nz4_to_bits(__funnelshift_r(v[k], v[k + 1], sh)) << (4 * k);
-        return n >= 32 ? w : w & ((1u << n) - 1u);
-    }
-    uint32_t w = 0;
-    for (int b = 0; b < n; b++) w |= (uint32_t)(p[b] != 0) << b;
-    return w;
-}
-
 template <typename T>
 __device__ __forceinline__ uint32_t pack_word_mode(const T *p, int n, int mode, long long room, long long lead = 0)
 {
     return mode == 0 ? pack_word<T, 0>(p, n, room, lead) : mode == 1 ? pack_word<T, 1>(p, n, room, lead)
                                                                      : pack_word<T, 2>(p, n, room, lead);
-}
-
-__device__ __forceinline__ int dtype_bytes(int dtype)
-{
-    return dtype == BGT_F64 ? 8 : (dtype == BGT_U32 || dtype == BGT_I32 || dtype == BGT_F32) ? 4
-                                  : (dtype == BGT_U16 || dtype == BGT_I16) ? 2 : 1;
 }
 
 __device__ __forceinline__ int find_io(const IODesc *io, int n, long long g, bool unpack)
@@ -571,10 +498,6 @@ __global__ void pack_all_kernel(const Inst *__restrict__ insts, const IODesc *__
         }
     }
 }
-
-// 4 bits -> 4 bytes of value 0/1 (bit k to byte k): the multiplier places bit
-// k at 8k and the mask drops the other partial products (all at distinct bits).
-__device__ __forceinline__ uint32_t bits4_to_bytes(uint32_t nib) { return (nib * 0x00204081u) & 0x01010101u; }
 
 template <typename T>
 __device__ __forceinline__ void unpack_word(uint32_t w, T *o, int n)

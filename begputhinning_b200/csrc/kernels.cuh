@@ -88,9 +88,6 @@ int res_rows_fit2d(int W);
 bool res_fits3d(int W, int ny, int nz);
 constexpr int kResHalo3D = 6;  // one iteration: six subiterations, one row and plane each
 cudaError_t res_occupancy(int *per_sm);  // resident CTAs per SM
-cudaError_t launch_resident(int grid, Inst *d_insts, int ninst, const ResItem *d_items, int nitems,
-                            ResSched *d_rs, ResTrace *d_trace, long long timeout_ns, cudaStream_t st);
-
 // Per-instance input/output of a batch-wide pack/unpack launch.
 // Unsigned 32-bit division by a divisor fixed per instance, as a multiply
 // and shifts (Granlund and Montgomery, "Division by invariant integers using
@@ -130,6 +127,12 @@ struct alignas(16) IODesc {
     // used words per row ceil(W/32), and the core tile extents TW, TH, TZ
     FastDiv dP, dH, dW, dWW, dTW, dTH, dTZ;
 };
+
+// pixels: instances are read from and written to their pixel arrays (d_io by
+// instance, or `one` for a batch of one instance); else buf[0] holds them.
+cudaError_t launch_resident(int grid, Inst *d_insts, int ninst, const ResItem *d_items, int nitems,
+                            ResSched *d_rs, ResTrace *d_trace, long long timeout_ns, const IODesc *d_io,
+                            const IODesc *one, bool pixels, cudaStream_t st);
 
 // Launchers (stream-ordered, no host synchronisation).
 // bytes: every input is one byte wide and tested "byte != 0" (see pack_all_kernel)

@@ -1,0 +1,207 @@
+// pixels.cuh -- pixels <-> bit words: the binarisation of every pixel type on
+// the way in, 0/1 in the pixel type on the way out.  Shared by the batch-wide
+// pack and unpack kernels and by the resident kernel, which reads and writes
+// the pixels of its instances itself.
+#pragma once
+#include <cstdint>
+#include <type_traits>
+
+#include "common.cuh"
+#include "kernels.cuh"
+
+namespace bgt {
+
+// Foreground tests of the reference's binarisation.  2D: (unsigned int)v > 0
+// evaluated on the device (2D/CUDA_DeviceHelperFunctions.cuh:101), i.e. a
+// saturating conversion for floating types.  3D: int(v) > 0 as the host
+// evaluates it (3D/CenterlineExtraction.cpp:44; x86-64 conversion of
+// out-of-range floats gives INT_MIN).
+template <typename T>
+__device__ __forceinline__ bool fg2(T v) { return (unsigned int)v > 0u; }
+template <>
+__device__ __forceinline__ bool fg2<bool>(bool v) { return v; }
+
+template <typename T>
+__device__ __forceinline__ bool fg3(T v) { return (int)v > 0; }
+template <>
+__device__ __forceinline__ bool fg3<float>(float v) { return v >= 1.0f && v < 2147483648.0f; }
+template <>
+__device__ __forceinline__ bool fg3<double>(double v) { return v >= 1.0 && v < 2147483648.0; }
+template <>
+__device__ __forceinline__ bool fg3<bool>(bool v) { return v; }
+
+__device__ __forceinline__ int dtype_bytes(int dtype)
+{
+    return dtype == BGT_F64 ? 8 : (dtype == BGT_U32 || dtype == BGT_I32 || dtype == BGT_F32) ? 4
+                                  : (dtype == BGT_U16 || dtype == BGT_I16) ? 2 : 1;
+}
+
+// MSB-of-byte gather: multiplying the MSB mask by 0x00204081 moves bits 7,
+// 15, 23, 31 to 28..31 without carries.
+__device__ __forceinline__ uint32_t bytes4_to_bits(uint32_t cmp)
+{
+    return ((cmp & 0x80808080u) * 0x00204081u) >> 28;
+}
+
+// 4 bytes -> 4 bits "byte != 0" (bit k for byte k) with integer ALU ops only:
+// the low seven bits of each byte plus 0x7F carry into the byte's MSB
+// exactly when they are nonzero (no carry leaves the byte), and OR-ing the
+// byte back in covers the MSB itself.  With `neg` all ones, "byte > 0" of
+// signed bytes: those whose own MSB is set are taken out again.
+__device__ __forceinline__ uint32_t nz4_to_bits(uint32_t c, uint32_t neg = 0u)
+{
+    return bytes4_to_bits((((c & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | c) & ~(c & neg));
+}
+
+// 4 bits -> 4 bytes of value 0/1 (bit k to byte k): the multiplier places bit
+// k at 8k and the mask drops the other partial products (all at distinct bits).
+__device__ __forceinline__ uint32_t bits4_to_bytes(uint32_t nib) { return (nib * 0x00204081u) & 0x01010101u; }
+
+// 32 one-byte pixels from p (n < 32 at a row's ragged end) -> "byte != 0"
+// bits (neg all ones: "byte > 0", signed), without branches that depend on p's
+// alignment: three aligned 16-byte loads (two for an aligned p) cover p .. p+31 (they may run past
+// the row into the next one, never past the input: `room` = bytes readable
+// from p onward, `lead` = bytes readable before p), the 12 loaded words are
+// shifted by p's word offset in two conditional-select stages and by its byte
+// offset with funnel shifts, and bits at and past n are cleared.  Words too
+// close to either end of the input take the byte loop.
+__device__ __forceinline__ uint32_t pack_bytes32(const uint8_t *p, int n, long long room, long long lead,
+                                                 uint32_t neg = 0u)
+{
+    const uintptr_t pa = reinterpret_cast<uintptr_t>(p);
+    const unsigned o = (unsigned)(pa & 15u);
+    if ((long long)o <= lead && (long long)(o ? 48u - o : 32u) <= room) {
+        const uint4 *a16 = reinterpret_cast<const uint4 *>(pa & ~uintptr_t(15));
+        const uint4 A = __ldg(a16), B = __ldg(a16 + 1), C = o ? __ldg(a16 + 2) : make_uint4(0, 0, 0, 0);
+        const uint32_t u[12] = {A.x, A.y, A.z, A.w, B.x, B.y, B.z, B.w, C.x, C.y, C.z, C.w};
+        const bool s2 = (o & 8u) != 0, s1 = (o & 4u) != 0;
+        uint32_t t[10], v[9];
+#pragma unroll
+        for (int i = 0; i < 10; i++) t[i] = s2 ? u[i + 2] : u[i];
+#pragma unroll
+        for (int i = 0; i < 9; i++) v[i] = s1 ? t[i + 1] : t[i];
+        const unsigned sh = (o & 3u) * 8u;
+        uint32_t w = 0;
+#pragma unroll
+        for (int k = 0; k < 8; k++) w |= nz4_to_bits(__funnelshift_r(v[k], v[k + 1], sh), neg) << (4 * k);
+        return n >= 32 ? w : w & ((1u << n) - 1u);
+    }
+    uint32_t w = 0;
+    for (int b = 0; b < n; b++) w |= (uint32_t)(p[b] != 0 && !(p[b] & neg & 0x80u)) << b;
+    return w;
+}
+
+// The packed word of `cnt` (0..32) one-byte pixels from element `off` of the input.
+__device__ __forceinline__ uint32_t pixel_bytes(const IODesc &d, uint32_t off, int cnt, uint32_t neg)
+{
+    if (cnt <= 0) return 0u;
+    const long long total = (long long)d.inW * d.inH * d.inD;
+    return pack_bytes32((const uint8_t *)d.in + off, cnt, total - off, off, neg);
+}
+// the `neg` of an input's pixel type and rule
+__device__ __forceinline__ uint32_t pixel_neg(const IODesc &d)
+{
+    return d.mode == 1 && (d.dtype == BGT_I8 || (d.dtype == BGT_CHAR && std::is_signed<char>::value)) ? 0xffffffffu : 0u;
+}
+
+// Wider pixels: the warp builds its 32 lanes' words one after the other, a
+// lane per pixel (coalesced whatever the alignment) and a vote per word.
+template <typename T, int MODE>
+__device__ __forceinline__ uint32_t pixel_vote(const T *p, uint32_t off, int cnt)
+{
+    const int lane = threadIdx.x & 31;
+    uint32_t w = 0;
+#pragma unroll 8
+    for (int k = 0; k < 32; k++) {
+        const uint32_t o = __shfl_sync(kFull, off, k);
+        const int c = __shfl_sync(kFull, cnt, k);
+        bool f = false;
+        if (lane < c) {
+            const T v = __ldg(p + (size_t)o + lane);
+            f = MODE == 0 ? fg2<T>(v) : fg3<T>(v);
+        }
+        const uint32_t m = __ballot_sync(kFull, f);
+        if (lane == k) w = m;
+    }
+    return w;
+}
+template <typename T>
+__device__ __forceinline__ uint32_t pixel_vote_mode(const IODesc &d, uint32_t off, int cnt)
+{
+    return d.mode == 0 ? pixel_vote<T, 0>((const T *)d.in, off, cnt) : pixel_vote<T, 1>((const T *)d.in, off, cnt);
+}
+// Every lane of the warp calls it (cnt = 0 for none).
+static __device__ __noinline__ uint32_t pixel_word_wide(const IODesc &d, uint32_t off, int cnt)
+{
+    switch (d.dtype) {
+    case BGT_U16: return pixel_vote_mode<uint16_t>(d, off, cnt);
+    case BGT_I16: return pixel_vote_mode<int16_t>(d, off, cnt);
+    case BGT_U32: return pixel_vote_mode<uint32_t>(d, off, cnt);
+    case BGT_I32: return pixel_vote_mode<int32_t>(d, off, cnt);
+    case BGT_F32: return pixel_vote_mode<float>(d, off, cnt);
+    default: return pixel_vote_mode<double>(d, off, cnt);
+    }
+}
+
+// The same way out: lane l writes pixel l of the warp's k-th word.
+template <typename T>
+__device__ __forceinline__ void pixel_spread(T *p, uint32_t off, int cnt, uint32_t w)
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll 4
+    for (int k = 0; k < 32; k++) {
+        const uint32_t o = __shfl_sync(kFull, off, k), v = __shfl_sync(kFull, w, k);
+        const int c = __shfl_sync(kFull, cnt, k);
+        if (lane < c) p[(size_t)o + lane] = (T)((v >> lane) & 1u);
+    }
+}
+static __device__ __noinline__ void pixel_store_wide(const IODesc &d, uint32_t off, int cnt, uint32_t w)
+{
+    switch (dtype_bytes(d.dtype)) {
+    case 2: pixel_spread((uint16_t *)d.out, off, cnt, w); break;
+    case 4:
+        if (d.dtype == BGT_F32) pixel_spread((float *)d.out, off, cnt, w);
+        else pixel_spread((uint32_t *)d.out, off, cnt, w);
+        break;
+    default: pixel_spread((double *)d.out, off, cnt, w); break;
+    }
+}
+
+// 32-byte-aligned chunk c of the one-byte pixels of `rows` consecutive rows of
+// W pixels that start at `out`; row(r) = the packed words of row r, readable
+// one word past the row's last.  Two 128-bit stores where the chunk lies
+// inside the rows and spans at most two of them, bytes otherwise.
+template <class Row>
+__device__ __forceinline__ void pixel_chunk(uint8_t *out, uint32_t rows, int W, const FastDiv &dW, uint32_t c, Row row)
+{
+    const uintptr_t o = reinterpret_cast<uintptr_t>(out), end = o + (uintptr_t)rows * W;
+    const uintptr_t a = (o & ~uintptr_t(31)) + (uintptr_t)c * 32u;
+    const uintptr_t lo = a > o ? a : o, hi = a + 32 < end ? a + 32 : end;
+    if (lo >= hi) return;
+    const uint32_t f = (uint32_t)(lo - o);
+    uint32_t r = fdiv(dW, f);
+    int x = (int)(f - r * (uint32_t)W);
+    if (hi - lo == 32 && W >= 32) {
+        const uint32_t *s = row(r);
+        uint32_t bits = __funnelshift_r(s[x >> 5], s[(x >> 5) + 1], x & 31);
+        if (x + 32 > W) {  // the chunk runs into the next row
+            const int n0 = W - x;
+            bits = (bits & ((1u << n0) - 1u)) | row(r + 1)[0] << n0;
+        }
+        uint4 *q = reinterpret_cast<uint4 *>(a);
+        q[0] = make_uint4(bits4_to_bytes(bits & 15u), bits4_to_bytes((bits >> 4) & 15u),
+                          bits4_to_bytes((bits >> 8) & 15u), bits4_to_bytes((bits >> 12) & 15u));
+        q[1] = make_uint4(bits4_to_bytes((bits >> 16) & 15u), bits4_to_bytes((bits >> 20) & 15u),
+                          bits4_to_bytes((bits >> 24) & 15u), bits4_to_bytes(bits >> 28));
+        return;
+    }
+    for (uintptr_t b = lo; b < hi; b++) {
+        *reinterpret_cast<uint8_t *>(b) = (uint8_t)((row(r)[x >> 5] >> (x & 31)) & 1u);
+        if (++x == W) {
+            x = 0;
+            r++;
+        }
+    }
+}
+
+}  // namespace bgt

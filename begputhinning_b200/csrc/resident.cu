@@ -51,6 +51,7 @@
 #include <algorithm>
 
 #include "kernels.cuh"
+#include "pixels.cuh"
 #include "rules.cuh"
 #include "tiles.cuh"
 
@@ -153,6 +154,139 @@ __device__ __forceinline__ int res_take(int *c)
     int k = 0;
     if ((threadIdx.x & 31) == 0) k = atomicAdd(c, 1);
     return __shfl_sync(kFull, k, 0);
+}
+
+// Positions of the words of an ny x nz grid of rows of wl words, in raster
+// order, for a thread that takes every kResThreads-th one.
+struct WordPos {
+    int x, y, z;
+};
+struct WordWalk {
+    int wl, ny, dx, dy, dz;
+    __device__ __forceinline__ WordWalk(int wl_, int ny_) : wl(wl_), ny(ny_)
+    {
+        const int q = kResThreads / wl;
+        dx = kResThreads - q * wl;
+        dz = q / ny;
+        dy = q - dz * ny;
+    }
+    __device__ __forceinline__ WordPos first() const
+    {
+        const int r = (int)threadIdx.x / wl;
+        return WordPos{(int)threadIdx.x - r * wl, r % ny, r / ny};
+    }
+    __device__ __forceinline__ void next(WordPos &q) const
+    {
+        q.x += dx;
+        q.y += dy;
+        q.z += dz;
+        if (q.x >= wl) {
+            q.x -= wl;
+            q.y++;
+        }
+        if (q.y >= ny) {
+            q.y -= ny;
+            q.z++;
+        }
+    }
+};
+
+// Where an instance's words come from and go to: its pixels, or (pix false)
+// its packed buffer.
+struct ResIO {
+    const IODesc *d;
+    bool pix;
+};
+
+// put(pos, word) for every word of the grid of rows whose first pixel row and
+// plane are y0, z0 (warps stay together: put may hold warp-wide votes; `live`
+// is false for lanes past the end, whose word is 0).  U words of a thread are
+// in flight at once: at 768 threads and 48 bytes per word of one-byte pixels,
+// two cover the latency of HBM.
+template <int U, class Fetch, class Put>
+__device__ __forceinline__ void res_load_loop(const WordWalk &walk, int n, Fetch fetch, Put put)
+{
+    const int lane = threadIdx.x & 31;
+    WordPos q = walk.first();
+    for (int i = threadIdx.x; i - lane < n; i += U * kResThreads) {
+        uint32_t v[U];
+        WordPos at[U];
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+            at[k] = q;
+            v[k] = fetch(i + k * kResThreads < n, q);
+            walk.next(q);
+        }
+#pragma unroll
+        for (int k = 0; k < U; k++) put(i + k * kResThreads < n, at[k], v[k]);
+    }
+}
+template <class Put>
+__device__ __forceinline__ void res_load(const Inst &in, const ResIO &io, const WordWalk &walk, int n, int y0, int z0,
+                                         Put put)
+{
+    if (!io.pix) {
+        const uint32_t *g = in.buf[0];
+        const int H = in.H, P = in.P;
+        res_load_loop<4>(walk, n, [&](bool live, const WordPos &q) {
+            return live ? __ldcg(g + ((size_t)(z0 + q.z) * H + (y0 + q.y)) * P + q.x) : 0u;
+        }, put);
+        return;
+    }
+    const IODesc &d = *io.d;
+    const int inW = d.inW, inH = d.inH, inD = d.inD;
+    auto count = [&](bool live, const WordPos &q, uint32_t &off) {
+        const int y = y0 + q.y, z = z0 + q.z;
+        off = ((uint32_t)z * (uint32_t)inH + (uint32_t)y) * (uint32_t)inW + 32u * (uint32_t)q.x;
+        return live && y < inH && z < inD ? max(0, min(32, inW - 32 * q.x)) : 0;
+    };
+    if (dtype_bytes(d.dtype) == 1) {
+        const uint32_t neg = pixel_neg(d);
+        res_load_loop<2>(walk, n, [&](bool live, const WordPos &q) {
+            uint32_t off;
+            const int cnt = count(live, q, off);
+            return pixel_bytes(d, off, cnt, neg);
+        }, put);
+    } else {
+        res_load_loop<1>(walk, n, [&](bool live, const WordPos &q) {
+            uint32_t off;
+            const int cnt = count(live, q, off);
+            return pixel_word_wide(d, off, cnt);
+        }, put);
+    }
+}
+
+// The way back for rows [y0, y0 + ny) of planes [z0, z0 + nz): row(y, z) = the
+// packed words of grid row y of grid plane z.
+template <class Row>
+__device__ __forceinline__ void res_store(const Inst &in, const ResIO &io, int ny, int nz, int y0, int z0, Row row)
+{
+    const int lane = threadIdx.x & 31, wl = (in.W + 31) >> 5;
+    const WordWalk walk(wl, ny);
+    const int n = nz * ny * wl;
+    if (!io.pix || !io.d->out) {
+        uint32_t *g = in.buf[0];
+        WordPos q = walk.first();
+        for (int i = threadIdx.x; i < n; i += kResThreads, walk.next(q))
+            g[((size_t)(z0 + q.z) * in.H + (y0 + q.y)) * in.P + q.x] = row(q.y, q.z)[q.x];
+        return;
+    }
+    const IODesc &d = *io.d;
+    if (dtype_bytes(d.dtype) == 1) {
+        const uint32_t per = ((uint32_t)ny * (uint32_t)in.W + 31u) / 32u + 1u;  // chunks a plane's rows touch at most
+        for (uint32_t i = threadIdx.x; i < per * (uint32_t)nz; i += kResThreads) {
+            const uint32_t z = nz == 1 ? 0u : i / per;
+            uint8_t *out = (uint8_t *)d.out + ((size_t)(z0 + (int)z) * in.H + y0) * in.W;
+            pixel_chunk(out, (uint32_t)ny, in.W, d.dW, i - z * per, [&](uint32_t r) { return row((int)r, (int)z); });
+        }
+        return;
+    }
+    WordPos q = walk.first();
+    for (int i = threadIdx.x; i - lane < n; i += kResThreads, walk.next(q)) {
+        const bool live = i < n;
+        const uint32_t off = ((uint32_t)(z0 + q.z) * (uint32_t)in.H + (uint32_t)(y0 + q.y)) * (uint32_t)in.W + 32u * (uint32_t)q.x;
+        pixel_store_wide(d, off, live ? min(32, in.W - 32 * q.x) : 0, live ? row(q.y, q.z)[q.x] : 0u);
+    }
 }
 
 // ------------------------------------------------------------ 2D ----------
@@ -327,7 +461,7 @@ __device__ uint32_t res_pass2d(const Band2D &b, int q, int *take, unsigned long 
     return core;
 }
 
-__device__ void res_run2d(Inst &in, const ResItem &it, uint32_t *sm, ResSched *S, int *take)
+__device__ void res_run2d(Inst &in, const ResIO &io, const ResItem &it, uint32_t *sm, ResSched *S, int *take)
 {
     __shared__ int s_flag;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -348,22 +482,24 @@ __device__ void res_run2d(Inst &in, const ResItem &it, uint32_t *sm, ResSched *S
     const int pp = b.pp;
     const int nunits = b.nstrips * b.nchunks;
 
-    for (int i = threadIdx.x; i < pp; i += kResThreads) b.zero[i] = 0u;
+    // zero row and row copies (their words left and right of the image stay zero)
+    {
+        const int total = pp * (1 + 2 * b.nrows);
+        for (int i = threadIdx.x; i < total / 4; i += kResThreads)
+            reinterpret_cast<uint4 *>(sm)[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (threadIdx.x < (total & 3)) sm[(total & ~3) + threadIdx.x] = 0u;
+    }
     for (int i = threadIdx.x; i < nunits; i += kResThreads) b.until[i] = -1;
     if (threadIdx.x < 2) take[threadIdx.x] = 0;
     __syncthreads();
-    const uint32_t *g0 = in.buf[0];
-    for (int r = warp; r < b.nrows; r += kWarps) {
-        const uint32_t *grow = g0 + (size_t)(b.a + r) * in.P;
-        uint32_t *r0p = b.buf0 + (size_t)r * pp, *r1p = b.buf1 + (size_t)r * pp;
-        for (int w = lane; w < pp; w += 32) {
-            const uint32_t v = (w >= 1 && w <= b.wl) ? __ldcg(grow + (w - 1)) : 0u;
-            r0p[w] = v;
-            r1p[w] = v;
-            // units holding foreground start active
-            if (v) b.until[(r / kUnitRows) * b.nchunks + (w - 1) / kUnitWords] = 0;
-        }
-    }
+    res_load(in, io, WordWalk(b.wl, b.nrows), b.nrows * b.wl, b.a, 0, [&](bool, const WordPos &q, uint32_t v) {
+        if (!v) return;
+        const int w = q.y * pp + q.x + 1;
+        b.buf0[w] = v;
+        b.buf1[w] = v;
+        // units holding foreground start active
+        b.until[(q.y / kUnitRows) * b.nchunks + q.x / kUnitWords] = 0;
+    });
     __syncthreads();
 
     int result = 0;  // 1 converged, -1 pass cap or failed wait
@@ -436,15 +572,10 @@ __device__ void res_run2d(Inst &in, const ResItem &it, uint32_t *sm, ResSched *S
             break;
         }
     }
-    // the converged core rows (in buf[(q+1)&1]) -> buf[0]
+    // the converged core rows (in buf[(q+1)&1])
     __syncthreads();
-    const uint32_t *fin = (q & 1) ? b.buf0 : b.buf1;
-    uint32_t *g0w = in.buf[0];
-    for (int r = b.r0 - b.a + warp; r < b.r1 - b.a; r += kWarps) {
-        const uint32_t *srow = fin + (size_t)r * pp;
-        uint32_t *grow = g0w + (size_t)(b.a + r) * in.P;
-        for (int w = lane; w < b.wl; w += 32) grow[w] = srow[w + 1];
-    }
+    const uint32_t *fin = ((q & 1) ? b.buf0 : b.buf1) + (size_t)(b.r0 - b.a) * pp + 1;
+    res_store(in, io, b.r1 - b.r0, 1, b.r0, 0, [&](int y, int) { return fin + (size_t)y * pp; });
     if (lane == 0 && words) atomicAdd(&in.work_words, words);  // core words per pass (one iteration)
     if (threadIdx.x == 0) {
         if (it.band == 0) in.passes_run = q + 1;
@@ -559,12 +690,12 @@ __device__ __forceinline__ void box_subiteration1(const Box3D b, uint32_t e, uin
 // whole (24 us per iteration): a 97 x 75 x 66 tree volume 214 -> 72 us, a
 // 187 x 203 x 161 one 955 -> 150 us, a 256^3 one, whose bricks did not fit,
 // 1330 us on the tile rings -> 176 us.
-__device__ void res_run3d(Inst &in, const ResItem &it, uint8_t *smb, ResSched *S)
+__device__ void res_run3d(Inst &in, const ResIO &io, const ResItem &it, uint8_t *smb, ResSched *S)
 {
     __shared__ int s_n[4];  // lengths: word list, active words, candidates, messages
     __shared__ int s_flag;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int W = in.W, H = in.H, D = in.D, P = in.P, wl = (W + 31) >> 5;
+    const int H = in.H, D = in.D, wl = (in.W + 31) >> 5;
     const bool team = it.bands > 1;
     const int z0 = max(0, it.r0 - it.halo), z1 = min(D, it.r1 + it.halo);
     const int y0 = max(0, it.c0 - it.halo), y1 = min(H, it.c1 + it.halo);
@@ -590,58 +721,19 @@ __device__ void res_run3d(Inst &in, const ResItem &it, uint8_t *smb, ResSched *S
     for (size_t i = threadIdx.x; i < off / 16; i += kResThreads) reinterpret_cast<uint4 *>(smb)[i] = make_uint4(0, 0, 0, 0);
     if (threadIdx.x < 4) s_n[threadIdx.x] = 0;
     __syncthreads();
-    const uint32_t *g0 = in.buf[0];
-    // words of the box in raster order, a thread every kResThreads-th one
     const int nbox = nz * ny * wl;
-    const int qr = kResThreads / wl, dx = kResThreads - qr * wl, dz = qr / ny, dy = qr - dz * ny;
-    struct Pos {
-        int x, y, z;
-    };
-    auto first_pos = [&]() {
-        const int r = (int)threadIdx.x / wl;
-        return Pos{(int)threadIdx.x - r * wl, r % ny, r / ny};
-    };
-    auto advance = [&](Pos &q) {
-        q.x += dx;
-        q.y += dy;
-        q.z += dz;
-        if (q.x >= wl) {
-            q.x -= wl;
-            q.y++;
-        }
-        if (q.y >= ny) {
-            q.y -= ny;
-            q.z++;
-        }
-    };
-    auto dist_of = [&](const Pos &q) {
+    const WordWalk walk(wl, ny);
+    auto dist_of = [&](const WordPos &q) {
         const int y = y0 + q.y, z = z0 + q.z;
         return max(max(max(it.c0 - y, y - it.c1 + 1), max(it.r0 - z, z - it.r1 + 1)), 0);
     };
-    auto index_of = [&](const Pos &q) { return ((q.z + 1) * ny2 + q.y + 1) * b.p + 1 + q.x; };
-    {
-        constexpr int U = 4;  // loads in flight per thread
-        Pos q = first_pos();
-        for (int i = threadIdx.x; i - lane < nbox; i += U * kResThreads) {
-            uint32_t v[U];
-            Pos at[U];
-#pragma unroll
-            for (int k = 0; k < U; k++) {
-                at[k] = q;
-                v[k] = i + k * kResThreads < nbox ? __ldcg(g0 + ((size_t)(z0 + q.z) * H + (y0 + q.y)) * P + q.x) : 0u;
-                advance(q);
-            }
-#pragma unroll
-            for (int k = 0; k < U; k++) {
-                const int d = dist_of(at[k]);
-                const int idx = v[k] ? index_of(at[k]) : 0;
-                if (v[k]) b.state[idx] = v[k];
-                const int pos = warp_append(v[k] != 0u && d <= 5, &s_n[0]);
-                if (pos >= 0 && pos < list_cap)
-                    list[pos] = (uint32_t)idx | (uint32_t)(at[k].x >> xs) << 16 | (uint32_t)d << 21;
-            }
-        }
-    }
+    auto index_of = [&](const WordPos &q) { return ((q.z + 1) * ny2 + q.y + 1) * b.p + 1 + q.x; };
+    res_load(in, io, walk, nbox, y0, z0, [&](bool, const WordPos &q, uint32_t v) {
+        const int d = dist_of(q), idx = v ? index_of(q) : 0;
+        if (v) b.state[idx] = v;
+        const int pos = warp_append(v != 0u && d <= 5, &s_n[0]);
+        if (pos >= 0 && pos < list_cap) list[pos] = (uint32_t)idx | (uint32_t)(q.x >> xs) << 16 | (uint32_t)d << 21;
+    });
     __syncthreads();
     const int nl = s_n[0];
     MeetState meet;
@@ -766,8 +858,8 @@ __device__ void res_run3d(Inst &in, const ResItem &it, uint8_t *smb, ResSched *S
                 changed(ent_idx(e), ent_col(e), msg);
             }
         } else {
-            Pos q = first_pos();
-            for (int i = threadIdx.x; i < nbox; i += kResThreads, advance(q)) {
+            WordPos q = walk.first();
+            for (int i = threadIdx.x; i < nbox; i += kResThreads, walk.next(q)) {
                 const int idx = index_of(q), d = dist_of(q);
                 const uint32_t *s = b.state + idx;
                 uint32_t un = 0, du = 0;
@@ -786,16 +878,16 @@ __device__ void res_run3d(Inst &in, const ResItem &it, uint8_t *smb, ResSched *S
 #pragma unroll 1
             for (int j = 0; j < 6; j++) {
                 // deletions of subiteration j were found: apply them, then find the next one's
-                q = first_pos();
-                for (int i = threadIdx.x; i < nbox; i += kResThreads, advance(q)) {
+                q = walk.first();
+                for (int i = threadIdx.x; i < nbox; i += kResThreads, walk.next(q)) {
                     const int idx = index_of(q);
                     const uint32_t del = b.cdel[idx];
                     if (del) b.state[idx] &= ~del;
                 }
                 __syncthreads();
                 if (j == 5) break;
-                q = first_pos();
-                for (int i = threadIdx.x; i < nbox; i += kResThreads, advance(q)) {
+                q = walk.first();
+                for (int i = threadIdx.x; i < nbox; i += kResThreads, walk.next(q)) {
                     const int idx = index_of(q), d = dist_of(q);
                     const uint32_t cand = b.state[idx] & b.cU[idx];
                     uint32_t del = 0;
@@ -814,8 +906,8 @@ __device__ void res_run3d(Inst &in, const ResItem &it, uint8_t *smb, ResSched *S
                 __syncthreads();
             }
             // only voxels of the union were deleted: a word changed when it lost some of its union
-            q = first_pos();
-            for (int i = threadIdx.x; i < nbox; i += kResThreads, advance(q)) {
+            q = walk.first();
+            for (int i = threadIdx.x; i < nbox; i += kResThreads, walk.next(q)) {
                 const int idx = index_of(q);
                 if (!(b.cU[idx] & ~b.state[idx]) || dist_of(q) != 0) continue;
                 core = true;
@@ -887,16 +979,10 @@ __device__ void res_run3d(Inst &in, const ResItem &it, uint8_t *smb, ResSched *S
         // (chg is next written after the barriers of the next iteration)
     }
     __syncthreads();
-    // the converged core -> buf[0]
-    {
-        uint32_t *g0w = in.buf[0];
-        Pos q = first_pos();
-        for (int i = threadIdx.x; i < nbox; i += kResThreads, advance(q)) {
-            const int y = y0 + q.y, z = z0 + q.z;
-            if (y >= it.c0 && y < it.c1 && z >= it.r0 && z < it.r1)
-                g0w[((size_t)z * H + y) * P + q.x] = b.state[index_of(q)];
-        }
-    }
+    // the converged core
+    res_store(in, io, it.c1 - it.c0, it.r1 - it.r0, it.c0, it.r0, [&](int y, int z) {
+        return b.state + ((z + it.r0 - z0 + 1) * ny2 + (y + it.c0 - y0 + 1)) * b.p + 1;
+    });
     words = __reduce_add_sync(kFull, words);
     entries = __reduce_add_sync(kFull, entries);
     if (lane == 0 && words) {
@@ -939,7 +1025,8 @@ __device__ __forceinline__ int res_smid()
 }
 
 __global__ void __launch_bounds__(kResThreads, kResCtasPerSm)
-    resident_kernel(Inst *insts, const ResItem *items, ResSched *S, ResTrace *trace)
+    resident_kernel(Inst *insts, const ResItem *items, ResSched *S, ResTrace *trace, const IODesc *ios, bool pix,
+                    const __grid_constant__ IODesc one)
 {
     extern __shared__ __align__(16) uint8_t res_smem[];
     __shared__ int s_item;
@@ -953,10 +1040,11 @@ __global__ void __launch_bounds__(kResThreads, kResCtasPerSm)
         const ResItem it = items[k];
         Inst &in = insts[it.inst];
         const long long t0 = (long long)globaltimer();
+        const ResIO io{ios ? ios + it.inst : &one, pix};
         if (in.dims == 2)
-            res_run2d(in, it, reinterpret_cast<uint32_t *>(res_smem), S, s_take);
+            res_run2d(in, io, it, reinterpret_cast<uint32_t *>(res_smem), S, s_take);
         else
-            res_run3d(in, it, res_smem, S);
+            res_run3d(in, io, it, res_smem, S);
         if (threadIdx.x == 0) trace[k] = ResTrace{t0, (long long)globaltimer(), res_smid(), 0};
     }
 }
@@ -971,8 +1059,10 @@ cudaError_t res_occupancy(int *per_sm)
 }
 
 cudaError_t launch_resident(int grid, Inst *d_insts, int ninst, const ResItem *d_items, int nitems,
-                            ResSched *d_rs, ResTrace *d_trace, long long timeout_ns, cudaStream_t st)
+                            ResSched *d_rs, ResTrace *d_trace, long long timeout_ns, const IODesc *d_io,
+                            const IODesc *one, bool pixels, cudaStream_t st)
 {
+    if (nitems == 0) return cudaSuccess;
     static bool attr_done = false;
     if (!attr_done) {
         cudaError_t e = cudaFuncSetAttribute(resident_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
@@ -984,11 +1074,11 @@ cudaError_t launch_resident(int grid, Inst *d_insts, int ninst, const ResItem *d
     resident_reset_kernel<<<std::max(1, std::min(64, (ninst + 255) / 256)), 256, 0, st>>>(d_insts, ninst, d_rs, nitems,
                                                                                        timeout_ns);
     cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess || nitems == 0) return e;
+    if (e != cudaSuccess) return e;
     // cooperative: all CTAs are resident at once, which the bands of an image
     // (waiting for one another) rely on
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = dim3(std::min(grid, nitems));
     cfg.blockDim = dim3(kResThreads);
     cfg.dynamicSmemBytes = kSmemBytes;
     cfg.stream = st;
@@ -997,7 +1087,8 @@ cudaError_t launch_resident(int grid, Inst *d_insts, int ninst, const ResItem *d
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, resident_kernel, d_insts, d_items, d_rs, d_trace);
+    return cudaLaunchKernelEx(&cfg, resident_kernel, d_insts, d_items, d_rs, d_trace, one ? nullptr : d_io, pixels,
+                              one ? *one : IODesc{});
 }
 
 }  // namespace bgt
