@@ -264,23 +264,21 @@ extern "C" int bgt_batch_add3d(bgt_batch *b, int w, int h, int d, int cfg, int *
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-// Which instances the resident engine takes and how large 2D images are cut
-// into bands: a band holds at most what one CTA's shared memory does, and an
-// image is cut further while it is a large share of the batch's work (so a
-// batch of few large images still spreads over the SMs), keeping at least 32
-// core rows per band.  Items are ordered volumes first (largest first: their
-// chains of iterations are the longest), then images largest first, the bands
-// of one image consecutive.
+// Which instances the resident engine takes and how they are cut into boxes: a
+// box holds at most what one CTA's shared memory does, and an instance is cut
+// further while it is a large share of the batch's work (so a batch of few
+// large instances still spreads over the SMs).  Items are ordered volumes
+// first (largest first: their chains of iterations are the longest), then
+// images largest first, the boxes of one instance consecutive.
 static void plan_resident(bgt_batch *b)
 {
-    constexpr int kHalo = kResHalo2D, kMinCore = 32;  // 2D band halo
     b->res_items.clear();
     b->any_ring = false;
     const int N = (int)b->items.size();
     const bool rings_only = b->engine_mode == 1 || (getenv("BGT_ENGINE") && !strcmp(getenv("BGT_ENGINE"), "rings"));
     double total = 0;
     for (const BatchItem &it : b->items) total += (double)((it.W + 31) / 32) * it.H * it.D;
-    const double target = std::max(total / std::max(1, b->res_grid), 4096.0);
+    const double all = total, target = std::max(total / std::max(1, b->res_grid), 4096.0);
     std::vector<std::pair<double, int>> vols, imgs;
     for (int i = 0; i < N; i++) {
         const BatchItem &it = b->items[i];
@@ -315,7 +313,7 @@ static void plan_resident(bgt_batch *b)
         auto extent = [](int n, int g) {  // longest box along an axis of n cut into g, halo included
             return (n + g - 1) / g + (g == 1 ? 0 : g == 2 ? kResHalo3D : 2 * kResHalo3D);
         };
-        int share = (int)std::ceil(words / std::max(target, box_words));
+        int share = (int)(words / std::max(target, box_words));
         if (slab) share = (int)std::ceil(v.first / std::max(1.0e4, atof(slab)));
         share = std::max(1, std::min(share, b->res_grid));
         // the cut into at most `boxes` boxes with the smallest box, or (fewest) the fewest boxes
@@ -347,27 +345,47 @@ static void plan_resident(bgt_batch *b)
         }
         in.res_bands = G;
     }
+    // An image is cut into boxes of rows and words, as many as its share of the
+    // batch's work is worth (at least box_words2 words each), or as few as fit
+    // one CTA each.  A box costs its units' word steps, halo included; of the
+    // cuts with at most that many boxes the one with the cheapest box is taken.
+    // Shares are rounded down, so that the boxes of a batch of a few images do
+    // not exceed the CTAs by some (16 images of 1024^2: 128 boxes 121 us, 160
+    // boxes 183 us).  512 and 1024 words measured the same on lone images
+    // (512^2: 42 us), 2048 and 4096 longer (57 and 63 us).
+    double box_words2 = 1024.0;
+    if (const char *e = getenv("BGT_RES2D_BOX_WORDS")) box_words2 = std::max(1.0, atof(e));
     for (auto &m : imgs) {
         const int i = m.second;
         const BatchItem &it = b->items[i];
-        const int fit = res_rows_fit2d(it.W);
-        int G = 1;
-        if (it.H > fit) {
-            G = (it.H + (fit - 2 * kHalo) - 1) / std::max(1, fit - 2 * kHalo);
-            while ((it.H + G - 1) / G + 2 * kHalo > fit) G++;
-        }
-        const int G_work = (int)std::ceil(m.first / target);
-        const int G_rows = std::max(1, it.H / kMinCore);
-        G = std::max(G, std::min(G_work, G_rows));
-        G = std::min(G, b->res_grid);
-        const bool fits = G == 1 ? it.H <= fit : (it.H + G - 1) / G + 2 * kHalo <= fit && it.H / G >= kHalo;
-        if (!fits) {
-            b->h[i].res = 0;  // cannot be cut into bands that fit: the rings take it
+        const int wl = (it.W + 31) / 32;
+        constexpr int kHalo = 4 * kResPeriod2D, kMinRows = 24, kMinWords = 4;
+        const int share = std::max(1, std::min((int)(m.first / std::max(all / std::max(1, b->res_grid), box_words2)),
+                                               b->res_grid));
+        int gx = 0, gy = 0;
+        auto search = [&](int boxes, bool fewest) {
+            double best = 1e30;
+            for (int x = 1; x <= std::min(boxes, std::max(1, wl / kMinWords)); x++)
+                for (int y = 1; x * y <= boxes && y <= std::max(1, it.H / kMinRows); y++) {
+                    const bool cut = x * y > 1;
+                    const int nw = std::min(wl, (wl + x - 1) / x + (x == 1 ? 0 : x == 2 ? 1 : 2));
+                    const int nr = std::min(it.H, (it.H + y - 1) / y + (!cut || y == 1 ? 0 : y == 2 ? kHalo : 2 * kHalo));
+                    if (!res_fits2d(nw, nr)) continue;
+                    const double cost = res_cost2d(nw, nr) + (fewest ? 1e9 : 1e-3) * x * y;
+                    if (cost < best) best = cost, gx = x, gy = y;
+                }
+            return gx > 0;
+        };
+        if (!search(share, false) && !search(b->res_grid, true)) {
+            b->h[i].res = 0;  // cannot be cut into boxes that fit: the rings take it
             continue;
         }
+        const int G = gx * gy;
         for (int k = 0; k < G; k++) {
-            const int r0 = (int)((long long)k * it.H / G), r1 = (int)((long long)(k + 1) * it.H / G);
-            b->res_items.push_back(ResItem{i, k, G, r0, r1, G > 1 ? kHalo : 0, 0, it.W});
+            const int ky = k / gx, kx = k % gx;
+            const int r0 = (int)((long long)ky * it.H / gy), r1 = (int)((long long)(ky + 1) * it.H / gy);
+            const int c0 = (int)((long long)kx * wl / gx), c1 = (int)((long long)(kx + 1) * wl / gx);
+            b->res_items.push_back(ResItem{i, k, G, r0, r1, G > 1 ? kHalo : 0, c0, c1});
         }
     }
     for (int i = 0; i < N; i++)

@@ -46,16 +46,15 @@ struct Sched {
     long long timeout_ns;
 };
 
-// Resident engine (resident.cu).  A work item is one instance, or one band
-// of rows of a 2D image too large for one CTA (the bands of an image run
-// together and trade `halo` boundary rows through global memory after every
-// iteration).  Items are taken in order by one fetch-and-add.
+// Resident engine (resident.cu).  A work item is one instance, or one box of
+// it (the boxes of an instance run together and trade what lies along their
+// edges through global memory).  Items are taken in order by one fetch-and-add.
 struct ResItem {
     int inst;        // instance index
-    int band, bands; // band (3D: box) index and number of bands (1: the whole instance)
-    int r0, r1;      // 2D: core rows [r0, r1) of the band; 3D: core planes of the box
-    int halo;        // rows (3D: and planes) kept on each side of the core (0 for a single band)
-    int c0, c1;      // 3D: core rows of the box
+    int band, bands; // box index and number of boxes (1: the whole instance)
+    int r0, r1;      // core rows [r0, r1) of the box; 3D: core planes
+    int halo;        // rows (3D: and planes) kept on each side of the core (0 for a single box)
+    int c0, c1;      // core words of the box; 3D: core rows
 };
 struct ResSched {
     int head;        // next item
@@ -69,21 +68,22 @@ struct ResTrace {
     long long t0, t1;
     int sm, pad;
 };
-// 2D bands of one image meet every kResPassesPerExchange passes; wrong
-// values entering at a band's edge move at most 4 rows per pass, so the
-// bands keep 4 halo rows per pass of the period
-#ifndef BGT_RES_PASSES_PER_EXCHANGE
-#define BGT_RES_PASSES_PER_EXCHANGE 4  // measured: 1, 2, 3, 4 -> mixed batch 1.20, 1.11, 1.10, 1.09 ms
-#endif
-constexpr int kResPassesPerExchange = BGT_RES_PASSES_PER_EXCHANGE;
-constexpr int kResHalo2D = 4 * kResPassesPerExchange;
+// One CTA per SM: two of 384 threads with 112 KB each took the mixed batch
+// from 1.19 to 1.35 ms and three of 256 to 1.52 ms (smaller boxes, more halo),
+// lone images and volumes as long or longer.
 constexpr int kResThreads = 768;
 constexpr int kResCtasPerSm = 1;
-constexpr int kResSmemBytes = 230400;  // dynamic shared memory of one CTA (one per SM)
+constexpr int kResSmemBytes = 230400;  // dynamic shared memory of one CTA
 // Dynamic shared memory of the resident kernel (one CTA per SM).
 int res_smem_bytes();
-// Rows of a W-wide 2D band (core plus halo) that one CTA holds.
-int res_rows_fit2d(int W);
+// Whether a 2D box of nrows rows of wl words (halo included) fits one CTA.
+bool res_fits2d(int wl, int nrows);
+// Its cost: word steps of a pass over all of its units.
+double res_cost2d(int wl, int nrows);
+// Passes between two meetings of the boxes of an image (4 halo rows each): 1,
+// 2, 3 and 4 took a 4096^2 image 155, 119, 120 and 114 us, a 512^2 one 54, 47,
+// 47 and 43 us.
+constexpr int kResPeriod2D = 4;
 // Whether a 3D box (ny rows x nz planes of a volume W wide, halo included) fits one CTA.
 bool res_fits3d(int W, int ny, int nz);
 constexpr int kResHalo3D = 6;  // one iteration: six subiterations, one row and plane each

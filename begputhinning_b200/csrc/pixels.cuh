@@ -111,7 +111,7 @@ __device__ __forceinline__ uint32_t pixel_vote(const T *p, uint32_t off, int cnt
 {
     const int lane = threadIdx.x & 31;
     uint32_t w = 0;
-#pragma unroll 8
+#pragma unroll 16
     for (int k = 0; k < 32; k++) {
         const uint32_t o = __shfl_sync(kFull, off, k);
         const int c = __shfl_sync(kFull, cnt, k);
@@ -200,6 +200,37 @@ __device__ __forceinline__ void pixel_chunk(uint8_t *out, uint32_t rows, int W, 
         if (++x == W) {
             x = 0;
             r++;
+        }
+    }
+}
+
+// Chunk c of a run of n one-byte pixels at `out` whose words are s (readable
+// one word past the last).
+__device__ __forceinline__ void pixel_run_chunk(uint8_t *out, int n, uint32_t c, const uint32_t *s)
+{
+    const uintptr_t o = reinterpret_cast<uintptr_t>(out), end = o + (uintptr_t)n;
+    const uintptr_t a = (o & ~uintptr_t(31)) + (uintptr_t)c * 32u;
+    const uintptr_t lo = a > o ? a : o, hi = a + 32 < end ? a + 32 : end;
+    if (lo >= hi) return;
+    const int x = (int)(lo - o);
+    const uint32_t bits = __funnelshift_r(s[x >> 5], s[(x >> 5) + 1], x & 31);
+    if (hi - lo == 32) {
+        uint4 *q = reinterpret_cast<uint4 *>(a);
+        q[0] = make_uint4(bits4_to_bytes(bits & 15u), bits4_to_bytes((bits >> 4) & 15u),
+                          bits4_to_bytes((bits >> 8) & 15u), bits4_to_bytes((bits >> 12) & 15u));
+        q[1] = make_uint4(bits4_to_bytes((bits >> 16) & 15u), bits4_to_bytes((bits >> 20) & 15u),
+                          bits4_to_bytes((bits >> 24) & 15u), bits4_to_bytes(bits >> 28));
+        return;
+    }
+    // an end of the run: whole 4-byte groups, then the bytes left
+    for (uintptr_t b = lo; b < hi;) {
+        const unsigned k = (unsigned)(b - lo);
+        if ((b & 3) == 0 && b + 4 <= hi) {
+            *reinterpret_cast<uint32_t *>(b) = bits4_to_bytes((bits >> k) & 15u);
+            b += 4;
+        } else {
+            *reinterpret_cast<uint8_t *>(b) = (uint8_t)((bits >> k) & 1u);
+            b++;
         }
     }
 }

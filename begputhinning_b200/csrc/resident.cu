@@ -1,36 +1,19 @@
 // resident.cu -- the resident engine: every work item (an instance, or one
-// band of rows of a 2D image too large for one CTA) is loaded once into one
+// box of it) is loaded once into one
 // CTA's shared memory and thinned there from its first subiteration to its
-// fixed point; only the bands of a large image (every fourth iteration) and
-// the slabs of a large volume (every iteration) meet to trade boundary rows
-// through global memory.
+// fixed point; only the boxes of a large image (every few iterations) and of
+// a large volume (every iteration) meet to trade their edges through global
+// memory.
 // One CTA of 768 threads per SM holds up to 225 KB (measured against two
 // CTAs of 384 threads with 111 KB each: larger bands and slabs won).
 //
-// 2D band (dense).  Rows of the band (core plus `halo` rows on each side,
-// clamped to the image) lie twice in shared memory (subiteration t reads one
-// copy and writes the other) with an odd pitch of 2*ceil(wl/2)+3 words
-// (wl = ceil(W/32); a zero word left of every row and zero words right of
-// it).  A subiteration hands units (a strip of 32 rows x a chunk of words,
-// chunks sized so that there are about two units per warp) to warps
-// dynamically; lane = row, walking the chunk in pairs of words: each lane
-// loads its own row and the rows above and below straight from shared
-// memory and forms the x-neighbours by funnel shifts.  A unit whose 3x3
-// neighbourhood of units did not change during the last four subiterations
-// -- one of each direction -- is a fixed point for the next one and is
-// skipped (a unit processed without a change wrote identical data to both
-// copies, so a skipped unit is current in both).  A
-// single band stops after four consecutive subiterations without a deletion
-// (a fixed point of N, S, E and W: the reference's result, whatever the
-// alignment).  Bands of one image run their iterations (N, S, E, W) in
-// lockstep, meeting after every kResPassesPerExchange-th one: then a band
-// writes its first and last `halo` core rows to global memory, meets the
-// other bands at a per-image counter, stops if no band's core changed in
-// that iteration, and otherwise reads its halo rows from its neighbours.
-// With halo = 4 rows per iteration of the period, wrong values entering at a
-// band's outer edge between two meetings (4 rows per iteration at most)
-// reach at most its halo rows; if an iteration before the meeting was
-// already a fixed point, the one at the meeting is too.
+// 2D image (dense).  The rows of the image, or of a box of it (core plus halo),
+// lie twice in shared memory (pass q reads one copy and writes the other) with
+// an odd pitch and zero words left and right of every row.  A pass hands units
+// (24 rows x 2, 4 or 8 words) to warps dynamically; units whose surroundings
+// did not change in the previous pass are skipped.  One box stops after a pass
+// without a deletion: a fixed point of N, S, E and W, the reference's result.
+// The boxes of a larger image meet after every few passes.
 //
 // 3D volume (dense boxes, word lists).  A box of the volume (rows x planes,
 // full width) lies once in shared memory.  Deletion never adds foreground,
@@ -65,51 +48,71 @@ __host__ __device__ inline size_t up16(size_t v) { return (v + 15) & ~size_t(15)
 }  // namespace
 
 // ------------------------------------------------------------ geometry ----
-#ifndef BGT_RES_LANE_ROWS
-#define BGT_RES_LANE_ROWS 1
-#endif
-constexpr int kLaneRows = BGT_RES_LANE_ROWS;  // rows of a 2D unit per lane (1 or 2)
-constexpr int kUnitRowsH = 32 * kLaneRows - 8, kUnitWordsH = 8;  // 2D unit (see the 2D section)
+constexpr int kUnitRows = 24;  // core rows of a 2D unit (see the 2D section)
 
-// words of shared memory a 2D band of nrows rows needs: zero row, two row
-// copies and the activity record of its units
-__host__ __device__ inline size_t res_words2d(int W, int nrows)
+// Core words of the units of a 2D box of nrows rows of wl words: the width
+// whose pass is shortest when every unit is active.  A unit of UW words costs
+// UW + 1 word steps (one for its halo); a pass of few units takes as long as
+// the units of one warp one after the other, a pass of many is bound by the
+// ALU, which takes about kUnitLatency units in the time of one.  Widths of 8,
+// 4 and 2 words for all boxes took the mixed batch 1.20, 1.23 and 1.38 ms, 16
+// images of 1024^2 120, 116 and 121 us, a 200 x 160 image 21.1, 20.6 and 19.3 us.
+constexpr int kUnitLatency = 11;
+__host__ __device__ inline long long res_unit_cost(int nrows, int wl, int uw)
 {
-    const int wl = (W + 31) >> 5;
-    const int nch = (wl + kUnitWordsH - 1) / kUnitWordsH;
-    const int pp = (nch * kUnitWordsH + 2) | 1;
-    const int ns = (nrows + kUnitRowsH - 1) / kUnitRowsH;
-    return (size_t)pp * (1 + 2 * (size_t)nrows) + (size_t)ns * nch;
+    const long long units = (long long)((nrows + kUnitRows - 1) / kUnitRows) * ((wl + uw - 1) / uw);
+    const long long lat = (units + kWarps - 1) / kWarps * kUnitLatency * (uw + 1), alu = units * (uw + 1);
+    return lat > alu ? lat : alu;
+}
+__host__ __device__ inline int res_unit_words(int nrows, int wl)
+{
+    int best = 8;
+    for (int uw = 4; uw >= 2; uw /= 2)
+        if (res_unit_cost(nrows, wl, uw) < res_unit_cost(nrows, wl, best)) best = uw;
+    return best;
+}
+__host__ __device__ inline int res_pitch2d(int wl, int uw)
+{
+    return ((wl + uw - 1) / uw * uw + 2) | 1;  // zero word left, zero words right, odd
+}
+// words of shared memory a 2D box of nrows rows of wl words (halo included)
+// needs with units of uw words: zero row, two row copies and the activity
+// record of its units
+inline size_t res_words2d(int wl, int nrows, int uw)
+{
+    return (size_t)res_pitch2d(wl, uw) * (1 + 2 * (size_t)nrows) +
+           (size_t)((nrows + kUnitRows - 1) / kUnitRows) * ((wl + uw - 1) / uw);
 }
 
-// bytes of shared memory a box of ny x nz rows of wl words (halo included)
-// needs: its state, the rows' masks and, in the dense form, two more words
-// per word (the lists take what they find there, up to 44% non-empty words)
+// A 3D box of ny x nz rows of wl words (halo included) holds its state and the
+// rows' masks in shared memory, and lists of its non-empty words; the planner
+// leaves room for kListFill of the words.  A box with more non-empty words
+// than its lists hold goes over all of its words, at most kDenseWords per
+// thread, whose unions and deletions that thread keeps (in local memory).
 constexpr size_t kBoxListBytes = 4 + 4 + 4 + 4 + 2;  // list, candidate, union, deletions, active list
-__host__ __device__ inline size_t res_bytes3d(int wl, int ny, int nz)
-{
-    const size_t rows2 = (size_t)(ny + 2) * (nz + 2), words = rows2 * (wl + 1) + 1;
-    return up16(words * 4) + 2 * up16(rows2 * 4) + 2 * words * 4 + 80;
-}
+constexpr double kListFill = 0.25;
+constexpr int kDenseWords = 32;
 
 int res_smem_bytes() { return kSmemBytes; }
 
-int res_rows_fit2d(int W)
+double res_cost2d(int wl, int nrows) { return (double)res_unit_cost(nrows, wl, res_unit_words(nrows, wl)); }
+
+bool res_fits2d(int wl, int nrows)
 {
-    int lo = 0, hi = 32767;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) / 2;
-        if (res_words2d(W, mid) * 4 <= (size_t)kSmemBytes) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
+    // with units of any width: the boxes of an image differ in size (those at
+    // its edges have less halo), so a smaller one may take wider units
+    for (int uw = 2; uw <= 8; uw *= 2)
+        if (res_words2d(wl, nrows, uw) * 4 > (size_t)kSmemBytes) return false;
+    return true;
 }
 
 bool res_fits3d(int W, int ny, int nz)
 {
     const int wl = (W + 31) / 32;
+    const double rows2 = (double)(ny + 2) * (nz + 2), held = rows2 * (wl + 1) + 1, words = (double)wl * ny * nz;
     // words are indexed by 16 bits
-    return (long long)(ny + 2) * (nz + 2) * (wl + 1) < 65535 && res_bytes3d(wl, ny, nz) <= (size_t)kSmemBytes;
+    return held < 65535 && words <= (double)kDenseWords * kResThreads &&
+           held * 4 + rows2 * 8 + kListFill * words * kBoxListBytes + 128 <= (double)kSmemBytes;
 }
 
 // ------------------------------------------------------------ helpers -----
@@ -198,8 +201,8 @@ struct ResIO {
     bool pix;
 };
 
-// put(pos, word) for every word of the grid of rows whose first pixel row and
-// plane are y0, z0 (warps stay together: put may hold warp-wide votes; `live`
+// put(pos, word) for every word of the grid of rows whose first word, row and
+// plane are x0, y0, z0 (warps stay together: put may hold warp-wide votes; `live`
 // is false for lanes past the end, whose word is 0).  U words of a thread are
 // in flight at once: at 768 threads and 48 bytes per word of one-byte pixels,
 // two cover the latency of HBM.
@@ -222,23 +225,23 @@ __device__ __forceinline__ void res_load_loop(const WordWalk &walk, int n, Fetch
     }
 }
 template <class Put>
-__device__ __forceinline__ void res_load(const Inst &in, const ResIO &io, const WordWalk &walk, int n, int y0, int z0,
+__device__ __forceinline__ void res_load(const Inst &in, const ResIO &io, const WordWalk &walk, int n, int x0, int y0, int z0,
                                          Put put)
 {
     if (!io.pix) {
         const uint32_t *g = in.buf[0];
         const int H = in.H, P = in.P;
         res_load_loop<4>(walk, n, [&](bool live, const WordPos &q) {
-            return live ? __ldcg(g + ((size_t)(z0 + q.z) * H + (y0 + q.y)) * P + q.x) : 0u;
+            return live ? __ldcg(g + ((size_t)(z0 + q.z) * H + (y0 + q.y)) * P + (x0 + q.x)) : 0u;
         }, put);
         return;
     }
     const IODesc &d = *io.d;
     const int inW = d.inW, inH = d.inH, inD = d.inD;
     auto count = [&](bool live, const WordPos &q, uint32_t &off) {
-        const int y = y0 + q.y, z = z0 + q.z;
-        off = ((uint32_t)z * (uint32_t)inH + (uint32_t)y) * (uint32_t)inW + 32u * (uint32_t)q.x;
-        return live && y < inH && z < inD ? max(0, min(32, inW - 32 * q.x)) : 0;
+        const int x = 32 * (x0 + q.x), y = y0 + q.y, z = z0 + q.z;
+        off = ((uint32_t)z * (uint32_t)inH + (uint32_t)y) * (uint32_t)inW + (uint32_t)x;
+        return live && y < inH && z < inD ? max(0, min(32, inW - x)) : 0;
     };
     if (dtype_bytes(d.dtype) == 1) {
         const uint32_t neg = pixel_neg(d);
@@ -256,24 +259,27 @@ __device__ __forceinline__ void res_load(const Inst &in, const ResIO &io, const 
     }
 }
 
-// The way back for rows [y0, y0 + ny) of planes [z0, z0 + nz): row(y, z) = the
-// packed words of grid row y of grid plane z.
+// The way back for words [x0, x1) of rows [y0, y0 + ny) of planes [z0, z0 + nz):
+// row(y, z) = the packed words from x0 on of grid row y of grid plane z.
 template <class Row>
-__device__ __forceinline__ void res_store(const Inst &in, const ResIO &io, int ny, int nz, int y0, int z0, Row row)
+__device__ __forceinline__ void res_store(const Inst &in, const ResIO &io, int x0, int x1, int ny, int nz, int y0,
+                                          int z0, Row row)
 {
-    const int lane = threadIdx.x & 31, wl = (in.W + 31) >> 5;
+    const int lane = threadIdx.x & 31, wl = x1 - x0;
     const WordWalk walk(wl, ny);
     const int n = nz * ny * wl;
     if (!io.pix || !io.d->out) {
         uint32_t *g = in.buf[0];
         WordPos q = walk.first();
         for (int i = threadIdx.x; i < n; i += kResThreads, walk.next(q))
-            g[((size_t)(z0 + q.z) * in.H + (y0 + q.y)) * in.P + q.x] = row(q.y, q.z)[q.x];
+            g[((size_t)(z0 + q.z) * in.H + (y0 + q.y)) * in.P + x0 + q.x] = row(q.y, q.z)[q.x];
         return;
     }
     const IODesc &d = *io.d;
-    if (dtype_bytes(d.dtype) == 1) {
-        const uint32_t per = ((uint32_t)ny * (uint32_t)in.W + 31u) / 32u + 1u;  // chunks a plane's rows touch at most
+    const int np = min(in.W, 32 * x1) - 32 * x0;  // pixels per row
+    if (dtype_bytes(d.dtype) == 1 && np == in.W) {
+        // whole rows: one run of pixels per plane
+        const uint32_t per = ((uint32_t)ny * (uint32_t)in.W + 31u) / 32u + 1u;  // chunks it touches at most
         for (uint32_t i = threadIdx.x; i < per * (uint32_t)nz; i += kResThreads) {
             const uint32_t z = nz == 1 ? 0u : i / per;
             uint8_t *out = (uint8_t *)d.out + ((size_t)(z0 + (int)z) * in.H + y0) * in.W;
@@ -281,106 +287,73 @@ __device__ __forceinline__ void res_store(const Inst &in, const ResIO &io, int n
         }
         return;
     }
+    if (dtype_bytes(d.dtype) == 1) {
+        // parts of rows: a run per row (wl + 1 aligned chunks hold it)
+        const WordWalk chunks(wl + 1, ny);
+        WordPos q = chunks.first();
+        for (int i = threadIdx.x; i < nz * ny * (wl + 1); i += kResThreads, chunks.next(q)) {
+            uint8_t *out = (uint8_t *)d.out + ((size_t)(z0 + q.z) * in.H + (y0 + q.y)) * in.W + 32 * x0;
+            const uint32_t *s = row(q.y, q.z);
+            pixel_run_chunk(out, np, (uint32_t)q.x, s);
+        }
+        return;
+    }
     WordPos q = walk.first();
     for (int i = threadIdx.x; i - lane < n; i += kResThreads, walk.next(q)) {
         const bool live = i < n;
-        const uint32_t off = ((uint32_t)(z0 + q.z) * (uint32_t)in.H + (uint32_t)(y0 + q.y)) * (uint32_t)in.W + 32u * (uint32_t)q.x;
-        pixel_store_wide(d, off, live ? min(32, in.W - 32 * q.x) : 0, live ? row(q.y, q.z)[q.x] : 0u);
+        const int x = 32 * (x0 + q.x);
+        const uint32_t off = ((uint32_t)(z0 + q.z) * (uint32_t)in.H + (uint32_t)(y0 + q.y)) * (uint32_t)in.W + (uint32_t)x;
+        pixel_store_wide(d, off, live ? min(32, in.W - x) : 0, live ? row(q.y, q.z)[q.x] : 0u);
     }
 }
 
 // ------------------------------------------------------------ 2D ----------
 // A pass is one iteration (N, S, E, W) run on register tiles: a warp loads a
-// unit -- 24 core rows plus 4 halo rows above and below (lane = row) by 8
-// core words plus one halo word on either side -- from the pass-start copy,
-// runs the four subiterations in registers (rows above and below by
-// shuffles, x-neighbours by funnel shifts) and writes its core to the other
-// copy.  Wrong values entering at a unit's edge move one row (or bit) per
-// subiteration, so after four they reach only its halo.
-// BGT_RES_LANE_ROWS=2 builds units of 56 core rows, two adjacent rows per
-// lane (each other's vertical neighbours, half the shuffles per row, less
-// halo): measured slower on stroke images (1.13 against 1.06 ms for 512
-// images), as the larger units stay active for longer.
-constexpr int kUnitRows = 32 * kLaneRows - 2 * 4;  // core rows of a unit (K = 4)
-constexpr int kUnitWords = 8;                      // core words of a unit
-constexpr int kHaloLanes = 4 / kLaneRows;          // lanes holding the top (or bottom) halo rows
+// unit -- 24 core rows plus 4 halo rows above and below (lane = row) by UW
+// core words plus a halo word -- from the pass-start copy, runs the four
+// subiterations in registers (rows above and below by shuffles, x-neighbours
+// by funnel shifts) and writes its core to the other copy.  Wrong values
+// entering at a unit's edge move one row (or bit) per subiteration, so after
+// four they reach only its halo.  Of the words left and right of the unit
+// only the four pixels next to it matter, so one halo word holds both: its
+// low half is the right one's, its high half the left one's, and the words
+// form a ring (wrong values from the seam in its middle stay 12 bits away):
+// 9 word steps per subiteration for 8 core words instead of 10.
 
-// The rule on word j of a lane's two rows a (upper) and b (lower): o the
-// words, n/p the words after/before them (pass-start values).
-template <int DIR>
-__device__ __forceinline__ void word2d_pair(uint32_t oa, uint32_t na, uint32_t pa, uint32_t ob, uint32_t nb,
-                                            uint32_t pb, uint32_t &ra, uint32_t &rb)
+// One subiteration on the ring of UW core words and the halo word v[UW];
+// pairs of words empty in every lane are skipped.  The last subiteration
+// leaves the halo word alone.
+template <int UW, int DIR, bool LAST>
+__device__ __forceinline__ void subit2d_ring(uint32_t (&v)[UW + 1])
 {
-    const uint32_t xpa = at_xp1(oa, na), xma = at_xm1(oa, pa);
-    const uint32_t xpb = at_xp1(ob, nb), xmb = at_xm1(ob, pb);
-    uint32_t A[8], B[8];
-    A[0] = __shfl_up_sync(kFull, ob, 1);   // row above a: the lower row of the lane above
-    A[1] = __shfl_up_sync(kFull, xpb, 1);
-    A[7] = __shfl_up_sync(kFull, xmb, 1);
-    A[2] = xpa;
-    A[6] = xma;
-    A[4] = ob;
-    A[3] = xpb;
-    A[5] = xmb;
-    B[4] = __shfl_down_sync(kFull, oa, 1);  // row below b: the upper row of the lane below
-    B[3] = __shfl_down_sync(kFull, xpa, 1);
-    B[5] = __shfl_down_sync(kFull, xma, 1);
-    B[2] = xpb;
-    B[6] = xmb;
-    B[0] = oa;
-    B[1] = xpa;
-    B[7] = xma;
-    ra = keep2d<DIR>(oa, A);
-    rb = keep2d<DIR>(ob, B);
-}
-
-// One subiteration on the lane's two rows of S+2 words (words j0..j1-1 are
-// processed; the rest keep their values).  Words that are empty in both
-// rows of every lane are skipped.
-template <int S, int DIR, int J0, int J1>
-__device__ __forceinline__ void subit2d_pair(uint32_t (&a)[S + 2], uint32_t (&b)[S + 2])
-{
-    uint32_t pa = J0 > 0 ? a[J0 - 1] : 0u, pb = J0 > 0 ? b[J0 - 1] : 0u;
+    const uint32_t first = v[0];
+    uint32_t prev = v[UW];
 #pragma unroll
-    for (int j = J0; j < J1; j++) {
-        const uint32_t oa = a[j], ob = b[j];
-        const uint32_t na = j + 1 < S + 2 ? a[j + 1] : 0u, nb = j + 1 < S + 2 ? b[j + 1] : 0u;
-        if (__any_sync(kFull, (oa | ob) != 0u)) word2d_pair<DIR>(oa, na, pa, ob, nb, pb, a[j], b[j]);
-        pa = oa;
-        pb = ob;
+    for (int j = 0; j < UW; j += 2) {
+        const uint32_t o0 = v[j], o1 = v[j + 1], on = v[j + 2];
+        if (__any_sync(kFull, (o0 | o1) != 0u)) {
+            v[j] = word2d<DIR>(o0, o1, prev);
+            v[j + 1] = word2d<DIR>(o1, on, o0);
+        }
+        prev = o1;
+    }
+    if constexpr (!LAST) {
+        const uint32_t o = v[UW];
+        if (__any_sync(kFull, o != 0u)) v[UW] = word2d<DIR>(o, first, prev);
     }
 }
 
-// K subiterations from phase PH; the last one only on the core words.
-template <int K, int S, int PH, int I = 0>
-__device__ __forceinline__ void run_subits2d_pair(uint32_t (&a)[S + 2], uint32_t (&b)[S + 2])
-{
-    if constexpr (I + 1 < K) {
-        subit2d_pair<S, (PH + I) & 3, 0, S + 2>(a, b);
-        run_subits2d_pair<K, S, PH, I + 1>(a, b);
-    } else if constexpr (I + 1 == K) {
-        subit2d_pair<S, (PH + I) & 3, 1, S + 1>(a, b);
-    }
-}
-
-__host__ __device__ inline int res_pitch2d_tiles(int W)
-{
-    const int wl = (W + 31) >> 5;
-    const int nch = (wl + kUnitWords - 1) / kUnitWords;
-    return (nch * kUnitWords + 2) | 1;  // zero word left, zero words right, odd
-}
-
-struct Band2D {
-    uint32_t *zero;     // pp zero words
+struct Box2D {
+    uint32_t *zero;         // pp zero words
     uint32_t *buf0, *buf1;  // nrows x pp each: pass q reads buf[q & 1], writes buf[(q + 1) & 1]
-    int *until;         // [nstrips][nchunks]: the unit is processed while q <= until (a unit in
-                        // its 3x3 neighbourhood deleted something in the previous pass)
+    int *until;             // [nstrips][nchunks]: the unit is processed while q <= until (a unit in
+                            // its 3x3 neighbourhood deleted something in the previous pass)
     int pp, wl, nrows, nstrips, nchunks;
-    int a;              // image row of the band's first row in shared memory
-    int r0, r1;         // core rows (image coordinates)
+    int rlo, rhi;           // core rows and words, within the box
+    int wlo, whi;
 };
 
-// One pass q over the band's units.  A unit none of whose inputs for the
+// One pass q over the box's units.  A unit none of whose inputs for the
 // pass -- its core and the 4-pixel border bands of its 3x3 neighbours -- had
 // a deletion in the previous pass (one subiteration of every direction) is
 // skipped: that region is a fixed point, and a unit processed without a
@@ -388,8 +361,9 @@ struct Band2D {
 // extends `until` to q + 1 for itself and for each neighbour whose border
 // band the deletions reach (a reader in the same pass may see the new value:
 // it then processes a unit it could have skipped).
-// Returns this thread's deleted core bits (band core rows only).
-__device__ uint32_t res_pass2d(const Band2D &b, int q, int *take, unsigned long long *words)
+// Returns this thread's deleted core bits (of the box's core only).
+template <int UW>
+__device__ uint32_t res_pass2d(const Box2D &b, int q, int *take, unsigned long long *words)
 {
     const int lane = threadIdx.x & 31;
     const uint32_t *IN = (q & 1) ? b.buf1 : b.buf0;
@@ -401,39 +375,33 @@ __device__ uint32_t res_pass2d(const Band2D &b, int q, int *take, unsigned long 
         if (u >= nunits) break;
         if (b.until[u] < q) continue;
         const int s = u / b.nchunks, c = u - s * b.nchunks;
-        const int x0 = 1 + kUnitWords * c;
-        const int rbase = kUnitRows * s - 4 + kLaneRows * lane;  // band row of the lane's first row
-        uint32_t v[kLaneRows][kUnitWords + 2];
-        const uint32_t *in[kLaneRows];
-        bool valid[kLaneRows];
+        const int x0 = 1 + UW * c;
+        const int r = kUnitRows * s - 4 + lane;  // box row of this lane
+        const bool valid = r >= 0 && r < b.nrows;
+        const uint32_t *in = (valid ? IN + (size_t)r * b.pp : b.zero) + x0;
+        uint32_t v[UW + 1];
 #pragma unroll
-        for (int i = 0; i < kLaneRows; i++) {
-            const int r = rbase + i;
-            valid[i] = r >= 0 && r < b.nrows;
-            in[i] = valid[i] ? IN + (size_t)r * b.pp : b.zero;
-#pragma unroll
-            for (int k = 0; k < kUnitWords + 2; k++) v[i][k] = in[i][x0 - 1 + k];
-        }
-        if constexpr (kLaneRows == 2) run_subits2d_pair<4, kUnitWords, 0>(v[0], v[1]);
-        else run_subits2d<4, kUnitWords, 0>(v[0]);
-        const bool core_lane = lane >= kHaloLanes && lane < 32 - kHaloLanes;
+        for (int k = 0; k < UW; k++) v[k] = in[k];
+        v[UW] = (in[-1] & 0xFFFF0000u) | (in[UW] & 0xFFFFu);
+        subit2d_ring<UW, 0, false>(v);
+        subit2d_ring<UW, 1, false>(v);
+        subit2d_ring<UW, 2, false>(v);
+        subit2d_ring<UW, 3, true>(v);
         uint32_t chg = 0, lft = 0, rgt = 0;
+        if (valid && lane >= 4 && lane < 28) {
+            uint32_t *out = OUT + (size_t)r * b.pp + x0;
+            const int klo = b.wlo - UW * c, khi = b.whi - UW * c;
+            uint32_t cc = 0;
 #pragma unroll
-        for (int i = 0; i < kLaneRows; i++) {
-            if (!(valid[i] && core_lane)) continue;
-            uint32_t *out = OUT + (size_t)(rbase + i) * b.pp;
-            uint32_t ci = 0;
-#pragma unroll
-            for (int k = 0; k < kUnitWords; k++) {
-                const uint32_t d = v[i][1 + k] ^ in[i][x0 + k];
-                ci |= d;
-                if (k == 0) lft |= d & 0xFu;                     // within 4 pixels of the left edge
-                if (k == kUnitWords - 1) rgt |= d & 0xF0000000u;  // ... of the right edge
-                out[x0 + k] = v[i][1 + k];
+            for (int k = 0; k < UW; k++) {
+                const uint32_t d = v[k] ^ in[k];
+                chg |= d;
+                if (k >= klo && k < khi) cc |= d;
+                if (k == 0) lft = d & 0xFu;                 // within 4 pixels of the left edge
+                if (k == UW - 1) rgt = d & 0xF0000000u;     // ... of the right edge
+                out[k] = v[k];
             }
-            chg |= ci;
-            const int gy = b.a + rbase + i;
-            if (gy >= b.r0 && gy < b.r1) core |= ci;
+            if (r >= b.rlo && r < b.rhi) core |= cc;
         }
         // The next pass of a neighbour depends on this unit only through the
         // 4 pixels next to their common border (four subiterations reach 4
@@ -443,8 +411,7 @@ __device__ uint32_t res_pass2d(const Band2D &b, int q, int *take, unsigned long 
         if (m_any) {
             const unsigned m_l = __ballot_sync(kFull, lft != 0u), m_r = __ballot_sync(kFull, rgt != 0u);
             // lanes holding the first and last 4 core rows
-            constexpr unsigned band_top = ((1u << kHaloLanes) - 1u) << kHaloLanes;
-            constexpr unsigned band_bot = ((1u << kHaloLanes) - 1u) << (32 - 2 * kHaloLanes);
+            constexpr unsigned band_top = 0xF0u, band_bot = 0x0F000000u;
             if (lane < 9) {
                 const int dy = lane / 3 - 1, dx = lane % 3 - 1;
                 const unsigned rows = dy < 0 ? band_top : dy > 0 ? band_bot : ~0u;
@@ -455,26 +422,45 @@ __device__ uint32_t res_pass2d(const Band2D &b, int q, int *take, unsigned long 
             }
         }
         if (lane == 0)
-            *words += (unsigned long long)min(kUnitRows, b.nrows - kUnitRows * s) *
-                      min(kUnitWords, b.wl - kUnitWords * c);
+            *words += (unsigned long long)min(kUnitRows, b.nrows - kUnitRows * s) * min(UW, b.wl - UW * c);
     }
     return core;
 }
 
+// Bound: in a large batch the ALU (13 half-rate operations per word step) and
+// the passes' tails; for a lone image the latency of its passes (1.5 us each
+// in a box of a 512^2 image) and meetings (4 us with the exchange).  Boxes of
+// rows and words against bands of full-width rows: a 4096^2 image 127 -> 102 us,
+// a 1501 x 1003 float image 154 -> 92 us, a 512^2 one 59 -> 43 us, the mixed
+// batch (with the exchange flattened over the threads) 1.24 -> 1.19 ms.
+//
+// One image, or one box of it: rows [r0, r1) of words [c0, c1) are the core;
+// `halo` rows above and below it and one word left and right (clamped to the
+// image) are held too.  Boxes run passes in lockstep and meet after every
+// halo / 4-th one: then a box writes the edge of its core to global memory,
+// meets the others, stops if no box's core changed in that pass, and reads
+// its halo.  Wrong values entering at a box's outer edge move at most 4 rows
+// or pixels per pass, so halo rows (and the 32 pixels of a word, for up to 8
+// passes) keep the core exact; if a pass before the meeting was a fixed point
+// already, the one at the meeting is too.
+template <int UW>
 __device__ void res_run2d(Inst &in, const ResIO &io, const ResItem &it, uint32_t *sm, ResSched *S, int *take)
 {
     __shared__ int s_flag;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    Band2D b;
-    b.wl = (in.W + 31) >> 5;
-    b.pp = res_pitch2d_tiles(in.W);
-    b.nchunks = (b.wl + kUnitWords - 1) / kUnitWords;
-    b.r0 = it.r0;
-    b.r1 = it.r1;
-    b.a = max(0, it.r0 - it.halo);
-    const int bend = min(in.H, it.r1 + it.halo);
-    b.nrows = bend - b.a;
+    const int lane = threadIdx.x & 31;
+    const int wl_img = (in.W + 31) >> 5;
+    const int a = max(0, it.r0 - it.halo), e0 = it.halo ? max(0, it.c0 - 1) : 0;  // first row and word held
+    const int aend = min(in.H, it.r1 + it.halo), e1 = it.halo ? min(wl_img, it.c1 + 1) : wl_img;
+    Box2D b;
+    b.wl = e1 - e0;
+    b.pp = res_pitch2d(b.wl, UW);
+    b.nchunks = (b.wl + UW - 1) / UW;
+    b.nrows = aend - a;
     b.nstrips = (b.nrows + kUnitRows - 1) / kUnitRows;
+    b.rlo = it.r0 - a;
+    b.rhi = it.r1 - a;
+    b.wlo = it.c0 - e0;
+    b.whi = it.c1 - e0;
     b.zero = sm;
     b.buf0 = sm + b.pp;
     b.buf1 = b.buf0 + (size_t)b.nrows * b.pp;
@@ -482,7 +468,7 @@ __device__ void res_run2d(Inst &in, const ResIO &io, const ResItem &it, uint32_t
     const int pp = b.pp;
     const int nunits = b.nstrips * b.nchunks;
 
-    // zero row and row copies (their words left and right of the image stay zero)
+    // zero row and row copies (their words left and right of the box stay zero)
     {
         const int total = pp * (1 + 2 * b.nrows);
         for (int i = threadIdx.x; i < total / 4; i += kResThreads)
@@ -492,45 +478,46 @@ __device__ void res_run2d(Inst &in, const ResIO &io, const ResItem &it, uint32_t
     for (int i = threadIdx.x; i < nunits; i += kResThreads) b.until[i] = -1;
     if (threadIdx.x < 2) take[threadIdx.x] = 0;
     __syncthreads();
-    res_load(in, io, WordWalk(b.wl, b.nrows), b.nrows * b.wl, b.a, 0, [&](bool, const WordPos &q, uint32_t v) {
+    res_load(in, io, WordWalk(b.wl, b.nrows), b.nrows * b.wl, e0, a, 0, [&](bool, const WordPos &q, uint32_t v) {
         if (!v) return;
         const int w = q.y * pp + q.x + 1;
         b.buf0[w] = v;
         b.buf1[w] = v;
         // units holding foreground start active
-        b.until[(q.y / kUnitRows) * b.nchunks + q.x / kUnitWords] = 0;
+        b.until[(q.y / kUnitRows) * b.nchunks + q.x / UW] = 0;
     });
     __syncthreads();
 
     int result = 0;  // 1 converged, -1 pass cap or failed wait
     MeetState meet;
     unsigned long long words = 0;
-    int q = 0;
+    const int period = it.halo / 4;
+    int q = 0, since = 0, e = 0;  // pass, passes since the last meeting, meetings
     for (;; q++) {
         // the counter of this pass was cleared during the previous one;
         // clear the next one's (nobody uses it before the barrier below)
         if (threadIdx.x == 0) take[(q + 1) & 1] = 0;
-        const uint32_t core = res_pass2d(b, q, take + (q & 1), &words);
+        const uint32_t core = res_pass2d<UW>(b, q, take + (q & 1), &words);
         const bool any = __syncthreads_or(core != 0u);
         if (it.bands == 1) {
             if (!any) {
                 result = 1;
                 break;
             }
-        } else if (q % kResPassesPerExchange == kResPassesPerExchange - 1) {
-            // end of pass q (state in buf[(q+1)&1]), the last of an exchange
-            // period: trade boundary rows with the neighbouring bands
-            const int h = it.halo;
-            const int e = q / kResPassesPerExchange;  // exchange index
+        } else if (++since == period) {
+            since = 0;
             uint32_t *cur = (q & 1) ? b.buf0 : b.buf1;
-            uint32_t *gx = in.buf[(e + 1) & 1];  // buf[0] holds the start state other bands may still load
-            for (int k = warp; k < 2 * h; k += kWarps) {
-                const bool top = k < h;
-                if (top ? it.band == 0 : it.band + 1 == it.bands) continue;
-                const int gy = top ? b.r0 + k : b.r1 - 2 * h + k;
-                const uint32_t *srow = cur + (size_t)(gy - b.a) * pp;
-                uint32_t *grow = gx + (size_t)gy * in.P;
-                for (int w = lane; w < b.wl; w += 32) grow[w] = srow[w + 1];
+            uint32_t *gx = in.buf[(e + 1) & 1];  // buf[0] may hold the start state other boxes still load
+            // the edge of the core: its first and last `halo` rows, its first and last words
+            const int cw = it.c1 - it.c0, ch = it.r1 - it.r0;
+            const int top = it.r0 > 0 ? min(it.halo, ch) : 0, bot = it.r1 < in.H ? min(it.halo, ch - top) : 0;
+            for (int i = threadIdx.x; i < (top + bot) * cw; i += kResThreads) {
+                const int r = i / cw, w = it.c0 + i - r * cw, y = r < top ? it.r0 + r : it.r1 - bot + (r - top);
+                gx[(size_t)y * in.P + w] = cur[(y - a) * pp + 1 + w - e0];
+            }
+            for (int i = threadIdx.x; i < 2 * ch; i += kResThreads) {
+                const int y = it.r0 + (i >> 1), w = (i & 1) ? it.c1 - 1 : it.c0;
+                if ((i & 1) ? it.c1 < wl_img : it.c0 > 0) gx[(size_t)y * in.P + w] = cur[(y - a) * pp + 1 + w - e0];
             }
             __syncthreads();
             if (threadIdx.x == 0) {
@@ -543,28 +530,28 @@ __device__ void res_run2d(Inst &in, const ResIO &io, const ResItem &it, uint32_t
                 result = f == 0 ? 1 : -1;
                 break;
             }
-            // halo rows: the neighbours' boundary core rows after pass q
-            const int ntop = b.r0 - b.a, nh = ntop + (bend - b.r1);
-            uint32_t hc = 0;
-            for (int k = warp; k < nh; k += kWarps) {
-                const int r = k < ntop ? k : (b.r1 - b.a) + (k - ntop);
-                const uint32_t *grow = gx + (size_t)(b.a + r) * in.P;
-                uint32_t *srow = cur + (size_t)r * pp;
-                for (int w = lane; w < b.wl; w += 32) {
-                    const uint32_t v = __ldcg(grow + w);
-                    hc |= v ^ srow[w + 1];
-                    srow[w + 1] = v;
-                }
+            e++;
+            // the halo: a word that changed makes its unit, and the units it is within 4 pixels of, active
+            auto take_over = [&](int y, int w, uint32_t v) {
+                const int r = y - a, x = w - e0;
+                uint32_t *p = cur + r * pp + 1 + x;
+                if (*p == v) return;
+                *p = v;
+                const int s = r / kUnitRows, c = x / UW, rr = r - s * kUnitRows, cc = x - c * UW;
+                for (int dy = rr < 4 && s > 0 ? -1 : 0; dy <= (rr >= kUnitRows - 4 && s + 1 < b.nstrips ? 1 : 0); dy++)
+                    for (int dx = cc == 0 && c > 0 ? -1 : 0; dx <= (cc == UW - 1 && c + 1 < b.nchunks ? 1 : 0); dx++)
+                        b.until[(s + dy) * b.nchunks + c + dx] = q + 1;
+            };
+            const int htop = it.r0 - a, hrows = htop + (aend - it.r1);
+            for (int i = threadIdx.x; i < hrows * b.wl; i += kResThreads) {
+                const int r = i / b.wl, w = e0 + i - r * b.wl, y = r < htop ? a + r : it.r1 + (r - htop);
+                take_over(y, w, __ldcg(gx + (size_t)y * in.P + w));
             }
-            if (__syncthreads_or(hc != 0u)) {
-                // units within reach of the halo rows go on next pass
-                for (int u = threadIdx.x; u < nunits; u += kResThreads) {
-                    const int st = u / b.nchunks;
-                    const int ga = b.a + kUnitRows * st - kUnitRows, gb = b.a + kUnitRows * st + 2 * kUnitRows;
-                    if (ga < b.r0 || gb > b.r1) b.until[u] = q + 1;
-                }
-                __syncthreads();
+            for (int i = threadIdx.x; i < 2 * ch; i += kResThreads) {
+                const int y = it.r0 + (i >> 1), w = (i & 1) ? it.c1 : e0;
+                if ((i & 1) ? e1 > it.c1 : e0 < it.c0) take_over(y, w, __ldcg(gx + (size_t)y * in.P + w));
             }
+            __syncthreads();
         }
         if (q >= in.pass_cap) {
             if (threadIdx.x == 0) atomicOr(&S->status, kErrPassLimit);
@@ -572,11 +559,11 @@ __device__ void res_run2d(Inst &in, const ResIO &io, const ResItem &it, uint32_t
             break;
         }
     }
-    // the converged core rows (in buf[(q+1)&1])
+    // the converged core (in buf[(q+1)&1])
     __syncthreads();
-    const uint32_t *fin = ((q & 1) ? b.buf0 : b.buf1) + (size_t)(b.r0 - b.a) * pp + 1;
-    res_store(in, io, b.r1 - b.r0, 1, b.r0, 0, [&](int y, int) { return fin + (size_t)y * pp; });
-    if (lane == 0 && words) atomicAdd(&in.work_words, words);  // core words per pass (one iteration)
+    const uint32_t *fin = ((q & 1) ? b.buf0 : b.buf1) + (size_t)b.rlo * pp + 1 + b.wlo;
+    res_store(in, io, it.c0, it.c1, it.r1 - it.r0, 1, it.r0, 0, [&](int y, int) { return fin + (size_t)y * pp; });
+    if (lane == 0 && words) atomicAdd(&in.work_words, words);  // words per pass (one iteration)
     if (threadIdx.x == 0) {
         if (it.band == 0) in.passes_run = q + 1;
         if (result < 0) atomicMin(&in.converged, -1);
@@ -728,7 +715,7 @@ __device__ void res_run3d(Inst &in, const ResIO &io, const ResItem &it, uint8_t 
         return max(max(max(it.c0 - y, y - it.c1 + 1), max(it.r0 - z, z - it.r1 + 1)), 0);
     };
     auto index_of = [&](const WordPos &q) { return ((q.z + 1) * ny2 + q.y + 1) * b.p + 1 + q.x; };
-    res_load(in, io, walk, nbox, y0, z0, [&](bool, const WordPos &q, uint32_t v) {
+    res_load(in, io, walk, nbox, 0, y0, z0, [&](bool, const WordPos &q, uint32_t v) {
         const int d = dist_of(q), idx = v ? index_of(q) : 0;
         if (v) b.state[idx] = v;
         const int pos = warp_append(v != 0u && d <= 5, &s_n[0]);
@@ -737,12 +724,11 @@ __device__ void res_run3d(Inst &in, const ResIO &io, const ResItem &it, uint8_t 
     __syncthreads();
     const int nl = s_n[0];
     MeetState meet;
-    // more non-empty words than the lists hold: go over all words of the box,
-    // with the union and the deletions stored per word
+    // more non-empty words than the lists hold: go over all words of the box
     const bool dense = off + (size_t)nl * kBoxListBytes + 64 > (size_t)kSmemBytes;
     b.cidx = list + nl;
-    b.cU = dense ? list : b.cidx + nl;
-    b.cdel = b.cU + (dense ? nwords : nl);
+    b.cU = b.cidx + nl;
+    b.cdel = b.cU + nl;
     uint16_t *const alist = reinterpret_cast<uint16_t *>(b.cdel + nl);
     for (int r = threadIdx.x; r < rows2; r += kResThreads) act[r] = kFull;
     __syncthreads();
@@ -858,58 +844,58 @@ __device__ void res_run3d(Inst &in, const ResIO &io, const ResItem &it, uint8_t 
                 changed(ent_idx(e), ent_col(e), msg);
             }
         } else {
+            uint32_t un[kDenseWords], del[kDenseWords];  // of this thread's words
             WordPos q = walk.first();
-            for (int i = threadIdx.x; i < nbox; i += kResThreads, walk.next(q)) {
-                const int idx = index_of(q), d = dist_of(q);
-                const uint32_t *s = b.state + idx;
-                uint32_t un = 0, du = 0;
+            int k = 0;
+            for (int i = threadIdx.x; i < nbox; i += kResThreads, walk.next(q), k++) {
+                const int d = dist_of(q);
+                const uint32_t *s = b.state + index_of(q);
+                un[k] = del[k] = 0;
                 if (d <= 5 && *s && ((act[(q.z + 1) * ny2 + q.y + 1] >> (q.x >> xs)) & 1u)) {
                     uint32_t g[27];
                     box_window(s, b.p, b.ps, g);
-                    du = rule3d<0>(g) & g[13];
-                    un = (du | rule3d<1>(g) | rule3d<2>(g) | rule3d<3>(g) | rule3d<4>(g) | rule3d<5>(g)) & g[13];
+                    const uint32_t du = rule3d<0>(g) & g[13];
+                    del[k] = du;
+                    un[k] = (du | rule3d<1>(g) | rule3d<2>(g) | rule3d<3>(g) | rule3d<4>(g) | rule3d<5>(g)) & g[13];
                     words += d == 0;
                     entries++;
                 }
-                b.cU[idx] = un;
-                b.cdel[idx] = du;
             }
             __syncthreads();
 #pragma unroll 1
             for (int j = 0; j < 6; j++) {
                 // deletions of subiteration j were found: apply them, then find the next one's
                 q = walk.first();
-                for (int i = threadIdx.x; i < nbox; i += kResThreads, walk.next(q)) {
-                    const int idx = index_of(q);
-                    const uint32_t del = b.cdel[idx];
-                    if (del) b.state[idx] &= ~del;
-                }
+                k = 0;
+                for (int i = threadIdx.x; i < nbox; i += kResThreads, walk.next(q), k++)
+                    if (del[k]) b.state[index_of(q)] &= ~del[k];
                 __syncthreads();
                 if (j == 5) break;
                 q = walk.first();
-                for (int i = threadIdx.x; i < nbox; i += kResThreads, walk.next(q)) {
-                    const int idx = index_of(q), d = dist_of(q);
-                    const uint32_t cand = b.state[idx] & b.cU[idx];
-                    uint32_t del = 0;
-                    if (cand && d <= 4 - j) {
-                        uint32_t g[27];
-                        box_window(b.state + idx, b.p, b.ps, g);
-                        del = cand & (j == 0   ? rule3d<1>(g)
-                                      : j == 1 ? rule3d<2>(g)
-                                      : j == 2 ? rule3d<3>(g)
-                                      : j == 3 ? rule3d<4>(g)
-                                               : rule3d<5>(g));
-                        words += d == 0;
-                    }
-                    b.cdel[idx] = del;
+                k = 0;
+                for (int i = threadIdx.x; i < nbox; i += kResThreads, walk.next(q), k++) {
+                    del[k] = 0;
+                    if (!un[k] || dist_of(q) > 4 - j) continue;
+                    const uint32_t *s = b.state + index_of(q);
+                    const uint32_t cand = *s & un[k];
+                    if (!cand) continue;
+                    uint32_t g[27];
+                    box_window(s, b.p, b.ps, g);
+                    del[k] = cand & (j == 0   ? rule3d<1>(g)
+                                     : j == 1 ? rule3d<2>(g)
+                                     : j == 2 ? rule3d<3>(g)
+                                     : j == 3 ? rule3d<4>(g)
+                                              : rule3d<5>(g));
+                    words += dist_of(q) == 0;
                 }
                 __syncthreads();
             }
             // only voxels of the union were deleted: a word changed when it lost some of its union
             q = walk.first();
-            for (int i = threadIdx.x; i < nbox; i += kResThreads, walk.next(q)) {
+            k = 0;
+            for (int i = threadIdx.x; i < nbox; i += kResThreads, walk.next(q), k++) {
                 const int idx = index_of(q);
-                if (!(b.cU[idx] & ~b.state[idx]) || dist_of(q) != 0) continue;
+                if (!(un[k] & ~b.state[idx]) || dist_of(q) != 0) continue;
                 core = true;
                 changed((uint32_t)idx, (uint32_t)(q.x >> xs), msg);
             }
@@ -933,10 +919,10 @@ __device__ void res_run3d(Inst &in, const ResIO &io, const ResItem &it, uint8_t 
                 result = f == 0 ? 1 : -1;
                 break;
             }
-            // three warps per neighbouring box take over its messages
+            // kWarps / 8 warps per neighbouring box take over its messages
             const int k8 = warp & 7, k9 = k8 < 4 ? k8 : k8 + 1;
             const int nbz = bz + k9 / 3 - 1, nby = by + k9 % 3 - 1;
-            if (nbz >= 0 && nbz < gz && nby >= 0 && nby < gy) {
+            if (warp < kWarps / 8 * 8 && nbz >= 0 && nbz < gz && nby >= 0 && nby < gy) {
                 const int nb = nbz * gy + nby;
                 const uint2 *m = in.res_msg + ((size_t)(iter & 1) * it.bands + nb) * in.res_stride;
                 const int k0 = (warp >> 3) * 32 + lane;
@@ -980,7 +966,7 @@ __device__ void res_run3d(Inst &in, const ResIO &io, const ResItem &it, uint8_t 
     }
     __syncthreads();
     // the converged core
-    res_store(in, io, it.c1 - it.c0, it.r1 - it.r0, it.c0, it.r0, [&](int y, int z) {
+    res_store(in, io, 0, wl, it.c1 - it.c0, it.r1 - it.r0, it.c0, it.r0, [&](int y, int z) {
         return b.state + ((z + it.r0 - z0 + 1) * ny2 + (y + it.c0 - y0 + 1)) * b.p + 1;
     });
     words = __reduce_add_sync(kFull, words);
@@ -1041,9 +1027,17 @@ __global__ void __launch_bounds__(kResThreads, kResCtasPerSm)
         Inst &in = insts[it.inst];
         const long long t0 = (long long)globaltimer();
         const ResIO io{ios ? ios + it.inst : &one, pix};
-        if (in.dims == 2)
-            res_run2d(in, io, it, reinterpret_cast<uint32_t *>(res_smem), S, s_take);
-        else
+        if (in.dims == 2) {
+            const int wl = (in.W + 31) >> 5;
+            const int nw = it.halo ? min(wl, it.c1 + 1) - max(0, it.c0 - 1) : wl;
+            const int nr = min(in.H, it.r1 + it.halo) - max(0, it.r0 - it.halo);
+            uint32_t *sm = reinterpret_cast<uint32_t *>(res_smem);
+            switch (res_unit_words(nr, nw)) {
+            case 2: res_run2d<2>(in, io, it, sm, S, s_take); break;
+            case 4: res_run2d<4>(in, io, it, sm, S, s_take); break;
+            default: res_run2d<8>(in, io, it, sm, S, s_take); break;
+            }
+        } else
             res_run3d(in, io, it, res_smem, S);
         if (threadIdx.x == 0) trace[k] = ResTrace{t0, (long long)globaltimer(), res_smid(), 0};
     }

@@ -1,13 +1,13 @@
-"""GPU parity of the resident kernel's 3D boxes (begputhinning_b200/csrc/resident.cu)
+"""GPU parity of the resident kernel's boxes (begputhinning_b200/csrc/resident.cu)
 against the oracle: one box, cuts along y, along z and along both, boxes whose
 cores are as thin as the halo, ragged and word-boundary widths, change masks
 with more than one word per column, and boxes with more non-empty words than
-their lists hold."""
+their lists hold; images cut along rows, along words and along both."""
 import numpy as np
 import pytest
 
 from oracle import pyoracle as po
-from tests.helpers import blobs3d, random3d
+from tests.helpers import blobs2d, blobs3d, random2d, random3d
 
 pytestmark = pytest.mark.gpu
 
@@ -56,3 +56,16 @@ def test_boxes_dense(ctx, density):
     for g, v, s in zip(got, vols, stats):
         assert s["converged"] == 1
         assert np.array_equal(g, po.thin3d(v)[0]), f"{plans}"
+
+
+@pytest.mark.parametrize("box_words", [30, 200, 1000000])
+@pytest.mark.parametrize("shape", [(24, 300), (75, 260), (200, 129), (333, 1001), (97, 4000), (1500, 40)])
+def test_image_boxes(ctx, shape, box_words, monkeypatch):
+    monkeypatch.setenv("BGT_RES2D_BOX_WORDS", str(box_words))
+    rng = np.random.default_rng(sum(shape))
+    for v in (random2d(rng, *shape, 0.5), blobs2d(rng, *shape, max(2, np.prod(shape) // 3000), rmax=14),
+              np.ones(shape, np.uint8)):
+        (got,), (plan,), (stat,) = _thin(ctx, [v])
+        want, _ = po.thin2d(v)
+        assert plan[0] and stat["converged"] == 1
+        assert np.array_equal(got, want), f"plan {plan}: {(got != want).sum()} pixels differ"
