@@ -115,7 +115,8 @@ extern "C" int bgt_segments3d_device(bgt_ctx *c, int dtype, const void *d_vol, i
 //  * kept segments are renumbered in order (prefix sums of the keep flags
 //    and of the kept point counts give each one its CSR slot);
 //  * each kept segment is smoothed by one thread with the reference's float
-//    running sum (integer coordinates added to and subtracted from it one at
+//    running sum (the tail of segments_graph.cu does it point by point where
+//    that sum is exact) (integer coordinates added to and subtracted from it one at
 //    a time, IEEE round-to-nearest adds and divide by float(count)), so the
 //    float outputs are bit-identical.  A negative smoothing_span is treated
 //    as 0 (the reference indexes out of bounds there).
@@ -271,8 +272,14 @@ static int prune_smooth_device(bgt_ctx *c, const DevSegs &s, int dims, int max_s
     return BGT_OK;
 }
 
-// Thin the padded image with the engine and extract segments on the device.
-static int centerline_segments(bgt_ctx *c, int dims, int dtype, const void *in, int w, int h, int d, DevSegs *ds)
+// The whole path: thin the padded image, extract its segments, prune, smooth
+// and flatten.  The resident kernel and the segment kernel with its centreline
+// tail run back to back and everything the host needs comes with one copy;
+// images beyond that kernel (and spans whose running sums could round) take
+// the extraction and prune_smooth_device one after the other.
+static int centerline(bgt_ctx *c, int dims, int dtype, const void *in, int w, int h, int d, int max_segment_length,
+                      int smoothing_span, float **ox, float **oy, float **oz, unsigned int **oidx,
+                      unsigned int *nsegs)
 {
     if (!c || !in) return fail(BGT_ERR_ARG, "null argument");
     const size_t es = dtype_size(dtype);
@@ -301,10 +308,52 @@ static int centerline_segments(bgt_ctx *c, int dims, int dtype, const void *in, 
     if (rc == BGT_OK) rc = bgt_batch_set_io(b, 0, dtype, d_in, nullptr);
     if (rc == BGT_OK) rc = batch_set_input_extent(b, 0, w, h, d);
     if (rc == BGT_OK) rc = bgt_batch_run(b, 0, 0);
-    if (rc == BGT_OK) rc = batch_check(b);
     if (rc != BGT_OK) return rc;
-    const Inst &inst = b->h[0];
-    return segments_device_arrays(c, dims, inst.buf[0], pw, ph, pd, inst.P, ds);
+    const uint32_t *packed = b->h[0].buf[0];
+    const int P = b->h[0].P;
+    SegTail tail;
+    tail.max_segment_length = max_segment_length;
+    tail.span = smoothing_span;
+    batch_status_words(b, tail.check);
+    SegResult r;
+    rc = 1;
+    if ((long long)pw * ph * pd < (1LL << 32) - 1 && !getenv("BGT_SEGMENTS_PIXEL_WALK"))
+        rc = segments_graph(c, dims, packed, pw, ph, pd, P, &tail, &r);
+    if (rc == BGT_OK && r.checked) return batch_status(r.checked);
+    if (rc == 1) {
+        rc = batch_check(b);
+        DevSegs ds;
+        if (rc == BGT_OK) rc = segments_device_arrays(c, dims, packed, pw, ph, pd, P, &ds);
+        if (rc == BGT_OK)
+            rc = prune_smooth_device(c, ds, dims, max_segment_length, smoothing_span, ox, oy, oz, oidx, nsegs);
+        return rc;
+    }
+    if (rc != BGT_OK) return rc;
+    const size_t n = (size_t)r.npts;
+    float *X = (float *)malloc(sizeof(float) * std::max<size_t>(1, n));
+    float *Y = (float *)malloc(sizeof(float) * std::max<size_t>(1, n));
+    float *Z = dims == 3 ? (float *)malloc(sizeof(float) * std::max<size_t>(1, n)) : nullptr;
+    unsigned *I = (unsigned *)malloc(sizeof(unsigned) * ((size_t)r.nseg + 1));
+    if (!X || !Y || !I || (dims == 3 && !Z)) {
+        free(X);
+        free(Y);
+        free(Z);
+        free(I);
+        return fail(BGT_ERR_NOMEM, "host allocation of centreline arrays");
+    }
+    if (n > 0) {
+        memcpy(X, r.fx, n * 4);
+        memcpy(Y, r.fy, n * 4);
+        if (Z) memcpy(Z, r.fz, n * 4);
+    }
+    if (r.nseg > 0) memcpy(I, r.idx, (size_t)r.nseg * 4);
+    I[r.nseg] = (unsigned)n;
+    *ox = X;
+    *oy = Y;
+    if (oz) *oz = Z;
+    *oidx = I;
+    *nsegs = (unsigned)r.nseg;
+    return BGT_OK;
 }
 
 extern "C" int bgt_centerline2d(bgt_ctx *c, int dtype, const void *in, int w, int h, int max_segment_length,
@@ -312,11 +361,8 @@ extern "C" int bgt_centerline2d(bgt_ctx *c, int dtype, const void *in, int w, in
                                 unsigned int *nsegs)
 {
     if (!out_x || !out_y || !out_idx || !nsegs) return fail(BGT_ERR_ARG, "null output");
-    DevSegs ds;
-    int rc = centerline_segments(c, 2, dtype, in, w, h, 1, &ds);
-    if (rc == BGT_OK)
-        rc = prune_smooth_device(c, ds, 2, max_segment_length, smoothing_span, out_x, out_y, nullptr, out_idx, nsegs);
-    return rc;
+    return centerline(c, 2, dtype, in, w, h, 1, max_segment_length, smoothing_span, out_x, out_y, nullptr, out_idx,
+                      nsegs);
 }
 
 extern "C" int bgt_centerline3d(bgt_ctx *c, int dtype, const void *in, int w, int h, int d, int max_segment_length,
@@ -324,9 +370,6 @@ extern "C" int bgt_centerline3d(bgt_ctx *c, int dtype, const void *in, int w, in
                                 unsigned int **out_idx, unsigned int *nsegs)
 {
     if (!out_x || !out_y || !out_z || !out_idx || !nsegs) return fail(BGT_ERR_ARG, "null output");
-    DevSegs ds;
-    int rc = centerline_segments(c, 3, dtype, in, w, h, d, &ds);
-    if (rc == BGT_OK)
-        rc = prune_smooth_device(c, ds, 3, max_segment_length, smoothing_span, out_x, out_y, out_z, out_idx, nsegs);
-    return rc;
+    return centerline(c, 3, dtype, in, w, h, d, max_segment_length, smoothing_span, out_x, out_y, out_z, out_idx,
+                      nsegs);
 }

@@ -1154,22 +1154,35 @@ extern "C" int bgt_batch_run(bgt_batch *b, int mode, int use_graph)
     return BGT_OK;
 }
 
-// Synchronise and turn the kernels' status word into an error code.
-int bgt::batch_check(bgt_batch *b)
+void bgt::batch_status_words(const bgt_batch *b, const int *(&words)[2])
 {
-    cudaError_t e = cudaStreamSynchronize(b->ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "batch run");
-    int status = 0, rstatus = 0;
-    if (b->last_mode != 0 || b->any_ring)
-        e = cudaMemcpy(&status, &b->d_sched->status, sizeof(int), cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess && b->last_mode == 0 && !b->res_items.empty())
-        e = cudaMemcpy(&rstatus, &b->d_rs->status, sizeof(int), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return cuda_fail(e, "status readback");
-    status |= rstatus;
+    words[0] = b->last_mode != 0 || b->any_ring ? &b->d_sched->status : nullptr;
+    words[1] = b->last_mode == 0 && !b->res_items.empty() ? &b->d_rs->status : nullptr;
+}
+
+int bgt::batch_status(int status)
+{
     if (status & (kErrTmaTimeout | kErrQueueTimeout | kErrQueueFull))
         return fail(BGT_ERR_TIMEOUT, "device wait gave up (status bits 0x%x)", status);
     if (status & kErrPassLimit) return fail(BGT_ERR_LIMIT, "an instance hit the pass cap");
     return BGT_OK;
+}
+
+// Synchronise and turn the kernels' status words into an error code.
+int bgt::batch_check(bgt_batch *b)
+{
+    cudaError_t e = cudaStreamSynchronize(b->ctx->stream);
+    if (e != cudaSuccess) return cuda_fail(e, "batch run");
+    const int *words[2];
+    batch_status_words(b, words);
+    int status = 0;
+    for (const int *w : words) {
+        int v = 0;
+        if (w) e = cudaMemcpy(&v, w, sizeof(int), cudaMemcpyDeviceToHost);
+        if (e != cudaSuccess) return cuda_fail(e, "status readback");
+        status |= v;
+    }
+    return batch_status(status);
 }
 
 extern "C" int bgt_batch_instance_stats(bgt_batch *b, int id, int *passes, int *converged, int *cfg)

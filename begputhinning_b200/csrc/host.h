@@ -50,6 +50,10 @@ int ctx_scratch(bgt_ctx *c, int slot, size_t bytes, void **out);
 int ctx_pinned(bgt_ctx *c, size_t bytes, void **out);
 int single_batch(bgt_ctx *c, int dims, int W, int H, int D, bgt_batch **out);
 int batch_check(bgt_batch *b);
+// Status words of the batch's last run (device pointers, null: none), and
+// their bits as an error code.
+void batch_status_words(const bgt_batch *b, const int *(&words)[2]);
+int batch_status(int bits);
 int batch_set_input_extent(bgt_batch *b, int id, int inW, int inH, int inD);
 size_t batch_pool_bytes(const std::vector<BatchItem> &items);
 // Lay a batch out in caller-provided device memory (the serving runtime's
@@ -70,11 +74,29 @@ struct DevSegs {
     uint8_t *is_end = nullptr;
     int16_t *px = nullptr, *py = nullptr, *pz = nullptr;
 };
+// The rest of CenterlineExtraction: pruning and smoothing; status words of the
+// kernels that made the image, read back with the results.
+struct SegTail {
+    int max_segment_length = 0, span = 0;
+    const int *check[2] = {nullptr, nullptr};
+};
+// Results in the context's pinned memory, valid until its next use (idx, fx,
+// fy, fz with a tail, start .. pz without), and the device arrays (without).
+struct SegResult {
+    int nseg = 0, npts = 0, checked = 0;
+    const int32_t *start = nullptr;
+    const uint8_t *is_end = nullptr;
+    const int16_t *px = nullptr, *py = nullptr, *pz = nullptr;
+    const uint32_t *idx = nullptr;
+    const float *fx = nullptr, *fy = nullptr, *fz = nullptr;
+    DevSegs dev;
+};
+// One cooperative launch (segments_graph.cu); 1 = beyond its range.
+int segments_graph(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, int D, int P, const SegTail *tail,
+                   SegResult *r);
 // Device ExtractSegmentsV on a packed image (P words per row): arrays left in
 // the context's scratch, or copied to host memory.
 int segments_device_arrays(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, int D, int P, DevSegs *out);
-// The same as one cooperative launch (segments_graph.cu); 1 = beyond its index range.
-int segments_graph(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, int D, int P, DevSegs *out);
 int segments_packed(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, int D, int P, HostSegs *out);
 // Exclusive prefix sum of n ints on the context's stream (CUB temporary
 // storage in scratch slot `slot`).
@@ -90,6 +112,7 @@ struct bgt_ctx {
     std::vector<bgt::Scratch> scratch;
     bgt::Scratch pinned;
     size_t seg_chains = 0, seg_nodes = 0;  // list sizes of the segment extraction (grown on demand)
+    size_t seg_read = 0;                   // bytes its last result took (read back with the header)
     std::map<std::tuple<int, int, int, int>, bgt_batch *> cache;
 };
 

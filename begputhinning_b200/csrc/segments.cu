@@ -466,7 +466,9 @@ int segments_device_arrays(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, i
     const long long npx = (long long)W * H * D;
     // BGT_SEGMENTS_PIXEL_WALK=1 selects the per-component pixel walk below (tests compare both)
     if (npx < (1LL << 32) - 1 && !getenv("BGT_SEGMENTS_PIXEL_WALK")) {
-        const int grc = segments_graph(c, dims, d_buf, W, H, D, P, out);
+        SegResult r;
+        const int grc = segments_graph(c, dims, d_buf, W, H, D, P, nullptr, &r);
+        *out = r.dev;
         if (grc != 1) return grc;  // done, or an error
     }
     if (npx >= (1LL << 32) - 1) return fail(BGT_ERR_LIMIT, "segment extraction limited to < 2^32 pixels");
@@ -631,12 +633,35 @@ int segments_device_arrays(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, i
 // The same, with the segment arrays copied to host memory (malloc).
 int segments_packed(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, int D, int P, HostSegs *out)
 {
-    DevSegs ds;
-    int rc = segments_device_arrays(c, dims, d_buf, W, H, D, P, &ds);
-    if (rc != BGT_OK) return rc;
-    cudaStream_t st = c->stream;
-    const int S = ds.nseg, Np = ds.npts;
     *out = HostSegs();
+    SegResult r;
+    int rc = 1;
+    if ((long long)W * H * D < (1LL << 32) - 1 && !getenv("BGT_SEGMENTS_PIXEL_WALK"))
+        rc = segments_graph(c, dims, d_buf, W, H, D, P, nullptr, &r);
+    if (rc == 1) {
+        // the pixel walk leaves its arrays on the device, one behind the other
+        rc = segments_device_arrays(c, dims, d_buf, W, H, D, P, &r.dev);
+        if (rc != BGT_OK) return rc;
+        r.nseg = r.dev.nseg;
+        r.npts = r.dev.npts;
+        if (r.nseg > 0) {
+            const char *first = (const char *)r.dev.start;
+            const size_t span = (size_t)((const char *)((dims == 3 ? r.dev.pz : r.dev.py) + r.npts) - first);
+            void *pin = nullptr;
+            if ((rc = ctx_pinned(c, span, &pin))) return rc;
+            cudaError_t e = cudaMemcpyAsync(pin, first, span, cudaMemcpyDeviceToHost, c->stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+            if (e != cudaSuccess) return cuda_fail(e, "segment readback");
+            auto host = [&](const void *d) { return (const char *)pin + ((const char *)d - first); };
+            r.start = (const int32_t *)host(r.dev.start);
+            r.is_end = (const uint8_t *)host(r.dev.is_end);
+            r.px = (const int16_t *)host(r.dev.px);
+            r.py = (const int16_t *)host(r.dev.py);
+            r.pz = dims == 3 ? (const int16_t *)host(r.dev.pz) : nullptr;
+        }
+    }
+    if (rc != BGT_OK) return rc;
+    const int S = r.nseg, Np = r.npts;
     out->nseg = S;
     out->npts = Np;
     out->start = (int32_t *)malloc((size_t)(S + 1) * 4);
@@ -644,29 +669,18 @@ int segments_packed(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, i
     out->px = (int16_t *)malloc((size_t)Np * 2 + 2);
     out->py = (int16_t *)malloc((size_t)Np * 2 + 2);
     out->pz = dims == 3 ? (int16_t *)malloc((size_t)Np * 2 + 2) : nullptr;
-    if (!out->start || !out->is_end || !out->px || !out->py || (dims == 3 && !out->pz))
+    if (!out->start || !out->is_end || !out->px || !out->py || (dims == 3 && !out->pz)) {
+        free_host_segs(out);
         return fail(BGT_ERR_NOMEM, "host allocation of segment arrays");
-    if (S == 0) {
-        out->start[0] = 0;
-        return BGT_OK;
     }
-    // the arrays lie one behind the other: one copy to pinned memory, then to the caller's arrays
-    const char *first = (const char *)ds.start;
-    const size_t span = (size_t)((const char *)((dims == 3 ? ds.pz : ds.py) + Np) - first);
-    void *pin = nullptr;
-    int prc = ctx_pinned(c, span, &pin);
-    if (prc != BGT_OK) return prc;
-    cudaError_t e = cudaMemcpyAsync(pin, first, span, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e == cudaSuccess) {
-        auto host = [&](const void *d) { return (const char *)pin + ((const char *)d - first); };
-        memcpy(out->start, host(ds.start), (size_t)(S + 1) * 4);
-        memcpy(out->is_end, host(ds.is_end), (size_t)S);
-        memcpy(out->px, host(ds.px), (size_t)Np * 2);
-        memcpy(out->py, host(ds.py), (size_t)Np * 2);
-        if (dims == 3) memcpy(out->pz, host(ds.pz), (size_t)Np * 2);
+    out->start[0] = 0;
+    if (S > 0) {
+        memcpy(out->start, r.start, (size_t)(S + 1) * 4);
+        memcpy(out->is_end, r.is_end, (size_t)S);
+        memcpy(out->px, r.px, (size_t)Np * 2);
+        memcpy(out->py, r.py, (size_t)Np * 2);
+        if (dims == 3) memcpy(out->pz, r.pz, (size_t)Np * 2);
     }
-    if (e != cudaSuccess) return cuda_fail(e, "segment readback");
     return BGT_OK;
 }
 

@@ -36,6 +36,9 @@
 //      cycles without a node, which the reference never walks)
 //   D  segments and points per node;  E  prefix sums, node outputs
 //   F  chain points write their coordinates
+//   G, H (CenterlineExtraction only) pruning, smoothing and flattening
+//      (2D/CenterlineExtraction.cpp:51-131, 3D/CenterlineExtraction.cpp:56-144),
+//      so the whole path needs one readback and no count on the host
 //
 // Bound: latency -- about 7 + log4(longest chain) grid barriers of 1-2 us,
 // and in phase A of a volume the read of its packed words.  Measured on a
@@ -81,6 +84,21 @@ __host__ __device__ inline SegLayout seg_layout(unsigned S, unsigned N, int dims
     return L;
 }
 
+// Output block of the centreline tail: header, I[nsegs + 1], X[N], Y[N], Z[N].
+struct TailLayout {
+    size_t idx, x, y, z, total;
+};
+__host__ __device__ inline TailLayout tail_layout(unsigned S, unsigned N, int dims)
+{
+    TailLayout L;
+    L.idx = kSegHeaderBytes;
+    L.x = L.idx + seg_up16((size_t)(S + 1) * 4);
+    L.y = L.x + seg_up16((size_t)N * 4);
+    L.z = L.y + seg_up16((size_t)N * 4);
+    L.total = L.z + (dims == 3 ? seg_up16((size_t)N * 4) : 0);
+    return L;
+}
+
 struct SegArgs {
     const uint32_t *buf;  // packed image, P words per row
     int W, H, D, P;
@@ -99,17 +117,25 @@ struct SegArgs {
     uint8_t *ndeg;        // foreground neighbours
     uint2 *ncnt;          // segments, points
     uint32_t cap_n;
-    uint2 *bsum, *bsum2;  // per block: nodes and chain points; segments and points
+    uint2 *bsum, *bsum2, *bsum3;  // per block: nodes and chain points; segments and points; kept ones
     int *sync;
     uint8_t *out;
     unsigned long long out_bytes;
     long long timeout_ns;
+    // centreline tail
+    uint32_t *keep;       // segment -> its first output point, kNone: pruned
+    uint8_t *tail;
+    unsigned long long tail_bytes, maxlen;
+    int span;
+    const int *check[2];  // status words of the kernels before this one (or null)
 };
 
-// Header of the output block.
+// Header of the output blocks.
 struct SegHeader {
     uint32_t nodes, chains, segs, pts;
-    int status;  // 0 done, 1 lists too small, 2 output too small, 4 a wait ran out, 8 sums past 32 bits
+    int status;   // 0 done, 1 lists too small, 2 output too small, 4 a wait ran out, 8 sums past 32 bits
+    int checked;  // the status words, OR-ed
+    uint32_t kept, kept_pts;
 };
 
 // Grid barrier (cooperative launch: every block is resident).  Bounded; false
@@ -130,7 +156,10 @@ __device__ bool seg_barrier(const SegArgs &a, unsigned &gen)
                 good = false;
                 break;
             }
-        if (!good) atomicOr(a.sync + 1, 4);
+        if (!good) {
+            atomicOr(a.sync + 1, 4);
+            atomicOr(&reinterpret_cast<SegHeader *>(a.tail ? a.tail : a.out)->status, 4);
+        }
         ok = good && !(ld_acquire(a.sync + 1) & 4);
     }
     __syncthreads();
@@ -376,12 +405,38 @@ __device__ __forceinline__ uint2 seg_visit(const SegArgs &a, uint32_t r, uint32_
     return make_uint2(si - si0, pi - pi0);
 }
 
+// A kept segment's points, smoothed, by one warp.  Point q is the mean of the
+// points within min(span, q, n - 1 - q) of it.  The reference keeps a float
+// running sum of integer coordinates, which is exact while it stays below
+// 2^24 (spans up to kTailSpan: 2 * span + 2 coordinates of 15 bits), so the
+// sum is taken as an integer here and the quotient is the same.
+constexpr int kTailSpan = 255;
 template <int DIMS>
+__device__ __forceinline__ void tail_segment(const SegArgs &a, const int16_t *px, const int16_t *py, const int16_t *pz,
+                                             int first, int n, uint32_t to, float *X, float *Y, float *Z)
+{
+    const int span = min(a.span, (n - 1) / 2);
+    for (int q = threadIdx.x & 31; q < n; q += 32) {
+        const int h = min(span, min(q, n - 1 - q));
+        int x = 0, y = 0, z = 0;
+        for (int k = first + q - h; k <= first + q + h; k++) {
+            x += __ldcg(px + k);
+            y += __ldcg(py + k);
+            if (DIMS == 3) z += __ldcg(pz + k);
+        }
+        const float c = (float)(2 * h + 1);
+        X[to + q] = __fdiv_rn((float)x, c);
+        Y[to + q] = __fdiv_rn((float)y, c);
+        if (DIMS == 3) Z[to + q] = __fdiv_rn((float)z, c);
+    }
+}
+
+template <int DIMS, bool TAIL>
 __global__ void __launch_bounds__(kSegThreads, 1) segments_graph_kernel(const SegArgs a)
 {
     unsigned gen = 0;
     const uint32_t tid = blockIdx.x * kSegThreads + threadIdx.x, nthr = gridDim.x * kSegThreads;
-    SegHeader *hdr = reinterpret_cast<SegHeader *>(a.out);
+    SegHeader *hdr = reinterpret_cast<SegHeader *>(TAIL ? a.tail : a.out);
     unsigned long long total, before[2], all[2];
 
     // A: masks and counts of this block's range of words
@@ -404,8 +459,10 @@ __global__ void __launch_bounds__(kSegThreads, 1) segments_graph_kernel(const Se
     // B: lists in raster order
     seg_block_prefix(a.bsum, before, all);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        *hdr = SegHeader{(uint32_t)min(all[0], (unsigned long long)kNone), (uint32_t)min(all[1], (unsigned long long)kNone),
-                         0u, 0u, all[0] > a.cap_n || all[1] > a.cap_c ? 1 : 0};
+        hdr->nodes = (uint32_t)min(all[0], (unsigned long long)kNone);
+        hdr->chains = (uint32_t)min(all[1], (unsigned long long)kNone);
+        hdr->checked = (a.check[0] ? __ldcg(a.check[0]) : 0) | (a.check[1] ? __ldcg(a.check[1]) : 0);
+        if (all[0] > a.cap_n || all[1] > a.cap_c) atomicOr(&hdr->status, 1);
     }
     if (all[0] > a.cap_n || all[1] > a.cap_c) return;
     const uint32_t nn = (uint32_t)all[0], nc = (uint32_t)all[1];
@@ -519,7 +576,7 @@ __global__ void __launch_bounds__(kSegThreads, 1) segments_graph_kernel(const Se
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         hdr->segs = (uint32_t)all[0];
         hdr->pts = (uint32_t)all[1];
-        hdr->status = wide ? 8 : L.total > a.out_bytes ? 2 : 0;
+        if (wide || L.total > a.out_bytes) atomicOr(&hdr->status, wide ? 8 : 2);
     }
     if (wide || L.total > a.out_bytes) return;
     int32_t *start = reinterpret_cast<int32_t *>(a.out + L.start);
@@ -560,19 +617,71 @@ __global__ void __launch_bounds__(kSegThreads, 1) segments_graph_kernel(const Se
         px[pos] = (int16_t)at.y;
         py[pos] = (int16_t)y;
     }
+    if constexpr (TAIL) {
+        if (!seg_barrier(a, gen)) return;
+        // G: segments kept (more than maxlen points, or not an end segment)
+        const uint32_t S = (uint32_t)all[0];
+        const uint32_t sper = (S + gridDim.x - 1) / gridDim.x;
+        const uint32_t k0 = min(S, sper * blockIdx.x), k1 = min(S, k0 + sper);
+        auto points = [&](uint32_t k) {
+            const uint32_t n = (uint32_t)(__ldcg(start + k + 1) - __ldcg(start + k));
+            return (unsigned long long)n > a.maxlen || !__ldcg(is_end + k) ? n : 0u;
+        };
+        unsigned long long kept = 0;
+        for (uint32_t k = k0 + threadIdx.x; k < k1; k += kSegThreads) {
+            const uint32_t n = points(k);
+            kept += n ? 1ull << 32 | n : 0ull;
+        }
+        seg_exscan(kept, &total);
+        if (threadIdx.x == 0) a.bsum3[blockIdx.x] = make_uint2((uint32_t)(total >> 32), (uint32_t)total);
+        if (!seg_barrier(a, gen)) return;
+        seg_block_prefix(a.bsum3, before, all);
+        const TailLayout T = tail_layout((unsigned)all[0], (unsigned)all[1], DIMS);
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            hdr->kept = (uint32_t)all[0];
+            hdr->kept_pts = (uint32_t)all[1];
+            if (T.total > a.tail_bytes) atomicOr(&hdr->status, 2);
+        }
+        if (T.total > a.tail_bytes) return;
+        uint32_t *I = reinterpret_cast<uint32_t *>(a.tail + T.idx);
+        float *X = reinterpret_cast<float *>(a.tail + T.x), *Y = reinterpret_cast<float *>(a.tail + T.y),
+              *Z = reinterpret_cast<float *>(a.tail + T.z);
+        if (blockIdx.x == 0 && threadIdx.x == 0) I[all[0]] = (uint32_t)all[1];
+        uint32_t to = (uint32_t)before[0], pt = (uint32_t)before[1];
+        for (uint32_t base = k0; base < k1; base += kSegThreads) {
+            const uint32_t k = base + threadIdx.x;
+            const uint32_t n = k < k1 ? points(k) : 0u;
+            const unsigned long long o = seg_exscan(n ? 1ull << 32 | n : 0ull, &total);
+            if (k < k1) a.keep[k] = n ? pt + (uint32_t)o : kNone;
+            if (n) I[to + (uint32_t)(o >> 32)] = pt + (uint32_t)o;
+            to += (uint32_t)(total >> 32);
+            pt += (uint32_t)total;
+        }
+        __syncthreads();
+        // H: the block's segments, a warp each
+        for (uint32_t k = k0 + (threadIdx.x >> 5); k < k1; k += kSegWarps) {
+            const uint32_t p = a.keep[k];
+            if (p == kNone) continue;
+            const int first = __ldcg(start + k), n = __ldcg(start + k + 1) - first;
+            tail_segment<DIMS>(a, px, py, pz, first, n, p, X, Y, Z);
+        }
+    }
 }
 }  // namespace
 
-// Device segment extraction of a packed image.  Returns BGT_OK with *out
-// filled (arrays in the context's scratch until its next extraction), 1 when
-// the image is beyond this path's index range, or an error.  The lists and
-// the output live in scratch sized by what the context has met so far; an
-// image that needs more reports its counts and is run once more.
-int segments_graph(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, int D, int P, DevSegs *out)
+// Device segment extraction of a packed image and, with `tail`, the rest of
+// CenterlineExtraction.  Returns BGT_OK with *r filled, 1 when the image is
+// beyond this path's index range, or an error.  The lists and the outputs
+// live in scratch sized by what the context has met so far; an image that
+// needs more reports its counts and is run once more.  The results are read
+// back to pinned memory: with the header as much as the last result had, the
+// rest, if any, by a second copy.
+int segments_graph(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, int D, int P, const SegTail *tail,
+                   SegResult *r)
 {
-    *out = DevSegs();
+    *r = SegResult();
     const long long rows = (long long)H * D, ww = (W + 31) / 32, nw = rows * ww, npx = (long long)W * rows;
-    if (nw >= (1LL << 31) || rows >= (1LL << 31)) return 1;
+    if (nw >= (1LL << 31) || rows >= (1LL << 31) || (tail && tail->span > kTailSpan)) return 1;
     cudaStream_t st = c->stream;
     SegArgs a{};
     a.buf = d_buf;
@@ -592,17 +701,20 @@ int segments_graph(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, in
     void *p_rec, *p_out, *p_list, *p_sync, *h_pin;
     int rc;
     if ((rc = ctx_scratch(c, 30, (size_t)nw * sizeof(uint4), &p_rec)) ||
-        (rc = ctx_scratch(c, 33, kSyncInts * sizeof(int) + 2 * (size_t)c->sms * sizeof(uint2), &p_sync)) ||
-        (rc = ctx_pinned(c, 4096, &h_pin)))
+        (rc = ctx_scratch(c, 33, kSyncInts * sizeof(int) + 3 * (size_t)c->sms * sizeof(uint2), &p_sync)))
         return rc;
     a.rec = (uint4 *)p_rec;
     a.sync = (int *)p_sync;
     a.bsum = (uint2 *)((char *)p_sync + kSyncInts * sizeof(int));
     a.bsum2 = a.bsum + c->sms;
-    size_t out_bytes = 0;
-    for (int attempt = 0; attempt < 4; attempt++) {
+    a.bsum3 = a.bsum2 + c->sms;
+    size_t out_segs = 0, out_pts = 0;
+    for (int attempt = 0; attempt < 5; attempt++) {
         const size_t nc = c->seg_chains, nn = c->seg_nodes;
         if (nc >= (1u << 30) || nn >= (1u << 31)) return 1;
+        // points: the chain points and two per segment, about two segments per node
+        out_segs = std::max(out_segs, std::min<size_t>(4 * nn, 1u << 30));
+        out_pts = std::max(out_pts, std::min<size_t>(nc + 8 * nn, 1u << 30));
         size_t off = 0;
         auto take = [&](size_t bytes) {
             const size_t o = off;
@@ -610,7 +722,8 @@ int segments_graph(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, in
             return o;
         };
         const size_t o_cpt = take(nc * 8), o_cdir = take(nc * 2), o_pair = take(nc * 16), o_exit = take(nc * 8),
-                     o_base = take(nc * 8), o_npt = take(nn * 8), o_deg = take(nn), o_cnt = take(nn * 8);
+                     o_base = take(nc * 8), o_npt = take(nn * 8), o_deg = take(nn), o_cnt = take(nn * 8),
+                     o_keep = take(tail ? out_segs * 4 : 0);
         if ((rc = ctx_scratch(c, 31, off, &p_list))) return rc;
         char *l = (char *)p_list;
         a.cpt = (uint2 *)(l + o_cpt);
@@ -621,15 +734,28 @@ int segments_graph(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, in
         a.npt = (uint2 *)(l + o_npt);
         a.ndeg = (uint8_t *)(l + o_deg);
         a.ncnt = (uint2 *)(l + o_cnt);
+        a.keep = (uint32_t *)(l + o_keep);
         a.cap_c = (uint32_t)nc;
         a.cap_n = (uint32_t)nn;
-        // points: the chain points and two per segment, about two segments per node
-        out_bytes = std::max(out_bytes, seg_layout((unsigned)std::min<size_t>(4 * nn, 1u << 30),
-                                                   (unsigned)std::min<size_t>(nc + 8 * nn, 1u << 30), dims).total);
-        if ((rc = ctx_scratch(c, 19, out_bytes, &p_out))) return rc;
+        a.out_bytes = seg_layout((unsigned)out_segs, (unsigned)out_pts, dims).total;
+        if ((rc = ctx_scratch(c, 19, a.out_bytes, &p_out))) return rc;
         a.out = (uint8_t *)p_out;
-        a.out_bytes = c->scratch[19].bytes;
+        uint8_t *block = a.out;
+        size_t block_bytes = a.out_bytes;
+        if (tail) {
+            void *p_tail;
+            block_bytes = a.tail_bytes = tail_layout((unsigned)out_segs, (unsigned)out_pts, dims).total;
+            if ((rc = ctx_scratch(c, 22, block_bytes, &p_tail))) return rc;
+            block = a.tail = (uint8_t *)p_tail;
+            a.maxlen = (unsigned long long)(long long)tail->max_segment_length;
+            a.span = std::max(0, tail->span);
+            a.check[0] = tail->check[0];
+            a.check[1] = tail->check[1];
+        }
+        const size_t first = std::min(block_bytes, std::min<size_t>(std::max<size_t>(c->seg_read, 32 << 10), 2 << 20));
+        if ((rc = ctx_pinned(c, first, &h_pin))) return rc;
         cudaError_t e = cudaMemsetAsync(a.sync, 0, kSyncInts * sizeof(int), st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(block, 0, sizeof(SegHeader), st);
         if (e != cudaSuccess) return cuda_fail(e, "segment sync reset");
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(grid);
@@ -640,36 +766,65 @@ int segments_graph(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, in
         attr[0].val.cooperative = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        e = dims == 2 ? cudaLaunchKernelEx(&cfg, segments_graph_kernel<2>, a)
-                      : cudaLaunchKernelEx(&cfg, segments_graph_kernel<3>, a);
+        e = dims == 2 ? (tail ? cudaLaunchKernelEx(&cfg, segments_graph_kernel<2, true>, a)
+                              : cudaLaunchKernelEx(&cfg, segments_graph_kernel<2, false>, a))
+                      : (tail ? cudaLaunchKernelEx(&cfg, segments_graph_kernel<3, true>, a)
+                              : cudaLaunchKernelEx(&cfg, segments_graph_kernel<3, false>, a));
         if (e != cudaSuccess) return cuda_fail(e, "segment kernel");
-        int *h_sync = (int *)((char *)h_pin + kSegHeaderBytes);
-        e = cudaMemcpyAsync(h_pin, a.out, sizeof(SegHeader), cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(h_sync, a.sync, 2 * sizeof(int), cudaMemcpyDeviceToHost, st);
+        e = cudaMemcpyAsync(h_pin, block, first, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return cuda_fail(e, "segment extraction");
         const SegHeader h = *(const SegHeader *)h_pin;
-        if (h_sync[1] & 4) return fail(BGT_ERR_TIMEOUT, "segment extraction: a device wait gave up");
-        if (h.status == 8) return fail(BGT_ERR_LIMIT, "segment output bound exceeds 2^31 entries");
-        if (h.status == 1) {
+        r->checked = h.checked;
+        if (h.checked) return BGT_OK;  // the image is not valid: the caller reports why
+        if (h.status & 4) return fail(BGT_ERR_TIMEOUT, "segment extraction: a device wait gave up");
+        if (h.status & 8) return fail(BGT_ERR_LIMIT, "segment output bound exceeds 2^31 entries");
+        if (h.status & 1) {
             c->seg_chains = std::max(c->seg_chains, (size_t)h.chains + h.chains / 8);
             c->seg_nodes = std::max(c->seg_nodes, (size_t)h.nodes + h.nodes / 8);
             continue;
         }
-        const SegLayout L = seg_layout(h.segs, h.pts, dims);
-        if (h.status == 2) {
-            out_bytes = L.total;
+        if (h.status & 2) {
+            out_segs = std::max(out_segs, (size_t)h.segs);
+            out_pts = std::max(out_pts, (size_t)h.pts);
             continue;
         }
-        out->nseg = (int)h.segs;
-        out->npts = (int)h.pts;
+        const SegLayout L = seg_layout(h.segs, h.pts, dims);
+        const TailLayout T = tail_layout(h.kept, h.kept_pts, dims);
+        const size_t total = tail ? T.total : L.total;
+        c->seg_read = total + total / 8;
+        if (total > first) {
+            if ((rc = ctx_pinned(c, total, &h_pin))) return rc;
+            e = cudaMemcpyAsync(h_pin, block, total, cudaMemcpyDeviceToHost, st);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+            if (e != cudaSuccess) return cuda_fail(e, "segment readback");
+        }
+        const char *o = (const char *)h_pin;
+        if (tail) {
+            r->nseg = (int)h.kept;
+            r->npts = (int)h.kept_pts;
+            r->idx = (const uint32_t *)(o + T.idx);
+            r->fx = (const float *)(o + T.x);
+            r->fy = (const float *)(o + T.y);
+            r->fz = (const float *)(o + T.z);
+            return BGT_OK;
+        }
+        r->nseg = (int)h.segs;
+        r->npts = (int)h.pts;
+        r->start = (const int32_t *)(o + L.start);
+        r->is_end = (const uint8_t *)(o + L.is_end);
+        r->px = (const int16_t *)(o + L.x);
+        r->py = (const int16_t *)(o + L.y);
+        r->pz = (const int16_t *)(o + L.z);
+        DevSegs &d = r->dev;
+        d.nseg = r->nseg;
+        d.npts = r->npts;
         if (h.segs == 0) return BGT_OK;
-        uint8_t *o = a.out;
-        out->start = (int32_t *)(o + L.start);
-        out->is_end = o + L.is_end;
-        out->px = (int16_t *)(o + L.x);
-        out->py = (int16_t *)(o + L.y);
-        out->pz = dims == 3 ? (int16_t *)(o + L.z) : nullptr;
+        d.start = (int32_t *)(a.out + L.start);
+        d.is_end = a.out + L.is_end;
+        d.px = (int16_t *)(a.out + L.x);
+        d.py = (int16_t *)(a.out + L.y);
+        d.pz = dims == 3 ? (int16_t *)(a.out + L.z) : nullptr;
         return BGT_OK;
     }
     return fail(BGT_ERR_NOMEM, "segment extraction: the counts kept growing");

@@ -133,3 +133,18 @@ def test_kernel_edges(ctx, kind):
     for _ in range(2):  # the second call finds the lists of the first
         got = ExtractSegmentsV(a, ctx)
         assert got.as_lists() == want.as_lists()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prune,span", [(0, 0), (3, 1), (12, 7), (-1, 2), (2, -3), (5, 255), (5, 256), (1, 6000)])
+@pytest.mark.parametrize("kind", ["serpentine", "frame", "rings", "129x65", "1x1", "thin3"])
+def test_centerline_edges(ctx, kind, prune, span):
+    """Pruning, smoothing (spans up to and past the one whose running sums stay
+    exact) and flattening: the same floats, bit for bit."""
+    from begputhinning_b200 import CenterlineExtraction
+    a = _mask(kind)
+    got = CenterlineExtraction(a, prune, span, ctx)
+    want = (po.centerline2d if a.ndim == 2 else po.centerline3d)(a, prune, span)
+    arrays = [want.x, want.y] + ([want.z] if a.ndim == 3 else []) + [want.idx]
+    for g, w in zip(got, arrays, strict=True):
+        assert np.array_equal(g, w)
