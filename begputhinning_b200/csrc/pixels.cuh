@@ -118,7 +118,7 @@ __device__ __forceinline__ uint32_t pixel_vote(const T *p, uint32_t off, int cnt
         bool f = false;
         if (lane < c) {
             const T v = __ldg(p + (size_t)o + lane);
-            f = MODE == 0 ? fg2<T>(v) : fg3<T>(v);
+            f = MODE == 0 ? fg2<T>(v) : MODE == 1 ? fg3<T>(v) : v != (T)0;
         }
         const uint32_t m = __ballot_sync(kFull, f);
         if (lane == k) w = m;
@@ -128,7 +128,9 @@ __device__ __forceinline__ uint32_t pixel_vote(const T *p, uint32_t off, int cnt
 template <typename T>
 __device__ __forceinline__ uint32_t pixel_vote_mode(const IODesc &d, uint32_t off, int cnt)
 {
-    return d.mode == 0 ? pixel_vote<T, 0>((const T *)d.in, off, cnt) : pixel_vote<T, 1>((const T *)d.in, off, cnt);
+    return d.mode == 0   ? pixel_vote<T, 0>((const T *)d.in, off, cnt)
+           : d.mode == 1 ? pixel_vote<T, 1>((const T *)d.in, off, cnt)
+                         : pixel_vote<T, 2>((const T *)d.in, off, cnt);
 }
 // Every lane of the warp calls it (cnt = 0 for none).
 static __device__ __noinline__ uint32_t pixel_word_wide(const IODesc &d, uint32_t off, int cnt)
