@@ -67,6 +67,7 @@ struct alignas(16) Inst {
     // resident engine (resident.cu)
     int res;                  // 1: thinned by the resident engine, 0: by the tile rings
     unsigned long long res_meet[2];  // meetings of its CTAs in turn: arrivals (low half), changes reported (high half)
+    int res_left;             // CTAs of the instance that are done with it (the last one clears the meetings)
     int res_bands;            // 3D: boxes the volume is cut into
     int res_gy;               // 3D: boxes along y (band = z index * res_gy + y index)
     int res_stride;           // 3D: messages a box may send per iteration (its core words)

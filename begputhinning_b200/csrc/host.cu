@@ -336,7 +336,7 @@ static void plan_resident(bgt_batch *b)
         }
         const int G = gy * gz;
         in.res_gy = gy;
-        in.res_stride = ((it.H + gy - 1) / gy) * ((it.D + gz - 1) / gz) * wl;
+        in.res_stride = ((it.H + gy - 1) / gy) * ((it.D + gz - 1) / gz) * res_words3d(it.W);
         for (int k = 0; k < G; k++) {
             const int kz = k / gy, ky = k % gy;
             const int r0 = (int)((long long)kz * it.D / gz), r1 = (int)((long long)(kz + 1) * it.D / gz);
@@ -575,6 +575,17 @@ extern "C" int bgt_batch_finalize(bgt_batch *b)
     if (e == cudaSuccess && !b->res_items.empty())
         e = cudaMemcpyAsync(b->d_res_items, b->res_items.data(), b->res_items.size() * sizeof(ResItem),
                             cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess && !b->res_items.empty()) {
+        b->res_teams = false;
+        for (const ResItem &r : b->res_items) b->res_teams |= r.bands > 1;
+        b->rs_host = ResSched{};
+        b->rs_host.nitems = (int)b->res_items.size();
+        // the boxes of an instance wait for one another only for the length of
+        // the slowest one's passes between two meetings, and at first until
+        // the last of them is taken: 4 s is far beyond any legitimate wait
+        b->rs_host.timeout_ns = 4000000000LL;
+        e = cudaMemcpyAsync(b->d_rs, &b->rs_host, sizeof(ResSched), cudaMemcpyHostToDevice, st);
+    }
     if (e != cudaSuccess) {
         if (!b->reserved) batch_free_device(b);
         return cuda_fail(e, "batch table upload");
@@ -928,11 +939,8 @@ static int enqueue_engine(bgt_batch *b, cudaStream_t st, bool capturing)
         sched_reset_kernel<<<std::min<unsigned>(1024, (b->cap + 255) / 256), 256, 0, st>>>(
             b->d_sched, b->d_seq, b->d_item, b->cap, 20000000000LL, b->grid);
     stage_event(b, 1, st, capturing);
-    // bands of an image wait for one another only for the length of one
-    // iteration of the slowest band: 4 s is far beyond any legitimate wait
-    e = launch_resident(b->res_grid, b->d_insts, N, b->d_res_items, (int)b->res_items.size(), b->d_rs,
-                        b->d_rtrace, 4000000000LL, b->d_io, N == 1 && b->pack_words == 0 ? &b->io_host[0] : nullptr,
-                        b->pixels, st);
+    e = launch_resident(b->res_grid, b->d_insts, b->d_res_items, (int)b->res_items.size(), b->d_rs, b->d_rtrace,
+                        b->d_io, N == 1 && b->pack_words == 0 ? &b->io_host[0] : nullptr, b->pixels, b->res_teams, st);
     if (e != cudaSuccess) return cuda_fail(e, "resident engine launch");
     stage_event(b, 2, st, capturing);
     if (b->any_ring) {
@@ -1185,19 +1193,50 @@ int bgt::batch_check(bgt_batch *b)
     return batch_status(status);
 }
 
+// Per-instance passes, convergence and work of the last run, from the
+// instance table and, for instances of the resident kernel, its item records.
+struct RunRecord {
+    int passes = 0, converged = 0;
+    unsigned long long tiles = 0, words = 0;
+};
+static int read_records(bgt_batch *b, std::vector<RunRecord> &rec)
+{
+    int rc = batch_check(b);
+    if (rc != BGT_OK) return rc;
+    const size_t n = b->items.size();
+    std::vector<Inst> tmp(n);
+    cudaError_t e = cudaMemcpy(tmp.data(), b->d_insts, n * sizeof(Inst), cudaMemcpyDeviceToHost);
+    std::vector<ResTrace> tr(b->last_mode == 0 ? b->res_items.size() : 0);
+    if (e == cudaSuccess && !tr.empty())
+        e = cudaMemcpy(tr.data(), b->d_rtrace, tr.size() * sizeof(ResTrace), cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) return cuda_fail(e, "stats readback");
+    rec.assign(n, RunRecord());
+    for (size_t i = 0; i < n; i++)
+        if (b->last_mode != 0 || !b->h[i].res)
+            rec[i] = RunRecord{tmp[i].passes_run, tmp[i].converged, tmp[i].tiles_run, tmp[i].work_words};
+        else
+            rec[i].converged = 1;
+    for (size_t k = 0; k < tr.size(); k++) {
+        RunRecord &r = rec[b->res_items[k].inst];
+        if (b->res_items[k].band == 0) r.passes = tr[k].passes;
+        r.converged = std::min(r.converged, tr[k].result);
+        r.tiles += tr[k].tiles;
+        r.words += tr[k].words;
+    }
+    return BGT_OK;
+}
+
 extern "C" int bgt_batch_instance_stats(bgt_batch *b, int id, int *passes, int *converged, int *cfg)
 {
     if (!b || !b->finalized) return fail(BGT_ERR_STATE, "batch not finalized");
     if (id < 0 || id >= (int)b->items.size()) return fail(BGT_ERR_ARG, "bad instance id");
     if (!b->stats_valid) {
-        int rc = batch_check(b);
+        std::vector<RunRecord> rec;
+        int rc = read_records(b, rec);
         if (rc != BGT_OK) return rc;
-        std::vector<Inst> tmp(b->items.size());
-        cudaError_t e = cudaMemcpy(tmp.data(), b->d_insts, tmp.size() * sizeof(Inst), cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) return cuda_fail(e, "stats readback");
-        for (size_t i = 0; i < tmp.size(); i++) {
-            b->stats[i].passes = tmp[i].passes_run;
-            b->stats[i].converged = tmp[i].converged;
+        for (size_t i = 0; i < rec.size(); i++) {
+            b->stats[i].passes = rec[i].passes;
+            b->stats[i].converged = rec[i].converged;
         }
         b->stats_valid = true;
     }
@@ -1210,15 +1249,13 @@ extern "C" int bgt_batch_instance_stats(bgt_batch *b, int id, int *passes, int *
 extern "C" int bgt_batch_work(bgt_batch *b, unsigned long long *tiles, unsigned long long *words)
 {
     if (!b || !b->finalized) return fail(BGT_ERR_STATE, "batch not finalized");
-    int rc = batch_check(b);
+    std::vector<RunRecord> rec;
+    int rc = read_records(b, rec);
     if (rc != BGT_OK) return rc;
-    std::vector<Inst> tmp(b->items.size());
-    cudaError_t e = cudaMemcpy(tmp.data(), b->d_insts, tmp.size() * sizeof(Inst), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return cuda_fail(e, "work readback");
     unsigned long long t = 0, w = 0;
-    for (const Inst &in : tmp) {
-        t += in.tiles_run;
-        w += in.work_words;
+    for (const RunRecord &r : rec) {
+        t += r.tiles;
+        w += r.words;
     }
     if (tiles) *tiles = t;
     if (words) *words = w;

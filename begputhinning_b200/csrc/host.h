@@ -159,6 +159,8 @@ struct bgt_batch {
     bgt::ResSched *d_rs = nullptr;
     bgt::ResTrace *d_rtrace = nullptr;  // per-item timeline of the last resident run
     int res_grid = 0;
+    bool res_teams = false;           // some instance is cut into several boxes
+    bgt::ResSched rs_host{};          // kept alive for its stream-ordered upload
     bool any_ring = false;            // some instance is planned for the tile rings
     cudaGraphExec_t gexec = nullptr;
     bool graph_valid = false;

@@ -58,15 +58,20 @@ struct ResItem {
 };
 struct ResSched {
     int head;        // next item
+    int done;        // CTAs that have left the kernel (the last one resets both for the next run)
     int nitems;
-    int status;      // error bits
-    int pad;
+    int status;      // error bits of the run
     long long timeout_ns;
 };
-// Timeline of one work item of the last run (global timer, ns; SM id).
+// What became of one work item in the last run: its timeline (global timer,
+// ns; SM id), outcome and work.
 struct ResTrace {
     long long t0, t1;
-    int sm, pad;
+    int sm;
+    int result;      // 1 converged, -1 pass cap or failed wait
+    int passes;      // passes (3D: subiterations) run
+    int pad;
+    unsigned long long words, tiles;  // packed core words processed; units of work
 };
 // One CTA per SM: two of 384 threads with 112 KB each took the mixed batch
 // from 1.19 to 1.35 ms and three of 256 to 1.52 ms (smaller boxes, more halo),
@@ -86,6 +91,8 @@ double res_cost2d(int wl, int nrows);
 constexpr int kResPeriod2D = 4;
 // Whether a 3D box (ny rows x nz planes of a volume W wide, halo included) fits one CTA.
 bool res_fits3d(int W, int ny, int nz);
+// Words of its rows (30 voxels each).
+int res_words3d(int W);
 constexpr int kResHalo3D = 6;  // one iteration: six subiterations, one row and plane each
 cudaError_t res_occupancy(int *per_sm);  // resident CTAs per SM
 // Per-instance input/output of a batch-wide pack/unpack launch.
@@ -130,9 +137,10 @@ struct alignas(16) IODesc {
 
 // pixels: instances are read from and written to their pixel arrays (d_io by
 // instance, or `one` for a batch of one instance); else buf[0] holds them.
-cudaError_t launch_resident(int grid, Inst *d_insts, int ninst, const ResItem *d_items, int nitems,
-                            ResSched *d_rs, ResTrace *d_trace, long long timeout_ns, const IODesc *d_io,
-                            const IODesc *one, bool pixels, cudaStream_t st);
+// teams: some instance is cut into several boxes.
+cudaError_t launch_resident(int grid, Inst *d_insts, const ResItem *d_items, int nitems,
+                            ResSched *d_rs, ResTrace *d_trace, const IODesc *d_io, const IODesc *one, bool pixels,
+                            bool teams, cudaStream_t st);
 
 // Launchers (stream-ordered, no host synchronisation).
 // bytes: every input is one byte wide and tested "byte != 0" (see pack_all_kernel)

@@ -170,11 +170,10 @@ static __device__ __noinline__ void pixel_store_wide(const IODesc &d, uint32_t o
 }
 
 // 32-byte-aligned chunk c of the one-byte pixels of `rows` consecutive rows of
-// W pixels that start at `out`; row(r) = the packed words of row r, readable
-// one word past the row's last.  Two 128-bit stores where the chunk lies
+// W pixels that start at `out`; bits(r, x) = 32 pixels of row r from x on.  Two 128-bit stores where the chunk lies
 // inside the rows and spans at most two of them, bytes otherwise.
-template <class Row>
-__device__ __forceinline__ void pixel_chunk(uint8_t *out, uint32_t rows, int W, const FastDiv &dW, uint32_t c, Row row)
+template <class Bits>
+__device__ __forceinline__ void pixel_chunk(uint8_t *out, uint32_t rows, int W, const FastDiv &dW, uint32_t c, Bits pix)
 {
     const uintptr_t o = reinterpret_cast<uintptr_t>(out), end = o + (uintptr_t)rows * W;
     const uintptr_t a = (o & ~uintptr_t(31)) + (uintptr_t)c * 32u;
@@ -184,11 +183,10 @@ __device__ __forceinline__ void pixel_chunk(uint8_t *out, uint32_t rows, int W, 
     uint32_t r = fdiv(dW, f);
     int x = (int)(f - r * (uint32_t)W);
     if (hi - lo == 32 && W >= 32) {
-        const uint32_t *s = row(r);
-        uint32_t bits = __funnelshift_r(s[x >> 5], s[(x >> 5) + 1], x & 31);
+        uint32_t bits = pix(r, x);
         if (x + 32 > W) {  // the chunk runs into the next row
             const int n0 = W - x;
-            bits = (bits & ((1u << n0) - 1u)) | row(r + 1)[0] << n0;
+            bits = (bits & ((1u << n0) - 1u)) | pix(r + 1, 0) << n0;
         }
         uint4 *q = reinterpret_cast<uint4 *>(a);
         q[0] = make_uint4(bits4_to_bytes(bits & 15u), bits4_to_bytes((bits >> 4) & 15u),
@@ -198,7 +196,7 @@ __device__ __forceinline__ void pixel_chunk(uint8_t *out, uint32_t rows, int W, 
         return;
     }
     for (uintptr_t b = lo; b < hi; b++) {
-        *reinterpret_cast<uint8_t *>(b) = (uint8_t)((row(r)[x >> 5] >> (x & 31)) & 1u);
+        *reinterpret_cast<uint8_t *>(b) = (uint8_t)(pix(r, x) & 1u);
         if (++x == W) {
             x = 0;
             r++;
@@ -206,16 +204,16 @@ __device__ __forceinline__ void pixel_chunk(uint8_t *out, uint32_t rows, int W, 
     }
 }
 
-// Chunk c of a run of n one-byte pixels at `out` whose words are s (readable
-// one word past the last).
-__device__ __forceinline__ void pixel_run_chunk(uint8_t *out, int n, uint32_t c, const uint32_t *s)
+// Chunk c of a run of n one-byte pixels at `out`; pix(x) = 32 of them from x on.
+template <class Bits>
+__device__ __forceinline__ void pixel_run_chunk(uint8_t *out, int n, uint32_t c, Bits pix)
 {
     const uintptr_t o = reinterpret_cast<uintptr_t>(out), end = o + (uintptr_t)n;
     const uintptr_t a = (o & ~uintptr_t(31)) + (uintptr_t)c * 32u;
     const uintptr_t lo = a > o ? a : o, hi = a + 32 < end ? a + 32 : end;
     if (lo >= hi) return;
     const int x = (int)(lo - o);
-    const uint32_t bits = __funnelshift_r(s[x >> 5], s[(x >> 5) + 1], x & 31);
+    const uint32_t bits = pix(x);
     if (hi - lo == 32) {
         uint4 *q = reinterpret_cast<uint4 *>(a);
         q[0] = make_uint4(bits4_to_bytes(bits & 15u), bits4_to_bytes((bits >> 4) & 15u),

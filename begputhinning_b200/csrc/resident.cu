@@ -106,16 +106,21 @@ bool res_fits2d(int wl, int nrows)
     return true;
 }
 
+int res_words3d(int W) { return (W + 29) / 30; }
+
 bool res_fits3d(int W, int ny, int nz)
 {
-    const int wl = (W + 31) / 32;
-    const double rows2 = (double)(ny + 2) * (nz + 2), held = rows2 * (wl + 1) + 1, words = (double)wl * ny * nz;
+    const int wl = res_words3d(W);
+    const double held = (double)(((ny + 2) * (wl | 1)) | 1) * (nz + 2), words = (double)wl * ny * nz;
+    const double rows2 = (double)((ny + 5) & ~3) * (nz + 2);
     // words are indexed by 16 bits
     return held < 65535 && words <= (double)kDenseWords * kResThreads &&
-           held * 4 + rows2 * 8 + kListFill * words * kBoxListBytes + 128 <= (double)kSmemBytes;
+           held * 4 + rows2 * 2 + kListFill * words * kBoxListBytes + 128 <= (double)kSmemBytes;
 }
 
 // ------------------------------------------------------------ helpers -----
+extern __shared__ __align__(16) uint8_t res_smem[];  // dynamic shared memory of the CTA
+
 // The CTAs of one instance meet for the k-th time: each adds 1 to the low half
 // of meet[k & 1], and 1 to its high half when something of its own changed
 // since the last meeting; the wait (bounded) ends when all `bands` arrived.
@@ -125,7 +130,7 @@ bool res_fits3d(int W, int ny, int nz)
 // writes to global memory.  Returns 0 when nobody changed anything, 1 when
 // somebody did, 2 when the wait ran out.
 struct MeetState {
-    unsigned k = 0, seen0 = 0, seen1 = 0;  // meetings so far, high halves after the last one of either word
+    unsigned k, seen0, seen1;  // meetings so far, high halves after the last one of either word
 };
 __device__ __forceinline__ int res_meet(unsigned long long *meet, unsigned bands, bool changed, MeetState &m,
                                         long long timeout_ns)
@@ -201,7 +206,8 @@ struct ResIO {
     bool pix;
 };
 
-// put(pos, word) for every word of the grid of rows whose first word, row and
+// put(pos, word) for every word (W30: the 30-voxel words of full rows, see the
+// 3D section) of the grid of rows whose first word, row and
 // plane are x0, y0, z0 (warps stay together: put may hold warp-wide votes; `live`
 // is false for lanes past the end, whose word is 0).  U words of a thread are
 // in flight at once: at 768 threads and 48 bytes per word of one-byte pixels,
@@ -224,7 +230,7 @@ __device__ __forceinline__ void res_load_loop(const WordWalk &walk, int n, Fetch
         for (int k = 0; k < U; k++) put(i + k * kResThreads < n, at[k], v[k]);
     }
 }
-template <class Put>
+template <bool W30, class Put>
 __device__ __forceinline__ void res_load(const Inst &in, const ResIO &io, const WordWalk &walk, int n, int x0, int y0, int z0,
                                          Put put)
 {
@@ -232,38 +238,47 @@ __device__ __forceinline__ void res_load(const Inst &in, const ResIO &io, const 
         const uint32_t *g = in.buf[0];
         const int H = in.H, P = in.P;
         res_load_loop<4>(walk, n, [&](bool live, const WordPos &q) {
-            return live ? __ldcg(g + ((size_t)(z0 + q.z) * H + (y0 + q.y)) * P + (x0 + q.x)) : 0u;
+            if (!live) return 0u;
+            const uint32_t *r = g + ((size_t)(z0 + q.z) * H + (y0 + q.y)) * P;
+            if (!W30) return __ldcg(r + x0 + q.x);
+            if (q.x == 0) return __ldcg(r) << 1;
+            const int x = 30 * q.x - 1, j = x >> 5;
+            return __funnelshift_r(__ldcg(r + j), j + 1 < P ? __ldcg(r + j + 1) : 0u, x & 31);
         }, put);
         return;
     }
     const IODesc &d = *io.d;
     const int inW = d.inW, inH = d.inH, inD = d.inD;
+    // first pixel and number of pixels of a word; a row's first 30-voxel word starts one pixel late
     auto count = [&](bool live, const WordPos &q, uint32_t &off) {
-        const int x = 32 * (x0 + q.x), y = y0 + q.y, z = z0 + q.z;
+        const bool late = W30 && q.x == 0;
+        const int x = late ? 0 : W30 ? 30 * q.x - 1 : 32 * (x0 + q.x), y = y0 + q.y, z = z0 + q.z;
         off = ((uint32_t)z * (uint32_t)inH + (uint32_t)y) * (uint32_t)inW + (uint32_t)x;
-        return live && y < inH && z < inD ? max(0, min(32, inW - x)) : 0;
+        return live && y < inH && z < inD ? max(0, min(late ? 31 : 32, inW - x)) : 0;
     };
+    auto place = [&](const WordPos &q, uint32_t w) { return W30 && q.x == 0 ? w << 1 : w; };
     if (dtype_bytes(d.dtype) == 1) {
         const uint32_t neg = pixel_neg(d);
         res_load_loop<2>(walk, n, [&](bool live, const WordPos &q) {
             uint32_t off;
             const int cnt = count(live, q, off);
-            return pixel_bytes(d, off, cnt, neg);
+            return place(q, pixel_bytes(d, off, cnt, neg));
         }, put);
     } else {
         res_load_loop<1>(walk, n, [&](bool live, const WordPos &q) {
             uint32_t off;
             const int cnt = count(live, q, off);
-            return pixel_word_wide(d, off, cnt);
+            return place(q, pixel_word_wide(d, off, cnt));
         }, put);
     }
 }
 
 // The way back for words [x0, x1) of rows [y0, y0 + ny) of planes [z0, z0 + nz):
-// row(y, z) = the packed words from x0 on of grid row y of grid plane z.
-template <class Row>
+// bits(y, z, x) = 32 pixels from the x-th one on of grid row y of grid plane z
+// (what lies past the row's last pixel, or word x1, does not matter).
+template <class Bits>
 __device__ __forceinline__ void res_store(const Inst &in, const ResIO &io, int x0, int x1, int ny, int nz, int y0,
-                                          int z0, Row row)
+                                          int z0, Bits bits)
 {
     const int lane = threadIdx.x & 31, wl = x1 - x0;
     const WordWalk walk(wl, ny);
@@ -271,8 +286,11 @@ __device__ __forceinline__ void res_store(const Inst &in, const ResIO &io, int x
     if (!io.pix || !io.d->out) {
         uint32_t *g = in.buf[0];
         WordPos q = walk.first();
-        for (int i = threadIdx.x; i < n; i += kResThreads, walk.next(q))
-            g[((size_t)(z0 + q.z) * in.H + (y0 + q.y)) * in.P + x0 + q.x] = row(q.y, q.z)[q.x];
+        for (int i = threadIdx.x; i < n; i += kResThreads, walk.next(q)) {
+            const int left = in.W - 32 * (x0 + q.x);  // pixels from the word's first one on
+            const uint32_t w = bits(q.y, q.z, 32 * q.x);
+            g[((size_t)(z0 + q.z) * in.H + (y0 + q.y)) * in.P + x0 + q.x] = left >= 32 ? w : w & ((1u << left) - 1u);
+        }
         return;
     }
     const IODesc &d = *io.d;
@@ -283,7 +301,8 @@ __device__ __forceinline__ void res_store(const Inst &in, const ResIO &io, int x
         for (uint32_t i = threadIdx.x; i < per * (uint32_t)nz; i += kResThreads) {
             const uint32_t z = nz == 1 ? 0u : i / per;
             uint8_t *out = (uint8_t *)d.out + ((size_t)(z0 + (int)z) * in.H + y0) * in.W;
-            pixel_chunk(out, (uint32_t)ny, in.W, d.dW, i - z * per, [&](uint32_t r) { return row((int)r, (int)z); });
+            pixel_chunk(out, (uint32_t)ny, in.W, d.dW, i - z * per,
+                        [&](uint32_t r, int x) { return bits((int)r, (int)z, x); });
         }
         return;
     }
@@ -293,8 +312,7 @@ __device__ __forceinline__ void res_store(const Inst &in, const ResIO &io, int x
         WordPos q = chunks.first();
         for (int i = threadIdx.x; i < nz * ny * (wl + 1); i += kResThreads, chunks.next(q)) {
             uint8_t *out = (uint8_t *)d.out + ((size_t)(z0 + q.z) * in.H + (y0 + q.y)) * in.W + 32 * x0;
-            const uint32_t *s = row(q.y, q.z);
-            pixel_run_chunk(out, np, (uint32_t)q.x, s);
+            pixel_run_chunk(out, np, (uint32_t)q.x, [&](int x) { return bits(q.y, q.z, x); });
         }
         return;
     }
@@ -303,8 +321,41 @@ __device__ __forceinline__ void res_store(const Inst &in, const ResIO &io, int x
         const bool live = i < n;
         const int x = 32 * (x0 + q.x);
         const uint32_t off = ((uint32_t)(z0 + q.z) * (uint32_t)in.H + (uint32_t)(y0 + q.y)) * (uint32_t)in.W + (uint32_t)x;
-        pixel_store_wide(d, off, live ? min(32, in.W - x) : 0, live ? row(q.y, q.z)[q.x] : 0u);
+        pixel_store_wide(d, off, live ? min(32, in.W - x) : 0, live ? bits(q.y, q.z, 32 * q.x) : 0u);
     }
+}
+
+// An item is done: its outcome and work (words and tiles: this thread's share)
+// go to its record, and the last CTA of an instance clears the meetings for
+// the next run.  All threads call it; ends with a barrier.
+__device__ void res_done(Inst &in, const ResItem &it, int result, int passes, unsigned long long words,
+                         unsigned long long tiles, ResTrace *tr)
+{
+    __shared__ unsigned long long s_work[2];
+    if (threadIdx.x < 2) s_work[threadIdx.x] = 0;
+    __syncthreads();
+    // one add per warp: a 64-bit add to shared memory is a loop that 768 threads would take 40 us for
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        words += __shfl_xor_sync(kFull, words, o);
+        tiles += __shfl_xor_sync(kFull, tiles, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&s_work[0], words);
+        atomicAdd(&s_work[1], tiles);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        tr->result = result;
+        tr->passes = passes;
+        tr->words = s_work[0];
+        tr->tiles = s_work[1];
+        if (it.bands > 1 && atomicAdd(&in.res_left, 1) == it.bands - 1) {
+            in.res_meet[0] = in.res_meet[1] = 0;
+            in.res_left = 0;
+        }
+    }
+    __syncthreads();
 }
 
 // ------------------------------------------------------------ 2D ----------
@@ -444,10 +495,10 @@ __device__ uint32_t res_pass2d(const Box2D &b, int q, int *take, unsigned long l
 // passes) keep the core exact; if a pass before the meeting was a fixed point
 // already, the one at the meeting is too.
 template <int UW>
-__device__ void res_run2d(Inst &in, const ResIO &io, const ResItem &it, uint32_t *sm, ResSched *S, int *take)
+__device__ void res_run2d(Inst &in, const ResIO &io, const ResItem &it, uint32_t *sm, ResSched *S, int *take,
+                          ResTrace *tr)
 {
     __shared__ int s_flag;
-    const int lane = threadIdx.x & 31;
     const int wl_img = (in.W + 31) >> 5;
     const int a = max(0, it.r0 - it.halo), e0 = it.halo ? max(0, it.c0 - 1) : 0;  // first row and word held
     const int aend = min(in.H, it.r1 + it.halo), e1 = it.halo ? min(wl_img, it.c1 + 1) : wl_img;
@@ -478,7 +529,7 @@ __device__ void res_run2d(Inst &in, const ResIO &io, const ResItem &it, uint32_t
     for (int i = threadIdx.x; i < nunits; i += kResThreads) b.until[i] = -1;
     if (threadIdx.x < 2) take[threadIdx.x] = 0;
     __syncthreads();
-    res_load(in, io, WordWalk(b.wl, b.nrows), b.nrows * b.wl, e0, a, 0, [&](bool, const WordPos &q, uint32_t v) {
+    res_load<false>(in, io, WordWalk(b.wl, b.nrows), b.nrows * b.wl, e0, a, 0, [&](bool, const WordPos &q, uint32_t v) {
         if (!v) return;
         const int w = q.y * pp + q.x + 1;
         b.buf0[w] = v;
@@ -489,7 +540,7 @@ __device__ void res_run2d(Inst &in, const ResIO &io, const ResItem &it, uint32_t
     __syncthreads();
 
     int result = 0;  // 1 converged, -1 pass cap or failed wait
-    MeetState meet;
+    MeetState meet{0, 0, 0};
     unsigned long long words = 0;
     const int period = it.halo / 4;
     int q = 0, since = 0, e = 0;  // pass, passes since the last meeting, meetings
@@ -562,42 +613,123 @@ __device__ void res_run2d(Inst &in, const ResIO &io, const ResItem &it, uint32_t
     // the converged core (in buf[(q+1)&1])
     __syncthreads();
     const uint32_t *fin = ((q & 1) ? b.buf0 : b.buf1) + (size_t)b.rlo * pp + 1 + b.wlo;
-    res_store(in, io, it.c0, it.c1, it.r1 - it.r0, 1, it.r0, 0, [&](int y, int) { return fin + (size_t)y * pp; });
-    if (lane == 0 && words) atomicAdd(&in.work_words, words);  // words per pass (one iteration)
-    if (threadIdx.x == 0) {
-        if (it.band == 0) in.passes_run = q + 1;
-        if (result < 0) atomicMin(&in.converged, -1);
-        atomicAdd(&in.tiles_run, 1ull);
-    }
-    __syncthreads();
+    res_store(in, io, it.c0, it.c1, it.r1 - it.r0, 1, it.r0, 0, [&](int y, int, int x) {
+        const uint32_t *s = fin + y * pp + (x >> 5);
+        return __funnelshift_r(s[0], s[1], x & 31);
+    });
+    res_done(in, it, result, q + 1, words, threadIdx.x == 0, tr);
 }
 
 // ------------------------------------------------------------ 3D ----------
 // Entry of a box's word list: word index in shared memory (16 bits), its
-// column in the rows' change masks (5 bits), its distance from the box's core
-// (3 bits, 0 = core), and, in the candidate list, whether it changed.
-constexpr uint32_t kEntChanged = 1u << 24;
+// column in the rows' change masks (3 bits), its distance from the box's core
+// (3 bits, 0 = core), whether its row goes on to its left and right, and, in
+// the candidate list, whether it changed.
+constexpr uint32_t kEntChanged = 1u << 24, kEntLeft = 1u << 25, kEntRight = 1u << 26;
 __device__ __forceinline__ uint32_t ent_idx(uint32_t e) { return e & 0xffffu; }
-__device__ __forceinline__ uint32_t ent_col(uint32_t e) { return (e >> 16) & 31u; }
+__device__ __forceinline__ uint32_t ent_col(uint32_t e) { return (e >> 16) & 7u; }
 __device__ __forceinline__ int ent_dist(uint32_t e) { return (int)((e >> 21) & 7u); }
 
+// Words of a 3D box hold 30 voxels: bit 1 + k of word j is voxel x = 30 j + k, and
+// bits 0 and 31 repeat the voxels next to them, which are the neighbouring
+// words' bits 30 and 1.  A word's 3x3x3 neighbourhood is then 9 words of
+// shared memory instead of 27 (whose loads, at two to four lanes per bank, set
+// the time of a subiteration), and a deletion at either end of a word is
+// applied to the neighbour's copy as well.
+constexpr int kVox = 30;
+constexpr uint32_t kCoreBits = 0x7FFFFFFEu;
+
+// Everything about the box that all threads share lies in shared memory and is
+// read where it is needed: at 80 registers a thread, 27 of them the window,
+// values kept over an iteration would be spilled to local memory, and every
+// acquire of a meeting empties the L1 that holds the spills.
 struct Box3D {
-    uint32_t *state;      // [nz + 2][ny + 2] rows of wl words, a zero word between rows, a zero word at the end
-    uint32_t *cidx, *cU, *cdel;  // candidates of this iteration: entry, union, deletions of the subiteration
-    int p, ps;            // words between rows, between planes
+    ResItem it;
+    int H, D, wl;              // volume rows, planes; words per row
+    int y0, y1, z0, z1;        // rows and planes held
+    int p, ps;                 // words between rows, between planes
+    uint32_t mp, mps;          // reciprocals: idx / p and idx / ps by mulhi, exact for 16-bit idx
+    int my, mrows;             // rows of the masks: per plane (a multiple of 4), in all
+    int xs;                    // words per column of the masks: 1 << xs
+    int act, chg, list;        // offsets of the masks and of the word list
+    int nl;                    // its length
+    int gy, gz, by, bz;        // boxes along y and z; this box
+    int stride;                // messages a box may send
+    uint2 *msgs;
+    int *counts;
+    MeetState meet;            // (used by thread 0)
+    int n[4];                  // lengths: word list, active words, candidates, messages
+    int flag;
 };
 
-// The 3x3x3 neighbourhood words of the word at s.
-__device__ __forceinline__ void box_window(const uint32_t *s, int p, int ps, uint32_t (&g)[27])
+__device__ __forceinline__ uint32_t *box_state() { return reinterpret_cast<uint32_t *>(res_smem); }
+__device__ __forceinline__ uint32_t *box_words(int off) { return reinterpret_cast<uint32_t *>(res_smem + off); }
+// the lists, one behind the other: non-empty words, then the candidates'
+// entries, unions and deletions, then the active words (positions in `list`)
+__device__ __forceinline__ uint32_t *box_list(const Box3D &v, int k) { return box_words(v.list) + k * v.nl; }
+
+// plane and row of a word, padding included
+__device__ __forceinline__ uint32_t box_plane_row(const Box3D &v, uint32_t idx, uint32_t &y2)
+{
+    const uint32_t z2 = __umulhi(idx, v.mps);
+    y2 = __umulhi(idx - z2 * (uint32_t)v.ps, v.mp);
+    return z2;
+}
+__device__ __forceinline__ int box_index(const Box3D &v, const WordPos &q)
+{
+    return (q.z + 1) * v.ps + (q.y + 1) * v.p + q.x;
+}
+__device__ __forceinline__ int box_dist(const Box3D &v, const WordPos &q)
+{
+    const int y = v.y0 + q.y, z = v.z0 + q.z;
+    return max(max(max(v.it.c0 - y, y - v.it.c1 + 1), max(v.it.r0 - z, z - v.it.r1 + 1)), 0);
+}
+__device__ __forceinline__ uint32_t box_entry(const Box3D &v, const WordPos &q, int idx, int d)
+{
+    return (uint32_t)idx | (uint32_t)(q.x >> v.xs) << 16 | (uint32_t)d << 21 | (q.x > 0 ? kEntLeft : 0u) |
+           (q.x + 1 < v.wl ? kEntRight : 0u);
+}
+__device__ __forceinline__ void box_mark(const Box3D &v, int row, int col)
+{
+    atomicOr(box_words(v.chg) + (row >> 2), 1u << (8 * (row & 3) + col));
+}
+// a word of the core changed: mark it, and tell the boxes around when it lies near the core's edge
+__device__ __forceinline__ void box_changed(Box3D &v, uint32_t idx, uint32_t col, int iter)
+{
+    uint32_t y2;
+    const uint32_t z2 = box_plane_row(v, idx, y2);
+    box_mark(v, (int)(z2 * (uint32_t)v.my + y2), (int)col);
+    if (v.it.bands == 1) return;
+    const int y = v.y0 + (int)y2 - 1, z = v.z0 + (int)z2 - 1, h = v.it.halo;
+    if ((v.it.r0 > 0 && z < v.it.r0 + h) || (v.it.r1 < v.D && z >= v.it.r1 - h) || (v.it.c0 > 0 && y < v.it.c0 + h) ||
+        (v.it.c1 < v.H && y >= v.it.c1 - h)) {
+        const int x = (int)idx - (int)z2 * v.ps - (int)y2 * v.p;
+        uint2 *msg = v.msgs + ((size_t)(iter & 1) * v.it.bands + v.it.band) * v.stride;
+        msg[atomicAdd(&v.n[3], 1)] =
+            make_uint2(((uint32_t)z * (uint32_t)v.H + (uint32_t)y) * (uint32_t)v.wl + (uint32_t)x, box_state()[idx]);
+    }
+}
+
+// The 3x3x3 neighbourhood of the word at s; returns its own voxels.
+__device__ __forceinline__ uint32_t box_window(const uint32_t *s, int p, int ps, uint32_t (&g)[27])
 {
 #pragma unroll
     for (int k = 0; k < 9; k++) {
-        const uint32_t *r = s + (k / 3 - 1) * ps + (k % 3 - 1) * p;
-        const uint32_t l = r[-1], c = r[0], n = r[1];
-        g[3 * k] = at_xm1(c, l);
+        const uint32_t c = s[(k / 3 - 1) * ps + (k % 3 - 1) * p];
+        g[3 * k] = c << 1;
         g[3 * k + 1] = c;
-        g[3 * k + 2] = at_xp1(c, n);
+        g[3 * k + 2] = c >> 1;
     }
+    return g[13] & kCoreBits;
+}
+
+// Delete voxels of the word of entry e (other threads may do so to the copies in it).
+__device__ __forceinline__ void box_delete(uint32_t e, uint32_t del)
+{
+    uint32_t *s = box_state() + ent_idx(e);
+    atomicAnd(s, ~del);
+    if ((del & 2u) && (e & kEntLeft)) atomicAnd(s - 1, ~(1u << 31));
+    if ((del & (1u << kVox)) && (e & kEntRight)) atomicAnd(s + 1, ~1u);
 }
 
 // Position of this lane's element in a list the warp appends to (-1: none).
@@ -615,50 +747,212 @@ __device__ __forceinline__ int warp_append(bool take, int *count)
 // alone: what they read may be wrong by now, and nothing reads them before
 // their owner sends them.
 template <int J>
-__device__ __forceinline__ uint32_t box_deletions(const Box3D &b, uint32_t e, uint32_t cand)
+__device__ __forceinline__ uint32_t box_deletions(const Box3D &v, uint32_t e, uint32_t un)
 {
-    if (ent_dist(e) > 5 - J || cand == 0u) return 0u;
+    const uint32_t *s = box_state() + ent_idx(e);
+    if (ent_dist(e) > 5 - J || !(*s & un)) return 0u;
     uint32_t g[27];
-    box_window(b.state + ent_idx(e), b.p, b.ps, g);
-    return cand & rule3d<J>(g);
+    return box_window(s, v.p, v.ps, g) & un & rule3d<J>(g);
 }
 
 // ... with any number of candidates per thread
 template <int J>
-__device__ __forceinline__ void box_subiteration(const Box3D b, int nc, unsigned &words)
+__device__ __forceinline__ void box_subiteration(const Box3D &v, int nc, unsigned &words)
 {
     bool any = false;
     for (int c = threadIdx.x; c < nc; c += kResThreads) {
-        const uint32_t e = b.cidx[c];
-        const uint32_t del = box_deletions<J>(b, e, b.state[ent_idx(e)] & b.cU[c]);
+        const uint32_t e = box_list(v, 1)[c];
+        const uint32_t del = box_deletions<J>(v, e, box_list(v, 2)[c]);
         words += ent_dist(e) == 0;
         any |= del != 0u;
-        b.cdel[c] = del;
+        box_list(v, 3)[c] = del;
     }
     if (!__syncthreads_or(any)) return;
     for (int c = threadIdx.x; c < nc; c += kResThreads) {
-        const uint32_t del = b.cdel[c];
+        const uint32_t del = box_list(v, 3)[c];
         if (del) {
-            const uint32_t e = b.cidx[c];
-            b.state[ent_idx(e)] &= ~del;
-            b.cidx[c] = e | kEntChanged;
+            const uint32_t e = box_list(v, 1)[c];
+            box_delete(e, del);
+            box_list(v, 1)[c] = e | kEntChanged;
         }
     }
     __syncthreads();
 }
 
-// ... with at most one: its word, union and entry stay in registers
+// ... with at most one: its union and entry stay in registers
 template <int J>
-__device__ __forceinline__ void box_subiteration1(const Box3D b, uint32_t e, uint32_t un, uint32_t &val, unsigned &words)
+__device__ __forceinline__ void box_subiteration1(const Box3D &v, uint32_t &e, uint32_t un, unsigned &words)
 {
-    const uint32_t del = box_deletions<J>(b, e, val & un);
+    const uint32_t del = un ? box_deletions<J>(v, e, un) : 0u;
     words += un != 0u && ent_dist(e) == 0;
     if (!__syncthreads_or(del != 0u)) return;
     if (del) {
-        val &= ~del;
-        b.state[ent_idx(e)] = val;
+        box_delete(e, del);
+        e |= kEntChanged;
     }
     __syncthreads();
+}
+
+// An iteration on the lists.  Returns whether a word of the core changed.
+__device__ __forceinline__ bool box_iteration(Box3D &v, int iter, unsigned &words, unsigned &entries)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t *const list = box_list(v, 0);
+    uint16_t *const alist = reinterpret_cast<uint16_t *>(box_list(v, 4));
+    const int nl = v.nl;
+    // active words: a word of the row's 3x3 rows that is at most one column
+    // away changed in the previous iteration (otherwise its union is empty),
+    // and some voxel of it misses one of its face neighbours
+    for (int base = warp * 32; base < nl; base += kResThreads) {
+        const int k = base + lane;
+        bool on = false;
+        if (k < nl) {
+            const uint32_t e = list[k], idx = ent_idx(e);
+            uint32_t y2;
+            const uint32_t z2 = box_plane_row(v, idx, y2);
+            if ((res_smem[v.act + (int)(z2 * (uint32_t)v.my + y2)] >> ent_col(e)) & 1u) {
+                const uint32_t *s = box_state() + idx;
+                const uint32_t c = *s;
+                const uint32_t faces = (c << 1) & (c >> 1) & s[v.p] & s[-v.p] & s[v.ps] & s[-v.ps];
+                on = (c & kCoreBits & ~faces) != 0u;
+            }
+        }
+        const int pos = warp_append(on, &v.n[1]);
+        if (pos >= 0) alist[pos] = (uint16_t)k;
+    }
+    __syncthreads();
+    const int na = v.n[1];
+    // pre-test and U
+    for (int base = warp * 32; base < na; base += kResThreads) {
+        const int k = base + lane;
+        uint32_t e = 0, un = 0, du = 0;
+        if (k < na) {
+            e = list[alist[k]];
+            uint32_t g[27];
+            const uint32_t val = box_window(box_state() + ent_idx(e), v.p, v.ps, g);
+            du = rule3d<0>(g) & val;
+            un = (du | rule3d<1>(g) | rule3d<2>(g) | rule3d<3>(g) | rule3d<4>(g) | rule3d<5>(g)) & val;
+            words += ent_dist(e) == 0;
+            entries++;
+        }
+        const int c = warp_append(un != 0u, &v.n[2]);
+        if (c >= 0) {
+            box_list(v, 1)[c] = e;
+            box_list(v, 2)[c] = un;
+            box_list(v, 3)[c] = du;
+        }
+    }
+    __syncthreads();
+    const int nc = v.n[2];
+    bool core = false;
+    if (nc > kResThreads) {
+        for (int c = threadIdx.x; c < nc; c += kResThreads) {
+            const uint32_t del = box_list(v, 3)[c];
+            if (del) {
+                const uint32_t e = box_list(v, 1)[c];
+                box_delete(e, del);
+                box_list(v, 1)[c] = e | kEntChanged;
+            }
+        }
+        __syncthreads();
+        box_subiteration<1>(v, nc, words);
+        box_subiteration<2>(v, nc, words);
+        box_subiteration<3>(v, nc, words);
+        box_subiteration<4>(v, nc, words);
+        box_subiteration<5>(v, nc, words);
+        for (int c = threadIdx.x; c < nc; c += kResThreads) {
+            const uint32_t e = box_list(v, 1)[c];
+            if (!(e & kEntChanged) || ent_dist(e) != 0) continue;
+            core = true;
+            box_changed(v, ent_idx(e), ent_col(e), iter);
+        }
+    } else if (nc > 0) {
+        const int c = threadIdx.x;
+        uint32_t e = 0, un = 0;
+        if (c < nc) {
+            e = box_list(v, 1)[c];
+            un = box_list(v, 2)[c];
+            const uint32_t del = box_list(v, 3)[c];
+            if (del) {
+                box_delete(e, del);
+                e |= kEntChanged;
+            }
+        }
+        __syncthreads();
+        box_subiteration1<1>(v, e, un, words);
+        box_subiteration1<2>(v, e, un, words);
+        box_subiteration1<3>(v, e, un, words);
+        box_subiteration1<4>(v, e, un, words);
+        box_subiteration1<5>(v, e, un, words);
+        if ((e & kEntChanged) && ent_dist(e) == 0) {
+            core = true;
+            box_changed(v, ent_idx(e), ent_col(e), iter);
+        }
+    }
+    return core;
+}
+
+// The same on all words of the box, for one with more non-empty words than its
+// lists hold: a thread keeps the unions and deletions of its words.
+static __device__ __noinline__ bool box_iteration_dense(Box3D &v, int iter, unsigned &words, unsigned &entries)
+{
+    uint32_t un[kDenseWords], del[kDenseWords];
+    bool core = false;
+    const int nbox = (v.z1 - v.z0) * (v.y1 - v.y0) * v.wl;
+    const WordWalk walk(v.wl, v.y1 - v.y0);
+    WordPos q = walk.first();
+    int k = 0;
+    for (int i = threadIdx.x; i < nbox; i += kResThreads, walk.next(q), k++) {
+        const int d = box_dist(v, q);
+        const uint32_t *s = box_state() + box_index(v, q);
+        un[k] = del[k] = 0;
+        if (d <= 5 && (*s & kCoreBits) && ((res_smem[v.act + (q.z + 1) * v.my + q.y + 1] >> (q.x >> v.xs)) & 1u)) {
+            uint32_t g[27];
+            const uint32_t val = box_window(s, v.p, v.ps, g), du = rule3d<0>(g) & val;
+            del[k] = du;
+            un[k] = (du | rule3d<1>(g) | rule3d<2>(g) | rule3d<3>(g) | rule3d<4>(g) | rule3d<5>(g)) & val;
+            words += d == 0;
+            entries++;
+        }
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int j = 0; j < 6; j++) {
+        // deletions of subiteration j were found: apply them, then find the next one's
+        q = walk.first();
+        k = 0;
+        for (int i = threadIdx.x; i < nbox; i += kResThreads, walk.next(q), k++)
+            if (del[k]) box_delete(box_entry(v, q, box_index(v, q), 0), del[k]);
+        __syncthreads();
+        if (j == 5) break;
+        q = walk.first();
+        k = 0;
+        for (int i = threadIdx.x; i < nbox; i += kResThreads, walk.next(q), k++) {
+            del[k] = 0;
+            if (!un[k] || box_dist(v, q) > 4 - j) continue;
+            const uint32_t *s = box_state() + box_index(v, q);
+            if (!(*s & un[k])) continue;
+            uint32_t g[27];
+            const uint32_t cand = box_window(s, v.p, v.ps, g) & un[k];
+            del[k] = cand & (j == 0   ? rule3d<1>(g)
+                             : j == 1 ? rule3d<2>(g)
+                             : j == 2 ? rule3d<3>(g)
+                             : j == 3 ? rule3d<4>(g)
+                                      : rule3d<5>(g));
+            words += box_dist(v, q) == 0;
+        }
+        __syncthreads();
+    }
+    // only voxels of the union were deleted: a word changed when it lost some of its union
+    q = walk.first();
+    k = 0;
+    for (int i = threadIdx.x; i < nbox; i += kResThreads, walk.next(q), k++) {
+        const int idx = box_index(v, q);
+        if (!(un[k] & ~box_state()[idx]) || box_dist(v, q) != 0) continue;
+        core = true;
+        box_changed(v, (uint32_t)idx, (uint32_t)(q.x >> v.xs), iter);
+    }
+    return core;
 }
 
 // One volume, or one box of it: rows [c0, c1) of planes [r0, r1) are the
@@ -670,339 +964,157 @@ __device__ __forceinline__ void box_subiteration1(const Box3D b, uint32_t e, uin
 // edge that changed to a list in global memory, the boxes meet, and each
 // takes over what lies in its halo from its neighbours' lists.
 //
-// Bound: the latency of an iteration (about 10 us: six dependent subiterations
+// Bound: the latency of an iteration (8 to 12 us: six dependent subiterations
 // with two barriers each, then the meeting), not throughput: a box has some
 // hundred active words.  Against warps marching through sparse bricks of
 // 32 x 32 x 4 voxels, every brick of the neighbourhood of a change evaluated
-// whole (24 us per iteration): a 97 x 75 x 66 tree volume 214 -> 72 us, a
-// 187 x 203 x 161 one 955 -> 150 us, a 256^3 one, whose bricks did not fit,
-// 1330 us on the tile rings -> 176 us.
-__device__ void res_run3d(Inst &in, const ResIO &io, const ResItem &it, uint8_t *smb, ResSched *S)
+// whole (24 us per iteration): a 97 x 75 x 66 tree volume 214 -> 85 us, a
+// 187 x 203 x 161 one (16-bit pixels, transfers included) 955 -> 221 us, a
+// 256^3 one, whose bricks did not fit, 1330 us on the tile rings -> 179 us.
+// Words of 32 voxels took the last two 238 and 193 us.
+__device__ void res_run3d(Inst &in, const ResIO &io, const ResItem &item, ResSched *S, ResTrace *tr)
 {
-    __shared__ int s_n[4];  // lengths: word list, active words, candidates, messages
-    __shared__ int s_flag;
+    __shared__ Box3D v;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int H = in.H, D = in.D, wl = (in.W + 31) >> 5;
-    const bool team = it.bands > 1;
-    const int z0 = max(0, it.r0 - it.halo), z1 = min(D, it.r1 + it.halo);
-    const int y0 = max(0, it.c0 - it.halo), y1 = min(H, it.c1 + it.halo);
-    const int nz = z1 - z0, ny = y1 - y0, ny2 = ny + 2, rows2 = (nz + 2) * ny2;
-    int xs = 0;  // words per column of the change masks: 1 << xs
-    while (((wl - 1) >> xs) > 31) xs++;
-    Box3D b;
-    b.p = wl + 1;
-    b.ps = ny2 * b.p;
-    const uint32_t mp = 0xffffffffu / (uint32_t)b.p + 1u;
-    const uint32_t mny = 0xffffffffu / (uint32_t)ny2 + 1u;
-    const int nwords = rows2 * b.p + 1;
-    size_t off = 0;
-    b.state = reinterpret_cast<uint32_t *>(smb);
-    off += up16((size_t)nwords * 4);
-    uint32_t *const act = reinterpret_cast<uint32_t *>(smb + off);
-    off += up16((size_t)rows2 * 4);
-    uint32_t *const chg = reinterpret_cast<uint32_t *>(smb + off);
-    off += up16((size_t)rows2 * 4);
-    uint32_t *const list = reinterpret_cast<uint32_t *>(smb + off);
-    const int list_cap = (int)(((size_t)kSmemBytes - off) / 4);
-
-    for (size_t i = threadIdx.x; i < off / 16; i += kResThreads) reinterpret_cast<uint4 *>(smb)[i] = make_uint4(0, 0, 0, 0);
-    if (threadIdx.x < 4) s_n[threadIdx.x] = 0;
+    if (threadIdx.x == 0) {
+        v.it = item;
+        v.H = in.H;
+        v.D = in.D;
+        v.wl = (in.W + kVox - 1) / kVox;
+        v.z0 = max(0, item.r0 - item.halo);
+        v.z1 = min(in.D, item.r1 + item.halo);
+        v.y0 = max(0, item.c0 - item.halo);
+        v.y1 = min(in.H, item.c1 + item.halo);
+        const int nz = v.z1 - v.z0, ny = v.y1 - v.y0;
+        v.p = v.wl | 1;  // odd strides: rows and planes start on different banks
+        v.ps = ((ny + 2) * v.p) | 1;
+        v.mp = 0xffffffffu / (uint32_t)v.p + 1u;
+        v.mps = 0xffffffffu / (uint32_t)v.ps + 1u;
+        v.my = (ny + 5) & ~3;
+        v.mrows = (nz + 2) * v.my;
+        v.xs = 0;
+        while (((v.wl - 1) >> v.xs) > 7) v.xs++;
+        v.act = (int)up16((size_t)(nz + 2) * v.ps * 4);
+        v.chg = v.act + (int)up16((size_t)v.mrows);
+        v.list = v.chg + (int)up16((size_t)v.mrows);
+        v.gy = in.res_gy;
+        v.gz = item.bands / v.gy;
+        v.bz = item.band / v.gy;
+        v.by = item.band - v.bz * v.gy;
+        v.stride = in.res_stride;
+        v.msgs = in.res_msg;
+        v.counts = in.res_cnt;
+        v.meet = MeetState{0, 0, 0};
+        v.nl = 0;
+        for (int k = 0; k < 4; k++) v.n[k] = 0;
+    }
     __syncthreads();
-    const int nbox = nz * ny * wl;
-    const WordWalk walk(wl, ny);
-    auto dist_of = [&](const WordPos &q) {
-        const int y = y0 + q.y, z = z0 + q.z;
-        return max(max(max(it.c0 - y, y - it.c1 + 1), max(it.r0 - z, z - it.r1 + 1)), 0);
-    };
-    auto index_of = [&](const WordPos &q) { return ((q.z + 1) * ny2 + q.y + 1) * b.p + 1 + q.x; };
-    res_load(in, io, walk, nbox, 0, y0, z0, [&](bool, const WordPos &q, uint32_t v) {
-        const int d = dist_of(q), idx = v ? index_of(q) : 0;
-        if (v) b.state[idx] = v;
-        const int pos = warp_append(v != 0u && d <= 5, &s_n[0]);
-        if (pos >= 0 && pos < list_cap) list[pos] = (uint32_t)idx | (uint32_t)(q.x >> xs) << 16 | (uint32_t)d << 21;
-    });
+    for (int i = threadIdx.x; i < v.list / 16; i += kResThreads) reinterpret_cast<uint4 *>(res_smem)[i] = make_uint4(0, 0, 0, 0);
     __syncthreads();
-    const int nl = s_n[0];
-    MeetState meet;
+    {
+        const int list_cap = (kSmemBytes - v.list) / 4, nz = v.z1 - v.z0, ny = v.y1 - v.y0;
+        res_load<true>(in, io, WordWalk(v.wl, ny), nz * ny * v.wl, 0, v.y0, v.z0,
+                       [&](bool, const WordPos &q, uint32_t w) {
+                           const int d = box_dist(v, q), idx = w ? box_index(v, q) : 0;
+                           if (w) box_state()[idx] = w;
+                           const int pos = warp_append((w & kCoreBits) != 0u && d <= 5, &v.n[0]);
+                           if (pos >= 0 && pos < list_cap) box_words(v.list)[pos] = box_entry(v, q, idx, d);
+                       });
+    }
+    for (int r = threadIdx.x; r < v.mrows / 4; r += kResThreads) box_words(v.act)[r] = kFull;
+    __syncthreads();
     // more non-empty words than the lists hold: go over all words of the box
-    const bool dense = off + (size_t)nl * kBoxListBytes + 64 > (size_t)kSmemBytes;
-    b.cidx = list + nl;
-    b.cU = b.cidx + nl;
-    b.cdel = b.cU + nl;
-    uint16_t *const alist = reinterpret_cast<uint16_t *>(b.cdel + nl);
-    for (int r = threadIdx.x; r < rows2; r += kResThreads) act[r] = kFull;
+    const bool dense = v.list + (size_t)v.n[0] * kBoxListBytes + 64 > (size_t)kSmemBytes;
+    if (threadIdx.x == 0) v.nl = v.n[0];
     __syncthreads();
 
-    const int gy = in.res_gy;  // boxes along y
-    const int bz = it.band / gy, by = it.band - bz * gy, gz = it.bands / gy;
     int iter = 0, result = 0;
     unsigned words = 0, entries = 0;
-    const int cap_it = in.pass_cap / 6 + 1;
-    // a word of the core changed: mark it, and tell the boxes around when it lies near the core's edge
-    auto changed = [&](uint32_t idx, uint32_t col, uint2 *msg) {
-        const uint32_t row = __umulhi(idx, mp);
-        atomicOr(&chg[row], 1u << col);
-        if (!team) return;
-        const int zz = (int)__umulhi(row, mny), y = y0 + (int)row - zz * ny2 - 1, z = z0 + zz - 1;
-        const int h = it.halo;
-        if ((it.r0 > 0 && z < it.r0 + h) || (it.r1 < D && z >= it.r1 - h) || (it.c0 > 0 && y < it.c0 + h) ||
-            (it.c1 < H && y >= it.c1 - h)) {
-            const int x = (int)idx - (int)row * b.p - 1;
-            msg[atomicAdd(&s_n[3], 1)] =
-                make_uint2(((uint32_t)z * (uint32_t)H + (uint32_t)y) * (uint32_t)wl + (uint32_t)x, b.state[idx]);
-        }
-    };
     for (;; iter++) {
-        bool core = false;
-        uint2 *msg = nullptr;
-        if (team) msg = in.res_msg + ((size_t)(iter & 1) * it.bands + it.band) * in.res_stride;
-        if (!dense) {
-            // active words: a word of the row's 3x3 rows that is at most one
-            // column away changed in the previous iteration (otherwise its union
-            // is empty), and some voxel of it misses one of its face neighbours
-            for (int base = warp * 32; base < nl; base += kResThreads) {
-                const int k = base + lane;
-                bool on = false;
-                if (k < nl) {
-                    const uint32_t e = list[k], idx = ent_idx(e);
-                    if ((act[__umulhi(idx, mp)] >> ent_col(e)) & 1u) {
-                        const uint32_t *s = b.state + idx;
-                        const uint32_t c = *s;
-                        const uint32_t faces = at_xm1(c, s[-1]) & at_xp1(c, s[1]) & s[b.p] & s[-b.p] & s[b.ps] & s[-b.ps];
-                        on = (c & ~faces) != 0u;
-                    }
-                }
-                const int pos = warp_append(on, &s_n[1]);
-                if (pos >= 0) alist[pos] = (uint16_t)k;
-            }
-            __syncthreads();
-            const int na = s_n[1];
-            // pre-test and U
-            for (int base = warp * 32; base < na; base += kResThreads) {
-                const int k = base + lane;
-                uint32_t e = 0, un = 0, du = 0;
-                if (k < na) {
-                    e = list[alist[k]];
-                    const uint32_t *s = b.state + ent_idx(e);
-                    uint32_t g[27];
-                    box_window(s, b.p, b.ps, g);
-                    du = rule3d<0>(g) & g[13];
-                    un = (du | rule3d<1>(g) | rule3d<2>(g) | rule3d<3>(g) | rule3d<4>(g) | rule3d<5>(g)) & g[13];
-                    words += ent_dist(e) == 0;
-                    entries++;
-                }
-                const int c = warp_append(un != 0u, &s_n[2]);
-                if (c >= 0) {
-                    b.cidx[c] = e;
-                    b.cU[c] = un;
-                    b.cdel[c] = du;
-                }
-            }
-            __syncthreads();
-            const int nc = s_n[2];
-            if (nc > kResThreads) {
-                for (int c = threadIdx.x; c < nc; c += kResThreads) {
-                    const uint32_t del = b.cdel[c];
-                    if (del) {
-                        const uint32_t e = b.cidx[c];
-                        b.state[ent_idx(e)] &= ~del;
-                        b.cidx[c] = e | kEntChanged;
-                    }
-                }
-                __syncthreads();
-                box_subiteration<1>(b, nc, words);
-                box_subiteration<2>(b, nc, words);
-                box_subiteration<3>(b, nc, words);
-                box_subiteration<4>(b, nc, words);
-                box_subiteration<5>(b, nc, words);
-            } else if (nc > 0) {
-                const int c = threadIdx.x;
-                uint32_t e = 0, un = 0, val = 0, del = 0;
-                if (c < nc) {
-                    e = b.cidx[c];
-                    un = b.cU[c];
-                    del = b.cdel[c];
-                    val = b.state[ent_idx(e)];
-                }
-                const uint32_t before = val;
-                if (del) {
-                    val &= ~del;
-                    b.state[ent_idx(e)] = val;
-                }
-                __syncthreads();
-                box_subiteration1<1>(b, e, un, val, words);
-                box_subiteration1<2>(b, e, un, val, words);
-                box_subiteration1<3>(b, e, un, val, words);
-                box_subiteration1<4>(b, e, un, val, words);
-                box_subiteration1<5>(b, e, un, val, words);
-                if (val != before) b.cidx[c] = e | kEntChanged;
-            }
-            for (int c = threadIdx.x; c < nc; c += kResThreads) {
-                const uint32_t e = b.cidx[c];
-                if (!(e & kEntChanged) || ent_dist(e) != 0) continue;
-                core = true;
-                changed(ent_idx(e), ent_col(e), msg);
-            }
-        } else {
-            uint32_t un[kDenseWords], del[kDenseWords];  // of this thread's words
-            WordPos q = walk.first();
-            int k = 0;
-            for (int i = threadIdx.x; i < nbox; i += kResThreads, walk.next(q), k++) {
-                const int d = dist_of(q);
-                const uint32_t *s = b.state + index_of(q);
-                un[k] = del[k] = 0;
-                if (d <= 5 && *s && ((act[(q.z + 1) * ny2 + q.y + 1] >> (q.x >> xs)) & 1u)) {
-                    uint32_t g[27];
-                    box_window(s, b.p, b.ps, g);
-                    const uint32_t du = rule3d<0>(g) & g[13];
-                    del[k] = du;
-                    un[k] = (du | rule3d<1>(g) | rule3d<2>(g) | rule3d<3>(g) | rule3d<4>(g) | rule3d<5>(g)) & g[13];
-                    words += d == 0;
-                    entries++;
-                }
-            }
-            __syncthreads();
-#pragma unroll 1
-            for (int j = 0; j < 6; j++) {
-                // deletions of subiteration j were found: apply them, then find the next one's
-                q = walk.first();
-                k = 0;
-                for (int i = threadIdx.x; i < nbox; i += kResThreads, walk.next(q), k++)
-                    if (del[k]) b.state[index_of(q)] &= ~del[k];
-                __syncthreads();
-                if (j == 5) break;
-                q = walk.first();
-                k = 0;
-                for (int i = threadIdx.x; i < nbox; i += kResThreads, walk.next(q), k++) {
-                    del[k] = 0;
-                    if (!un[k] || dist_of(q) > 4 - j) continue;
-                    const uint32_t *s = b.state + index_of(q);
-                    const uint32_t cand = *s & un[k];
-                    if (!cand) continue;
-                    uint32_t g[27];
-                    box_window(s, b.p, b.ps, g);
-                    del[k] = cand & (j == 0   ? rule3d<1>(g)
-                                     : j == 1 ? rule3d<2>(g)
-                                     : j == 2 ? rule3d<3>(g)
-                                     : j == 3 ? rule3d<4>(g)
-                                              : rule3d<5>(g));
-                    words += dist_of(q) == 0;
-                }
-                __syncthreads();
-            }
-            // only voxels of the union were deleted: a word changed when it lost some of its union
-            q = walk.first();
-            k = 0;
-            for (int i = threadIdx.x; i < nbox; i += kResThreads, walk.next(q), k++) {
-                const int idx = index_of(q);
-                if (!(un[k] & ~b.state[idx]) || dist_of(q) != 0) continue;
-                core = true;
-                changed((uint32_t)idx, (uint32_t)(q.x >> xs), msg);
-            }
-        }
+        const bool core = dense ? box_iteration_dense(v, iter, words, entries) : box_iteration(v, iter, words, entries);
         const bool any = __syncthreads_or(core);
         bool any_chg = any;
-        if (!team) {
+        if (v.it.bands == 1) {
             if (!any) {
                 result = 1;
                 break;
             }
         } else {
             if (threadIdx.x == 0) {
-                in.res_cnt[(iter & 1) * it.bands + it.band] = s_n[3];
-                s_flag = res_meet(in.res_meet, it.bands, any, meet, S->timeout_ns);
-                if (s_flag == 2) atomicOr(&S->status, kErrQueueTimeout);
+                v.counts[(iter & 1) * v.it.bands + v.it.band] = v.n[3];
+                v.flag = res_meet(in.res_meet, v.it.bands, any, v.meet, S->timeout_ns);
+                if (v.flag == 2) atomicOr(&S->status, kErrQueueTimeout);
             }
             __syncthreads();
-            const int f = s_flag;
-            if (f != 1) {
-                result = f == 0 ? 1 : -1;
+            if (v.flag != 1) {
+                result = v.flag == 0 ? 1 : -1;
                 break;
             }
             // kWarps / 8 warps per neighbouring box take over its messages
             const int k8 = warp & 7, k9 = k8 < 4 ? k8 : k8 + 1;
-            const int nbz = bz + k9 / 3 - 1, nby = by + k9 % 3 - 1;
-            if (warp < kWarps / 8 * 8 && nbz >= 0 && nbz < gz && nby >= 0 && nby < gy) {
-                const int nb = nbz * gy + nby;
-                const uint2 *m = in.res_msg + ((size_t)(iter & 1) * it.bands + nb) * in.res_stride;
+            const int nbz = v.bz + k9 / 3 - 1, nby = v.by + k9 % 3 - 1;
+            if (warp < kWarps / 8 * 8 && nbz >= 0 && nbz < v.gz && nby >= 0 && nby < v.gy) {
+                const int nb = nbz * v.gy + nby;
+                const uint2 *m = v.msgs + ((size_t)(iter & 1) * v.it.bands + nb) * v.stride;
                 const int k0 = (warp >> 3) * 32 + lane;
                 // the first message is loaded beside the count, whether it is one or not
-                uint2 v = k0 < in.res_stride ? __ldcg(m + k0) : make_uint2(0u, 0u);
-                const int n = __ldcg(in.res_cnt + (iter & 1) * it.bands + nb);
+                uint2 w = k0 < v.stride ? __ldcg(m + k0) : make_uint2(0u, 0u);
+                const int n = __ldcg(v.counts + (iter & 1) * v.it.bands + nb);
                 for (int k = k0; k < n;) {
-                    const int r = (int)(v.x / (uint32_t)wl), x = (int)v.x - r * wl, z = r / H, y = r - z * H;
-                    if (z >= z0 && z < z1 && y >= y0 && y < y1) {
-                        const int row = (z - z0 + 1) * ny2 + (y - y0 + 1);
-                        b.state[row * b.p + 1 + x] = v.y;
-                        atomicOr(&chg[row], 1u << (x >> xs));
+                    const int r = (int)(w.x / (uint32_t)v.wl), x = (int)w.x - r * v.wl, z = r / v.H, y = r - z * v.H;
+                    if (z >= v.z0 && z < v.z1 && y >= v.y0 && y < v.y1) {
+                        uint32_t *s = box_state() + (z - v.z0 + 1) * v.ps + (y - v.y0 + 1) * v.p + x;
+                        atomicAnd(s, w.y);
+                        if (!(w.y & 2u) && x > 0) atomicAnd(s - 1, ~(1u << 31));
+                        if (!(w.y & (1u << kVox)) && x + 1 < v.wl) atomicAnd(s + 1, ~1u);
+                        box_mark(v, (z - v.z0 + 1) * v.my + (y - v.y0 + 1), x >> v.xs);
                         any_chg = true;
                     }
                     k += (kWarps / 8) * 32;
-                    if (k < n) v = __ldcg(m + k);
+                    if (k < n) w = __ldcg(m + k);
                 }
             }
             any_chg = __syncthreads_or(any_chg);
         }
-        if (iter + 1 >= cap_it) {
+        if (iter + 1 >= in.pass_cap / 6 + 1) {
             if (threadIdx.x == 0) atomicOr(&S->status, kErrPassLimit);
             result = -1;
             break;
         }
-        // rows to look at in the next iteration
-        for (int r = threadIdx.x + ny2; r < rows2 - ny2; r += kResThreads) {
+        // rows to look at in the next iteration, four at a time, a byte each (my
+        // is a multiple of 4; the bytes before the first and after the last row
+        // belong to rows of padding)
+        const int my4 = v.my / 4;
+        for (int w = threadIdx.x + my4; w < v.mrows / 4 - my4; w += kResThreads) {
             uint32_t m = 0;
             if (any_chg) {
-                const uint32_t *c = chg + r;
+                const uint32_t *c = box_words(v.chg) + w;
 #pragma unroll
-                for (int k = 0; k < 9; k++) m |= c[(k / 3 - 1) * ny2 + (k % 3 - 1)];
+                for (int dz = -1; dz <= 1; dz++) {
+                    const uint32_t *r = c + dz * my4;
+                    m |= r[0] | __funnelshift_l(r[-1], r[0], 8) | __funnelshift_r(r[0], r[1], 8);
+                }
             }
-            act[r] = m | m << 1 | m >> 1;
+            box_words(v.act)[w] = m | ((m << 1) & 0xFEFEFEFEu) | ((m >> 1) & 0x7F7F7F7Fu);
         }
-        if (threadIdx.x >= 1 && threadIdx.x < 4) s_n[threadIdx.x] = 0;
+        if (threadIdx.x >= 1 && threadIdx.x < 4) v.n[threadIdx.x] = 0;
         __syncthreads();
         if (any_chg)
-            for (int r = threadIdx.x; r < rows2; r += kResThreads) chg[r] = 0u;
+            for (int r = threadIdx.x; r < v.mrows / 4; r += kResThreads) box_words(v.chg)[r] = 0u;
         // (chg is next written after the barriers of the next iteration)
     }
     __syncthreads();
     // the converged core
-    res_store(in, io, 0, wl, it.c1 - it.c0, it.r1 - it.r0, it.c0, it.r0, [&](int y, int z) {
-        return b.state + ((z + it.r0 - z0 + 1) * ny2 + (y + it.c0 - y0 + 1)) * b.p + 1;
+    res_store(in, io, 0, (in.W + 31) >> 5, v.it.c1 - v.it.c0, v.it.r1 - v.it.r0, v.it.c0, v.it.r0, [&](int y, int z, int x) {
+        // 32 voxels from x on: the rest of its word, then the next word's from its second voxel on
+        const int j = x / kVox, o = x - j * kVox;
+        const uint32_t *s = box_state() + (z + v.it.r0 - v.z0 + 1) * v.ps + (y + v.it.c0 - v.y0 + 1) * v.p + j;
+        return s[0] >> (o + 1) | (j + 1 < v.wl ? s[1] >> 2 << (kVox + 1 - o) : 0u);
     });
-    words = __reduce_add_sync(kFull, words);
-    entries = __reduce_add_sync(kFull, entries);
-    if (lane == 0 && words) {
-        atomicAdd(&in.work_words, (unsigned long long)words);
-        atomicAdd(&in.tiles_run, (unsigned long long)entries);
-    }
-    if (threadIdx.x == 0) {
-        if (it.band == 0) in.passes_run = 6 * (iter + 1);
-        if (result < 0) atomicMin(&in.converged, -1);
-    }
-    __syncthreads();
+    res_done(in, v.it, result, 6 * (iter + 1), words, entries, tr);
 }
 
 // ------------------------------------------------------------ kernels -----
-__global__ void resident_reset_kernel(Inst *insts, int n, ResSched *S, int nitems, long long timeout_ns)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        Inst &in = insts[i];
-        in.res_meet[0] = in.res_meet[1] = 0;
-        if (in.res) {
-            in.converged = 1;  // lowered to -1 by a band that fails
-            in.passes_run = 0;
-            in.tiles_run = 0;
-            in.work_words = 0;
-        }
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        S->head = 0;
-        S->nitems = nitems;
-        S->status = 0;
-        S->timeout_ns = timeout_ns;
-    }
-}
-
 __device__ __forceinline__ int res_smid()
 {
     int v;
@@ -1014,11 +1126,14 @@ __global__ void __launch_bounds__(kResThreads, kResCtasPerSm)
     resident_kernel(Inst *insts, const ResItem *items, ResSched *S, ResTrace *trace, const IODesc *ios, bool pix,
                     const __grid_constant__ IODesc one)
 {
-    extern __shared__ __align__(16) uint8_t res_smem[];
     __shared__ int s_item;
     __shared__ int s_take[2];
     for (;;) {
-        if (threadIdx.x == 0) s_item = atomicAdd(&S->head, 1);
+        if (threadIdx.x == 0) {
+            s_item = atomicAdd(&S->head, 1);
+            // the run's errors come after its first item was taken: waits of seconds and pass caps
+            if (s_item == 0) S->status = 0;
+        }
         __syncthreads();
         const int k = s_item;
         __syncthreads();
@@ -1033,13 +1148,22 @@ __global__ void __launch_bounds__(kResThreads, kResCtasPerSm)
             const int nr = min(in.H, it.r1 + it.halo) - max(0, it.r0 - it.halo);
             uint32_t *sm = reinterpret_cast<uint32_t *>(res_smem);
             switch (res_unit_words(nr, nw)) {
-            case 2: res_run2d<2>(in, io, it, sm, S, s_take); break;
-            case 4: res_run2d<4>(in, io, it, sm, S, s_take); break;
-            default: res_run2d<8>(in, io, it, sm, S, s_take); break;
+            case 2: res_run2d<2>(in, io, it, sm, S, s_take, trace + k); break;
+            case 4: res_run2d<4>(in, io, it, sm, S, s_take, trace + k); break;
+            default: res_run2d<8>(in, io, it, sm, S, s_take, trace + k); break;
             }
         } else
-            res_run3d(in, io, it, res_smem, S);
-        if (threadIdx.x == 0) trace[k] = ResTrace{t0, (long long)globaltimer(), res_smid(), 0};
+            res_run3d(in, io, it, S, trace + k);
+        if (threadIdx.x == 0) {
+            trace[k].t0 = t0;
+            trace[k].t1 = (long long)globaltimer();
+            trace[k].sm = res_smid();
+        }
+    }
+    // the last CTA leaves the item counter as the next run needs it
+    if (threadIdx.x == 0 && atomicAdd(&S->done, 1) == (int)gridDim.x - 1) {
+        S->head = 0;
+        S->done = 0;
     }
 }
 
@@ -1052,9 +1176,9 @@ cudaError_t res_occupancy(int *per_sm)
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, resident_kernel, kResThreads, kSmemBytes);
 }
 
-cudaError_t launch_resident(int grid, Inst *d_insts, int ninst, const ResItem *d_items, int nitems,
-                            ResSched *d_rs, ResTrace *d_trace, long long timeout_ns, const IODesc *d_io,
-                            const IODesc *one, bool pixels, cudaStream_t st)
+cudaError_t launch_resident(int grid, Inst *d_insts, const ResItem *d_items, int nitems, ResSched *d_rs,
+                            ResTrace *d_trace, const IODesc *d_io, const IODesc *one, bool pixels, bool teams,
+                            cudaStream_t st)
 {
     if (nitems == 0) return cudaSuccess;
     static bool attr_done = false;
@@ -1065,10 +1189,6 @@ cudaError_t launch_resident(int grid, Inst *d_insts, int ninst, const ResItem *d
         if (e != cudaSuccess) return e;
         attr_done = true;
     }
-    resident_reset_kernel<<<std::max(1, std::min(64, (ninst + 255) / 256)), 256, 0, st>>>(d_insts, ninst, d_rs, nitems,
-                                                                                       timeout_ns);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
     // cooperative: all CTAs are resident at once, which the bands of an image
     // (waiting for one another) rely on
     cudaLaunchConfig_t cfg = {};
@@ -1080,7 +1200,7 @@ cudaError_t launch_resident(int grid, Inst *d_insts, int ninst, const ResItem *d
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = teams ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, resident_kernel, d_insts, d_items, d_rs, d_trace, one ? nullptr : d_io, pixels,
                               one ? *one : IODesc{});
 }
