@@ -15,7 +15,7 @@ EXPORTS = [
     "bgt_ctx_create", "bgt_ctx_destroy", "bgt_ctx_set_stream", "bgt_last_error", "bgt_version",
     "bgt_thin2d", "bgt_thin3d", "bgt_thin2d_device", "bgt_thin3d_device", "bgt_thin2d_device_noalloc",
     "bgt_centerline2d", "bgt_centerline3d", "bgt_free", "bgt_matlab_segments",
-    "bgt_segments2d_device", "bgt_segments3d_device",
+    "bgt_segments2d_device", "bgt_segments3d_device", "bgt_segments_begin", "bgt_segments_take",
     "bgt_batch_create", "bgt_batch_destroy", "bgt_batch_add2d", "bgt_batch_add3d", "bgt_batch_finalize",
     "bgt_batch_reserve", "bgt_batch_reset", "bgt_batch_set_grid",
     "bgt_batch_set_io", "bgt_batch_run", "bgt_batch_instance_stats", "bgt_batch_device_bytes", "bgt_batch_work", "bgt_batch_stage_ms",
@@ -58,6 +58,8 @@ def _declare(L):
         "bgt_thin2d_device_noalloc": [I, I, vp, I, I, vp, vp],
         "bgt_centerline2d": [vp, I, vp, I, I, I, I, fpp, fpp, upp, up],
         "bgt_centerline3d": [vp, I, vp, I, I, I, I, I, fpp, fpp, fpp, upp, up],
+        "bgt_segments_begin": [vp, I, I, vp, I, I, I, ip, ip],
+        "bgt_segments_take": [vp, vp, vp, vp],
         "bgt_segments2d_device": [vp, I, vp, I, I, C.POINTER(C.POINTER(C.c_int32)),
                                   C.POINTER(C.POINTER(C.c_uint8)), C.POINTER(C.POINTER(C.c_int16)),
                                   C.POINTER(C.POINTER(C.c_int16)), ip, ip],

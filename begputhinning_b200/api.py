@@ -221,27 +221,16 @@ def ExtractSegmentsV(data, ctx: Context | None = None) -> Segments:
     t = t.cuda().contiguous() if not t.is_cuda else t.contiguous()
     ctx = ctx or default_context(t.device.index or 0)
     code = torch_dtype_code(t)
-    st = C.POINTER(C.c_int32)()
-    ie = C.POINTER(C.c_uint8)()
-    px, py, pz = C.POINTER(C.c_int16)(), C.POINTER(C.c_int16)(), C.POINTER(C.c_int16)()
+    dims = 2 if t.dim() == 2 else 3
+    d, h, w = (1, t.shape[0], t.shape[1]) if dims == 2 else (t.shape[0], t.shape[1], t.shape[2])
     ns, npt = C.c_int(), C.c_int()
     torch.cuda.current_stream(t.device).synchronize()
-    if t.dim() == 2:
-        check(lib().bgt_segments2d_device(ctx.h, code, t.data_ptr(), t.shape[1], t.shape[0], C.byref(st),
-                                          C.byref(ie), C.byref(px), C.byref(py), C.byref(ns), C.byref(npt)))
-        dims = 2
-    else:
-        check(lib().bgt_segments3d_device(ctx.h, code, t.data_ptr(), t.shape[2], t.shape[1], t.shape[0],
-                                          C.byref(st), C.byref(ie), C.byref(px), C.byref(py), C.byref(pz),
-                                          C.byref(ns), C.byref(npt)))
-        dims = 3
+    check(lib().bgt_segments_begin(ctx.h, dims, code, t.data_ptr(), w, h, d, C.byref(ns), C.byref(npt)))
     n, m = ns.value, npt.value
-    start = _take(st, n + 1, np.int32)
-    is_end = _take(ie, n, np.uint8)
-    cols = [_take(px, m, np.int16), _take(py, m, np.int16)]
-    if dims == 3:
-        cols.append(_take(pz, m, np.int16))
-    pts = np.stack(cols, axis=1) if m else np.zeros((0, dims), np.int16)
+    start = np.empty(n + 1, np.int32)
+    is_end = np.empty(n, np.uint8)
+    pts = np.empty((m, dims), np.int16)
+    check(lib().bgt_segments_take(ctx.h, _vp(start), _vp(is_end), _vp(pts)))
     return Segments(start, is_end, pts)
 
 

@@ -23,8 +23,8 @@ NVCC = os.environ.get("NVCC", "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 CU_SOURCES = ["kernels.cu", "resident.cu", "host.cu", "segments.cu", "segments_graph.cu", "centerline.cu", "noalloc.cu", "serve.cu"]
-CXX_SOURCES = ["dropin.cpp"]
-HEADERS = ["common.cuh", "pixels.cuh", "rules.cuh", "tiles.cuh", "kernels.cuh", "host.h"]
+CXX_SOURCES = ["dropin.cpp", "hostpix.cpp"]
+HEADERS = ["common.cuh", "pixels.cuh", "rules.cuh", "tiles.cuh", "kernels.cuh", "host.h", "hostpix.h"]
 
 LIB = os.path.join(PKG, "libbgt.so")
 SYNTH = os.path.join(PKG, "libbgt_synth.so")

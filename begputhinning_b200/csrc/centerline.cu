@@ -56,20 +56,72 @@ extern "C" int bgt_tune_get(int dims, int cls, int *cfg)
 }
 
 // ------------------------------------------------------------ segments ----
-static int segments_device(bgt_ctx *c, int dims, int dtype, const void *d_img, int W, int H, int D, HostSegs *hs)
+// Pack the image for the extraction.
+static int segments_pack(bgt_ctx *c, int dtype, const void *d_img, int W, int H, int D, const uint32_t **packed, int *P)
 {
     if (!c || !d_img) return fail(BGT_ERR_ARG, "null argument");
     if (dtype_size(dtype) == 0) return fail(BGT_ERR_ARG, "bad dtype %d", dtype);
     if (W < 1 || H < 1 || D < 1) return fail(BGT_ERR_ARG, "bad size");
     cudaSetDevice(c->device);
-    const int P = ((W + 31) / 32 + 3) / 4 * 4;
+    *P = ((W + 31) / 32 + 3) / 4 * 4;
     void *buf = nullptr;
-    int rc = ctx_scratch(c, 20, (size_t)P * H * D * 4, &buf);
+    int rc = ctx_scratch(c, 20, (size_t)*P * H * D * 4, &buf);
     if (rc != BGT_OK) return rc;
+    *packed = (const uint32_t *)buf;
     // ExtractSegmentsV tests pdata != 0 (2D/ExtractSegments.cpp:36, 3D/ExtractSegments.cpp:158)
-    cudaError_t e = launch_pack(dtype, 2, d_img, W, H, D, W, H, D, P, (uint32_t *)buf, nullptr, c->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "pack");
-    return segments_packed(c, dims, (const uint32_t *)buf, W, H, D, P, hs);
+    cudaError_t e = launch_pack(dtype, 2, d_img, W, H, D, W, H, D, *P, (uint32_t *)buf, nullptr, c->stream);
+    return e == cudaSuccess ? BGT_OK : cuda_fail(e, "pack");
+}
+
+static int segments_device(bgt_ctx *c, int dims, int dtype, const void *d_img, int W, int H, int D, HostSegs *hs)
+{
+    const uint32_t *buf = nullptr;
+    int P = 0;
+    int rc = segments_pack(c, dtype, d_img, W, H, D, &buf, &P);
+    return rc == BGT_OK ? segments_packed(c, dims, buf, W, H, D, P, hs) : rc;
+}
+
+extern "C" int bgt_segments_begin(bgt_ctx *c, int dims, int dtype, const void *d_img, int w, int h, int d, int *nseg,
+                                  int *npts)
+{
+    if (dims != 2 && dims != 3) return fail(BGT_ERR_ARG, "dims must be 2 or 3");
+    if (!nseg || !npts) return fail(BGT_ERR_ARG, "null output");
+    const uint32_t *buf = nullptr;
+    int P = 0;
+    int rc = segments_pack(c, dtype, d_img, w, h, dims == 3 ? d : 1, &buf, &P);
+    SegResult r;
+    if (rc == BGT_OK) rc = segments_result(c, dims, buf, w, h, dims == 3 ? d : 1, P, &r);
+    if (rc != BGT_OK) return rc;
+    c->view = r;
+    c->view_dims = dims;
+    *nseg = r.nseg;
+    *npts = r.npts;
+    return BGT_OK;
+}
+
+extern "C" int bgt_segments_take(bgt_ctx *c, int32_t *start, uint8_t *is_end, int16_t *points)
+{
+    if (!c || !start || !is_end || !points) return fail(BGT_ERR_ARG, "null argument");
+    if (!c->view_dims) return fail(BGT_ERR_STATE, "no segments to take: call bgt_segments_begin first");
+    const SegResult &r = c->view;
+    start[0] = 0;
+    if (r.nseg > 0) {
+        memcpy(start, r.start, (size_t)(r.nseg + 1) * 4);
+        memcpy(is_end, r.is_end, (size_t)r.nseg);
+        if (c->view_dims == 2)
+            for (int i = 0; i < r.npts; i++) {
+                points[2 * i] = r.px[i];
+                points[2 * i + 1] = r.py[i];
+            }
+        else
+            for (int i = 0; i < r.npts; i++) {
+                points[3 * i] = r.px[i];
+                points[3 * i + 1] = r.py[i];
+                points[3 * i + 2] = r.pz[i];
+            }
+    }
+    c->view_dims = 0;
+    return BGT_OK;
 }
 
 extern "C" int bgt_segments2d_device(bgt_ctx *c, int dtype, const void *d_img, int w, int h, int32_t **start,
@@ -297,16 +349,20 @@ static int centerline(bgt_ctx *c, int dims, int dtype, const void *in, int w, in
         ph = (h + 31) / 32 * 32;
         pd = (d + 31) / 32 * 32;
     }
-    const size_t bytes = es * (size_t)w * h * d;
-    void *d_in = nullptr;
-    int rc = ctx_scratch(c, 0, bytes, &d_in);
-    if (rc != BGT_OK) return rc;
-    cudaError_t e = cudaMemcpyAsync(d_in, in, bytes, cudaMemcpyHostToDevice, c->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "H2D");
     bgt_batch *b = nullptr;
-    rc = single_batch(c, dims, pw, ph, pd, &b);
-    if (rc == BGT_OK) rc = bgt_batch_set_io(b, 0, dtype, d_in, nullptr);
-    if (rc == BGT_OK) rc = batch_set_input_extent(b, 0, w, h, d);
+    int rc = single_batch(c, dims, pw, ph, pd, &b);
+    if (rc == BGT_OK && batch_packs_host(b, dtype, w, h, d)) {
+        rc = batch_upload_packed(b, dtype, in, w, h, d);
+    } else if (rc == BGT_OK) {
+        const size_t bytes = es * (size_t)w * h * d;
+        void *d_in = nullptr;
+        rc = ctx_scratch(c, 0, bytes, &d_in);
+        if (rc != BGT_OK) return rc;
+        cudaError_t e = cudaMemcpyAsync(d_in, in, bytes, cudaMemcpyHostToDevice, c->stream);
+        if (e != cudaSuccess) return cuda_fail(e, "H2D");
+        rc = bgt_batch_set_io(b, 0, dtype, d_in, nullptr);
+        if (rc == BGT_OK) rc = batch_set_input_extent(b, 0, w, h, d);
+    }
     if (rc == BGT_OK) rc = bgt_batch_run(b, 0, 0);
     if (rc != BGT_OK) return rc;
     const uint32_t *packed = b->h[0].buf[0];

@@ -15,6 +15,7 @@
 #include <cudaTypedefs.h>
 
 #include "host.h"
+#include "hostpix.h"
 #include "kernels.cuh"
 
 using namespace bgt;
@@ -69,6 +70,7 @@ extern "C" int bgt_ctx_create(int device, bgt_ctx **out)
     }
     c->stream = c->own;
     cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
+    host_pool_retain();
     *out = c;
     return BGT_OK;
 }
@@ -83,6 +85,7 @@ extern "C" int bgt_ctx_destroy(bgt_ctx *c)
     for (auto &p : c->scratch) cudaFree(p.ptr);
     if (c->pinned.ptr) cudaFreeHost(c->pinned.ptr);
     if (c->own) cudaStreamDestroy(c->own);
+    host_pool_release();
     delete c;
     return BGT_OK;
 }
@@ -119,6 +122,7 @@ int bgt::ctx_scratch(bgt_ctx *c, int slot, size_t bytes, void **out)
 int bgt::ctx_pinned(bgt_ctx *c, size_t bytes, void **out)
 {
     Scratch &s = c->pinned;
+    c->view_dims = 0;  // its segments are about to be overwritten
     if (s.bytes < bytes) {
         if (s.ptr) {
             cudaStreamSynchronize(c->stream);
@@ -761,13 +765,44 @@ extern "C" int bgt_batch_set_io(bgt_batch *b, int id, int dtype, const void *d_i
     if (id < 0 || id >= (int)b->items.size()) return fail(BGT_ERR_ARG, "bad instance id %d", id);
     if (dtype_size(dtype) == 0) return fail(BGT_ERR_ARG, "bad dtype %d", dtype);
     IO &io = b->io[id];
-    if (io.in != d_in || io.out != d_out || io.dtype != dtype) {
+    if (io.in != d_in || io.out != d_out || io.dtype != dtype || io.packed) {
         b->graph_valid = b->pgraph_valid = false;
         b->io_dirty = true;
     }
     io.dtype = dtype;
     io.in = d_in;
     io.out = d_out;
+    io.packed = false;
+    return BGT_OK;
+}
+
+bool bgt::batch_packs_host(const bgt_batch *b, int dtype, int w, int h, int d)
+{
+    const Inst &in = b->h[0];
+    const size_t packed = (size_t)in.P * in.H * in.D * 4;
+    // worth it when it halves the bytes (narrow images have padded rows), in at most 64 MB of pinned memory
+    return b->items.size() == 1 && in.res && 2 * packed <= dtype_size(dtype) * (size_t)w * h * d && packed <= (64u << 20);
+}
+
+int bgt::batch_upload_packed(bgt_batch *b, int dtype, const void *in, int w, int h, int d)
+{
+    const Inst &inst = b->h[0];
+    const size_t bytes = (size_t)inst.P * inst.H * inst.D * 4;
+    void *pin = nullptr;
+    int rc = ctx_pinned(b->ctx, bytes, &pin);
+    if (rc != BGT_OK) return rc;
+    host_pack(dtype, inst.dims == 2 ? 0 : 1, in, w, h, d, inst.H, inst.D, inst.P, (uint32_t *)pin);
+    cudaError_t e = cudaMemcpyAsync(inst.buf[0], pin, bytes, cudaMemcpyHostToDevice, b->ctx->stream);
+    if (e != cudaSuccess) return cuda_fail(e, "H2D (packed)");
+    IO &io = b->io[0];
+    if (!io.packed) {
+        b->graph_valid = b->pgraph_valid = false;
+        b->io_dirty = true;
+    }
+    io = IO();
+    io.dtype = dtype;
+    io.in = inst.buf[0];
+    io.packed = true;
     return BGT_OK;
 }
 
@@ -861,7 +896,7 @@ static int upload_io(bgt_batch *b)
     std::vector<IODesc> &io = b->io_host;
     for (int i = 0; i < N; i++)
         if (!b->io[i].in) return fail(BGT_ERR_STATE, "instance %d has no input", i);
-    b->pixels = !io_crosses(b);
+    b->pixels = !io_crosses(b) && !b->io[0].packed;  // (packed: a batch of one)
     io.assign(N, IODesc());
     long long w = 0, g = 0;
     b->bytes_only = true;
@@ -885,7 +920,7 @@ static int upload_io(bgt_batch *b)
         io[i].dTW = make_fastdiv((uint32_t)in.TW);
         io[i].dTH = make_fastdiv((uint32_t)in.TH);
         io[i].dTZ = make_fastdiv((uint32_t)std::max(1, in.TZ));
-        if (in.res && b->pixels) continue;
+        if ((in.res && b->pixels) || s.packed) continue;
         const int dt = s.dtype;
         b->bytes_only &= dtype_size(dt) == 1 && (io[i].mode == 0 || dt == BGT_U8 || dt == BGT_BOOL);
         w += (long long)in.P * in.H * in.D;
@@ -1367,16 +1402,30 @@ static int thin_host(bgt_ctx *c, int dims, int dtype, const void *in, int W, int
     if (es == 0) return fail(BGT_ERR_ARG, "bad dtype %d", dtype);
     if (W < 1 || H < 1 || D < 1) return fail(BGT_ERR_ARG, "bad size %dx%dx%d", W, H, D);
     cudaSetDevice(c->device);
-    const size_t bytes = es * (size_t)W * H * D;
-    void *d_io = nullptr;
-    int rc = ctx_scratch(c, 0, bytes, &d_io);
-    if (rc != BGT_OK) return rc;
-    cudaError_t e = cudaMemcpyAsync(d_io, in, bytes, cudaMemcpyHostToDevice, c->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "H2D");
     bgt_batch *b = nullptr;
-    rc = single_batch(c, dims, W, H, D, &b);
+    int rc = single_batch(c, dims, W, H, D, &b);
     if (rc != BGT_OK) return rc;
-    rc = bgt_batch_set_io(b, 0, dtype, d_io, d_io);  // unpack after the engine: in place is safe
+    const size_t bytes = es * (size_t)W * H * D;
+    cudaError_t e;
+    if (batch_packs_host(b, dtype, W, H, D)) {
+        // one bit per pixel crosses the link in either direction
+        rc = batch_upload_packed(b, dtype, in, W, H, D);
+        if (rc == BGT_OK) rc = bgt_batch_run(b, 0, 0);
+        if (rc != BGT_OK) return rc;
+        const Inst &inst = b->h[0];
+        const uint32_t *pin = (const uint32_t *)c->pinned.ptr;
+        e = cudaMemcpyAsync(c->pinned.ptr, inst.buf[0], (size_t)inst.P * H * D * 4, cudaMemcpyDeviceToHost, c->stream);
+        if (e != cudaSuccess) return cuda_fail(e, "D2H (packed)");
+        rc = batch_check(b);
+        if (rc == BGT_OK) host_unpack(dtype, pin, W, H, D, inst.P, out);
+        return rc;
+    }
+    void *d_io = nullptr;
+    rc = ctx_scratch(c, 0, bytes, &d_io);
+    if (rc != BGT_OK) return rc;
+    e = cudaMemcpyAsync(d_io, in, bytes, cudaMemcpyHostToDevice, c->stream);
+    if (e != cudaSuccess) return cuda_fail(e, "H2D");
+    rc = bgt_batch_set_io(b, 0, dtype, d_io, d_io);  // in place is safe: an instance is read before it is written
     if (rc == BGT_OK) rc = bgt_batch_run(b, 0, 0);
     if (rc != BGT_OK) return rc;
     e = cudaMemcpyAsync(out, d_io, bytes, cudaMemcpyDeviceToHost, c->stream);

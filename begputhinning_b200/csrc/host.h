@@ -33,6 +33,7 @@ struct IO {
     const void *in = nullptr;
     void *out = nullptr;
     int inW = 0, inH = 0, inD = 0;  // input extents (0: the instance's own)
+    bool packed = false;            // buf[0] already holds the packed input (resident instances)
 };
 
 struct Stat {
@@ -54,6 +55,11 @@ int batch_check(bgt_batch *b);
 // their bits as an error code.
 void batch_status_words(const bgt_batch *b, const int *(&words)[2]);
 int batch_status(int bits);
+// Packed host transfers of the batch's only instance (w x h x d pixels of
+// `dtype` in it): whether they serve it, and the upload of its packed input in
+// place of set_io.
+bool batch_packs_host(const bgt_batch *b, int dtype, int w, int h, int d);
+int batch_upload_packed(bgt_batch *b, int dtype, const void *in, int w, int h, int d);
 int batch_set_input_extent(bgt_batch *b, int id, int inW, int inH, int inD);
 size_t batch_pool_bytes(const std::vector<BatchItem> &items);
 // Lay a batch out in caller-provided device memory (the serving runtime's
@@ -97,6 +103,8 @@ int segments_graph(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, in
 // Device ExtractSegmentsV on a packed image (P words per row): arrays left in
 // the context's scratch, or copied to host memory.
 int segments_device_arrays(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, int D, int P, DevSegs *out);
+// ... or in the context's pinned memory.
+int segments_result(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, int D, int P, SegResult *r);
 int segments_packed(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, int D, int P, HostSegs *out);
 // Exclusive prefix sum of n ints on the context's stream (CUB temporary
 // storage in scratch slot `slot`).
@@ -111,6 +119,8 @@ struct bgt_ctx {
     cudaStream_t stream = nullptr;
     std::vector<bgt::Scratch> scratch;
     bgt::Scratch pinned;
+    bgt::SegResult view;   // segments of bgt_segments_begin, until bgt_segments_take (in `pinned`)
+    int view_dims = 0;     // 0: none
     size_t seg_chains = 0, seg_nodes = 0;  // list sizes of the segment extraction (grown on demand)
     size_t seg_read = 0;                   // bytes its last result took (read back with the header)
     std::map<std::tuple<int, int, int, int>, bgt_batch *> cache;

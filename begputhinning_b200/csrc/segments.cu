@@ -630,36 +630,42 @@ int segments_device_arrays(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, i
     return BGT_OK;
 }
 
+// The same, with the segment arrays in the context's pinned memory.
+int segments_result(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, int D, int P, SegResult *out)
+{
+    SegResult &r = *out;
+    int rc = 1;
+    if ((long long)W * H * D < (1LL << 32) - 1 && !getenv("BGT_SEGMENTS_PIXEL_WALK"))
+        rc = segments_graph(c, dims, d_buf, W, H, D, P, nullptr, &r);
+    if (rc != 1) return rc;
+    // the pixel walk leaves its arrays on the device, one behind the other
+    rc = segments_device_arrays(c, dims, d_buf, W, H, D, P, &r.dev);
+    if (rc != BGT_OK) return rc;
+    r.nseg = r.dev.nseg;
+    r.npts = r.dev.npts;
+    if (r.nseg == 0) return BGT_OK;
+    const char *first = (const char *)r.dev.start;
+    const size_t span = (size_t)((const char *)((dims == 3 ? r.dev.pz : r.dev.py) + r.npts) - first);
+    void *pin = nullptr;
+    if ((rc = ctx_pinned(c, span, &pin))) return rc;
+    cudaError_t e = cudaMemcpyAsync(pin, first, span, cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (e != cudaSuccess) return cuda_fail(e, "segment readback");
+    auto host = [&](const void *d) { return (const char *)pin + ((const char *)d - first); };
+    r.start = (const int32_t *)host(r.dev.start);
+    r.is_end = (const uint8_t *)host(r.dev.is_end);
+    r.px = (const int16_t *)host(r.dev.px);
+    r.py = (const int16_t *)host(r.dev.py);
+    r.pz = dims == 3 ? (const int16_t *)host(r.dev.pz) : nullptr;
+    return BGT_OK;
+}
+
 // The same, with the segment arrays copied to host memory (malloc).
 int segments_packed(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, int D, int P, HostSegs *out)
 {
     *out = HostSegs();
     SegResult r;
-    int rc = 1;
-    if ((long long)W * H * D < (1LL << 32) - 1 && !getenv("BGT_SEGMENTS_PIXEL_WALK"))
-        rc = segments_graph(c, dims, d_buf, W, H, D, P, nullptr, &r);
-    if (rc == 1) {
-        // the pixel walk leaves its arrays on the device, one behind the other
-        rc = segments_device_arrays(c, dims, d_buf, W, H, D, P, &r.dev);
-        if (rc != BGT_OK) return rc;
-        r.nseg = r.dev.nseg;
-        r.npts = r.dev.npts;
-        if (r.nseg > 0) {
-            const char *first = (const char *)r.dev.start;
-            const size_t span = (size_t)((const char *)((dims == 3 ? r.dev.pz : r.dev.py) + r.npts) - first);
-            void *pin = nullptr;
-            if ((rc = ctx_pinned(c, span, &pin))) return rc;
-            cudaError_t e = cudaMemcpyAsync(pin, first, span, cudaMemcpyDeviceToHost, c->stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-            if (e != cudaSuccess) return cuda_fail(e, "segment readback");
-            auto host = [&](const void *d) { return (const char *)pin + ((const char *)d - first); };
-            r.start = (const int32_t *)host(r.dev.start);
-            r.is_end = (const uint8_t *)host(r.dev.is_end);
-            r.px = (const int16_t *)host(r.dev.px);
-            r.py = (const int16_t *)host(r.dev.py);
-            r.pz = dims == 3 ? (const int16_t *)host(r.dev.pz) : nullptr;
-        }
-    }
+    const int rc = segments_result(c, dims, d_buf, W, H, D, P, &r);
     if (rc != BGT_OK) return rc;
     const int S = r.nseg, Np = r.npts;
     out->nseg = S;

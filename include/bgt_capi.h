@@ -130,6 +130,15 @@ int bgt_segments3d_device(bgt_ctx *ctx, int dtype, const void *d_vol, int width,
                           int32_t **start, uint8_t **is_end, int16_t **px, int16_t **py, int16_t **pz, int *nseg,
                           int *npts);
 
+/* The same in two steps for callers that allocate the arrays themselves: begin
+ * extracts and reports the counts; take writes start[nseg + 1], is_end[nseg]
+ * and the points as npts x dims int16 (x, y[, z] of a point side by side).
+ * The segments wait in the context until they are taken or its next call
+ * that uses the host-side results. d is ignored when dims == 2. */
+int bgt_segments_begin(bgt_ctx *ctx, int dims, int dtype, const void *d_img, int width, int height, int depth,
+                       int *nseg, int *npts);
+int bgt_segments_take(bgt_ctx *ctx, int32_t *start, uint8_t *is_end, int16_t *points);
+
 /* ---- batched thinning ---------------------------------------------------
  * Hundreds of images/volumes of uneven size thinned together by one
  * persistent launch fed by a device-side queue of (instance, tile) work
