@@ -1380,6 +1380,8 @@ static int thin_device(bgt_ctx *c, int dims, int dtype, const void *d_in, int W,
     int rc = single_batch(c, dims, W, H, D, &b);
     if (rc != BGT_OK) return rc;
     rc = bgt_batch_set_io(b, 0, dtype, d_in, d_out);
+    // the cached batch of this shape may have served a padded input before
+    if (rc == BGT_OK) rc = batch_set_input_extent(b, 0, W, H, D);
     if (rc == BGT_OK) rc = bgt_batch_run(b, 0, 0);
     return rc;
 }
@@ -1426,6 +1428,7 @@ static int thin_host(bgt_ctx *c, int dims, int dtype, const void *in, int W, int
     e = cudaMemcpyAsync(d_io, in, bytes, cudaMemcpyHostToDevice, c->stream);
     if (e != cudaSuccess) return cuda_fail(e, "H2D");
     rc = bgt_batch_set_io(b, 0, dtype, d_io, d_io);  // in place is safe: an instance is read before it is written
+    if (rc == BGT_OK) rc = batch_set_input_extent(b, 0, W, H, D);
     if (rc == BGT_OK) rc = bgt_batch_run(b, 0, 0);
     if (rc != BGT_OK) return rc;
     e = cudaMemcpyAsync(out, d_io, bytes, cudaMemcpyDeviceToHost, c->stream);

@@ -85,3 +85,18 @@ def test_shared_arrays(ctx, dims):
     t.copy_(torch.from_numpy(a))
     _run(ctx, [(t, u), (u, v)])  # the second's input is overwritten by the first's output: all inputs are read first
     assert np.array_equal(u.cpu().numpy(), _want(a)) and np.array_equal(v.cpu().numpy(), _want(c))
+
+
+@pytest.mark.parametrize("dims", [2, 3])
+def test_padded_shape_then_plain(ctx, dims):
+    """The shape that CenterlineExtraction pads an input to, thinned afterwards
+    through the same context: the whole array is read."""
+    import torch
+    from begputhinning_b200 import CenterlineExtraction, Thinning2D, Thinning3D, thin_device
+    rng = np.random.default_rng(dims)
+    small, full = ((100, 20), (192, 32)) if dims == 2 else ((20, 25, 30), (32, 32, 32))
+    a = (rng.random(full) < 0.6).astype(np.uint8)
+    CenterlineExtraction((rng.random(small) < 0.6).astype(np.uint8), 2, 1, ctx)
+    assert np.array_equal(thin_device(torch.from_numpy(a).cuda(), ctx=ctx).cpu().numpy(), _want(a))
+    CenterlineExtraction((rng.random(small) < 0.6).astype(np.uint8), 2, 1, ctx)
+    assert np.array_equal((Thinning2D if dims == 2 else Thinning3D)(a, ctx), _want(a))
