@@ -40,13 +40,13 @@
 //      (2D/CenterlineExtraction.cpp:51-131, 3D/CenterlineExtraction.cpp:56-144),
 //      so the whole path needs one readback and no count on the host
 //
-// Bound: latency -- about 7 + log4(longest chain) grid barriers of 1-2 us,
-// and in phase A of a volume the read of its packed words.  Measured on a
-// B200, whole ExtractSegmentsV call, against a walk that followed each chain
-// with one thread and ran the nodes from a queue in the order of their
-// dependences: 2048^2 stroke image (226 k points) 5.72 -> 0.51 ms, 256^3
-// volume (2.3 k points) 0.86 -> 0.15 ms; CenterlineExtraction of a 512^2
-// image 1.24 -> 0.35 ms.
+// Bound: latency -- about 7 + log4(longest chain) grid barriers of 1-2 us and
+// as many chains of dependent loads.  Measured on a B200, this kernel alone:
+// 2048^2 stroke image (214 k points) 62 us, 256^3 volume (3.9 k points) 47 us
+// (84 and 57 us with one half-edge, one node and one strided word per thread at
+// a time).  Against a walk that followed each chain with one thread and ran the
+// nodes from a queue in the order of their dependences, whole ExtractSegmentsV
+// calls: 5.72 -> 0.24 ms and 0.86 -> 0.10 ms.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -196,25 +196,35 @@ __device__ unsigned long long seg_exscan(unsigned long long v, unsigned long lon
 // Sums of the per-block totals before this block, and of all blocks.
 __device__ void seg_block_prefix(const uint2 *sums, unsigned long long (&before)[2], unsigned long long (&all)[2])
 {
-    unsigned long long b0 = 0, b1 = 0, s0 = 0, s1 = 0;
+    __shared__ unsigned long long part[kSegWarps][4];
+    unsigned long long v[4] = {0, 0, 0, 0};
     for (unsigned k = threadIdx.x; k < gridDim.x; k += kSegThreads) {
-        const uint2 v = __ldcg(sums + k);
-        s0 += v.x;
-        s1 += v.y;
+        const uint2 u = __ldcg(sums + k);
+        v[2] += u.x;
+        v[3] += u.y;
         if (k < blockIdx.x) {
-            b0 += v.x;
-            b1 += v.y;
+            v[0] += u.x;
+            v[1] += u.y;
         }
     }
-    unsigned long long t;
-    seg_exscan(b0, &t);
-    before[0] = t;
-    seg_exscan(b1, &t);
-    before[1] = t;
-    seg_exscan(s0, &t);
-    all[0] = t;
-    seg_exscan(s1, &t);
-    all[1] = t;
+    const int warps = min(kSegWarps, (int)(gridDim.x + 31) >> 5);  // warps that hold any
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < warps) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int i = 0; i < 4; i++) v[i] += __shfl_xor_sync(kFull, v[i], o);
+        if (lane < 4) part[warp][lane] = lane == 0 ? v[0] : lane == 1 ? v[1] : lane == 2 ? v[2] : v[3];
+    }
+    __syncthreads();
+    before[0] = before[1] = all[0] = all[1] = 0;
+    for (int w = 0; w < warps; w++) {
+        before[0] += part[w][0];
+        before[1] += part[w][1];
+        all[0] += part[w][2];
+        all[1] += part[w][3];
+    }
+    __syncthreads();
 }
 
 template <int DIMS>
@@ -312,17 +322,25 @@ __device__ __forceinline__ void seg_masks(const SegArgs &a, uint32_t i, uint32_t
     chains = pts & two;
 }
 
-// What node r does at its visit; with EMIT its segments and end points are
-// written from segment si and point pi on (and the chains it walks learn
-// where their points go), else only counted.
+// What node r does at its visit, by a group of kSegGroup lanes that take its
+// neighbours side by side (a neighbour costs six dependent loads); with EMIT
+// its segments and end points are written from segment si and point pi on (and
+// the chains it walks learn where their points go), else only counted.  Whole
+// warps call it; lanes of groups without a node pass live = false.  Returns
+// the node's segments and points in every lane of its group.
+template <int DIMS>
+struct Group {
+    static constexpr int N = DIMS == 2 ? 4 : 8;
+};
 template <int DIMS, bool EMIT>
-__device__ __forceinline__ uint2 seg_visit(const SegArgs &a, uint32_t r, uint32_t si, uint32_t pi, int32_t *start,
-                                           uint8_t *is_end, int16_t *px, int16_t *py, int16_t *pz)
+__device__ __forceinline__ uint2 seg_visit(const SegArgs &a, bool live, uint32_t r, uint32_t si, uint32_t pi,
+                                           int32_t *start, uint8_t *is_end, int16_t *px, int16_t *py, int16_t *pz)
 {
-    constexpr int C = Win<DIMS>::C, q0 = DIMS == 2 ? 9 : 0;
-    const uint2 at = __ldcg(a.npt + r);
-    const uint32_t win = seg_window<DIMS>(a, at.x, at.y);
-    uint32_t todo = win & seg_interior<DIMS>(a, at.x, at.y);
+    constexpr int C = Win<DIMS>::C, q0 = DIMS == 2 ? 9 : 0, G = Group<DIMS>::N;
+    const int g = threadIdx.x & (G - 1);
+    const uint2 at = live ? __ldcg(a.npt + r) : make_uint2(0u, 0u);
+    const uint32_t win = live ? seg_window<DIMS>(a, at.x, at.y) : 0u;
+    uint32_t todo = live ? win & seg_interior<DIMS>(a, at.x, at.y) : 0u;
     const int n = __popc(win);
     const uint32_t pi0 = pi, si0 = si;
     uint32_t arrivals = 0;
@@ -336,73 +354,91 @@ __device__ __forceinline__ uint2 seg_visit(const SegArgs &a, uint32_t r, uint32_
         px[k] = (int16_t)p.y;
         py[k] = (int16_t)y;
     };
-    // a segment of `len` chain points that starts at r and ends at `end`
-    auto segment = [&](uint32_t len, uint2 end, bool e) {
-        if (EMIT) {
-            start[si] = (int32_t)pi;
-            is_end[si] = e || n < 2;
-            put(pi, at);
-            put(pi + 1 + len, end);
-        }
-        si++;
-        pi += len + 2;
-    };
-    while (todo) {
-        const int q = __ffs(todo) - 1;
-        todo &= todo - 1;
-        uint32_t id;
-        if (seg_point(a, at.x, at.y, q + q0, id)) {
-            if (q < C) {
-                arrivals++;
-                continue;
-            }
-            if (EMIT) segment(0, __ldcg(a.npt + id), __ldcg(a.ndeg + id) < 2);
-            else segment(0, at, false);
-            continue;
-        }
-        const int back = 2 * C - q;
-        const int sr = (__ldcg(a.cdir + id) & 0xff) == back ? 0 : 1;  // the side of the chain point that r is on
-        const unsigned long long pr = __ldcg(a.pair + 2 * (size_t)id + (1 - sr));
-        const uint32_t t = (uint32_t)pr & ~kFin, len = (uint32_t)(pr >> 32) + 1;
-        const uint32_t e = __ldcg(a.cexit + t);
-        const uint32_t home = 2 * id + sr;  // terminal half-edge of this end of the chain
-        if (e == kNone) {  // leads to the frame: the last point again
-            if (EMIT) a.cbase[home] = pi + 1;
-            segment(len, EMIT ? __ldcg(a.cpt + (t >> 1)) : at, false);
-        } else if (e == r) {
-            const uint16_t fd = __ldcg(a.cdir + (t >> 1));
-            const int far_q = 2 * C - ((t & 1) ? fd >> 8 : fd & 0xff);  // the cell of r that holds the far end
-            if (q < far_q) {
-                if (EMIT) a.cbase[home] = pi + 1;
-                segment(len, EMIT ? __ldcg(a.cpt + (t >> 1)) : at, false);
+    while (__any_sync(kFull, todo != 0u)) {
+        // this lane's neighbour: the g-th of those left
+        uint32_t m = todo;
+        for (int i = 0; i < g; i++) m &= m - 1;
+#pragma unroll
+        for (int i = 0; i < G; i++) todo &= todo - 1;
+        // what it gives: an arrival, or a segment of `len` chain points that ends at `end`
+        bool arrival = false, seg = false, end1 = false;
+        uint32_t len = 0, home = kNone;  // home: terminal half-edge of this end of the chain
+        uint2 end = at;
+        bool walked = false;
+        if (m) {
+            const int q = __ffs(m) - 1;
+            uint32_t id;
+            if (seg_point(a, at.x, at.y, q + q0, id)) {
+                arrival = q < C;
+                seg = !arrival;
+                if (EMIT && seg) {
+                    end = __ldcg(a.npt + id);
+                    end1 = __ldcg(a.ndeg + id) < 2;
+                }
             } else {
-                if (EMIT) a.cbase[home] = kNone;
-                segment(0, EMIT ? __ldcg(a.cpt + id) : at, false);
+                const int back = 2 * C - q;
+                const int sr = (__ldcg(a.cdir + id) & 0xff) == back ? 0 : 1;  // the side of the chain point that r is on
+                const unsigned long long pr = __ldcg(a.pair + 2 * (size_t)id + (1 - sr));
+                const uint32_t t = (uint32_t)pr & ~kFin;
+                const uint32_t e = __ldcg(a.cexit + t);
+                home = 2 * id + sr;
+                seg = true;
+                walked = true;
+                len = (uint32_t)(pr >> 32) + 1;
+                if (e == kNone) {  // leads to the frame: the last point again
+                    if (EMIT) end = __ldcg(a.cpt + (t >> 1));
+                } else if (e == r) {
+                    const uint16_t fd = __ldcg(a.cdir + (t >> 1));
+                    const int far_q = 2 * C - ((t & 1) ? fd >> 8 : fd & 0xff);  // the cell of r that holds the far end
+                    walked = q < far_q;
+                    if (!walked) len = 0;
+                    if (EMIT) end = __ldcg(a.cpt + (walked ? t >> 1 : id));
+                } else if (e > r) {
+                    if (EMIT) {
+                        end = __ldcg(a.npt + e);
+                        end1 = __ldcg(a.ndeg + e) < 2;
+                    }
+                } else {
+                    seg = walked = false;
+                    arrival = true;
+                }
             }
-        } else if (e > r) {
-            if (EMIT) {
-                a.cbase[home] = pi + 1;
-                segment(len, __ldcg(a.npt + e), __ldcg(a.ndeg + e) < 2);
-            } else {
-                segment(len, at, false);
-            }
-        } else {
-            if (EMIT) a.cbase[home] = kNone;
-            arrivals++;
         }
+        // places in the order of the neighbours
+        uint32_t segs = seg, pts = seg ? len + 2 : 0u;
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) {
+            const uint32_t s1 = __shfl_up_sync(kFull, segs, o, G), p1 = __shfl_up_sync(kFull, pts, o, G);
+            if (g >= o) {
+                segs += s1;
+                pts += p1;
+            }
+        }
+        if (EMIT && m) {
+            const uint32_t k = si + segs - 1, p = pi + pts - (len + 2);
+            if (home != kNone) a.cbase[home] = walked ? p + 1 : kNone;
+            if (seg) {
+                start[k] = (int32_t)p;
+                is_end[k] = end1 || n < 2;
+                put(p, at);
+                put(p + 1 + len, end);
+            }
+        }
+        si += __shfl_sync(kFull, segs, G - 1, G);
+        pi += __shfl_sync(kFull, pts, G - 1, G);
+        const unsigned arr = __ballot_sync(kFull, arrival);
+        arrivals += __popc((arr >> (threadIdx.x & 31 & ~(G - 1))) & ((1u << G) - 1u));
     }
     // the rest of the budget: single points
-    for (int left = max(n, 1) - (int)arrivals - (int)(si - si0); left > 0; left--) {
-        if (EMIT) {
-            start[si] = (int32_t)pi;
-            is_end[si] = n < 2;
-            put(pi, at);
+    const int left = live ? max(n, 1) - (int)arrivals - (int)(si - si0) : 0;
+    if (EMIT)
+        for (int k = g; k < left; k += G) {
+            start[si + k] = (int32_t)(pi + k);
+            is_end[si + k] = n < 2;
+            put(pi + k, at);
         }
-        si++;
-        pi++;
-    }
-    if (!EMIT) a.ndeg[r] = (uint8_t)n;
-    return make_uint2(si - si0, pi - pi0);
+    if (!EMIT && live && g == 0) a.ndeg[r] = (uint8_t)n;
+    return make_uint2(si - si0 + max(left, 0), pi - pi0 + max(left, 0));
 }
 
 // A kept segment's points, smoothed, by one warp.  Point q is the mean of the
@@ -439,11 +475,11 @@ __global__ void __launch_bounds__(kSegThreads, 1) segments_graph_kernel(const Se
     SegHeader *hdr = reinterpret_cast<SegHeader *>(TAIL ? a.tail : a.out);
     unsigned long long total, before[2], all[2];
 
-    // A: masks and counts of this block's range of words
-    const uint32_t per = (a.nw + gridDim.x - 1) / gridDim.x;
-    const uint32_t w0 = min(a.nw, per * blockIdx.x), w1 = min(a.nw, w0 + per);
+    // A: masks and counts of this thread's range of words
+    const uint32_t per = (a.nw + nthr - 1) / nthr;
+    const uint32_t w0 = min(a.nw, per * tid), w1 = min(a.nw, w0 + per);
     unsigned long long cnt = 0;
-    for (uint32_t i = w0 + threadIdx.x; i < w1; i += kSegThreads) {
+    for (uint32_t i = w0; i < w1; i++) {
         const uint32_t row = fdiv(a.dww, i);
         const uint32_t c = __ldg(a.buf + (size_t)row * a.P + (i - row * a.ww));
         if (!c) continue;
@@ -452,7 +488,7 @@ __global__ void __launch_bounds__(kSegThreads, 1) segments_graph_kernel(const Se
         a.rec[i] = make_uint4(nodes, chains, 0u, 0u);
         cnt += (unsigned long long)__popc(nodes) << 32 | __popc(chains);
     }
-    seg_exscan(cnt, &total);
+    const unsigned long long mine = seg_exscan(cnt, &total);
     if (threadIdx.x == 0) a.bsum[blockIdx.x] = make_uint2((uint32_t)(total >> 32), (uint32_t)total);
     if (!seg_barrier(a, gen)) return;
 
@@ -466,28 +502,18 @@ __global__ void __launch_bounds__(kSegThreads, 1) segments_graph_kernel(const Se
     }
     if (all[0] > a.cap_n || all[1] > a.cap_c) return;
     const uint32_t nn = (uint32_t)all[0], nc = (uint32_t)all[1];
-    uint32_t no = (uint32_t)before[0], co = (uint32_t)before[1];
-    for (uint32_t base = w0; base < w1; base += kSegThreads) {
-        const uint32_t i = base + threadIdx.x;
-        uint32_t row = 0, c = 0;
-        uint4 rc = make_uint4(0u, 0u, 0u, 0u);
-        if (i < w1) {
-            row = fdiv(a.dww, i);
-            c = __ldg(a.buf + (size_t)row * a.P + (i - row * a.ww));
-            if (c) rc = __ldcg(a.rec + i);
-        }
-        if (!__syncthreads_or((rc.x | rc.y) != 0u)) continue;
-        const unsigned long long o =
-            seg_exscan((unsigned long long)__popc(rc.x) << 32 | __popc(rc.y), &total);
-        if (c) {
-            uint32_t ni = no + (uint32_t)(o >> 32), ci = co + (uint32_t)o;
+    if (cnt) {
+        uint32_t ni = (uint32_t)before[0] + (uint32_t)(mine >> 32), ci = (uint32_t)before[1] + (uint32_t)mine;
+        for (uint32_t i = w0; i < w1; i++) {
+            const uint32_t row = fdiv(a.dww, i);
+            if (!__ldg(a.buf + (size_t)row * a.P + (i - row * a.ww))) continue;
+            const uint4 rc = a.rec[i];  // written by this thread
+            if (!(rc.x | rc.y)) continue;
             a.rec[i] = make_uint4(rc.x, rc.y, ni, ci);
             const uint32_t x0 = (i - row * a.ww) * 32;
             for (uint32_t m = rc.x; m; m &= m - 1) a.npt[ni++] = make_uint2(row, x0 + __ffs(m) - 1);
             for (uint32_t m = rc.y; m; m &= m - 1) a.cpt[ci++] = make_uint2(row, x0 + __ffs(m) - 1);
         }
-        no += (uint32_t)(total >> 32);
-        co += (uint32_t)total;
     }
     if (!seg_barrier(a, gen)) return;
 
@@ -526,19 +552,37 @@ __global__ void __launch_bounds__(kSegThreads, 1) segments_graph_kernel(const Se
     // finished one, so a round in which none finishes leaves only cycles.
     for (int round = 0; round < kMaxRounds; round++) {
         bool fin = false, left = false;
-        for (uint32_t h = tid; h < 2 * nc; h += nthr) {
-            unsigned long long v = __ldcg(a.pair + h);
-            if ((uint32_t)v & kFin) continue;
-            uint32_t p = (uint32_t)v, d = (uint32_t)(v >> 32);
-#pragma unroll 1
-            for (int k = 0; k < 4 && !(p & kFin); k++) {
-                const unsigned long long u = __ldcg(a.pair + p);
-                p = (uint32_t)u;
-                d += (uint32_t)(u >> 32);
+        // several half-edges of a thread at a time, so that their loads overlap
+        constexpr int U = 4;
+        for (uint32_t h0 = tid; h0 < 2 * nc; h0 += U * nthr) {
+            uint32_t p[U], d[U];
+            bool open[U];
+#pragma unroll
+            for (int i = 0; i < U; i++) {
+                const uint32_t h = h0 + i * nthr;
+                const unsigned long long v = h < 2 * nc ? __ldcg(a.pair + h) : (unsigned long long)kFin;
+                p[i] = (uint32_t)v;
+                d[i] = (uint32_t)(v >> 32);
+                open[i] = !(p[i] & kFin);
             }
-            __stcg(a.pair + h, (unsigned long long)d << 32 | p);
-            if (p & kFin) fin = true;
-            else left = true;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                unsigned long long u[U];
+#pragma unroll
+                for (int i = 0; i < U; i++) u[i] = p[i] & kFin ? (unsigned long long)p[i] : __ldcg(a.pair + p[i]);
+#pragma unroll
+                for (int i = 0; i < U; i++) {
+                    p[i] = (uint32_t)u[i];
+                    d[i] += (uint32_t)(u[i] >> 32);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < U; i++) {
+                if (!open[i]) continue;
+                __stcg(a.pair + h0 + i * nthr, (unsigned long long)d[i] << 32 | p[i]);
+                if (p[i] & kFin) fin = true;
+                else left = true;
+            }
         }
         const int any_left = __syncthreads_or(left), any_fin = __syncthreads_or(fin);
         if (threadIdx.x == 0) {
@@ -552,12 +596,18 @@ __global__ void __launch_bounds__(kSegThreads, 1) segments_graph_kernel(const Se
     // D: segments and points per node (a contiguous range of nodes per block)
     const uint32_t nper = (nn + gridDim.x - 1) / gridDim.x;
     const uint32_t n0 = min(nn, nper * blockIdx.x), n1 = min(nn, n0 + nper);
+    constexpr uint32_t G = Group<DIMS>::N;
+    const uint32_t group = threadIdx.x / G, groups = kSegThreads / G;
+    const bool lead = threadIdx.x % G == 0;
     unsigned long long s0 = 0, s1 = 0;
-    for (uint32_t r = n0 + threadIdx.x; r < n1; r += kSegThreads) {
-        const uint2 v = seg_visit<DIMS, false>(a, r, 0, 0, nullptr, nullptr, nullptr, nullptr, nullptr);
-        a.ncnt[r] = v;
-        s0 += v.x;
-        s1 += v.y;
+    for (uint32_t base = n0; base < n1; base += groups) {
+        const uint32_t r = base + group;
+        const uint2 v = seg_visit<DIMS, false>(a, r < n1, r, 0, 0, nullptr, nullptr, nullptr, nullptr, nullptr);
+        if (r < n1 && lead) {
+            a.ncnt[r] = v;
+            s0 += v.x;
+            s1 += v.y;
+        }
     }
     seg_exscan(s0, &total);
     s0 = total;
@@ -585,12 +635,12 @@ __global__ void __launch_bounds__(kSegThreads, 1) segments_graph_kernel(const Se
             *pz = reinterpret_cast<int16_t *>(a.out + L.z);
     if (blockIdx.x == 0 && threadIdx.x == 0) start[all[0]] = (int32_t)all[1];
     uint32_t so = (uint32_t)before[0], po = (uint32_t)before[1];
-    for (uint32_t base = n0; base < n1; base += kSegThreads) {
-        const uint32_t r = base + threadIdx.x;
-        const uint2 v = r < n1 ? __ldcg(a.ncnt + r) : make_uint2(0u, 0u);
-        const unsigned long long o = seg_exscan((unsigned long long)v.x << 32 | v.y, &total);
-        if (r < n1)
-            seg_visit<DIMS, true>(a, r, so + (uint32_t)(o >> 32), po + (uint32_t)o, start, is_end, px, py, pz);
+    for (uint32_t base = n0; base < n1; base += groups) {
+        const uint32_t r = base + group;
+        const uint2 v = r < n1 && lead ? __ldcg(a.ncnt + r) : make_uint2(0u, 0u);
+        unsigned long long o = seg_exscan((unsigned long long)v.x << 32 | v.y, &total);
+        o = __shfl_sync(kFull, o, 0, G);  // the group's
+        seg_visit<DIMS, true>(a, r < n1, r, so + (uint32_t)(o >> 32), po + (uint32_t)o, start, is_end, px, py, pz);
         so += (uint32_t)(total >> 32);
         po += (uint32_t)total;
     }
