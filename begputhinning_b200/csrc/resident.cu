@@ -10,7 +10,7 @@
 // 2D image (dense).  The rows of the image, or of a box of it (core plus halo),
 // lie twice in shared memory (pass q reads one copy and writes the other) with
 // an odd pitch and zero words left and right of every row.  A pass hands units
-// (24 rows x 2, 4 or 8 words) to warps dynamically; units whose surroundings
+// (24 rows x 2, 4 or 8 words) to warps dynamically; words whose surroundings
 // did not change in the previous pass are skipped.  One box stops after a pass
 // without a deletion: a fixed point of N, S, E and W, the reference's result.
 // The boxes of a larger image meet after every few passes.
@@ -371,18 +371,19 @@ __device__ void res_done(Inst &in, const ResItem &it, int result, int passes, un
 // form a ring (wrong values from the seam in its middle stay 12 bits away):
 // 9 word steps per subiteration for 8 core words instead of 10.
 
-// One subiteration on the ring of UW core words and the halo word v[UW];
-// pairs of words empty in every lane are skipped.  The last subiteration
-// leaves the halo word alone.
+// One subiteration on the ring of UW core words and the halo word v[UW], for
+// the active words only (bits of `act`, the same in every lane; a pair at a
+// time, so that two chains of operations overlap).  The last
+// subiteration leaves the halo word alone.
 template <int UW, int DIR, bool LAST>
-__device__ __forceinline__ void subit2d_ring(uint32_t (&v)[UW + 1])
+__device__ __forceinline__ void subit2d_ring(uint32_t (&v)[UW + 1], uint32_t act)
 {
     const uint32_t first = v[0];
     uint32_t prev = v[UW];
 #pragma unroll
     for (int j = 0; j < UW; j += 2) {
         const uint32_t o0 = v[j], o1 = v[j + 1], on = v[j + 2];
-        if (__any_sync(kFull, (o0 | o1) != 0u)) {
+        if (act & (3u << j)) {
             v[j] = word2d<DIR>(o0, o1, prev);
             v[j + 1] = word2d<DIR>(o1, on, o0);
         }
@@ -390,28 +391,27 @@ __device__ __forceinline__ void subit2d_ring(uint32_t (&v)[UW + 1])
     }
     if constexpr (!LAST) {
         const uint32_t o = v[UW];
-        if (__any_sync(kFull, o != 0u)) v[UW] = word2d<DIR>(o, first, prev);
+        if (act & (1u << UW)) v[UW] = word2d<DIR>(o, first, prev);
     }
 }
 
 struct Box2D {
     uint32_t *zero;         // pp zero words
     uint32_t *buf0, *buf1;  // nrows x pp each: pass q reads buf[q & 1], writes buf[(q + 1) & 1]
-    int *until;             // [nstrips][nchunks]: the unit is processed while q <= until (a unit in
-                            // its 3x3 neighbourhood deleted something in the previous pass)
+    uint32_t *act;          // [nstrips][nchunks]: the unit's active words, bit k (pass q even) or
+                            // 16 + k (odd) for word k
     int pp, wl, nrows, nstrips, nchunks;
     int rlo, rhi;           // core rows and words, within the box
     int wlo, whi;
 };
 
-// One pass q over the box's units.  A unit none of whose inputs for the
-// pass -- its core and the 4-pixel border bands of its 3x3 neighbours -- had
-// a deletion in the previous pass (one subiteration of every direction) is
-// skipped: that region is a fixed point, and a unit processed without a
-// change wrote identical data to both copies.  A unit that deletes something
-// extends `until` to q + 1 for itself and for each neighbour whose border
-// band the deletions reach (a reader in the same pass may see the new value:
-// it then processes a unit it could have skipped).
+// One pass q over the box's units.  Word k of a unit is active when the
+// previous pass deleted something in it or within 4 pixels or rows of it (one
+// subiteration of every direction reaches that far).  The others, and the
+// words next to them as far as the pass looks, are a fixed point: no
+// subiteration of the pass changes them, and both copies hold them already.
+// A pass that deletes something in a word makes the word active in the next
+// one, and each of its eight neighbours within 4 pixels or rows of the deletions.
 // Returns this thread's deleted core bits (of the box's core only).
 template <int UW>
 __device__ uint32_t res_pass2d(const Box2D &b, int q, int *take, unsigned long long *words)
@@ -424,7 +424,11 @@ __device__ uint32_t res_pass2d(const Box2D &b, int q, int *take, unsigned long l
     for (;;) {
         const int u = res_take(take);
         if (u >= nunits) break;
-        if (b.until[u] < q) continue;
+        const int sh = (q & 1) * 16;
+        const uint32_t act = (b.act[u] >> sh) & 0xffu;
+        if (!act) continue;
+        __syncwarp();
+        if (lane == 0) atomicAnd(b.act + u, 0xffff0000u >> sh);  // for pass q + 2
         const int s = u / b.nchunks, c = u - s * b.nchunks;
         const int x0 = 1 + UW * c;
         const int r = kUnitRows * s - 4 + lane;  // box row of this lane
@@ -434,56 +438,60 @@ __device__ uint32_t res_pass2d(const Box2D &b, int q, int *take, unsigned long l
 #pragma unroll
         for (int k = 0; k < UW; k++) v[k] = in[k];
         v[UW] = (in[-1] & 0xFFFF0000u) | (in[UW] & 0xFFFFu);
-        subit2d_ring<UW, 0, false>(v);
-        subit2d_ring<UW, 1, false>(v);
-        subit2d_ring<UW, 2, false>(v);
-        subit2d_ring<UW, 3, true>(v);
-        uint32_t chg = 0, lft = 0, rgt = 0;
+        // active words that are not empty by now, and the halo word where a word next to it is one
+        uint32_t some = v[UW] ? 1u << UW : 0u;
+#pragma unroll
+        for (int k = 0; k < UW; k++) some |= v[k] ? 1u << k : 0u;
+        some = __reduce_or_sync(kFull, some);
+        const uint32_t m = some & ((some & act & (1u | 1u << (UW - 1))) ? act | 1u << UW : act);
+        subit2d_ring<UW, 0, false>(v, m);
+        subit2d_ring<UW, 1, false>(v, m);
+        subit2d_ring<UW, 2, false>(v, m);
+        subit2d_ring<UW, 3, true>(v, m);
+        uint32_t chg = 0;  // bit 1 + k: word k to be active for the rows around, 0 and 1 + UW: the words left and right
         if (valid && lane >= 4 && lane < 28) {
             uint32_t *out = OUT + (size_t)r * b.pp + x0;
             const int klo = b.wlo - UW * c, khi = b.whi - UW * c;
             uint32_t cc = 0;
 #pragma unroll
             for (int k = 0; k < UW; k++) {
+                if (!(act & (1u << k))) continue;
                 const uint32_t d = v[k] ^ in[k];
-                chg |= d;
+                if (d) chg |= 2u << k;
+                if (d & 0xFu) chg |= 1u << k;
+                if (d & 0xF0000000u) chg |= 4u << k;
                 if (k >= klo && k < khi) cc |= d;
-                if (k == 0) lft = d & 0xFu;                 // within 4 pixels of the left edge
-                if (k == UW - 1) rgt = d & 0xF0000000u;     // ... of the right edge
                 out[k] = v[k];
             }
             if (r >= b.rlo && r < b.rhi) core |= cc;
         }
-        // The next pass of a neighbour depends on this unit only through the
-        // 4 pixels next to their common border (four subiterations reach 4
-        // pixels): activate the neighbours whose border band changed
-        // (border bands, as the tile engine does).
-        const unsigned m_any = __ballot_sync(kFull, chg != 0u);
-        if (m_any) {
-            const unsigned m_l = __ballot_sync(kFull, lft != 0u), m_r = __ballot_sync(kFull, rgt != 0u);
-            // lanes holding the first and last 4 core rows
-            constexpr unsigned band_top = 0xF0u, band_bot = 0x0F000000u;
-            if (lane < 9) {
-                const int dy = lane / 3 - 1, dx = lane % 3 - 1;
-                const unsigned rows = dy < 0 ? band_top : dy > 0 ? band_bot : ~0u;
-                const unsigned cols = dx < 0 ? m_l : dx > 0 ? m_r : m_any;
-                const int ns = s + dy, nc = c + dx;
-                if ((rows & cols & m_any) && ns >= 0 && ns < b.nstrips && nc >= 0 && nc < b.nchunks)
-                    b.until[ns * b.nchunks + nc] = q + 1;
-            }
+        // what changed in any row, in the first four and in the last four: ten bits each
+        chg = __reduce_or_sync(kFull, chg | (lane < 8 ? chg << 10 : 0u) | (lane >= 24 ? chg << 20 : 0u));
+        if (chg && lane < 9) {
+            const int dy = lane / 3 - 1, dx = lane % 3 - 1;
+            const uint32_t f = (chg >> (dy < 0 ? 10 : dy > 0 ? 20 : 0)) & 0x3ffu;
+            const uint32_t on = dx < 0 ? (f & 1u) << (UW - 1) : dx > 0 ? f >> (UW + 1) : (f >> 1) & ((1u << UW) - 1u);
+            const int ns = s + dy, nc = c + dx;
+            if (on && ns >= 0 && ns < b.nstrips && nc >= 0 && nc < b.nchunks)
+                atomicOr(b.act + ns * b.nchunks + nc, on << (16 - sh));
         }
         if (lane == 0)
-            *words += (unsigned long long)min(kUnitRows, b.nrows - kUnitRows * s) * min(UW, b.wl - UW * c);
+            *words += (unsigned long long)min(kUnitRows, b.nrows - kUnitRows * s) * __popc(m & ((1u << UW) - 1u));
     }
     return core;
 }
 
-// Bound: in a large batch the ALU (13 half-rate operations per word step) and
-// the passes' tails; for a lone image the latency of its passes (1.5 us each
+// Bound: in a large batch the latency of a word step's chain (6 warps per
+// scheduler issue on half of the cycles, the ALU is half busy) and the
+// passes' tails (27 % of the warps' time); for a lone image the latency of its passes (1.5 us each
 // in a box of a 512^2 image) and meetings (4 us with the exchange).  Boxes of
 // rows and words against bands of full-width rows: a 4096^2 image 127 -> 102 us,
 // a 1501 x 1003 float image 154 -> 92 us, a 512^2 one 59 -> 43 us, the mixed
 // batch (with the exchange flattened over the threads) 1.24 -> 1.19 ms.
+// Words active one by one against whole units with a vote per pair and
+// subiteration: 4096^2 103 -> 97 us, 16 images of 1024^2 121 -> 117 us, the
+// mixed batch 1.19 -> 1.17 ms (a branch per word instead of per pair: 1.21 ms;
+// 1024 threads: 1.18 ms).
 //
 // One image, or one box of it: rows [r0, r1) of words [c0, c1) are the core;
 // `halo` rows above and below it and one word left and right (clamped to the
@@ -515,7 +523,7 @@ __device__ void res_run2d(Inst &in, const ResIO &io, const ResItem &it, uint32_t
     b.zero = sm;
     b.buf0 = sm + b.pp;
     b.buf1 = b.buf0 + (size_t)b.nrows * b.pp;
-    b.until = reinterpret_cast<int *>(b.buf1 + (size_t)b.nrows * b.pp);
+    b.act = b.buf1 + (size_t)b.nrows * b.pp;
     const int pp = b.pp;
     const int nunits = b.nstrips * b.nchunks;
 
@@ -526,7 +534,7 @@ __device__ void res_run2d(Inst &in, const ResIO &io, const ResItem &it, uint32_t
             reinterpret_cast<uint4 *>(sm)[i] = make_uint4(0u, 0u, 0u, 0u);
         if (threadIdx.x < (total & 3)) sm[(total & ~3) + threadIdx.x] = 0u;
     }
-    for (int i = threadIdx.x; i < nunits; i += kResThreads) b.until[i] = -1;
+    for (int i = threadIdx.x; i < nunits; i += kResThreads) b.act[i] = 0;
     if (threadIdx.x < 2) take[threadIdx.x] = 0;
     __syncthreads();
     res_load<false>(in, io, WordWalk(b.wl, b.nrows), b.nrows * b.wl, e0, a, 0, [&](bool, const WordPos &q, uint32_t v) {
@@ -534,8 +542,13 @@ __device__ void res_run2d(Inst &in, const ResIO &io, const ResItem &it, uint32_t
         const int w = q.y * pp + q.x + 1;
         b.buf0[w] = v;
         b.buf1[w] = v;
-        // units holding foreground start active
-        b.until[(q.y / kUnitRows) * b.nchunks + q.x / UW] = 0;
+        // words with foreground start active, in the units within 4 rows of it
+        const int s = q.y / kUnitRows, rr = q.y - s * kUnitRows, c = q.x / UW;
+        volatile uint32_t *act = b.act + s * b.nchunks + c;
+        const uint32_t bit = 1u << (q.x - c * UW);
+        if (!(*act & bit)) atomicOr((uint32_t *)act, bit);
+        if (rr < 4 && s > 0 && !(act[-b.nchunks] & bit)) atomicOr((uint32_t *)act - b.nchunks, bit);
+        if (rr >= kUnitRows - 4 && s + 1 < b.nstrips && !(act[b.nchunks] & bit)) atomicOr((uint32_t *)act + b.nchunks, bit);
     });
     __syncthreads();
 
@@ -582,16 +595,19 @@ __device__ void res_run2d(Inst &in, const ResIO &io, const ResItem &it, uint32_t
                 break;
             }
             e++;
-            // the halo: a word that changed makes its unit, and the units it is within 4 pixels of, active
+            // the halo: a word that changed becomes active, and the words it is within 4 pixels or rows of
             auto take_over = [&](int y, int w, uint32_t v) {
                 const int r = y - a, x = w - e0;
                 uint32_t *p = cur + r * pp + 1 + x;
-                if (*p == v) return;
+                const uint32_t d = *p ^ v;
+                if (!d) return;
                 *p = v;
-                const int s = r / kUnitRows, c = x / UW, rr = r - s * kUnitRows, cc = x - c * UW;
-                for (int dy = rr < 4 && s > 0 ? -1 : 0; dy <= (rr >= kUnitRows - 4 && s + 1 < b.nstrips ? 1 : 0); dy++)
-                    for (int dx = cc == 0 && c > 0 ? -1 : 0; dx <= (cc == UW - 1 && c + 1 < b.nchunks ? 1 : 0); dx++)
-                        b.until[(s + dy) * b.nchunks + c + dx] = q + 1;
+                const int s = r / kUnitRows, rr = r - s * kUnitRows;
+                const int s0 = rr < 4 && s > 0 ? s - 1 : s, s1 = rr >= kUnitRows - 4 && s + 1 < b.nstrips ? s + 1 : s;
+                const int x0 = (d & 0xFu) && x > 0 ? x - 1 : x, x1 = (d & 0xF0000000u) && x + 1 < b.wl ? x + 1 : x;
+                for (int t = s0; t <= s1; t++)
+                    for (int k = x0; k <= x1; k++)
+                        atomicOr(b.act + t * b.nchunks + k / UW, 1u << ((q & 1 ? 0 : 16) + k % UW));
             };
             const int htop = it.r0 - a, hrows = htop + (aend - it.r1);
             for (int i = threadIdx.x; i < hrows * b.wl; i += kResThreads) {

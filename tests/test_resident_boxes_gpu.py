@@ -69,3 +69,22 @@ def test_image_boxes(ctx, shape, box_words, monkeypatch):
         want, _ = po.thin2d(v)
         assert plan[0] and stat["converged"] == 1
         assert np.array_equal(got, want), f"plan {plan}: {(got != want).sum()} pixels differ"
+
+
+def wedges2d(h, w):
+    """Wide wedges in all four directions: deletions travel along them for many
+    passes, so words fall out of a pass, come back, and pass on to their
+    neighbours at different times."""
+    y, x = np.mgrid[0:h, 0:w]
+    v = (np.abs(y - h // 2) * 3 < x % 150) | (np.abs(x - w // 2) * 3 < (h - y) % 130)
+    v[:, ::97] = 0
+    return v.astype(np.uint8)
+
+
+# units of 2, 4 and 8 words; unit rows and words cut anywhere
+@pytest.mark.parametrize("shape", [(60, 70), (97, 159), (230, 257), (310, 700), (767, 1025)])
+def test_active_words(ctx, shape):
+    for v in (wedges2d(*shape), wedges2d(shape[0], shape[1] + 5)[::-1, 5:].copy()):
+        (got,), _, (stat,) = _thin(ctx, [v])
+        assert stat["converged"] == 1
+        assert np.array_equal(got, po.thin2d(v)[0]), f"{(got != po.thin2d(v)[0]).sum()} pixels differ"
