@@ -105,32 +105,37 @@ __device__ __forceinline__ uint32_t pixel_neg(const IODesc &d)
 }
 
 // Wider pixels: the warp builds its 32 lanes' words one after the other, a
-// lane per pixel (coalesced whatever the alignment) and a vote per word.
+// lane per pixel (coalesced whatever the alignment) and a vote per word.  Every
+// lane loads, clamped to the input, and each lane masks its own word in the end,
+// so that the loads of 16 words are in flight at once (a branch around each
+// load left one in flight: the resident kernel on a 1501 x 1003 float image
+// 96 -> 85 us, on a 187 x 203 x 161 int16 volume 225 -> 190 us).
 template <typename T, int MODE>
-__device__ __forceinline__ uint32_t pixel_vote(const T *p, uint32_t off, int cnt)
+__device__ __forceinline__ uint32_t pixel_vote(const T *p, uint32_t last, uint32_t off, int cnt)
 {
+    constexpr int U = 16;
     const int lane = threadIdx.x & 31;
     uint32_t w = 0;
-#pragma unroll 16
-    for (int k = 0; k < 32; k++) {
-        const uint32_t o = __shfl_sync(kFull, off, k);
-        const int c = __shfl_sync(kFull, cnt, k);
-        bool f = false;
-        if (lane < c) {
-            const T v = __ldg(p + (size_t)o + lane);
-            f = MODE == 0 ? fg2<T>(v) : MODE == 1 ? fg3<T>(v) : v != (T)0;
+#pragma unroll
+    for (int k0 = 0; k0 < 32; k0 += U) {
+        T v[U];
+#pragma unroll
+        for (int k = 0; k < U; k++) v[k] = __ldg(p + min(__shfl_sync(kFull, off, k0 + k) + (uint32_t)lane, last));
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+            const uint32_t m = __ballot_sync(kFull, MODE == 0 ? fg2<T>(v[k]) : MODE == 1 ? fg3<T>(v[k]) : v[k] != (T)0);
+            if (lane == k0 + k) w = m;
         }
-        const uint32_t m = __ballot_sync(kFull, f);
-        if (lane == k) w = m;
     }
-    return w;
+    return cnt >= 32 ? w : w & ((1u << cnt) - 1u);
 }
 template <typename T>
 __device__ __forceinline__ uint32_t pixel_vote_mode(const IODesc &d, uint32_t off, int cnt)
 {
-    return d.mode == 0   ? pixel_vote<T, 0>((const T *)d.in, off, cnt)
-           : d.mode == 1 ? pixel_vote<T, 1>((const T *)d.in, off, cnt)
-                         : pixel_vote<T, 2>((const T *)d.in, off, cnt);
+    const uint32_t last = (uint32_t)d.inW * (uint32_t)d.inH * (uint32_t)d.inD - 1u;
+    return d.mode == 0   ? pixel_vote<T, 0>((const T *)d.in, last, off, cnt)
+           : d.mode == 1 ? pixel_vote<T, 1>((const T *)d.in, last, off, cnt)
+                         : pixel_vote<T, 2>((const T *)d.in, last, off, cnt);
 }
 // Every lane of the warp calls it (cnt = 0 for none).
 static __device__ __noinline__ uint32_t pixel_word_wide(const IODesc &d, uint32_t off, int cnt)
