@@ -139,9 +139,13 @@ struct SegHeader {
 };
 
 // Grid barrier (cooperative launch: every block is resident).  Bounded; false
-// once any block gave up.
+// once any block gave up (bit 30 of the arrivals, which ends every wait).  One
+// word says all, so that a block that arrives last reads once (a status word
+// of its own, read behind the wait: CenterlineExtraction of a 512^2 image 152 us
+// instead of 148, three 256^3 segment lists 96.1 instead of 95.6).
 __device__ bool seg_barrier(const SegArgs &a, unsigned &gen)
 {
+    constexpr int kGaveUp = 1 << 30;
     __shared__ int ok;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -150,22 +154,18 @@ __device__ bool seg_barrier(const SegArgs &a, unsigned &gen)
         atomicAdd(a.sync, 1);
         const int target = (int)(gen * gridDim.x);
         const unsigned long long t_end = globaltimer() + (unsigned long long)a.timeout_ns;
-        bool good = true;
-        for (int spin = 0; ld_acquire(a.sync) < target; spin++)
+        int v = ld_acquire(a.sync);
+        for (int spin = 0; v < target; v = ld_acquire(a.sync), spin++)
             if ((spin & 255) == 255 && globaltimer() > t_end) {
-                good = false;
+                atomicOr(a.sync, kGaveUp);
+                atomicOr(&reinterpret_cast<SegHeader *>(a.tail ? a.tail : a.out)->status, 4);
+                v = kGaveUp;
                 break;
             }
-        if (!good) {
-            atomicOr(a.sync + 1, 4);
-            atomicOr(&reinterpret_cast<SegHeader *>(a.tail ? a.tail : a.out)->status, 4);
-        }
-        ok = good && !(ld_acquire(a.sync + 1) & 4);
+        ok = !(v & kGaveUp);
     }
     __syncthreads();
-    const bool r = ok;
-    __syncthreads();
-    return r;
+    return ok;  // (thread 0 writes it again behind the next barrier's first __syncthreads)
 }
 
 // Exclusive prefix sum over the block of two counters packed in 64 bits.
