@@ -71,8 +71,9 @@ struct alignas(16) Inst {
     int res_bands;            // 3D: boxes the volume is cut into
     int res_gy;               // 3D: boxes along y (band = z index * res_gy + y index)
     int res_stride;           // 3D: messages a box may send per iteration (its core words)
-    uint2 *res_msg;           // 3D, several boxes: [2][boxes][res_stride] (word of the volume, value)
-    int *res_cnt;             // ... and their counts [2][boxes]
+    uint4 *res_msg;           // 3D, several boxes: [2][boxes][res_stride] (word of the volume, value, tag)
+    uint4 *res_head;          // ... and [2][boxes] (count, whether its core changed, tag); tag = run, iteration + 1
+    unsigned res_run;         // runs so far + 1 (the boxes' memory is zero at first)
 };
 
 // Core words of a tile (clamped to the image): the algorithmic unit of a pass.
@@ -217,6 +218,21 @@ __device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long l
 {
     unsigned long long v;
     asm volatile("ld.acquire.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// 16 bytes in one access: what is read was written by one store
+__device__ __forceinline__ void st_relaxed128(uint4 *p, const uint4 &v)
+{
+    asm volatile("{ .reg .b128 t; .reg .b64 a, b; mov.b64 a, {%1, %2}; mov.b64 b, {%3, %4}; mov.b128 t, {a, b}; "
+                 "st.relaxed.gpu.global.b128 [%0], t; }" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ uint4 ld_relaxed128(const uint4 *p)
+{
+    uint4 v;
+    asm volatile("{ .reg .b128 t; .reg .b64 a, b; ld.relaxed.gpu.global.b128 t, [%4]; mov.b128 {a, b}, t; "
+                 "mov.b64 {%0, %1}, a; mov.b64 {%2, %3}, b; }"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
     return v;
 }
 

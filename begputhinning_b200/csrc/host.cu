@@ -457,8 +457,8 @@ static PoolLayout layout_pool(const std::vector<Inst> &h, size_t n_res_items)
         // messages between the boxes of a volume (two iterations' worth)
         o.msg = o.cnt = 0;
         if (in.res && in.dims == 3 && in.res_bands > 1) {
-            o.msg = off; off = align_up(off + 2 * (size_t)in.res_bands * in.res_stride * sizeof(uint2), 256);
-            o.cnt = off; off = align_up(off + 2 * (size_t)in.res_bands * 4, 256);
+            o.msg = off; off = align_up(off + 2 * (size_t)in.res_bands * in.res_stride * sizeof(uint4), 256);
+            o.cnt = off; off = align_up(off + 2 * (size_t)in.res_bands * sizeof(uint4), 256);
         }
     }
     // all per-tile "last change" arrays in one block (one memset per run)
@@ -558,8 +558,9 @@ extern "C" int bgt_batch_finalize(bgt_batch *b)
         in.lc = (int *)(P + o.lc);
         in.act = (uint8_t *)(P + o.act);
         in.list = (int *)(P + o.list);
-        in.res_msg = o.msg ? (uint2 *)(P + o.msg) : nullptr;
-        in.res_cnt = o.cnt ? (int *)(P + o.cnt) : nullptr;
+        in.res_msg = o.msg ? (uint4 *)(P + o.msg) : nullptr;
+        in.res_head = o.cnt ? (uint4 *)(P + o.cnt) : nullptr;
+        in.res_run = 1;
         in.tmap = b->d_tmaps + kMapsPerInst * i;
         const CfgInfo &c = *cfg_info(in.cfg);
         CUtensorMap *m = &maps[(size_t)kMapsPerInst * i];
@@ -574,6 +575,11 @@ extern "C" int bgt_batch_finalize(bgt_batch *b)
     // tables are uploaded in stream order from host copies the batch keeps
     cudaStream_t st = b->ctx->stream;
     e = cudaMemcpyAsync(b->d_tmaps, maps.data(), maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice, st);
+    // the volumes' messages and headers (one block per volume) carry no tag of a run yet
+    for (int i = 0; i < N && e == cudaSuccess; i++)
+        if (offs[i].msg)
+            e = cudaMemsetAsync(P + offs[i].msg, 0,
+                                offs[i].cnt - offs[i].msg + 2 * (size_t)b->h[i].res_bands * sizeof(uint4), st);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(b->d_insts, b->h.data(), (size_t)N * sizeof(Inst), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && !b->res_items.empty())

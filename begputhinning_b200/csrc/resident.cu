@@ -5,7 +5,7 @@
 // a large volume (every iteration) meet to trade their edges through global
 // memory.
 // One CTA of 768 threads per SM holds up to 225 KB (measured against two
-// CTAs of 384 threads with 111 KB each: larger bands and slabs won).
+// CTAs of 384 threads with 111 KB each: larger boxes won).
 //
 // 2D image (dense).  The rows of the image, or of a box of it (core plus halo),
 // lie twice in shared memory (pass q reads one copy and writes the other) with
@@ -121,7 +121,7 @@ bool res_fits3d(int W, int ny, int nz)
 // ------------------------------------------------------------ helpers -----
 extern __shared__ __align__(16) uint8_t res_smem[];  // dynamic shared memory of the CTA
 
-// The CTAs of one instance meet for the k-th time: each adds 1 to the low half
+// The CTAs of one image meet for the k-th time: each adds 1 to the low half
 // of meet[k & 1], and 1 to its high half when something of its own changed
 // since the last meeting; the wait (bounded) ends when all `bands` arrived.
 // Two words in turn, so that a CTA that is already at the next meeting leaves
@@ -353,6 +353,7 @@ __device__ void res_done(Inst &in, const ResItem &it, int result, int passes, un
         if (it.bands > 1 && atomicAdd(&in.res_left, 1) == it.bands - 1) {
             in.res_meet[0] = in.res_meet[1] = 0;
             in.res_left = 0;
+            in.res_run++;
         }
     }
     __syncthreads();
@@ -671,9 +672,8 @@ struct Box3D {
     int nl;                    // its length
     int gy, gz, by, bz;        // boxes along y and z; this box
     int stride;                // messages a box may send
-    uint2 *msgs;
-    int *counts;
-    MeetState meet;            // (used by thread 0)
+    uint4 *msgs, *heads;
+    unsigned run;              // tags of this run's messages and headers
     int n[4];                  // lengths: word list, active words, candidates, messages
     int flag;
 };
@@ -720,9 +720,10 @@ __device__ __forceinline__ void box_changed(Box3D &v, uint32_t idx, uint32_t col
     if ((v.it.r0 > 0 && z < v.it.r0 + h) || (v.it.r1 < v.D && z >= v.it.r1 - h) || (v.it.c0 > 0 && y < v.it.c0 + h) ||
         (v.it.c1 < v.H && y >= v.it.c1 - h)) {
         const int x = (int)idx - (int)z2 * v.ps - (int)y2 * v.p;
-        uint2 *msg = v.msgs + ((size_t)(iter & 1) * v.it.bands + v.it.band) * v.stride;
-        msg[atomicAdd(&v.n[3], 1)] =
-            make_uint2(((uint32_t)z * (uint32_t)v.H + (uint32_t)y) * (uint32_t)v.wl + (uint32_t)x, box_state()[idx]);
+        uint4 *msg = v.msgs + ((size_t)(iter & 1) * v.it.bands + v.it.band) * v.stride;
+        st_relaxed128(msg + atomicAdd(&v.n[3], 1),
+                      make_uint4(((uint32_t)z * (uint32_t)v.H + (uint32_t)y) * (uint32_t)v.wl + (uint32_t)x,
+                                 box_state()[idx], v.run, (uint32_t)iter + 1u));
     }
 }
 
@@ -977,8 +978,14 @@ static __device__ __noinline__ bool box_iteration_dense(Box3D &v, int iter, unsi
 // A wrong value moves one row or plane per subiteration (the pre-test reads
 // the same neighbours as U), so with six halo rows and planes the core is
 // exact after an iteration; then every box sends the words near its core's
-// edge that changed to a list in global memory, the boxes meet, and each
-// takes over what lies in its halo from its neighbours' lists.
+// edge that changed to a list in global memory, waits for every box's header
+// (its count, and whether its core changed), and takes over what lies in its
+// halo from its neighbours' lists.  Headers and messages are 16 bytes, written
+// and read in one access, and carry the run and the iteration: each is waited
+// for by itself, so that no fence, counter or second trip stands between them
+// (97 x 75 x 66: 87 -> 82 us, 256^3: 176 -> 167 us, the int16 volume below 190 ->
+// 179 us).  Two sets in turn: a box writes the messages of iteration i + 2 when
+// it has every header of i + 1, which a box sends when it is done with those of i.
 //
 // Bound: the latency of an iteration (8 to 12 us: six dependent subiterations
 // with two barriers each, then the meeting), not throughput: a box has some
@@ -986,8 +993,8 @@ static __device__ __noinline__ bool box_iteration_dense(Box3D &v, int iter, unsi
 // 32 x 32 x 4 voxels, every brick of the neighbourhood of a change evaluated
 // whole (24 us per iteration): a 97 x 75 x 66 tree volume 214 -> 85 us, a
 // 187 x 203 x 161 one (16-bit pixels, transfers included) 955 -> 221 us, a
-// 256^3 one, whose bricks did not fit, 1330 us on the tile rings -> 179 us.
-// Words of 32 voxels took the last two 238 and 193 us.
+// 256^3 one, whose bricks did not fit, 1330 us on the tile rings -> 179 us
+// (both before the headers and messages above; words of 32 voxels took them 238 and 193 us).
 __device__ void res_run3d(Inst &in, const ResIO &io, const ResItem &item, ResSched *S, ResTrace *tr)
 {
     __shared__ Box3D v;
@@ -1019,8 +1026,9 @@ __device__ void res_run3d(Inst &in, const ResIO &io, const ResItem &item, ResSch
         v.by = item.band - v.bz * v.gy;
         v.stride = in.res_stride;
         v.msgs = in.res_msg;
-        v.counts = in.res_cnt;
-        v.meet = MeetState{0, 0, 0};
+        v.heads = in.res_head;
+        v.run = in.res_run;
+        v.flag = 0;
         v.nl = 0;
         for (int k = 0; k < 4; k++) v.n[k] = 0;
     }
@@ -1056,27 +1064,38 @@ __device__ void res_run3d(Inst &in, const ResIO &io, const ResItem &item, ResSch
                 break;
             }
         } else {
-            if (threadIdx.x == 0) {
-                v.counts[(iter & 1) * v.it.bands + v.it.band] = v.n[3];
-                v.flag = res_meet(in.res_meet, v.it.bands, any, v.meet, S->timeout_ns);
-                if (v.flag == 2) atomicOr(&S->status, kErrQueueTimeout);
-            }
-            __syncthreads();
-            if (v.flag != 1) {
-                result = v.flag == 0 ? 1 : -1;
-                break;
-            }
+            uint4 *const heads = v.heads + (iter & 1) * v.it.bands;
+            if (threadIdx.x == 0)
+                st_relaxed128(heads + v.it.band, make_uint4((unsigned)v.n[3], any ? 1u : 0u, v.run, (unsigned)iter + 1u));
+            const unsigned long long t_end = globaltimer() + (unsigned long long)S->timeout_ns;
+            // a header or message of this iteration, once it is there (bounded)
+            auto await = [&](const uint4 *p, uint4 w) {
+                for (int spin = 0; w.z != v.run || w.w != (unsigned)iter + 1u; w = ld_relaxed128(p), spin++) {
+                    if ((spin & 63) == 63 && globaltimer() > t_end) {
+                        v.flag = 2;
+                        w = make_uint4(0u, 0u, 0u, 0u);
+                        break;
+                    }
+                    if (spin >= 4096) __nanosleep(64);  // partners that have not started yet
+                }
+                return w;
+            };
             // kWarps / 8 warps per neighbouring box take over its messages
             const int k8 = warp & 7, k9 = k8 < 4 ? k8 : k8 + 1;
             const int nbz = v.bz + k9 / 3 - 1, nby = v.by + k9 % 3 - 1;
-            if (warp < kWarps / 8 * 8 && nbz >= 0 && nbz < v.gz && nby >= 0 && nby < v.gy) {
-                const int nb = nbz * v.gy + nby;
-                const uint2 *m = v.msgs + ((size_t)(iter & 1) * v.it.bands + nb) * v.stride;
-                const int k0 = (warp >> 3) * 32 + lane;
-                // the first message is loaded beside the count, whether it is one or not
-                uint2 w = k0 < v.stride ? __ldcg(m + k0) : make_uint2(0u, 0u);
-                const int n = __ldcg(v.counts + (iter & 1) * v.it.bands + nb);
+            const bool next = warp < kWarps / 8 * 8 && nbz >= 0 && nbz < v.gz && nby >= 0 && nby < v.gy;
+            const int nb = next ? nbz * v.gy + nby : v.it.band, k0 = (warp >> 3) * 32 + lane;
+            const uint4 *m = v.msgs + ((size_t)(iter & 1) * v.it.bands + nb) * v.stride;
+            // every thread's first header and message are on their way together, whether they are there or not
+            uint4 h = ld_relaxed128(heads + nb), w = ld_relaxed128(m + min(k0, v.stride - 1));
+            bool some = false;
+            for (int t = threadIdx.x; t < v.it.bands; t += kResThreads) some |= await(heads + t, ld_relaxed128(heads + t)).y != 0u;
+            if (next) {
+                h = await(heads + nb, h);
+                const int n = (int)h.x;
                 for (int k = k0; k < n;) {
+                    w = await(m + k, w);
+                    if (v.flag) break;
                     const int r = (int)(w.x / (uint32_t)v.wl), x = (int)w.x - r * v.wl, z = r / v.H, y = r - z * v.H;
                     if (z >= v.z0 && z < v.z1 && y >= v.y0 && y < v.y1) {
                         uint32_t *s = box_state() + (z - v.z0 + 1) * v.ps + (y - v.y0 + 1) * v.p + x;
@@ -1087,8 +1106,14 @@ __device__ void res_run3d(Inst &in, const ResIO &io, const ResItem &item, ResSch
                         any_chg = true;
                     }
                     k += (kWarps / 8) * 32;
-                    if (k < n) w = __ldcg(m + k);
+                    if (k < n) w = ld_relaxed128(m + k);
                 }
+            }
+            some = __syncthreads_or(some);
+            if (v.flag || !some) {
+                result = v.flag ? -1 : 1;
+                if (v.flag && threadIdx.x == 0) atomicOr(&S->status, kErrQueueTimeout);
+                break;
             }
             any_chg = __syncthreads_or(any_chg);
         }

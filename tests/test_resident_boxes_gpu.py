@@ -88,3 +88,32 @@ def test_active_words(ctx, shape):
         (got,), _, (stat,) = _thin(ctx, [v])
         assert stat["converged"] == 1
         assert np.array_equal(got, po.thin2d(v)[0]), f"{(got != po.thin2d(v)[0]).sum()} pixels differ"
+
+
+@pytest.mark.parametrize("slab_voxels", [10000, 40000])
+def test_messages_of_earlier_runs(ctx, slab_voxels, monkeypatch):
+    """A batch run again and again on other volumes, and batches made anew in the
+    memory that the last one left: the boxes take over this run's messages only."""
+    import torch
+    from begputhinning_b200 import Batch
+    monkeypatch.setenv("BGT_RES3D_SLAB_VOXELS", str(slab_voxels))
+    rng = np.random.default_rng(60)
+    shape = (31, 44, 70)
+    vols = [blobs3d(rng, *shape, 9, rmax=8), np.ones(shape, np.uint8), random3d(rng, *shape, 0.6),
+            blobs3d(rng, *shape, 30, rmax=5)]
+    wants = [po.thin3d(v)[0] for v in vols]
+    t = torch.empty(shape, dtype=torch.uint8, device="cuda")
+    o = torch.empty_like(t)
+    for k in range(3):
+        b = Batch(ctx)
+        i = b.add(shape)
+        b.finalize()
+        b.set_io(i, t, o)
+        assert b.plan(i)[1] > 1
+        for v, want in list(zip(vols, wants))[::-1 if k == 1 else 1]:
+            t.copy_(torch.from_numpy(v))
+            torch.cuda.synchronize()
+            b.run()
+            torch.cuda.synchronize()
+            assert np.array_equal(o.cpu().numpy(), want)
+        b.close()
