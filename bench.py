@@ -4,10 +4,10 @@
 Workload (per GPU): the mixed batch -- 512 2D images with sides log-uniform
 64..2048 px (aspect 0.5..2) of Bezier strokes, plus 32 3D volumes with sides
 log-uniform 64..192 of tubular trees -- uint8 {0,1}, seeded synthetic data.
-A step is one pass of the hot path over the whole batch: batch-wide pack of
-the uint8 inputs (resident in HBM) into bit-packed words, one persistent
-engine launch that thins every instance to its own fixed point, batch-wide
-unpack to uint8 outputs; replayed as one CUDA graph.  ``value`` is thinned
+A step is one pass of the hot path over the whole batch: one persistent launch
+that reads the uint8 inputs (resident in HBM) as bits, thins every instance to
+its own fixed point and writes uint8 outputs (instances of the tile rings are
+packed and unpacked by launches of their own); replayed as one CUDA graph.  ``value`` is thinned
 Mvoxel/s (pixels count as voxels) over all ranks.
 
 Also reported: ``e2e`` (the same step with inputs copied from pinned host
@@ -396,11 +396,12 @@ def run_bgt(args, rank, world, local):
     # the dominant kernel: the resident kernel when it takes the batch, else the tile-ring engine
     kernel, kms = ("resident_kernel", res) if res >= ring else ("engine_kernel", ring)
     alg_bytes = words * 8.0  # one 4-byte read + one 4-byte write per packed core word per pass
+    if kernel == "resident_kernel" and n_res == len(items):
+        alg_bytes += 2.0 * total  # it reads and writes the pixels as well
     achieved = alg_bytes / (kms * 1e-3) / 1e9
-    # kernels per step: batch pack, scheduler reset, resident reset, resident kernel, the
-    # tile-ring seed + engine (when some instance may use them), batch unpack
-    any_ring = n_res < len(items) or any(it.ndim == 3 for it in items)
-    launches_per_step = 4 + (1 if n_res else 0) + (2 if any_ring else 0)
+    # kernels per step: the resident kernel (which reads and writes the pixels itself), and for
+    # instances of the tile rings batch pack, scheduler reset, seed, engine and batch unpack
+    launches_per_step = (1 if n_res else 0) + (5 if n_res < len(items) else 0)
     n2 = sum(1 for it in items if it.ndim == 2)
     line = {
         "metric": METRIC,
@@ -418,7 +419,7 @@ def run_bgt(args, rank, world, local):
         "config": {"workload": WORKLOAD, "instances_2d": n2, "instances_3d": len(items) - n2,
                    "voxels_per_gpu": units, "input_bytes_per_gpu": total,
                    "l2": "inputs larger than L2 (uint8 inputs and outputs of several hundred MB per step)",
-                   "step": "batch-wide pack + persistent engine + batch-wide unpack, one CUDA graph",
+                   "step": "one resident launch that packs, thins and unpacks every instance, one CUDA graph",
                    "tile_configs": {f"{d}D class {c}": v for (d, c), v in sorted(table.items())},
                    "parallelism": f"instances per rank, {world} rank(s), no collective"},
         "e2e": {"value": units_all / (e2e_max * 1e-3) / 1e6, "unit": UNIT, "h2d_bytes_per_step": total,
@@ -486,7 +487,7 @@ def config_legs(local: int, peak: float, peak_kind: str, reps: int = 10) -> dict
     """The single-instance workloads at their named sizes: 512x512 Bezier
     strokes, 4096x4096 vessel trees with salt and holes, 256^3 tubular trees
     with ellipsoids.  Per workload, thinning and segment extraction are
-    timed separately: thinning device-resident (pack + engine + unpack of a
+    timed separately: thinning device-resident (one run of a
     one-instance batch, CUDA events on its stream, graph replay) and end to
     end through the host API (Thinning2D/Thinning3D: host buffers, copies
     included); segments by the device ExtractSegmentsV on the thinned image.

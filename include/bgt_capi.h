@@ -180,9 +180,9 @@ int bgt_batch_work(bgt_batch *b, unsigned long long *tiles, unsigned long long *
  * batch's stream): pack, engine (the thinning kernels), unpack */
 int bgt_batch_stage_ms(bgt_batch *b, float *pack_ms, float *engine_ms, float *unpack_ms);
 /* The engine stage split: the resident kernel (instances thinned inside
- * one CTA's shared memory, large images as bands of CTAs) and the tile-ring
- * engine after it (instances the resident kernel does not take, volumes
- * whose non-empty bricks did not fit). */
+ * one CTA's shared memory, large ones as boxes on several CTAs; it reads and
+ * writes their pixels) and the tile-ring engine after it (instances the
+ * resident kernel does not take). */
 int bgt_batch_engine_ms(bgt_batch *b, float *resident_ms, float *rings_ms);
 /* Engine choice for the next finalize: 0 = resident kernel wherever an
  * instance fits (default), 1 = tile rings only.  Instances added with an
