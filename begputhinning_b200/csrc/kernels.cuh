@@ -75,7 +75,7 @@ struct ResTrace {
 };
 // One CTA per SM: two of 384 threads with 112 KB each took the mixed batch
 // from 1.19 to 1.35 ms and three of 256 to 1.52 ms (smaller boxes, more halo),
-// lone images and volumes as long or longer.
+// lone images and volumes as long or longer; 1024 threads from 1.166 to 1.178 ms.
 constexpr int kResThreads = 768;
 constexpr int kResCtasPerSm = 1;
 constexpr int kResSmemBytes = 230400;  // dynamic shared memory of one CTA
@@ -85,9 +85,11 @@ int res_smem_bytes();
 bool res_fits2d(int wl, int nrows);
 // Its cost: word steps of a pass over all of its units.
 double res_cost2d(int wl, int nrows);
-// Passes between two meetings of the boxes of an image (4 halo rows each): 1,
-// 2, 3 and 4 took a 4096^2 image 155, 119, 120 and 114 us, a 512^2 one 54, 47,
-// 47 and 43 us.
+// Passes between two meetings of the boxes of an image (4 halo rows each): 3,
+// 4, 5 and 6 took a 4096^2 image 99, 98, 91 and 101 us, a 512^2 one 47, 44, 51
+// and 50 us, a 1501 x 1003 float one 85, 86, 89 and 86 us, the mixed batch 1.165,
+// 1.154, 1.156 and 1.175 ms (the passes that images need decide much of it: a
+// run ends at a meeting).
 constexpr int kResPeriod2D = 4;
 // Whether a 3D box (ny rows x nz planes of a volume W wide, halo included) fits one CTA.
 bool res_fits3d(int W, int ny, int nz);
