@@ -665,7 +665,7 @@ struct Box3D {
     int H, D, wl;              // volume rows, planes; words per row
     int y0, y1, z0, z1;        // rows and planes held
     int p, ps;                 // words between rows, between planes
-    uint32_t mp, mps;          // reciprocals: idx / p and idx / ps by mulhi, exact for 16-bit idx
+    uint32_t mp, mps;          // reciprocals of p and ps: see box_plane_row
     int my, mrows;             // rows of the masks: per plane (a multiple of 4), in all
     int xs;                    // words per column of the masks: 1 << xs
     int act, chg, list;        // offsets of the masks and of the word list
@@ -684,11 +684,15 @@ __device__ __forceinline__ uint32_t *box_words(int off) { return reinterpret_cas
 // entries, unions and deletions, then the active words (positions in `list`)
 __device__ __forceinline__ uint32_t *box_list(const Box3D &v, int k) { return box_words(v.list) + k * v.nl; }
 
-// plane and row of a word, padding included
+// Plane and row of a word, padding included.  n / d = mulhi(2 n, m) with
+// m = ceil(2^31 / d) = (2^31 + e) / d, e < d: the product exceeds n / d by
+// n e / (d 2^31), less than 1 / d for n < 2^16 and d <= 2^15 (a box has fewer than
+// 2^16 words in at least three planes of at least three rows).  2^31 and not
+// 2^32, whose quotient by 1 (rows of one word) does not fit 32 bits.
 __device__ __forceinline__ uint32_t box_plane_row(const Box3D &v, uint32_t idx, uint32_t &y2)
 {
-    const uint32_t z2 = __umulhi(idx, v.mps);
-    y2 = __umulhi(idx - z2 * (uint32_t)v.ps, v.mp);
+    const uint32_t z2 = __umulhi(2 * idx, v.mps);
+    y2 = __umulhi(2 * (idx - z2 * (uint32_t)v.ps), v.mp);
     return z2;
 }
 __device__ __forceinline__ int box_index(const Box3D &v, const WordPos &q)
@@ -1011,8 +1015,8 @@ __device__ void res_run3d(Inst &in, const ResIO &io, const ResItem &item, ResSch
         const int nz = v.z1 - v.z0, ny = v.y1 - v.y0;
         v.p = v.wl | 1;  // odd strides: rows and planes start on different banks
         v.ps = ((ny + 2) * v.p) | 1;
-        v.mp = 0xffffffffu / (uint32_t)v.p + 1u;
-        v.mps = 0xffffffffu / (uint32_t)v.ps + 1u;
+        v.mp = 0x7fffffffu / (uint32_t)v.p + 1u;
+        v.mps = 0x7fffffffu / (uint32_t)v.ps + 1u;
         v.my = (ny + 5) & ~3;
         v.mrows = (nz + 2) * v.my;
         v.xs = 0;
