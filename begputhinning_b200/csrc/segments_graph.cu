@@ -124,6 +124,7 @@ struct SegArgs {
     long long timeout_ns;
     // centreline tail
     uint32_t *keep;       // segment -> its first output point, kNone: pruned
+    uint32_t cap_s;       // segments it holds
     uint8_t *tail;
     unsigned long long tail_bytes, maxlen;
     int span;
@@ -623,12 +624,14 @@ __global__ void __launch_bounds__(kSegThreads, 1) segments_graph_kernel(const Se
     seg_block_prefix(a.bsum2, before, all);
     const bool wide = (ld_acquire(a.sync + 1) & 8) || all[0] >> 31 || all[1] >> 31;
     const SegLayout L = seg_layout((unsigned)all[0], (unsigned)all[1], DIMS);
+    // (many segments of few points fit the output block, but not `keep`)
+    const bool small = L.total > a.out_bytes || (TAIL && all[0] > a.cap_s);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         hdr->segs = (uint32_t)all[0];
         hdr->pts = (uint32_t)all[1];
-        if (wide || L.total > a.out_bytes) atomicOr(&hdr->status, wide ? 8 : 2);
+        if (wide || small) atomicOr(&hdr->status, wide ? 8 : 2);
     }
-    if (wide || L.total > a.out_bytes) return;
+    if (wide || small) return;
     int32_t *start = reinterpret_cast<int32_t *>(a.out + L.start);
     uint8_t *is_end = a.out + L.is_end;
     int16_t *px = reinterpret_cast<int16_t *>(a.out + L.x), *py = reinterpret_cast<int16_t *>(a.out + L.y),
@@ -785,6 +788,7 @@ int segments_graph(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, in
         a.ndeg = (uint8_t *)(l + o_deg);
         a.ncnt = (uint2 *)(l + o_cnt);
         a.keep = (uint32_t *)(l + o_keep);
+        a.cap_s = (uint32_t)out_segs;
         a.cap_c = (uint32_t)nc;
         a.cap_n = (uint32_t)nn;
         a.out_bytes = seg_layout((unsigned)out_segs, (unsigned)out_pts, dims).total;
