@@ -669,7 +669,8 @@ struct Box3D {
     int my, mrows;             // rows of the masks: per plane (a multiple of 4), in all
     int xs;                    // words per column of the masks: 1 << xs
     int act, chg, list;        // offsets of the masks and of the word list
-    int nl;                    // its length
+    int nl;                    // its length (0: the box goes over all of its words)
+    int cand, cap;             // offset of the candidates' lists, candidates they hold
     int gy, gz, by, bz;        // boxes along y and z; this box
     int stride;                // messages a box may send
     uint4 *msgs, *heads;
@@ -680,9 +681,8 @@ struct Box3D {
 
 __device__ __forceinline__ uint32_t *box_state() { return reinterpret_cast<uint32_t *>(res_smem); }
 __device__ __forceinline__ uint32_t *box_words(int off) { return reinterpret_cast<uint32_t *>(res_smem + off); }
-// the lists, one behind the other: non-empty words, then the candidates'
-// entries, unions and deletions, then the active words (positions in `list`)
-__device__ __forceinline__ uint32_t *box_list(const Box3D &v, int k) { return box_words(v.list) + k * v.nl; }
+// the candidates' entries, unions and deletions, one list behind the other
+__device__ __forceinline__ uint32_t *box_cand(const Box3D &v, int k) { return box_words(v.cand) + k * v.cap; }
 
 // Plane and row of a word, padding included.  n / d = mulhi(2 n, m) with
 // m = ceil(2^31 / d) = (2^31 + e) / d, e < d: the product exceeds n / d by
@@ -782,19 +782,19 @@ __device__ __forceinline__ void box_subiteration(const Box3D &v, int nc, unsigne
 {
     bool any = false;
     for (int c = threadIdx.x; c < nc; c += kResThreads) {
-        const uint32_t e = box_list(v, 1)[c];
-        const uint32_t del = box_deletions<J>(v, e, box_list(v, 2)[c]);
+        const uint32_t e = box_cand(v, 0)[c];
+        const uint32_t del = box_deletions<J>(v, e, box_cand(v, 1)[c]);
         words += ent_dist(e) == 0;
         any |= del != 0u;
-        box_list(v, 3)[c] = del;
+        box_cand(v, 2)[c] = del;
     }
     if (!__syncthreads_or(any)) return;
     for (int c = threadIdx.x; c < nc; c += kResThreads) {
-        const uint32_t del = box_list(v, 3)[c];
+        const uint32_t del = box_cand(v, 2)[c];
         if (del) {
-            const uint32_t e = box_list(v, 1)[c];
+            const uint32_t e = box_cand(v, 0)[c];
             box_delete(e, del);
-            box_list(v, 1)[c] = e | kEntChanged;
+            box_cand(v, 0)[c] = e | kEntChanged;
         }
     }
     __syncthreads();
@@ -814,12 +814,18 @@ __device__ __forceinline__ void box_subiteration1(const Box3D &v, uint32_t &e, u
     __syncthreads();
 }
 
-// An iteration on the lists.  Returns whether a word of the core changed.
-__device__ __forceinline__ bool box_iteration(Box3D &v, int iter, unsigned &words, unsigned &entries)
+// Voxels of the word c at s with all six face neighbours: no direction deletes them.
+__device__ __forceinline__ uint32_t box_faces(const Box3D &v, const uint32_t *s, uint32_t c)
+{
+    return (c << 1) & (c >> 1) & s[v.p] & s[-v.p] & s[v.ps] & s[-v.ps];
+}
+
+// Candidates of an iteration from the word list: pre-test and U on the active words.
+__device__ __forceinline__ void box_collect(Box3D &v, unsigned &words, unsigned &entries)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint32_t *const list = box_list(v, 0);
-    uint16_t *const alist = reinterpret_cast<uint16_t *>(box_list(v, 4));
+    uint32_t *const list = box_words(v.list);
+    uint16_t *const alist = reinterpret_cast<uint16_t *>(box_cand(v, 3));  // active words: positions in `list`
     const int nl = v.nl;
     // active words: a word of the row's 3x3 rows that is at most one column
     // away changed in the previous iteration (otherwise its union is empty),
@@ -834,8 +840,7 @@ __device__ __forceinline__ bool box_iteration(Box3D &v, int iter, unsigned &word
             if ((res_smem[v.act + (int)(z2 * (uint32_t)v.my + y2)] >> ent_col(e)) & 1u) {
                 const uint32_t *s = box_state() + idx;
                 const uint32_t c = *s;
-                const uint32_t faces = (c << 1) & (c >> 1) & s[v.p] & s[-v.p] & s[v.ps] & s[-v.ps];
-                on = (c & kCoreBits & ~faces) != 0u;
+                on = (c & kCoreBits & ~box_faces(v, s, c)) != 0u;
             }
         }
         const int pos = warp_append(on, &v.n[1]);
@@ -858,21 +863,63 @@ __device__ __forceinline__ bool box_iteration(Box3D &v, int iter, unsigned &word
         }
         const int c = warp_append(un != 0u, &v.n[2]);
         if (c >= 0) {
-            box_list(v, 1)[c] = e;
-            box_list(v, 2)[c] = un;
-            box_list(v, 3)[c] = du;
+            box_cand(v, 0)[c] = e;
+            box_cand(v, 1)[c] = un;
+            box_cand(v, 2)[c] = du;
         }
     }
     __syncthreads();
-    const int nc = v.n[2];
+}
+
+// ... from all words of the box, for one with more non-empty words than its
+// lists hold: most of them lie inside solid parts and are not candidates.  There may
+// be more candidates (v.n[2]) than their lists hold.  Returns this thread's work (words
+// of the core, words).
+static __device__ __noinline__ uint2 box_collect_all(Box3D &v)
+{
+    uint2 work = make_uint2(0u, 0u);
+    const int lane = threadIdx.x & 31, nbox = (v.z1 - v.z0) * (v.y1 - v.y0) * v.wl, cap = v.cap;
+    const WordWalk walk(v.wl, v.y1 - v.y0);
+    WordPos q = walk.first();
+    for (int i = threadIdx.x; i - lane < nbox; i += kResThreads, walk.next(q)) {
+        const int d = i < nbox ? box_dist(v, q) : 6;
+        uint32_t un = 0, du = 0;
+        int idx = 0;
+        if (d <= 5 && ((res_smem[v.act + (q.z + 1) * v.my + q.y + 1] >> (q.x >> v.xs)) & 1u)) {
+            idx = box_index(v, q);
+            const uint32_t *s = box_state() + idx;
+            const uint32_t c = *s;
+            if (c & kCoreBits & ~box_faces(v, s, c)) {
+                uint32_t g[27];
+                const uint32_t val = box_window(s, v.p, v.ps, g);
+                du = rule3d<0>(g) & val;
+                un = (du | rule3d<1>(g) | rule3d<2>(g) | rule3d<3>(g) | rule3d<4>(g) | rule3d<5>(g)) & val;
+                work.x += d == 0;
+                work.y++;
+            }
+        }
+        const int c = warp_append(un != 0u, &v.n[2]);
+        if (c >= 0 && c < cap) {
+            box_cand(v, 0)[c] = box_entry(v, q, idx, d);
+            box_cand(v, 1)[c] = un;
+            box_cand(v, 2)[c] = du;
+        }
+    }
+    __syncthreads();
+    return work;
+}
+
+// The rest of an iteration on its candidates.  Returns whether a word of the core changed.
+__device__ __forceinline__ bool box_thin(Box3D &v, int nc, int iter, unsigned &words)
+{
     bool core = false;
     if (nc > kResThreads) {
         for (int c = threadIdx.x; c < nc; c += kResThreads) {
-            const uint32_t del = box_list(v, 3)[c];
+            const uint32_t del = box_cand(v, 2)[c];
             if (del) {
-                const uint32_t e = box_list(v, 1)[c];
+                const uint32_t e = box_cand(v, 0)[c];
                 box_delete(e, del);
-                box_list(v, 1)[c] = e | kEntChanged;
+                box_cand(v, 0)[c] = e | kEntChanged;
             }
         }
         __syncthreads();
@@ -882,7 +929,7 @@ __device__ __forceinline__ bool box_iteration(Box3D &v, int iter, unsigned &word
         box_subiteration<4>(v, nc, words);
         box_subiteration<5>(v, nc, words);
         for (int c = threadIdx.x; c < nc; c += kResThreads) {
-            const uint32_t e = box_list(v, 1)[c];
+            const uint32_t e = box_cand(v, 0)[c];
             if (!(e & kEntChanged) || ent_dist(e) != 0) continue;
             core = true;
             box_changed(v, ent_idx(e), ent_col(e), iter);
@@ -891,9 +938,9 @@ __device__ __forceinline__ bool box_iteration(Box3D &v, int iter, unsigned &word
         const int c = threadIdx.x;
         uint32_t e = 0, un = 0;
         if (c < nc) {
-            e = box_list(v, 1)[c];
-            un = box_list(v, 2)[c];
-            const uint32_t del = box_list(v, 3)[c];
+            e = box_cand(v, 0)[c];
+            un = box_cand(v, 1)[c];
+            const uint32_t del = box_cand(v, 2)[c];
             if (del) {
                 box_delete(e, del);
                 e |= kEntChanged;
@@ -913,8 +960,9 @@ __device__ __forceinline__ bool box_iteration(Box3D &v, int iter, unsigned &word
     return core;
 }
 
-// The same on all words of the box, for one with more non-empty words than its
-// lists hold: a thread keeps the unions and deletions of its words.
+// An iteration on all words of the box, for one with more candidates than their
+// lists hold: a thread keeps the unions and deletions of its words (in local memory, so
+// that it takes about 100 us for the 12288 words of a 64^3 box).
 static __device__ __noinline__ bool box_iteration_dense(Box3D &v, int iter, unsigned &words, unsigned &entries)
 {
     uint32_t un[kDenseWords], del[kDenseWords];
@@ -1052,14 +1100,29 @@ __device__ void res_run3d(Inst &in, const ResIO &io, const ResItem &item, ResSch
     for (int r = threadIdx.x; r < v.mrows / 4; r += kResThreads) box_words(v.act)[r] = kFull;
     __syncthreads();
     // more non-empty words than the lists hold: go over all words of the box
-    const bool dense = v.list + (size_t)v.n[0] * kBoxListBytes + 64 > (size_t)kSmemBytes;
-    if (threadIdx.x == 0) v.nl = v.n[0];
+    if (threadIdx.x == 0) {
+        const bool dense = v.list + (size_t)v.n[0] * kBoxListBytes + 64 > (size_t)kSmemBytes;
+        v.nl = dense ? 0 : v.n[0];
+        v.cand = dense ? v.list : v.list + 4 * v.nl;
+        v.cap = dense ? (kSmemBytes - 64 - v.list) / 12 : v.nl;
+    }
     __syncthreads();
+    const bool dense = v.n[0] > v.nl;
 
     int iter = 0, result = 0;
     unsigned words = 0, entries = 0;
     for (;; iter++) {
-        const bool core = dense ? box_iteration_dense(v, iter, words, entries) : box_iteration(v, iter, words, entries);
+        if (dense) {
+            const uint2 work = box_collect_all(v);
+            if (v.n[2] <= v.cap) {
+                words += work.x;
+                entries += work.y;
+            }
+        } else {
+            box_collect(v, words, entries);
+        }
+        const int nc = v.n[2];
+        const bool core = nc > v.cap ? box_iteration_dense(v, iter, words, entries) : box_thin(v, nc, iter, words);
         const bool any = __syncthreads_or(core);
         bool any_chg = any;
         if (v.it.bands == 1) {
