@@ -351,7 +351,7 @@ static int centerline(bgt_ctx *c, int dims, int dtype, const void *in, int w, in
     }
     bgt_batch *b = nullptr;
     int rc = single_batch(c, dims, pw, ph, pd, &b);
-    if (rc == BGT_OK && batch_packs_host(b, dtype, w, h, d)) {
+    if (rc == BGT_OK && batch_packs_host(b, dtype, in, nullptr, w, h, d)) {
         rc = batch_upload_packed(b, dtype, in, w, h, d);
     } else if (rc == BGT_OK) {
         const size_t bytes = es * (size_t)w * h * d;

@@ -782,12 +782,24 @@ extern "C" int bgt_batch_set_io(bgt_batch *b, int id, int dtype, const void *d_i
     return BGT_OK;
 }
 
-bool bgt::batch_packs_host(const bgt_batch *b, int dtype, int w, int h, int d)
+bool bgt::batch_packs_host(const bgt_batch *b, int dtype, const void *in, const void *out, int w, int h, int d)
 {
-    const Inst &in = b->h[0];
-    const size_t packed = (size_t)in.P * in.H * in.D * 4;
+    const Inst &inst = b->h[0];
+    const size_t packed = (size_t)inst.P * inst.H * inst.D * 4, bytes = dtype_size(dtype) * (size_t)w * h * d;
     // worth it when it halves the bytes (narrow images have padded rows), in at most 64 MB of pinned memory
-    return b->items.size() == 1 && in.res && 2 * packed <= dtype_size(dtype) * (size_t)w * h * d && packed <= (64u << 20);
+    if (b->items.size() != 1 || !inst.res || 2 * packed > bytes || packed > (64u << 20)) return false;
+    bool pinned = false;
+    for (const void *p : {in, out}) {
+        cudaPointerAttributes a{};
+        if (p && cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+            cudaGetLastError();
+            a.type = cudaMemoryTypeUnregistered;
+        }
+        // memory that is not only the host's is left to the copies
+        if (p && a.type != cudaMemoryTypeUnregistered && a.type != cudaMemoryTypeHost) return false;
+        if (p == in) pinned = a.type == cudaMemoryTypeHost;
+    }
+    return host_pack_pays(dtype_size(dtype), bytes, pinned, host_pack_pays(dtype_size(dtype), bytes, pinned, 0) ? 0 : host_workers());
 }
 
 int bgt::batch_upload_packed(bgt_batch *b, int dtype, const void *in, int w, int h, int d)
@@ -1415,7 +1427,7 @@ static int thin_host(bgt_ctx *c, int dims, int dtype, const void *in, int W, int
     if (rc != BGT_OK) return rc;
     const size_t bytes = es * (size_t)W * H * D;
     cudaError_t e;
-    if (batch_packs_host(b, dtype, W, H, D)) {
+    if (batch_packs_host(b, dtype, in, out, W, H, D)) {
         // one bit per pixel crosses the link in either direction
         rc = batch_upload_packed(b, dtype, in, W, H, D);
         if (rc == BGT_OK) rc = bgt_batch_run(b, 0, 0);

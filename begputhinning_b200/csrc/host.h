@@ -56,9 +56,9 @@ int batch_check(bgt_batch *b);
 void batch_status_words(const bgt_batch *b, const int *(&words)[2]);
 int batch_status(int bits);
 // Packed host transfers of the batch's only instance (w x h x d pixels of
-// `dtype` in it): whether they serve it, and the upload of its packed input in
-// place of set_io.
-bool batch_packs_host(const bgt_batch *b, int dtype, int w, int h, int d);
+// `dtype` in it): whether they serve it (out: the output array, or null), and the
+// upload of its packed input in place of set_io.
+bool batch_packs_host(const bgt_batch *b, int dtype, const void *in, const void *out, int w, int h, int d);
 int batch_upload_packed(bgt_batch *b, int dtype, const void *in, int w, int h, int d);
 int batch_set_input_extent(bgt_batch *b, int id, int inW, int inH, int inD);
 size_t batch_pool_bytes(const std::vector<BatchItem> &items);

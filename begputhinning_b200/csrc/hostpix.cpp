@@ -48,6 +48,7 @@ public:
         cv_.notify_all();
         for (auto &t : th_) t.join();
     }
+    int size() const { return (int)th_.size(); }
     void run(Fn fn, void *arg, int parts)
     {
         std::unique_lock<std::mutex> busy(busy_, std::try_to_lock);
@@ -342,6 +343,17 @@ void host_unpack(int dtype, const uint32_t *words, int w, int h, int d, int P, v
     UnpackJob j{words, w, h, d, P, 1, out, by_type<Unpack, UnpackRows>(dtype)};
     j.parts = parts_of((size_t)w * h * d * by_type<Size, size_t>(dtype), (long long)h * d);
     run_parts(unpack_part, &j, j.parts);
+}
+
+bool host_pack_pays(size_t pixel, size_t bytes, bool pinned, int workers)
+{
+    return pinned ? pixel >= 4 && workers >= 3 : pixel >= 4 || bytes <= (2u << 20) || workers >= 1;
+}
+
+int host_workers()
+{
+    Pool *p = pool();
+    return p ? p->size() : 0;
 }
 
 void host_pool_retain()
