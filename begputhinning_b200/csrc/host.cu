@@ -621,6 +621,7 @@ extern "C" int bgt_batch_finalize(bgt_batch *b)
     }
     b->io.assign(N, IO());
     b->stats.assign(N, Stat());
+    b->ran = false;
     b->finalized = true;
     return BGT_OK;
 }
@@ -1041,6 +1042,7 @@ static int run_engine(bgt_batch *b, int use_graph)
     }
     b->stats_valid = false;
     b->last_mode = 0;
+    b->ran = true;
     return BGT_OK;
 }
 
@@ -1095,6 +1097,7 @@ static int run_plain(bgt_batch *b)
     cudaFreeHost(h_flag);
     b->stats_valid = true;
     b->last_mode = 1;
+    b->ran = true;
     return rc;
 }
 
@@ -1202,6 +1205,7 @@ static int run_plain_device(bgt_batch *b)
     if (e != cudaSuccess) return cuda_fail(e, "cudaGraphLaunch (plain)");
     b->stats_valid = false;
     b->last_mode = 2;
+    b->ran = true;
     return BGT_OK;
 }
 
@@ -1254,9 +1258,13 @@ struct RunRecord {
 };
 static int read_records(bgt_batch *b, std::vector<RunRecord> &rec)
 {
+    const size_t n = b->items.size();
+    if (!b->ran) {
+        rec.assign(n, RunRecord());
+        return BGT_OK;
+    }
     int rc = batch_check(b);
     if (rc != BGT_OK) return rc;
-    const size_t n = b->items.size();
     std::vector<Inst> tmp(n);
     cudaError_t e = cudaMemcpy(tmp.data(), b->d_insts, n * sizeof(Inst), cudaMemcpyDeviceToHost);
     std::vector<ResTrace> tr(b->last_mode == 0 ? b->res_items.size() : 0);

@@ -134,6 +134,7 @@ struct bgt_batch {
     std::vector<bgt::Stat> stats;
     bool finalized = false;
     bool stats_valid = false;
+    bool ran = false;        // since it was finalized: the device holds records of a run
     int last_mode = 0;
     void *pool = nullptr;
     size_t pool_bytes = 0;
