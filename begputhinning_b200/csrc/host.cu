@@ -273,13 +273,16 @@ static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 // further while it is a large share of the batch's work (so a batch of few
 // large instances still spreads over the SMs).  Items are ordered volumes
 // first (largest first: their chains of iterations are the longest), then
-// images largest first, the boxes of one instance consecutive.
-static void plan_resident(bgt_batch *b)
+// images largest first, the boxes of one instance consecutive.  For a reserved
+// pool that the plan does not fit: `level` 1 leaves volumes that need several boxes
+// to the tile rings (their boxes' messages are most of what such a plan adds: a
+// 256^3 volume takes 19 MB of them beside its 7 MB), level 2 everything.
+static void plan_resident(bgt_batch *b, int level)
 {
     b->res_items.clear();
     b->any_ring = false;
     const int N = (int)b->items.size();
-    const bool rings_only = b->engine_mode == 1 || (getenv("BGT_ENGINE") && !strcmp(getenv("BGT_ENGINE"), "rings"));
+    const bool rings_only = level == 2 || b->engine_mode == 1 || (getenv("BGT_ENGINE") && !strcmp(getenv("BGT_ENGINE"), "rings"));
     double total = 0;
     for (const BatchItem &it : b->items) total += (double)((it.W + 31) / 32) * it.H * it.D;
     const double all = total, target = std::max(total / std::max(1, b->res_grid), 4096.0);
@@ -333,7 +336,7 @@ static void plan_resident(bgt_batch *b)
                 }
             return gy > 0;
         };
-        const bool ok = search(share, false) || search(b->res_grid, true);
+        const bool ok = level == 1 ? search(1, false) : search(share, false) || search(b->res_grid, true);
         if (!ok) {
             in.res = 0;  // cannot be cut into boxes that fit: the rings take it
             continue;
@@ -515,8 +518,12 @@ extern "C" int bgt_batch_finalize(bgt_batch *b)
         else b->res_grid = 0;
         if (b->grid_cap > 0) b->res_grid = std::min(b->res_grid, b->grid_cap);
     }
-    plan_resident(b);
-    const PoolLayout L = layout_pool(b->h, b->res_items.size());
+    plan_resident(b, 0);
+    PoolLayout L = layout_pool(b->h, b->res_items.size());
+    for (int level = 1; level <= 2 && b->reserved && L.total > b->pool_bytes; level++) {
+        plan_resident(b, level);
+        L = layout_pool(b->h, b->res_items.size());
+    }
     const std::vector<InstOffs> &offs = L.offs;
     const size_t off = L.total, off_lc = L.off_lc, off_io = L.off_io, off_sched = L.off_sched,
                  off_seq = L.off_seq, off_item = L.off_item, off_inst = L.off_inst, off_tmap = L.off_tmap,

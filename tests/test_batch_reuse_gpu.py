@@ -44,3 +44,38 @@ def test_no_records_before_a_run(ctx):
             assert lib().bgt_batch_reset(b.h) == 0
     finally:
         b.close()
+
+
+def test_pools_too_small_for_messages(ctx):
+    """Reserved memory that holds the tile rings' plan takes the instances,
+    whichever engine then thins them."""
+    from begputhinning_b200 import Batch, lib
+    rng = np.random.default_rng(3)
+    items = [blobs3d(rng, 90, 100, 110, 30, rmax=9), blobs3d(rng, 20, 30, 40, 4)]
+    items += [random2d(rng, 80, 70 + k, 0.5) for k in range(12)]
+    rest = len(items) - 1
+
+    def sized(rings):
+        b = Batch(ctx)
+        b.set_engine(rings)
+        ids = _add(b, items)
+        b.finalize()
+        plan = [b.plan(i) for i in ids]
+        n = b.device_bytes()
+        b.close()
+        return n, plan
+
+    (rings, _), (boxes, plan) = sized(True), sized(False)
+    assert plan[0][1] > 1 and boxes > rings + (1 << 20)
+    for reserved, resident in ((boxes, [True] * (rest + 1)), (rings + 8192, [False] + [True] * rest),
+                               (rings, [False] * (rest + 1))):
+        b = Batch(ctx)
+        try:
+            assert lib().bgt_batch_reserve(b.h, C.c_size_t(reserved)) == 0
+            ids = _add(b, items)
+            b.finalize()
+            assert [b.plan(i)[0] for i in ids] == resident
+            _run(b, ids, items)
+            assert lib().bgt_batch_reset(b.h) == 0
+        finally:
+            b.close()
