@@ -120,7 +120,7 @@ extern "C" int bgt_segments_take(bgt_ctx *c, int32_t *start, uint8_t *is_end, in
                 points[3 * i + 2] = r.pz[i];
             }
     }
-    c->view_dims = 0;
+    ctx_pinned_done(c);
     return BGT_OK;
 }
 
@@ -403,6 +403,7 @@ static int centerline(bgt_ctx *c, int dims, int dtype, const void *in, int w, in
         if (Z) memcpy(Z, r.fz, n * 4);
     }
     if (r.nseg > 0) memcpy(I, r.idx, (size_t)r.nseg * 4);
+    ctx_pinned_done(c);
     I[r.nseg] = (unsigned)n;
     *ox = X;
     *oy = Y;

@@ -46,9 +46,11 @@ size_t dtype_size(int dtype);
 int default_cfg(int dims, int W, int H, int D);
 int tuned_cfg(int dims, int W, int H, int D);
 int ctx_scratch(bgt_ctx *c, int slot, size_t bytes, void **out);
-// Pinned host buffer of at least `bytes` (grown, never shrunk), for readbacks
-// that end before the call returns.
+// Host buffer of at least `bytes`, for readbacks that end before the call returns:
+// pinned and kept (grown, never shrunk) up to 256 MB, pageable beyond and given
+// back by ctx_pinned_done or the next ctx_pinned.
 int ctx_pinned(bgt_ctx *c, size_t bytes, void **out);
+void ctx_pinned_done(bgt_ctx *c);
 int single_batch(bgt_ctx *c, int dims, int W, int H, int D, bgt_batch **out);
 int batch_check(bgt_batch *b);
 // Status words of the batch's last run (device pointers, null: none), and
@@ -119,7 +121,8 @@ struct bgt_ctx {
     cudaStream_t stream = nullptr;
     std::vector<bgt::Scratch> scratch;
     bgt::Scratch pinned;
-    bgt::SegResult view;   // segments of bgt_segments_begin, until bgt_segments_take (in `pinned`)
+    void *large = nullptr; // in its place for results beyond its limit
+    bgt::SegResult view;   // segments of bgt_segments_begin, until bgt_segments_take (in `pinned` or `large`)
     int view_dims = 0;     // 0: none
     size_t seg_chains = 0, seg_nodes = 0;  // list sizes of the segment extraction (grown on demand)
     size_t seg_read = 0;                   // bytes its last result took (read back with the header)

@@ -687,6 +687,7 @@ int segments_packed(bgt_ctx *c, int dims, const uint32_t *d_buf, int W, int H, i
         memcpy(out->py, r.py, (size_t)Np * 2);
         if (dims == 3) memcpy(out->pz, r.pz, (size_t)Np * 2);
     }
+    ctx_pinned_done(c);
     return BGT_OK;
 }
 

@@ -39,3 +39,25 @@ def test_centerlines_of_checkerboards(ctx, n, prune, span):
         for g, w in zip(got, (want.x, want.y, want.z, want.idx), strict=True):
             assert np.array_equal(g, w)
     c.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["segments", "centerline"])
+def test_results_of_more_than_256_mb(ctx, kind):
+    """They come back through memory that the context does not keep."""
+    from begputhinning_b200 import CenterlineExtraction, ExtractSegmentsV
+    if kind == "segments":
+        a = (np.random.default_rng(4).random((4700, 5000)) < 0.5).astype(np.uint8)
+        want = po.segments2d(a)
+        assert 5 * want.nseg + 4 * len(want.pts) > 256 << 20
+        got = ExtractSegmentsV(a, ctx)
+        for g, w in ((got.start, want.start), (got.is_end, want.is_end), (got.pts, want.pts)):
+            assert np.array_equal(g, w)
+    else:
+        v = _checkerboard(150)
+        want = po.centerline3d(v, 1, 1)
+        assert 12 * len(want.x) + 4 * len(want.idx) > 256 << 20
+        for g, w in zip(CenterlineExtraction(v, 1, 1, ctx), (want.x, want.y, want.z, want.idx), strict=True):
+            assert np.array_equal(g, w)
+    small = (np.random.default_rng(5).random((60, 70)) < 0.3).astype(np.uint8)
+    assert ExtractSegmentsV(small, ctx).as_lists() == po.segments2d(small).as_lists()
