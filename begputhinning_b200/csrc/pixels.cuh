@@ -36,17 +36,11 @@ __device__ __forceinline__ int dtype_bytes(int dtype)
                                   : (dtype == BGT_U16 || dtype == BGT_I16) ? 2 : 1;
 }
 
-// MSB-of-byte gather: multiplying the MSB mask by 0x00204081 moves bits 7,
-// 15, 23, 31 to 28..31 without carries.
-__device__ __forceinline__ uint32_t bytes4_to_bits(uint32_t cmp)
-{
-    return ((cmp & 0x80808080u) * 0x00204081u) >> 28;
-}
-
 // 4 bytes -> 4 bits "byte != 0" (bit 28 + k for byte k, anything below them) with
 // integer ALU ops only: the low seven bits of each byte plus 0x7F carry into
 // the byte's MSB exactly when they are nonzero (no carry leaves the byte), and
-// OR-ing the byte back in covers the MSB itself.  With `neg` all ones, "byte > 0"
+// OR-ing the byte back in covers the MSB itself; multiplying the MSBs by 0x00204081
+// moves bits 7, 15, 23, 31 to 28..31 without carries.  With `neg` all ones, "byte > 0"
 // of signed bytes: those whose own MSB is set are taken out again.
 __device__ __forceinline__ uint32_t nz4_high(uint32_t c, uint32_t neg = 0u)
 {

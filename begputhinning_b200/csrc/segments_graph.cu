@@ -26,7 +26,7 @@
 // What is left is list ranking: every chain point has to know the two ends
 // of its chain and its distance to them.  Each chain point is two half-edges
 // (leaving it through its first or second neighbour); pointer jumping over
-// the half-edges takes about log4(longest chain) rounds, after which every
+// the half-edges takes at most log5(longest chain) rounds, after which every
 // point writes its own coordinates at its place in the output.  Phases (grid
 // barriers in between):
 //   A  node and chain masks per packed word (bit-sliced neighbour counts)
@@ -40,13 +40,13 @@
 //      (2D/CenterlineExtraction.cpp:51-131, 3D/CenterlineExtraction.cpp:56-144),
 //      so the whole path needs one readback and no count on the host
 //
-// Bound: latency -- about 7 + log4(longest chain) grid barriers of 1-2 us and
+// Bound: latency -- about 7 + log5(longest chain) grid barriers of 1-2 us and
 // as many chains of dependent loads.  Measured on a B200, this kernel alone:
 // 2048^2 stroke image (214 k points) 62 us, 256^3 volume (3.9 k points) 47 us
 // (84 and 57 us with one half-edge, one node and one strided word per thread at
 // a time).  Against a walk that followed each chain with one thread and ran the
 // nodes from a queue in the order of their dependences, whole ExtractSegmentsV
-// calls: 5.72 -> 0.24 ms and 0.86 -> 0.10 ms.
+// calls: 5.72 -> 0.29 ms and 0.86 -> 0.10 ms.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -143,7 +143,7 @@ struct SegHeader {
 // once any block gave up (bit 30 of the arrivals, which ends every wait).  One
 // word says all, so that a block that arrives last reads once (a status word
 // of its own, read behind the wait: CenterlineExtraction of a 512^2 image 152 us
-// instead of 148, three 256^3 segment lists 96.1 instead of 95.6).
+// instead of 148, segments of a 256^3 volume 96.1 instead of 95.6).
 __device__ bool seg_barrier(const SegArgs &a, unsigned &gen)
 {
     constexpr int kGaveUp = 1 << 30;

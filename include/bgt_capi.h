@@ -5,6 +5,8 @@
  * Every entry point returns BGT_OK (0) or a positive bgt_status; the message
  * of the last failure on the calling thread is available from
  * bgt_last_error().  Nothing here exits the process or reads stdin.
+ * A context and its batches serve one thread at a time; threads that work at
+ * the same time have a context each.
  *
  * Pixel data is row-major with x fastest: 2D data[y*width + x],
  * 3D data[(z*height + y)*width + x].  Foreground follows the reference's
